@@ -404,8 +404,8 @@ __global__ void __launch_bounds__(WT, 4) calib_shadow_kernel(const Scene S, cons
   TraceState st;
   float3 o = f3(0, 0, 0), d = f3(0, 0, 1);
   float tt = 0.0f;
-  uint32_t p = 0, j = 0;
-  bool active = false, exhausted = false;
+  uint32_t p = 0, j = 0, state = LANE_IDLE;
+  bool exhausted = false;
   const float4* srec = nullptr;
   auto next_sample = [&]() -> bool {
     for (; j < nl; j++) {
@@ -422,14 +422,10 @@ __global__ void __launch_bounds__(WT, 4) calib_shadow_kernel(const Scene S, cons
     tt = wb.nee[p].w;
     srec = wb.sh + size_t(p) * nl * 3;
     j = 0;
-    active = next_sample();
+    state = next_sample() ? LANE_NODE : LANE_IDLE;
   };
-  while (take_rays(active, exhausted, wb.fetch, n, cp.refill, start)) {
-    if (!active) continue;
-    const int r = trace_step<true>(S, 0.0f, st, stk);
-    bool done = r == 2;
-    if (r == 1) done = !trace_phase(S, cp.root, o, d, 0.0f, tt, 3u, skip, st, st.k + 1);
-    if (!done) continue;
+  auto next = [&]() {
+    if (st.best.tri == MISS && trace_phase(S, cp.root, o, d, 0.0f, tt, 3u, skip, st, st.k + 1)) { state = LANE_NODE; return; }
     if (st.best.tri != MISS) {
       const uint32_t vk = __float_as_uint(srec[3 * j + 2].z);
       rec[p].v[vk].q[j] = 0.0f;
@@ -437,8 +433,9 @@ __global__ void __launch_bounds__(WT, 4) calib_shadow_kernel(const Scene S, cons
       if (dec) dec[p].occ |= 1u << (vk * CAL_MAX_NL + j);
     }
     j++;
-    active = next_sample();
-  }
+    state = next_sample() ? LANE_NODE : LANE_IDLE;
+  };
+  while (serve_lanes(state, exhausted, wb.fetch, n, cp.refill, next, start)) trace_round<true>(S, 0.0f, st, stk, state);
 }
 
 // per pixel: the image value from the records in sub-sample order, its loss partial (forward); or the gradient of

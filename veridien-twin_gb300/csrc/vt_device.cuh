@@ -38,22 +38,7 @@ struct Scene {
   const float4* __restrict__ nstate;
   uint32_t* dbg;
   uint32_t mesh_off, mat_off, alb_off, prof_off, prof_n, emit_off, emit_n;
-  const float4* __restrict__ top;   // the static BVH's top levels, staged in shared memory by the traversal lanes
-  uint32_t n_top, top_root;
 };
-
-// Top levels of the static BVH held in shared memory by the persistent traversal lanes: the first VT_TOP_NODES
-// nodes of a breadth-first walk from the static root, each a copy of its 64-byte record whose interior-child
-// references into the set are rewritten as TOP_BIT | slot (slot 0 is the root). A traversal started at TOP_BIT
-// therefore reads these levels from shared memory and leaves the set through an ordinary global reference; the
-// visit order, and so every hit and counter, is that of the global records. Off by default: on the 657k-triangle
-// dome (640x480, 16 spp, depth 4) the frame takes 24.4 ms with 32 to 256 staged nodes against 21.9 ms without,
-// images identical; the top levels already hit in L1.
-#ifndef VT_TOP_NODES
-#define VT_TOP_NODES 0
-#endif
-constexpr uint32_t TOP_NODES = VT_TOP_NODES;
-constexpr uint32_t TOP_BIT = 0x80000000u;
 
 // ------------------------------------------------------------------------------------------------ float3 math
 __device__ __forceinline__ float3 f3(float x, float y, float z) { return make_float3(x, y, z); }
@@ -485,20 +470,17 @@ __device__ __forceinline__ Hit trace_scene(const Scene& S, uint32_t root, float3
 }
 
 // ------------------------------------------------------------------------------------------------ resumable trace
-// trace_scene split into single node visits, so that a warp of persistent lanes can take a new ray on any lane that
+// trace_scene split into node visits and leaves, so that a warp of persistent lanes can take a new ray on any lane that
 // finishes while the others keep traversing. Per ray the sequence of operations is trace_scene's: the static BVH,
 // then each posed body that passes the same culls, each traversed by the same ordered descent; so are the hits.
 struct TraceState {
   float3 ol, dl, inv;   // the ray in the current BVH's frame and its inverse direction
   Hit best;
-  uint32_t node, sp, visits;
+  uint32_t cur;         // next: a node, or LEAF_ITEM | 2 node + child for a leaf child of that node
+  uint32_t sp, visits;
   int k;                // current phase: -1 the static BVH, k >= 0 posed body k
-  // trace_step's node in progress: its children's entry distances (BIG once a leaf child is taken) and records (the
-  // triangle counts clamped to 16 bits: child 0's low, child 1's high), and the leaf being tested
-  float t0, t1;
-  uint32_t r0, r1, c01;
-  uint32_t lk, lend;    // triangles lk .. lend - 1 of the leaf are left (lk == lend: the next step visits st.node)
 };
+constexpr uint32_t LEAF_ITEM = 0x80000000u;
 
 // set up the first phase at or after `from` that has something to traverse; false when none is left
 __device__ __forceinline__ bool trace_phase(const Scene& S, uint32_t root, float3 o, float3 d, float tmin, float time, uint32_t mask,
@@ -506,8 +488,7 @@ __device__ __forceinline__ bool trace_phase(const Scene& S, uint32_t root, float
   int k = from;
   if (k < 0) {
     if (mask & 1u) {
-      st.k = -1; st.ol = o; st.dl = d; st.inv = safe_inv(d); st.node = root; st.sp = 0; st.visits = 0;
-      st.lk = st.lend = 0;
+      st.k = -1; st.ol = o; st.dl = d; st.inv = safe_inv(d); st.cur = root; st.sp = 0; st.visits = 0;
       return true;
     }
     k = 0;
@@ -528,10 +509,9 @@ __device__ __forceinline__ bool trace_phase(const Scene& S, uint32_t root, float
     st.ol = rtmul(R, o - p);
     st.dl = rtmul(R, d);
     st.inv = safe_inv(st.dl);
-    st.node = ldu(I + 11);
+    st.cur = ldu(I + 11);
     st.sp = 0;
     st.visits = 0;
-    st.lk = st.lend = 0;
     st.k = k;
     return true;
   }
@@ -547,7 +527,6 @@ __device__ __forceinline__ bool trace_phase(const Scene& S, uint32_t root, float
 constexpr uint32_t SH_DEPTH = VT_SH_DEPTH;
 struct LaneStack {
   uint2* sh;           // shared: SH_DEPTH x stride entries of (node, t bits)
-  const float4* top = nullptr;   // shared: the staged top levels (4 float4 per slot), when the kernel stages them
   uint32_t lane, stride;
   uint2 deep[STACK - SH_DEPTH];
   __device__ __forceinline__ void set(uint32_t i, uint32_t node, float t) {
@@ -557,125 +536,118 @@ struct LaneStack {
   __device__ __forceinline__ uint2 get(uint32_t i) const { return i < SH_DEPTH ? sh[i * stride + lane] : deep[i - SH_DEPTH]; }
 };
 
-// The current phase's traversal, one unit of traverse's loop per step: a step either visits a node (the child boxes,
-// and the first leaf child to test) or tests one triangle of that leaf. The node's children stay in the state until
-// its leaves are done; then the same step takes the next node from its interior children or the stack. Per ray the
-// sequence of operations is traverse's (child 0's leaf in triangle order, child 1's leaf only if its box is still
-// nearer than the best hit, then the push / pop with the updated best), so are the hits; a warp's lanes do not wait
-// for the longest leaf loop among them. The 2048-visit and 64-triangle caps and the parent-before-child check count
-// into dbg as in traverse. 0 continue, 1 the phase is finished, 2 an any-hit query found its hit.
-// the leaf of child c, when its box is nearer than the best hit: its triangles become the ones left, and the child's
-// distance BIG (traverse drops a tested leaf child from the push / pop the same way, after its loop)
-__device__ __forceinline__ bool leaf_enter(const Scene& S, TraceState& st, uint32_t c) {
-  const float tc = c == 0u ? st.t0 : st.t1;
-  const uint32_t cnt = (st.c01 >> (16u * c)) & 0xffffu, ref = c == 0u ? st.r0 : st.r1;
-  if (!(tc < st.best.t && cnt > 0u)) return false;
-  if (cnt > MAX_LEAF) atomicAdd(S.dbg + DBG_LEAF, 1u);
-  st.lk = ref;
-  st.lend = ref + min(cnt, MAX_LEAF);
-  if (c == 0u) st.t0 = BIG; else st.t1 = BIG;
-  return true;
+// Lane states of the persistent traversal loops: no ray; the current BVH is finished (or an any-hit query has its hit);
+// a node to visit; a leaf to test.
+enum { LANE_IDLE = 0, LANE_WAIT = 1, LANE_NODE = 2, LANE_LEAF = 3 };
+// Lanes at a leaf before a warp tests leaves. Few: the leaf code is issued for few lanes; many: lanes stand idle at
+// their leaf. 640x480, 16 spp, depth 4 on the 12k-triangle dome: 16.7 ms at 4, 15.6 at 8, 15.4 at 12 and 14; 1920x1200,
+// 8 spp, depth 6 with six instruments: 148, 139, 136, 136 ms; the same order on the pose batch and the twin frame
+#ifndef VT_LEAF_BATCH
+#define VT_LEAF_BATCH 12
+#endif
+
+// the next item off the stack that is nearer than the best hit: the lane's new state
+__device__ __forceinline__ uint32_t trace_pop(TraceState& st, const LaneStack& stk) {
+  while (st.sp > 0u) {
+    st.sp--;
+    const uint2 e = stk.get(st.sp);
+    if (__uint_as_float(e.y) < st.best.t) {
+      st.cur = e.x;
+      return (e.x & LEAF_ITEM) ? LANE_LEAF : LANE_NODE;
+    }
+  }
+  return LANE_WAIT;
 }
 
+// one node of traverse's loop: both child boxes, then the next item. traverse tests a node's leaf children in child
+// order before it descends, and what follows a leaf only while it is still nearer than the best hit. Here the first of
+// the two becomes the next item and the other goes on the stack, whose pop makes the same comparison: (leaf, leaf) child
+// 0 first, (leaf, interior) the leaf first, (interior, interior) the nearer first. The 2048-visit cap and the
+// parent-before-child check count into dbg as in traverse; so does the stack's clamp at 31 interior entries.
+__device__ __forceinline__ uint32_t trace_node(const Scene& S, float tmin, TraceState& st, LaneStack& stk) {
+  if (++st.visits > MAX_VISITS) { atomicAdd(S.dbg + DBG_VISITS, 1u); return LANE_WAIT; }
+  const uint32_t node = st.cur;
+  const float4* nb = S.nodes + 4u * node;
+  const float4 a0 = __ldg(nb), a1 = __ldg(nb + 1), a2 = __ldg(nb + 2), a3 = __ldg(nb + 3);
+  float t0, t1;
+  slab_pair(a0, a1, a2, a3, st.ol, st.inv, tmin, st.best.t, t0, t1);
+  const bool h0 = t0 < st.best.t, h1 = t1 < st.best.t;
+  const bool leaf0 = fu(a1.w) != 0u, leaf1 = fu(a3.w) != 0u;
+  if ((h0 && !leaf0 && fu(a0.w) <= node) || (h1 && !leaf1 && fu(a2.w) <= node)) { atomicAdd(S.dbg + DBG_CORRUPT, 1u); return LANE_WAIT; }
+  const uint32_t w0 = leaf0 ? (LEAF_ITEM | (2u * node)) : fu(a0.w), w1 = leaf1 ? (LEAF_ITEM | (2u * node + 1u)) : fu(a2.w);
+  if (!h0 && !h1) return trace_pop(st, stk);
+  const bool one = h1 && (!h0 || (!leaf0 && (leaf1 || t1 < t0)));   // child 1 comes first
+  st.cur = one ? w1 : w0;
+  if (h0 && h1) {
+    stk.set(st.sp, one ? w0 : w1, one ? t0 : t1);
+    st.sp = leaf0 || leaf1 ? st.sp + 1u : min(st.sp + 1u, STACK - 1u);
+  }
+  return (st.cur & LEAF_ITEM) ? LANE_LEAF : LANE_NODE;
+}
+
+// the triangles of a leaf in order (at most 64, counted into dbg beyond)
 template <bool ANY>
-__device__ __forceinline__ int trace_step(const Scene& S, float tmin, TraceState& st, LaneStack& stk) {
-  bool more;
-  if (st.lk == st.lend) {
-    if (++st.visits > MAX_VISITS) { atomicAdd(S.dbg + DBG_VISITS, 1u); return 1; }
-    const uint32_t node = st.node;
-#if VT_TOP_NODES
-    float4 a0, a1, a2, a3;
-    if ((node & TOP_BIT) != 0u) {
-      const float4* nb = stk.top + 4u * (node & 0xffffu);
-      a0 = nb[0]; a1 = nb[1]; a2 = nb[2]; a3 = nb[3];
-    } else {
-      const float4* nb = S.nodes + 4u * node;
-      a0 = __ldg(nb); a1 = __ldg(nb + 1); a2 = __ldg(nb + 2); a3 = __ldg(nb + 3);
-    }
-#else
-    const float4* nb = S.nodes + 4u * node;
-    const float4 a0 = __ldg(nb), a1 = __ldg(nb + 1), a2 = __ldg(nb + 2), a3 = __ldg(nb + 3);
-#endif
-    slab_pair(a0, a1, a2, a3, st.ol, st.inv, tmin, st.best.t, st.t0, st.t1);
-    st.c01 = min(fu(a1.w), 0xffffu) | (min(fu(a3.w), 0xffffu) << 16);
-    st.r0 = fu(a0.w); st.r1 = fu(a2.w);
-    more = leaf_enter(S, st, 0u) || leaf_enter(S, st, 1u);
-  } else {
-    const uint32_t k = st.lk++;
+__device__ __forceinline__ uint32_t trace_leaf(const Scene& S, float tmin, TraceState& st, LaneStack& stk) {
+  const float* rec = reinterpret_cast<const float*>(S.nodes) + 8u * size_t(st.cur & ~LEAF_ITEM);
+  uint32_t k = ldu(rec + 3);
+  const uint32_t cnt = ldu(rec + 7);
+  if (cnt > MAX_LEAF) atomicAdd(S.dbg + DBG_LEAF, 1u);
+  const uint32_t end = k + min(cnt, MAX_LEAF);
+  for (; k < end; k++) {
     float t, u, v;
     if (tri_hit(S, k, st.ol, st.dl, tmin, st.best.t, t, u, v)) {
       st.best.t = t; st.best.u = u; st.best.v = v; st.best.tri = k; st.best.inst = st.k < 0 ? MISS : uint32_t(st.k);
-      if (ANY) return 2;
+      if (ANY) return LANE_WAIT;
     }
-    // the leaf done: child 1's leaf next (when that was child 0's and child 1's box is still nearer)
-    more = st.lk != st.lend || leaf_enter(S, st, 1u);
   }
-  if (more) return 0;
-  const uint32_t node = st.node;
-#if VT_TOP_NODES
-  const bool staged = (node & TOP_BIT) != 0u;
-#else
-  constexpr bool staged = false;
-#endif
-  const float t0 = st.t0 < st.best.t ? st.t0 : BIG;
-  const float t1 = st.t1 < st.best.t ? st.t1 : BIG;
-  const uint32_t r0 = st.r0, r1 = st.r1;
-  if (!staged && ((t0 < BIG && (st.c01 & 0xffffu) == 0u && r0 <= node) || (t1 < BIG && (st.c01 >> 16) == 0u && r1 <= node))) {
-    atomicAdd(S.dbg + DBG_CORRUPT, 1u);
-    return 1;
-  }
-  const bool go0 = t0 < BIG, go1 = t1 < BIG;
-  if (go0 && go1) {
-    if (t1 < t0) { stk.set(st.sp, r0, t0); st.node = r1; }
-    else { stk.set(st.sp, r1, t1); st.node = r0; }
-    st.sp = min(st.sp + 1u, STACK - 1u);
-  } else if (go0) {
-    st.node = r0;
-  } else if (go1) {
-    st.node = r1;
+  return trace_pop(st, stk);
+}
+
+// One round of a warp's lanes (all call it): the lanes at a node visit it, until VT_LEAF_BATCH lanes wait at a leaf or
+// none is at a node; then those test their leaves. The warp issues one kind of work at a time: with a visit or a triangle
+// per lane in every step, both and the push / pop were issued for some lane in nearly each (328 warp instructions a step,
+// 10.4 lanes in the mean on secondary rays; now 16.3). With serve_lanes below: 640x480, 16 spp, depth 4: 19.6 -> 15.4 ms.
+template <bool ANY>
+__device__ __forceinline__ void trace_round(const Scene& S, float tmin, TraceState& st, LaneStack& stk, uint32_t& state) {
+  const uint32_t at_node = __ballot_sync(0xffffffffu, state == LANE_NODE), at_leaf = __ballot_sync(0xffffffffu, state == LANE_LEAF);
+  if (at_node && __popc(at_leaf) < VT_LEAF_BATCH) {
+    if (state == LANE_NODE) state = trace_node(S, tmin, st, stk);
   } else {
-    while (st.sp > 0u) {
-      st.sp--;
-      const uint2 e = stk.get(st.sp);
-      if (__uint_as_float(e.y) < st.best.t) { st.node = e.x; return 0; }
-    }
-    return 1;
+    if (state == LANE_LEAF) state = trace_leaf<ANY>(S, tmin, st, stk);
   }
-  return 0;
 }
 
-// Persistent traversal lanes: every lane keeps one ray in flight, one node visit per loop iteration; once `refill`
-// lanes of the warp are idle they take the next queue entries with one atomic. Lanes stay busy until the queue
-// drains instead of waiting for the warp's slowest ray (warp-level ray compaction).
-template <typename F>
-__device__ __forceinline__ bool take_rays(bool& active, bool& exhausted, uint32_t* head, uint32_t n, uint32_t refill, F&& start) {
-  const uint32_t lane = threadIdx.x & 31u;
-  const uint32_t idle = __ballot_sync(0xffffffffu, !active);
-  if (!exhausted && idle && (__popc(idle) >= int(refill) || idle == 0xffffffffu)) {
-    const uint32_t leader = __ffs(idle) - 1;
-    uint32_t base = 0;
-    if (lane == leader) base = atomicAdd(head, uint32_t(__popc(idle)));
-    base = __shfl_sync(0xffffffffu, base, leader);
-    if (base + uint32_t(__popc(idle)) >= n) exhausted = true;
-    if (!active) {
-      const uint32_t idx = base + __popc(idle & ((1u << lane) - 1u));
-      if (idx < n) start(idx);
+// Persistent traversal lanes: every lane keeps one ray in flight. A lane whose BVH is finished waits (LANE_WAIT) until
+// `refill` lanes of the warp are free (waiting, or idle while the queue has rays left), or until no lane traverses any
+// more; then the waiting lanes run next() together (the ray's next posed body, or its result; next() sets `state`) and
+// the idle ones take new queue entries with one atomic. next() and start() are some hundred instructions that a ray
+// needs once or twice among its ~40 visits and triangles: run for a lane at a time as its BVH ended, they were a good
+// part of what a warp issued. Near the queue's end, where no ray comes after, a quarter of the traversing lanes is enough.
+template <typename Next, typename Start>
+__device__ __forceinline__ bool serve_lanes(uint32_t& state, bool& exhausted, uint32_t* head, uint32_t n, uint32_t refill, Next&& next, Start&& start) {
+  const uint32_t tracing = __ballot_sync(0xffffffffu, state >= LANE_NODE);
+  const uint32_t waiting = __ballot_sync(0xffffffffu, state == LANE_WAIT);
+  const uint32_t free_lanes = exhausted ? waiting : ~tracing;
+  const int enough = exhausted ? min(int(refill), (__popc(tracing) + 3) / 4) : int(refill);
+  if (!free_lanes || (tracing && __popc(free_lanes) < enough)) return tracing != 0u;
+  if (state == LANE_WAIT) next();
+  __syncwarp();
+  if (!exhausted) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t idle = __ballot_sync(0xffffffffu, state == LANE_IDLE);
+    if (idle) {
+      const uint32_t leader = __ffs(idle) - 1;
+      uint32_t base = 0;
+      if (lane == leader) base = atomicAdd(head, uint32_t(__popc(idle)));
+      base = __shfl_sync(0xffffffffu, base, leader);
+      if (base + uint32_t(__popc(idle)) >= n) exhausted = true;
+      if (state == LANE_IDLE) {
+        const uint32_t idx = base + __popc(idle & ((1u << lane) - 1u));
+        if (idx < n) start(idx);
+      }
     }
   }
-  return __any_sync(0xffffffffu, active) || !exhausted;
-}
-
-// copy the staged top levels into the block's shared array; returns the root to start static traversals at
-__device__ __forceinline__ uint32_t stage_top(const Scene& S, float4* top_sh, uint32_t root) {
-#if VT_TOP_NODES
-  const uint32_t n = min(S.n_top, TOP_NODES) * 4u;
-  for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) top_sh[i] = __ldg(S.top + i);
-  __syncthreads();
-  return n && root == S.top_root ? TOP_BIT : root;
-#else
-  (void)S; (void)top_sh;
-  return root;
-#endif
+  return __any_sync(0xffffffffu, state != LANE_IDLE) || !exhausted;
 }
 
 // ------------------------------------------------------------------------------------------------ surfaces

@@ -51,8 +51,8 @@ __device__ __forceinline__ uint32_t landing_node(const Scene& S, const Hit& h, f
   return bb.y >= bb.z ? v1 : v2;
 }
 
-// The gather table's rays (node i, ray j at r = i K + j) on persistent closest-hit lanes (trace_step: one node visit
-// or triangle test per lane step, the same per-ray sequence as trace_scene's static descent, so the same hits); a
+// The gather table's rays (node i, ray j at r = i K + j) on persistent closest-hit lanes (trace_round:
+// node visits and leaves, the same per-ray sequence as trace_scene's static descent, so the same hits); a
 // lane takes the next ray when its own finishes. `head` counts the rays taken.
 __global__ void __launch_bounds__(256, VT_NODE_TRACE_BLOCKS) gather_build_kernel(const Scene S, uint32_t K, uint64_t r0, uint32_t total,
                                                                                  uint32_t* __restrict__ gtable, uint32_t* head) {
@@ -62,10 +62,11 @@ __global__ void __launch_bounds__(256, VT_NODE_TRACE_BLOCKS) gather_build_kernel
   TraceState st;
   float3 o = f3(0, 0, 0), d = f3(0, 0, 1);
   uint64_t r = 0;
-  bool active = false, exhausted = false;
-  auto finish = [&]() {
+  uint32_t state = LANE_IDLE;
+  bool exhausted = false;
+  auto next = [&]() {
     gtable[r] = landing_node(S, st.best, d);
-    active = false;
+    state = LANE_IDLE;
   };
   auto start = [&](uint32_t idx) {
     r = r0 + idx;
@@ -74,13 +75,9 @@ __global__ void __launch_bounds__(256, VT_NODE_TRACE_BLOCKS) gather_build_kernel
     d = gather_dir(i, j, K, n);
     o = p + n * EPS_OFF;
     st.best = Hit{BIG, 0.0f, 0.0f, MISS, MISS};
-    active = trace_phase(S, 0u, o, d, 0.0f, 0.5f, 1u, 0u, st, -1);
-    if (!active) { active = true; finish(); }
+    state = trace_phase(S, 0u, o, d, 0.0f, 0.5f, 1u, 0u, st, -1) ? LANE_NODE : LANE_WAIT;
   };
-  while (take_rays(active, exhausted, head, total, 8u, start)) {
-    if (!active) continue;
-    if (trace_step<false>(S, 0.0f, st, stk) != 0) finish();
-  }
+  while (serve_lanes(state, exhausted, head, total, 8u, next, start)) trace_round<false>(S, 0.0f, st, stk, state);
 }
 
 // escapes per node (gpu/wgsl/kernels.wgsl.js:326 gatherCount)
@@ -218,26 +215,23 @@ __global__ void __launch_bounds__(256, VT_NODE_TRACE_BLOCKS) node_direct_shadow(
   stk.sh = stack_sh; stk.lane = threadIdx.x; stk.stride = 256;
   TraceState st;
   float3 o = f3(0, 0, 0), d = f3(0, 0, 1);
-  uint32_t t = 0;
-  bool active = false, exhausted = false;
+  uint32_t t = 0, state = LANE_IDLE;
+  bool exhausted = false;
   auto visible = [&]() { b.term[t].w = __uint_as_float(__float_as_uint(b.term[t].w) | ND_VIS); };
   auto start = [&](uint32_t idx) {
     t = b.queue[idx];
     const float4 o4 = b.ro[t], d4 = b.rd[t];
     o = xyz(o4); d = xyz(d4);
     st.best = Hit{o4.w, 0.0f, 0.0f, MISS, MISS};
-    active = trace_phase(S, 0u, o, d, 0.0f, 0.5f, 3u, skip, st, -1);
-    if (!active) visible();
+    state = trace_phase(S, 0u, o, d, 0.0f, 0.5f, 3u, skip, st, -1) ? LANE_NODE : LANE_WAIT;
   };
-  while (take_rays(active, exhausted, b.counts + 1, n, refill, start)) {
-    if (!active) continue;
-    const int r = trace_step<true>(S, 0.0f, st, stk);
-    bool done = r == 2;
-    if (r == 1) done = !trace_phase(S, 0u, o, d, 0.0f, 0.5f, 3u, skip, st, st.k + 1);
-    if (!done) continue;
-    if (st.best.tri == MISS) visible();
-    active = false;
-  }
+  auto next = [&]() {
+    state = LANE_IDLE;
+    if (st.best.tri != MISS) return;
+    if (trace_phase(S, 0u, o, d, 0.0f, 0.5f, 3u, skip, st, st.k + 1)) state = LANE_NODE;
+    else visible();
+  };
+  while (serve_lanes(state, exhausted, b.counts + 1, n, refill, next, start)) trace_round<true>(S, 0.0f, st, stk, state);
 }
 
 __global__ void node_direct_sum(const Scene S, const uint32_t* __restrict__ active, uint32_t n_active, uint32_t NS, NodeDirectBufs b,

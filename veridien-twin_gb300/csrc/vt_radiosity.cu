@@ -444,8 +444,8 @@ __global__ void __launch_bounds__(FV_THREADS, 4) ff_visibility_kernel(const Scen
   const uint32_t skip = ldu(S.su + 7);
   const uint32_t total = n * n;
   float3 o = f3(0, 0, 0), d = f3(0, 0, 1);
-  uint32_t i = 0, j = 0, k = 0, vis = 0;
-  bool active = false, exhausted = false;
+  uint32_t i = 0, j = 0, k = 0, vis = 0, state = LANE_IDLE;
+  bool exhausted = false;
   auto next_ray = [&]() -> bool {
     for (; k < K; k++) {
       const float3 a = disc_point(C, N, A, i, kr(k, R2A, 0.5f), kr(k, R2B, 0.5f));
@@ -464,7 +464,7 @@ __global__ void __launch_bounds__(FV_THREADS, 4) ff_visibility_kernel(const Scen
   auto finish = [&]() {
     counts[size_t(i) * n + j] = uint8_t(vis);
     counts[size_t(j) * n + i] = uint8_t(vis);
-    active = false;
+    state = LANE_IDLE;
   };
   auto start = [&](uint32_t idx) {
     i = idx / n;
@@ -473,19 +473,19 @@ __global__ void __launch_bounds__(FV_THREADS, 4) ff_visibility_kernel(const Scen
     if (!facing(C, N, i, j)) { vis = 0; finish(); return; }
     k = 0;
     vis = 0;
-    active = true;
+    state = LANE_NODE;
     if (!next_ray()) finish();
   };
-  while (take_rays(active, exhausted, head, total, REFILL, start)) {
-    if (!active) continue;
-    const int r = trace_step<true>(S, 0.0f, st, stk);
-    bool done = r == 2;
-    if (r == 1) done = !trace_phase(S, 0u, o, d, 0.0f, 0.5f, 3u, skip, st, st.k + 1);
-    if (!done) continue;
-    if (st.best.tri == MISS) vis++;
+  auto next = [&]() {
+    state = LANE_NODE;
+    if (st.best.tri == MISS) {
+      if (trace_phase(S, 0u, o, d, 0.0f, 0.5f, 3u, skip, st, st.k + 1)) return;
+      vis++;
+    }
     k++;
     if (!next_ray()) finish();
-  }
+  };
+  while (serve_lanes(state, exhausted, head, total, REFILL, next, start)) trace_round<true>(S, 0.0f, st, stk, state);
 }
 
 __global__ void ff_rows_kernel(uint32_t n, const float* __restrict__ C, const float* __restrict__ N, const float* __restrict__ A,

@@ -147,25 +147,22 @@ __global__ void __launch_bounds__(WAVE_THREADS, VT_TRACE_BLOCKS) wave_extend(con
   const uint32_t n = *wb.count_in;
   if (wb.stats && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(wb.stats, (unsigned long long)n);
   __shared__ uint2 stack_sh[SH_DEPTH * WAVE_THREADS];
-  __shared__ float4 top_sh[4u * (TOP_NODES ? TOP_NODES : 1u)];
   LaneStack stk;
-  stk.sh = stack_sh; stk.lane = threadIdx.x; stk.stride = WAVE_THREADS; stk.top = top_sh;
+  stk.sh = stack_sh; stk.lane = threadIdx.x; stk.stride = WAVE_THREADS;
   TraceState st;
-  const uint32_t root = stage_top(S, top_sh, cp.root);
-  Scene Sl = S;
-  float3 o = f3(0, 0, 0), d = f3(0, 0, 1);
-  float tt = 0.0f;
+  const uint32_t root = cp.root;
   uint32_t p = 0, skip = 0;
-  bool active = false, exhausted = false;
+  uint32_t state = LANE_IDLE;
+  bool exhausted = false;
   auto finish = [&]() {
     wb.hit[p] = make_float4(st.best.t, st.best.u, st.best.v, __uint_as_float(st.best.tri));
     wb.hinst[p] = st.best.inst;
     if (VAR == WAVE_SHARED) {
       const uint64_t have = wb.bc.dirty[p];
-      const uint64_t bits = cull_bits(wb.bc, o, d, st.best.t, skip, have);
+      const uint64_t bits = cull_bits(wb.bc, xyz(wb.o[p]), xyz(wb.d[p]), st.best.t, wb.meta[p].w == 1 ? cp.skip : 0u, have);
       if (bits & ~have) wb.bc.dirty[p] = have | bits;
     }
-    active = false;
+    state = LANE_IDLE;
   };
   // static first-hit cache (camera rays of a fixed camera, gpu/wgsl/kernels.wgsl.js:82 staticFirstHit): a cached
   // entry replaces the static phase (the instance phases then start from it, exactly as after tracing it); an empty
@@ -174,10 +171,9 @@ __global__ void __launch_bounds__(WAVE_THREADS, VT_TRACE_BLOCKS) wave_extend(con
   auto start = [&](uint32_t idx) {
     p = wb.q_in[idx];
     const float4 o4 = wb.o[p], d4 = wb.d[p];
-    o = xyz(o4); d = xyz(d4); tt = o4.w;
     const uint4 meta = wb.meta[p];
     skip = meta.w == 1 ? cp.skip : 0u;
-    Sl = path_scene<VAR>(S, wb, p);
+    if (VAR == WAVE_SHARED) skip |= wb.bc.vary;
     st.best = Hit{BIG, 0.0f, 0.0f, MISS, MISS};
     int from = -1;
     ci = MISS;
@@ -186,22 +182,23 @@ __global__ void __launch_bounds__(WAVE_THREADS, VT_TRACE_BLOCKS) wave_extend(con
       const float4 h = wb.hcache[ci];
       if (h.x > 0.0f) { st.best = Hit{h.x, h.y, h.z, __float_as_uint(h.w), MISS}; from = 0; ci = MISS; }
     }
-    active = trace_phase(Sl, root, o, d, 0.0f, tt, 3u, VAR == WAVE_SHARED ? (skip | wb.bc.vary) : skip, st, from);
+    // a ray with nothing to traverse finishes at the next service
+    state = trace_phase(path_scene<VAR>(S, wb, p), root, xyz(o4), xyz(d4), 0.0f, o4.w, 3u, skip, st, from) ? LANE_NODE : LANE_WAIT;
     if (HC && ci != MISS && st.k != -1) {   // no static phase to wait for: the static hit is none
       wb.hcache[ci] = make_float4(BIG, 0.0f, 0.0f, __uint_as_float(MISS));
       ci = MISS;
     }
-    if (!active) { active = true; finish(); }
   };
-  while (take_rays(active, exhausted, wb.fetch, n, cp.refill, start)) {
-    if (!active) continue;
-    const int r = trace_step<false>(Sl, 0.0f, st, stk);
-    if (HC && r != 0 && VAR == WAVE_PLAIN && ci != MISS && st.k == -1) {
+  auto next = [&]() {
+    if (HC && VAR == WAVE_PLAIN && ci != MISS && st.k == -1) {
       wb.hcache[ci] = make_float4(st.best.t, st.best.u, st.best.v, __uint_as_float(st.best.tri));
       ci = MISS;
     }
-    if (r != 0 && !trace_phase(Sl, root, o, d, 0.0f, tt, 3u, VAR == WAVE_SHARED ? (skip | wb.bc.vary) : skip, st, st.k + 1)) finish();
-  }
+    const float4 o4 = wb.o[p], d4 = wb.d[p];   // read again: six registers less over the traversal
+    if (trace_phase(path_scene<VAR>(S, wb, p), root, xyz(o4), xyz(d4), 0.0f, o4.w, 3u, skip, st, st.k + 1)) state = LANE_NODE;
+    else finish();
+  };
+  while (serve_lanes(state, exhausted, wb.fetch, n, cp.refill, next, start)) trace_round<false>(S, 0.0f, st, stk, state);
 }
 
 template <int MODE, int VAR>
@@ -352,18 +349,18 @@ __global__ void __launch_bounds__(WAVE_THREADS, VT_TRACE_BLOCKS) wave_shadow(con
   const uint32_t skip0 = ldu(S0.su + 7);
   const uint32_t skip = VAR == WAVE_SHARED ? (skip0 | wb.bc.vary) : skip0;
   __shared__ uint2 stack_sh[SH_DEPTH * WAVE_THREADS];
-  __shared__ float4 top_sh[4u * (TOP_NODES ? TOP_NODES : 1u)];
   LaneStack stk;
-  stk.sh = stack_sh; stk.lane = threadIdx.x; stk.stride = WAVE_THREADS; stk.top = top_sh;
+  stk.sh = stack_sh; stk.lane = threadIdx.x; stk.stride = WAVE_THREADS;
   TraceState st;
-  const uint32_t root = stage_top(S0, top_sh, cp.root);
+  const uint32_t root = cp.root;
   Scene S = S0;
   float3 o = f3(0, 0, 0), d = f3(0, 0, 1);
   float4 nee = make_float4(0, 0, 0, 0);
   float3 Ld = f3(0, 0, 0);
   uint32_t p = 0, j = 0;
   uint64_t have = 0ull, bits = 0ull;
-  bool active = false, exhausted = false;
+  uint32_t state = LANE_IDLE;
+  bool exhausted = false;
   const float4* rec = nullptr;
   // the static-occlusion cache's bookkeeping of the current path (shade.wgsl.js:270-301): lit and visible samples,
   // their luminance range, a posed body blocking one, and the occlusion word to store
@@ -404,7 +401,7 @@ __global__ void __launch_bounds__(WAVE_THREADS, VT_TRACE_BLOCKS) wave_shadow(con
     }
     wb.L[p] = make_float4(v.x, v.y, v.z, __uint_as_float(key));
     if (VAR == WAVE_SHARED && bits) wb.bc.dirty[p] = have | bits;
-    active = false;
+    state = LANE_IDLE;
   };
   auto start = [&](uint32_t idx) {
     p = wb.q_sh[idx];
@@ -432,15 +429,11 @@ __global__ void __launch_bounds__(WAVE_THREADS, VT_TRACE_BLOCKS) wave_shadow(con
         lmax = 0.0f;
       }
     }
-    active = true;
-    if (!next_sample()) finish_path();
+    if (next_sample()) state = LANE_NODE;
+    else finish_path();
   };
-  while (take_rays(active, exhausted, wb.fetch, n, cp.refill, start)) {
-    if (!active) continue;
-    const int r = trace_step<true>(S, 0.0f, st, stk);
-    bool done = r == 2;
-    if (r == 1) done = !trace_phase(S, root, o, d, 0.0f, nee.w, 3u, skip, st, st.k + 1);
-    if (!done) continue;
+  auto next = [&]() {
+    if (st.best.tri == MISS && trace_phase(S, root, o, d, 0.0f, nee.w, 3u, skip, st, st.k + 1)) { state = LANE_NODE; return; }
     if (st.best.tri == MISS) {
       visible(j);
       if (VAR == WAVE_SHARED) bits |= cull_bits(wb.bc, o, d, rec[3 * j].w, skip0, have | bits);
@@ -449,8 +442,10 @@ __global__ void __launch_bounds__(WAVE_THREADS, VT_TRACE_BLOCKS) wave_shadow(con
       else dyn = true;                 // a posed body does
     }
     j++;
-    if (!next_sample()) finish_path();
-  }
+    if (next_sample()) state = LANE_NODE;
+    else finish_path();
+  };
+  while (serve_lanes(state, exhausted, wb.fetch, n, cp.refill, next, start)) trace_round<true>(S0, 0.0f, st, stk, state);
 }
 
 // per pixel, the wave's sub-samples in order i0..i0+n_i-1 added to the running sum; the last wave writes the pixel
