@@ -103,6 +103,8 @@ vt_status vt_create(const vt_scene_desc* scene, const vt_options* opts, vt_ctx**
   const vt::Prepared& S = ctx->S;
   vt_status s;
   if ((s = upload(ctx, &ctx->d_nodes, S.nodes.data(), S.nodes.size() * 4)) != VT_OK) return bail(s);
+  vtk::pack_nodes(ctx->d_nodes, S.node_count, ctx->stream);
+  if (cudaGetLastError() != cudaSuccess) return bail(VT_ERR_CUDA);
   if ((s = upload(ctx, &ctx->d_tris, S.tris.data(), S.tris.size() * 4)) != VT_OK) return bail(s);
   if ((s = upload(ctx, &ctx->d_verts, S.verts.data(), S.verts.size() * 4)) != VT_OK) return bail(s);
   if ((s = upload(ctx, &ctx->d_params, S.params.data(), S.params.size() * 4)) != VT_OK) return bail(s);

@@ -50,6 +50,8 @@ constexpr int TILE_W = 8, TILE_H = 4;
 constexpr uint32_t REFILL = 8;
 // padded pixel count of a w x h image in tile_w x tile_h tiles
 inline uint32_t tiled_pixels(uint32_t w, uint32_t h, uint32_t tw, uint32_t th) { return ((w + tw - 1) / tw) * ((h + th - 1) / th) * tw * th; }
+// the nodes of gpu/bvh.js's layout (n x 4 float4) into the traversal's, in place
+void pack_nodes(float4* nodes, uint32_t n, cudaStream_t st);
 void launch_trace(const vtd::Scene& S, const float4* o4, const float4* d4, uint32_t n, uint32_t mask, uint32_t any_hit, uint32_t root,
                   float4* out4, float* out_v, cudaStream_t st);
 void launch_visible(const vtd::Scene& S, float3 c, const float3* pts, uint32_t n, float tol, float time, uint32_t skip, uint8_t* out,

@@ -7,6 +7,23 @@
 namespace vtk {
 using namespace vtd;
 
+// Traversal layout of a node (64 B): per axis the planes (child 0 lo, child 1 lo, child 0 hi, child 1 hi), then the
+// children's words (child 0 ref, count, child 1 ref, count), so that a load leaves the two children's planes as the
+// register pairs of slab_pair's f32x2 operations
+__global__ void pack_nodes_kernel(float4* __restrict__ nodes, uint32_t n) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  float4* nb = nodes + size_t(4) * i;
+  const float4 a0 = nb[0], a1 = nb[1], a2 = nb[2], a3 = nb[3];   // c0.lo|ref, c0.hi|count, c1.lo|ref, c1.hi|count
+  nb[0] = make_float4(a0.x, a2.x, a1.x, a3.x);
+  nb[1] = make_float4(a0.y, a2.y, a1.y, a3.y);
+  nb[2] = make_float4(a0.z, a2.z, a1.z, a3.z);
+  nb[3] = make_float4(a0.w, a1.w, a2.w, a3.w);
+}
+void pack_nodes(float4* nodes, uint32_t n, cudaStream_t st) {
+  if (n) pack_nodes_kernel<<<(n + 255) / 256, 256, 0, st>>>(nodes, n);
+}
+
 // gpu/wgsl/kernels.wgsl.js:535 traceTest: one ray per thread
 __global__ void trace_kernel(const Scene S, const float4* __restrict__ o4, const float4* __restrict__ d4, uint32_t n, uint32_t mask,
                              uint32_t any_hit, uint32_t root, float4* __restrict__ out4, float* __restrict__ out_v) {
