@@ -966,9 +966,18 @@ vt_status vt_radiosity_solve(vt_ctx* ctx, vt_solve_req* q) {
   if (tma && dF && !aligned16(q->F)) return fail(ctx, VT_ERR_ARG, "solve: the bulk-copy matvec needs a 16-byte aligned F");
   const uint32_t max_blocks = std::max<uint32_t>(std::max<uint32_t>((n + 7) / 8, uint32_t((size_t(n) * R / 4 + 255) / 256)),
                                                  tma ? vtk::jacobi_matvec_tma_blocks(n) : 0u) + 8;
-  const size_t gemm_work = R > 1 ? vtk::jacobi_gemm_fp32_work(n, R) : 0;
-  const size_t need = (dF ? 0 : nf) + 3 * nb + size_t(n) * 4 + size_t(max_blocks) * 16 + gemm_work + 64 + 2048;
-  vt_status s = ensure_scratch(ctx, need);
+  // several right-hand sides: the tensor cores where F allows it (a host F is copied to aligned memory)
+  bool tc = q->precision == VT_PREC_FP32 && vtk::jacobi_tc_f32_ok(dF ? q->F : nullptr, n, R);
+  const size_t gemm_work = R > 1 ? std::max(vtk::jacobi_gemm_fp32_work(n, R), tc ? vtk::jacobi_tc_f32_work(n, R) : 0) : 0;
+  const uint32_t pitch = vtk::jacobi_tc_f32_pitch(n);
+  size_t nfp = tc && pitch != n ? size_t(n) * pitch * 4 : 0;   // F's copy in aligned rows
+  const size_t need = (dF ? 0 : nf) + 3 * nb + size_t(n) * 4 + size_t(max_blocks) * 16 + gemm_work + 64 + 2048 + 512;
+  vt_status s = ensure_scratch(ctx, need + nfp);
+  if (s != VT_OK && nfp) {   // no room for the copy
+    tc = false;
+    nfp = 0;
+    s = ensure_scratch(ctx, need);
+  }
   if (s != VT_OK) return s;
   char* base = static_cast<char*>(ctx->d_scratch);
   auto take = [&](size_t bytes) { char* p = base; base += (bytes + 255) / 256 * 256; return p; };
@@ -983,8 +992,26 @@ vt_status vt_radiosity_solve(vt_ctx* ctx, vt_solve_req* q) {
   if (!dF && (s = to_device(ctx, const_cast<float*>(Fd), q->F, nf)) != VT_OK) return s;
   if ((s = to_device(ctx, E, q->E, nb)) != VT_OK) return s;
   if ((s = to_device(ctx, rho, q->rho, size_t(n) * 4)) != VT_OK) return s;
-  if (q->warm_start) { if ((s = to_device(ctx, B0, q->B, nb)) != VT_OK) return s; }
-  else VT_CK(cudaMemcpyAsync(B0, E, nb, cudaMemcpyDeviceToDevice, ctx->stream));
+  auto first_iterate = [&]() -> vt_status {
+    if (q->warm_start) return to_device(ctx, B0, q->B, nb);
+    VT_CK(cudaMemcpyAsync(B0, E, nb, cudaMemcpyDeviceToDevice, ctx->stream));
+    return VT_OK;
+  };
+  if ((s = first_iterate()) != VT_OK) return s;
+  vtk::TcMap mF, mB;
+  uint32_t* wait_err = reinterpret_cast<uint32_t*>(norms + 4);   // a bounded wait ran out
+  if (tc) VT_CK(cudaMemsetAsync(wait_err, 0, 4, ctx->stream));
+  if (tc) {
+    int code = 0;
+    const float* Ft = Fd;
+    if (nfp) {
+      float* rows = reinterpret_cast<float*>(take(nfp));
+      vtk::jacobi_tc_f32_repitch(Fd, n, rows, ctx->stream);
+      Ft = rows;
+    }
+    if (!vtk::jacobi_tc_f32_setup(Ft, n, pitch, work, &mF, &mB, ctx->stream, &code))
+      return fail(ctx, VT_ERR_CUDA, "solve: tensor map encoding failed (" + std::to_string(code) + ")");
+  }
   const uint32_t check = q->check_every ? q->check_every : 8;
   const uint32_t max_it = q->max_iters ? q->max_iters : 1000;
   float* cur = B0;
@@ -998,6 +1025,7 @@ vt_status vt_radiosity_solve(vt_ctx* ctx, vt_solve_req* q) {
       if (j == 0) VT_CK(cudaEventRecord(ctx->ev2, ctx->stream));
       if (tma) vtk::launch_jacobi_matvec_tma(Fd, rho, E, cur, nxt, n, partials, &np, ctx->stream);
       else if (R == 1) vtk::launch_jacobi_matvec(Fd, rho, E, cur, nxt, n, partials, &np, ctx->stream);
+      else if (tc) vtk::launch_jacobi_tc_f32(mF, mB, it + j == 0, rho, E, cur, nxt, n, R, work, wait_err, partials, &np, ctx->stream);
       else vtk::launch_jacobi_gemm_fp32(Fd, rho, E, cur, nxt, n, R, work, partials, &np, ctx->stream);
       if (j == 0) VT_CK(cudaEventRecord(ctx->ev3, ctx->stream));
       std::swap(cur, nxt);
@@ -1006,9 +1034,23 @@ vt_status vt_radiosity_solve(vt_ctx* ctx, vt_solve_req* q) {
     it += k;
     vtk::launch_reduce_partials(partials, np, norms, ctx->stream);
     VT_CK(cudaGetLastError());
-    double h[2];
-    VT_CK(cudaMemcpyAsync(h, norms, 16, cudaMemcpyDeviceToHost, ctx->stream));
+    double h[5];   // the norms; wait_err in the first word of h[4]
+    VT_CK(cudaMemcpyAsync(h, norms, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
     VT_CK(cudaStreamSynchronize(ctx->stream));
+    if (tc) {
+      uint32_t e = 0;
+      memcpy(&e, h + 4, 4);
+      if (e) return fail(ctx, VT_ERR_TIMEOUT, "solve: a tensor-core pipeline wait ran out");
+    }
+    if (tc) {
+      if (!std::isfinite(h[0]) || !std::isfinite(h[1])) {
+        // an infinity or NaN (or a value past bf16's range) has no parts: the CUDA-core sweeps from the start
+        tc = false;
+        if ((s = first_iterate()) != VT_OK) return s;
+        cur = B0; nxt = B1; it = 0; sweep_n = 0; sweep_sum = 0;
+        continue;
+      }
+    }
     resid = h[1] > 0 ? std::sqrt(h[0] / h[1]) : 0.0;
     float gms = 0;
     cudaEventElapsedTime(&gms, ctx->ev2, ctx->ev3);

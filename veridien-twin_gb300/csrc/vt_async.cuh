@@ -27,15 +27,19 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 }
 // bounded wait for the completion of the phase with parity `parity`; false (and *err set) when it runs out
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_t* err, unsigned long long limit = WAIT_CYCLES) {
-  const unsigned long long t0 = clock64();
-  for (;;) {
+  auto try_wait = [&]() -> bool {
     uint32_t ok;
     asm volatile(
         "{\n .reg .pred P;\n mbarrier.try_wait.parity.shared::cta.b64 P, [%1], %2;\n selp.u32 %0, 1, 0, P;\n}"
         : "=r"(ok)
         : "r"(bar), "r"(parity)
         : "memory");
-    if (ok) return true;
+    return ok != 0u;
+  };
+  if (try_wait()) return true;
+  const unsigned long long t0 = clock64();
+  for (;;) {
+    if (try_wait()) return true;
     if (clock64() - t0 > limit) { atomicOr(err, 1u); return false; }
   }
 }

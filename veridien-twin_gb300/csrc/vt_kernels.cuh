@@ -78,6 +78,16 @@ uint32_t matvec_error(cudaStream_t st, bool reset);
 size_t jacobi_gemm_fp32_work(uint32_t n, uint32_t R);
 void launch_jacobi_gemm_fp32(const float* F, const float* rho, const float* E, const float* Bin, float* Bout, uint32_t n, uint32_t R,
                              float* work, double* partials, uint32_t* n_partials, cudaStream_t st);
+// the same sweep on the tensor cores in FP32 accuracy: whether this F can take it (n % 4 != 0: in a copy with rows of
+// jacobi_tc_f32_pitch), the bytes of `work` (16-byte aligned), the tensor maps (once per solve; false with the driver's code), a sweep (first: the solve's first; *err: a wait ran out)
+struct TcMap;
+bool jacobi_tc_f32_ok(const float* F, uint32_t n, uint32_t R);
+size_t jacobi_tc_f32_work(uint32_t n, uint32_t R);
+uint32_t jacobi_tc_f32_pitch(uint32_t n);
+void jacobi_tc_f32_repitch(const float* F, uint32_t n, float* out, cudaStream_t st);
+bool jacobi_tc_f32_setup(const float* F, uint32_t n, uint32_t pitch, void* work, TcMap* mF, TcMap* mB, cudaStream_t st, int* code);
+void launch_jacobi_tc_f32(const TcMap& mF, const TcMap& mB, bool first, const float* rho, const float* E, const float* Bin, float* Bout, uint32_t n,
+                          uint32_t R, void* work, uint32_t* err, double* partials, uint32_t* n_partials, cudaStream_t st);
 // sum the partials into out[0..1] (deterministic order)
 void launch_reduce_partials(const double* partials, uint32_t n, double* out, cudaStream_t st);
 void launch_form_factors(uint32_t n, const float* C, const float* N, const float* A, float* F, cudaStream_t st);

@@ -1,11 +1,12 @@
 // Node radiosity on sm_103a: B = E + diag(rho) F B by Jacobi sweeps (the twin's jacobiGather + jacobiUpdate with
-// Lambertian nodes, gpu/wgsl/kernels.wgsl.js:416-461), in plain FP32 on CUDA cores.
+// Lambertian nodes, gpu/wgsl/kernels.wgsl.js:416-461), in FP32.
 //
 //   jacobi_matvec   one right-hand side: one warp per row, F streamed with 128-bit loads (HBM- or L2-bound: 4 B of F
 //                   per 2 flops), B_in read from L1/L2; epilogue B_out = E + rho acc and the residual partials.
 //   jacobi_matvec_tma  the same sweep with F's rows fed into shared memory by bulk copies (VT_PREC_FP32_TMA; ~20%
 //                   slower than the plain kernel's 128-bit streaming loads on GB300, which stay the default).
-//   jacobi_gemm     R right-hand sides (R <= 64): a 128 x 64 output tile per 256-thread block, 8 x 4 outputs per
+//   jacobi_tc_f32   R right-hand sides: F B in FP32 accuracy on the tensor cores (vt_tc.cu), where F can come by TMA.
+//   jacobi_gemm     R right-hand sides (R <= 64) of a small or unaligned F: a 128 x 64 output tile per 256-thread block, 8 x 4 outputs per
 //                   thread, F and B staged through double-buffered shared memory in 16-wide K slices, K split across
 //                   blocks to fill the GPU. Compute-bound at 2 R flops per 4-byte element of F (R = 64: 32 flop/B)
 //                   on the FP32 pipes.
@@ -15,6 +16,7 @@
 
 #include "vt_async.cuh"
 #include "vt_kernels.cuh"
+#include "vt_tc.cuh"
 
 namespace vtk {
 using namespace vtd;
@@ -174,19 +176,27 @@ uint32_t matvec_error(cudaStream_t st, bool reset) {
   return e;
 }
 
-void launch_jacobi_matvec(const float* F, const float* rho, const float* E, const float* Bin, float* Bout, uint32_t n, double* partials,
-                          uint32_t* n_partials, cudaStream_t st) {
-  const uint32_t blocks = (n + MV_THREADS / 32 - 1) / (MV_THREADS / 32);
-  *n_partials = blocks;
+namespace {
+// F that is read with the cache's default policy: at most half the L2
+bool keep_f(uint32_t n) {
   static std::atomic<int> l2[MAX_DEVICES];
   const size_t l2_bytes = size_t(per_device_value(l2, [](int dev) {
     int b = 0;
     if (cudaDeviceGetAttribute(&b, cudaDevAttrL2CacheSize, dev) != cudaSuccess) { cudaGetLastError(); b = 0; }
     return b;
   }));
-  if (size_t(n) * n * 4 <= l2_bytes / 2) jacobi_matvec_kernel<true><<<blocks, MV_THREADS, 0, st>>>(F, rho, E, Bin, Bout, n, partials);
+  return size_t(n) * n * 4 <= l2_bytes / 2;
+}
+}  // namespace
+
+void launch_jacobi_matvec(const float* F, const float* rho, const float* E, const float* Bin, float* Bout, uint32_t n, double* partials,
+                          uint32_t* n_partials, cudaStream_t st) {
+  const uint32_t blocks = (n + MV_THREADS / 32 - 1) / (MV_THREADS / 32);
+  *n_partials = blocks;
+  if (keep_f(n)) jacobi_matvec_kernel<true><<<blocks, MV_THREADS, 0, st>>>(F, rho, E, Bin, Bout, n, partials);
   else jacobi_matvec_kernel<false><<<blocks, MV_THREADS, 0, st>>>(F, rho, E, Bin, Bout, n, partials);
 }
+
 
 // ---------------------------------------------------------------------------------------------- FP32 GEMM sweep
 // 128 x 64 output tile per 256-thread block (8 x 4 outputs per thread), K in 16-wide slices double-buffered through
@@ -357,6 +367,50 @@ void launch_jacobi_gemm_fp32(const float* F, const float* rho, const float* E, c
   const uint32_t blocks = uint32_t((size_t(n) * R / 4 + 255) / 256);
   *n_partials = blocks;
   jacobi_gemm_combine_kernel<<<blocks, 256, 0, st>>>(work, splits, rho, E, Bin, Bout, n, R, partials);
+}
+
+// ---------------------------------------------------------------------------------------------- FP32 tensor-core sweep
+// The same sweep with F B on the tensor cores in FP32 accuracy (vt_tc.cu tc_gemm_f32_kernel). F must come by TMA: rows
+// 16-byte aligned. An n that is no multiple of 4 is copied once per solve to rows that are (less than half a sweep of the FMA
+// kernel). Below 1536 nodes the FMA kernel stays: a sweep
+// is a few microseconds of work either way (n = 1000, 64 columns: 20.9 us there, 24.4 here; n = 2000: 29.4 and 25.7; n =
+// 4096: 73.6 and 30.4; n = 32768: 3197 and 755), and up to about there its rounding errors are the smaller ones.
+constexpr uint32_t TC_F32_MIN = 1536;
+bool jacobi_tc_f32_ok(const float* F, uint32_t n, uint32_t R) {
+  return R > 1 && n >= TC_F32_MIN && (n % 4u != 0u || (reinterpret_cast<uintptr_t>(F) & 15u) == 0u);
+}
+uint32_t jacobi_tc_f32_pitch(uint32_t n) { return (n + 3u) / 4u * 4u; }
+// rows of n floats to rows of `pitch` (a multiple of 4); the tail of a row is not read
+__global__ void __launch_bounds__(256) pitch_rows_kernel(const float* __restrict__ F, uint32_t n, uint32_t pitch, float* __restrict__ out) {
+  const float* src = F + size_t(blockIdx.x) * n;
+  float4* dst = reinterpret_cast<float4*>(out + size_t(blockIdx.x) * pitch);
+  for (uint32_t j = threadIdx.x; j < pitch / 4u; j += 256u) {
+    const uint32_t k = 4u * j;
+    dst[j] = make_float4(__ldcs(src + k), k + 1u < n ? __ldcs(src + k + 1u) : 0.0f, k + 2u < n ? __ldcs(src + k + 2u) : 0.0f,
+                         k + 3u < n ? __ldcs(src + k + 3u) : 0.0f);
+  }
+}
+void jacobi_tc_f32_repitch(const float* F, uint32_t n, float* out, cudaStream_t st) {
+  pitch_rows_kernel<<<n, 256, 0, st>>>(F, n, jacobi_tc_f32_pitch(n), out);
+}
+size_t jacobi_tc_f32_work(uint32_t n, uint32_t R) {
+  const uint32_t segs = tc_f32_segments(n, tc_f32_ctas(n, uint32_t(sm_count())));
+  return (tc_f32_parts_bytes(n) + 255) / 256 * 256 + size_t(segs) * n * R * 4 + 256;
+}
+// the maps of F and of the columns' parts (at the start of `work`), once per solve
+bool jacobi_tc_f32_setup(const float* F, uint32_t n, uint32_t pitch, void* work, TcMap* mF, TcMap* mB, cudaStream_t st, int* code) {
+  cudaMemsetAsync(work, 0, tc_f32_parts_bytes(n), st);   // columns past R are zero
+  return tc_encode(mF, F, n, n, 4, 128, code, pitch) && tc_encode(mB, work, tc_f32_pad(n), 192, 2, 192, code);
+}
+// first: Bin's parts are not in `work` yet (a sweep leaves its result's parts there)
+void launch_jacobi_tc_f32(const TcMap& mF, const TcMap& mB, bool first, const float* rho, const float* E, const float* Bin, float* Bout, uint32_t n,
+                          uint32_t R, void* work, uint32_t* err, double* partials, uint32_t* n_partials, cudaStream_t st) {
+  const uint32_t ctas = tc_f32_ctas(n, uint32_t(sm_count()));
+  uint16_t* parts = static_cast<uint16_t*>(work);
+  float* part = reinterpret_cast<float*>(static_cast<char*>(work) + (tc_f32_parts_bytes(n) + 255) / 256 * 256);
+  if (first) tc_pack_b_f32(Bin, n, R, parts, st);
+  tc_gemm_f32(&mF, &mB, n, R, ctas, part, err, st);
+  *n_partials = tc_combine_f32(part, ctas, rho, E, Bin, Bout, n, R, parts, partials, st);
 }
 
 __global__ void reduce_partials_kernel(const double* __restrict__ p, uint32_t n, double* __restrict__ out) {

@@ -19,6 +19,7 @@
 #include <mutex>
 
 #include "vt_async.cuh"
+#include "vt_kernels.cuh"
 #include "vt_tc.cuh"
 
 namespace vtk {
@@ -197,6 +198,323 @@ void launch_gemm(const TcMap* A, const TcMap* A2, const TcMap* B, const TcMap* B
                                                                                     partials, err);
 }
 
+// ------------------------------------------------------------------------------------------------ FP32 sweeps
+// F B in FP32 accuracy on the tensor cores. A float32 is the sum of three bf16 numbers (rounded to nearest at each step:
+// m at most 2^-9 and l at most 2^-18 of it), so the product of two is h h' + (h m' + m h') + (h l' + l h' + m m') to
+// 2^-26: six bf16 products, each exact. F stays FP32 in memory (no converted copy): its tiles arrive by TMA, converter warps
+// split them in registers and store the parts to TMEM, from where tcgen05.mma takes its A operand; B's parts are K-major
+// rows (h | m | l, 64 each) in shared memory.
+//
+// The tensor cores' accumulation drops what lies below the accumulator's last bit, which over a long sum of positive terms
+// is a drift (-6.4e-8 of the sum when it is taken up every 64 of K). So the h h' sums of each 32 of K go to an accumulator of
+// their own and four warps add a stage's two to FP32 registers, rounded to nearest, while the next stage's are made; the
+// small products (2^-8 of the sum) stay in theirs for a tile's whole range. Error of F B against FP64 (2-norm, positive
+// entries; the FMA chain of jacobi_gemm_fp32_kernel in brackets): n = 1540 6.3e-8 (6.9e-8), 4096 5.9e-8 (8.0e-8), 16384
+// 1.6e-7 (1.9e-7); signed entries 9.3e-8 (2.0e-7) to 2.5e-7 (7.3e-7).
+//
+// Bound: F from HBM. n = 32768, 64 columns: 755 us a sweep with its combine, 4.3 GB of F in ~725 us (0.87 of the measured
+// copy rate), against 3197 us on the FMA pipes. A stage is 32 KB of F, 1450 cycles of an SM's share of the bandwidth; its 24
+// MMAs take 768. What held it back on the way there: one lane's MMA code (72 cycles an MMA), two waits of the MMA warp
+// for each 32 of K (890 us), CTAs per tile and K split instead of one run each (a start and an end of ~5 us per 70 us).
+constexpr int FX_THREADS = 448;          // warps 0-3 drain, 4-11 convert, 12 TMA, 13 MMA
+constexpr int FX_STAGES = 4;
+constexpr uint32_t FX_F = 2 * 128 * 128, FX_B = 192 * 128, FX_STAGE = FX_F + FX_B;
+constexpr uint32_t FX_A = 96, FX_HH = 192, FX_R = 448;   // TMEM columns: A parts (2 x 96 from 0), h h' (2 x 2 x 64), the rest (64)
+constexpr size_t FX_SMEM = size_t(FX_STAGES) * FX_STAGE + 1024 + 256;
+
+// D (+)= A B: A in TMEM (a row per lane, two bf16 of K per column), B by descriptor
+__device__ __forceinline__ void mma_ta(uint32_t d, uint32_t a, uint64_t b, uint32_t accumulate) {
+  asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}" ::"r"(d), "r"(a), "l"(b),
+               "r"(IDESC_BF16), "r"(accumulate)
+               : "memory");
+}
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr), "r"(r[0]),
+      "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]),
+      "r"(r[14]), "r"(r[15])
+      : "memory");
+}
+__device__ __forceinline__ bool elect_one() {
+  uint32_t r;
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(r));
+  return r != 0u;
+}
+// 16 columns of two neighbouring accumulators of 64
+__device__ __forceinline__ void tmem_ld16x2(uint32_t taddr, float* v) {
+  uint32_t r[32];
+#pragma unroll
+  for (int q = 0; q < 2; q++) {
+    uint32_t* x = r + 16 * q;
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=r"(x[0]), "=r"(x[1]), "=r"(x[2]), "=r"(x[3]), "=r"(x[4]), "=r"(x[5]), "=r"(x[6]), "=r"(x[7]), "=r"(x[8]), "=r"(x[9]), "=r"(x[10]),
+          "=r"(x[11]), "=r"(x[12]), "=r"(x[13]), "=r"(x[14]), "=r"(x[15])
+        : "r"(taddr + 64u * q));
+  }
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < 32; i++) v[i] = __uint_as_float(r[i]);
+}
+// two floats' bf16 parts, packed (the first in the low half); x becomes the remainder
+__device__ __forceinline__ uint32_t take_bf16x2(float& x0, float& x1) {
+  uint32_t w;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(w) : "f"(x1), "f"(x0));
+  x0 -= __uint_as_float(w << 16);
+  x1 -= __uint_as_float(w & 0xffff0000u);
+  return w;
+}
+
+// One CTA per SM takes an equal run of the (row tile, K stage) pairs in tile order, across tiles without a break in the
+// pipeline (a CTA's start and end cost ~5 us); a tile's sum is then that of the few CTAs whose runs meet it, each in a
+// partial of its own. Stage g belongs to CTA fx_cta(g).
+__host__ __device__ inline uint32_t fx_cta(uint64_t g, uint64_t total, uint32_t ctas) { return uint32_t(((g + 1u) * ctas - 1u) / total); }
+
+__global__ void __launch_bounds__(FX_THREADS, 1)
+    tc_gemm_f32_kernel(const __grid_constant__ TcMap mF, const __grid_constant__ TcMap mB, uint32_t n, uint32_t R, float* __restrict__ partials,
+                       uint32_t* err) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + FX_STAGES * FX_STAGE);
+  // Stage kt has A buffer and h h' accumulators kt & 1. full[s]: a stage's tiles landed; empty[s]: its MMAs are done;
+  // ready[b]: its A parts are in TMEM, its B tile landed and its accumulators are free; done[b]: its MMAs are done; drained[b]:
+  // its h h' accumulators are read; rest: the small products of a tile are read; fin: the last MMA is done
+  auto full = [&](uint32_t s) { return smem_u32(bars + s); };
+  auto empty = [&](uint32_t s) { return smem_u32(bars + FX_STAGES + s); };
+  auto ready = [&](uint32_t a) { return smem_u32(bars + 2 * FX_STAGES + a); };
+  auto done = [&](uint32_t a) { return smem_u32(bars + 2 * FX_STAGES + 2 + a); };
+  auto drained = [&](uint32_t b) { return smem_u32(bars + 2 * FX_STAGES + 4 + b); };
+  const uint32_t rest = smem_u32(bars + 2 * FX_STAGES + 6), fin = smem_u32(bars + 2 * FX_STAGES + 7);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * FX_STAGES + 8);
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+  const uint32_t KT = (n + 63u) / 64u;
+  const uint64_t total = uint64_t((n + 127u) / 128u) * KT;
+  const uint64_t g0 = uint64_t(blockIdx.x) * total / gridDim.x;
+  const uint32_t nkt = uint32_t((uint64_t(blockIdx.x) + 1u) * total / gridDim.x - g0);
+  uint32_t tile = uint32_t(g0 / KT), kk = uint32_t(g0 % KT);   // of the role's next stage
+  if (threadIdx.x == 0) {
+    for (uint32_t s = 0; s < FX_STAGES; s++) { mbar_init(full(s), 1); mbar_init(empty(s), 1); }
+    for (uint32_t b = 0; b < 2; b++) { mbar_init(ready(b), 8); mbar_init(done(b), 1); mbar_init(drained(b), 4); }
+    mbar_init(rest, 4);
+    mbar_init(fin, 1);
+    mbar_fence_init();
+  }
+  if (warp == 13) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(tmem_slot)) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+
+  if (warp == 12) {
+    if (lane == 0) {
+      uint32_t issued = 0;
+      for (uint32_t kt = 0; kt < nkt; kt++) {
+        const uint32_t s = kt % FX_STAGES;
+        if (kt >= FX_STAGES && !mbar_wait(empty(s), ((kt / FX_STAGES) & 1u) ^ 1u, err)) break;
+        mbar_expect_tx(full(s), FX_STAGE);
+        const int32_t kx = int32_t(kk * 64u), m0 = int32_t(tile * 128u);
+        const uint32_t at = smem_u32(smem + s * FX_STAGE);
+        tma_load_2d(at, &mF, kx, m0, full(s));
+        tma_load_2d(at + FX_F / 2, &mF, kx + 32, m0, full(s));
+        tma_load_2d(at + FX_F, &mB, kx, 0, full(s));
+        if (++kk == KT) { kk = 0; tile++; }
+        issued++;
+      }
+      // drain: every stage this thread filled must have landed before the CTA may exit
+      for (uint32_t kt = issued > FX_STAGES ? issued - FX_STAGES : 0; kt < issued; kt++) mbar_wait(full(kt % FX_STAGES), (kt / FX_STAGES) & 1u, err);
+    }
+  } else if (warp == 13) {
+    // The whole warp runs the loop, so that the descriptors stay in uniform registers, and one elected lane issues (in one
+    // lane's code an MMA took 72 cycles to issue; N = 64 runs in 32). A wait costs this warp ~200 cycles beside the
+    // converters, so it makes one per stage: they wait for what `ready` stands for.
+    const bool el = elect_one();
+    const uint64_t B0 = sw128_desc(smem_u32(smem + FX_F));
+    uint32_t tiles = 0;   // tiles begun before this one
+    for (uint32_t kt = 0; kt < nkt; kt++) {
+      const uint32_t s = kt % FX_STAGES, b = kt & 1u;
+      const bool first = kt == 0u || kk == 0u;
+      bool ok = mbar_wait(ready(b), (kt >> 1) & 1u, err);
+      if (first) {
+        if (tiles) ok = ok && mbar_wait(rest, (tiles - 1u) & 1u, err);
+        tiles++;
+      }
+      if (++kk == KT) kk = 0;
+      if (!__all_sync(0xffffffffu, ok)) break;
+      tc_fence_after();
+      const uint64_t Bs = B0 + ((s * FX_STAGE) >> 4);   // rows h' | m' | l', 512 units of 16 bytes each
+      const uint32_t A = tmem + FX_A * b, hh = tmem + FX_HH + 128u * b, r = tmem + FX_R;
+      if (el) {
+#pragma unroll
+        for (uint32_t k = 0; k < 4; k++) {   // 16 of K each
+          const uint32_t h = A + 8 * k, m = h + 32, l = h + 64;
+          const uint64_t Bh = Bs + 2 * k, Bm = Bh + 512, Bl = Bh + 1024;
+          mma_ta(hh + 64u * (k >> 1), h, Bh, k & 1u);
+          mma_ta(r, h, Bm, k || !first);
+          mma_ta(r, m, Bh, 1u);
+          mma_ta(r, h, Bl, 1u);
+          mma_ta(r, l, Bh, 1u);
+          mma_ta(r, m, Bm, 1u);
+        }
+        mma_commit(empty(s));
+        mma_commit(done(b));
+      }
+      __syncwarp();
+    }
+    if (el) mma_commit(fin);
+    mbar_wait(fin, 0, err);   // no MMA in flight when the TMEM is given back
+  } else if (warp >= 4) {
+    // converters: warps 4-7 the stage's first 32 of K, 8-11 the others; a thread takes a row (its TMEM lane)
+    const uint32_t half = (warp - 4u) >> 2, row = (warp & 3u) * 32u + lane;
+    for (uint32_t kt = 0; kt < nkt; kt++) {
+      const uint32_t s = kt % FX_STAGES, b = kt & 1u;
+      bool ok = mbar_wait(full(s), (kt / FX_STAGES) & 1u, err);
+      if (kt >= 2u) ok = ok && mbar_wait(done(b), ((kt >> 1) - 1u) & 1u, err);   // the A buffer is free
+      if (!__all_sync(0xffffffffu, ok)) break;
+      tc_fence_after();
+      const float4* src = reinterpret_cast<const float4*>(smem + s * FX_STAGE + half * (FX_F / 2) + row * 128u);
+      const uint32_t taddr = tmem + FX_A * b + 16u * half + (((warp & 3u) * 32u) << 16);
+      uint32_t h[16], m[16], l[16];
+#pragma unroll
+      for (uint32_t c = 0; c < 8; c++) {
+        float4 x = src[c ^ (row & 7u)];   // 128-byte swizzle
+        h[2 * c] = take_bf16x2(x.x, x.y); h[2 * c + 1] = take_bf16x2(x.z, x.w);
+        m[2 * c] = take_bf16x2(x.x, x.y); m[2 * c + 1] = take_bf16x2(x.z, x.w);
+        l[2 * c] = take_bf16x2(x.x, x.y); l[2 * c + 1] = take_bf16x2(x.z, x.w);
+      }
+      tmem_st16(taddr, h);
+      tmem_st16(taddr + 32, m);
+      tmem_st16(taddr + 64, l);
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+      if (kt >= 2u && !__all_sync(0xffffffffu, mbar_wait(drained(b), ((kt >> 1) - 1u) & 1u, err))) break;
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(ready(b));
+    }
+  } else {
+    // drain: a stage's h h' sums in one rounding to nearest, in K order; at a tile's end the small products
+    float acc[64];
+#pragma unroll
+    for (int c = 0; c < 64; c++) acc[c] = 0.0f;
+    const uint32_t base = tmem + ((warp * 32u) << 16);
+    for (uint32_t kt = 0; kt < nkt; kt++) {
+      if (!__all_sync(0xffffffffu, mbar_wait(done(kt & 1u), (kt >> 1) & 1u, err))) break;
+      tc_fence_after();
+#pragma unroll
+      for (int g = 0; g < 4; g++) {
+        float v[32];
+        tmem_ld16x2(base + FX_HH + 128u * (kt & 1u) + 16u * g, v);
+#pragma unroll
+        for (int c = 0; c < 16; c++) acc[16 * g + c] += v[c] + v[16 + c];
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(drained(kt & 1u));
+      if (++kk < KT && kt + 1u < nkt) continue;
+      // the tile's end, or the run's: this CTA's partial of it
+#pragma unroll
+      for (int g = 0; g < 4; g++) {
+        float v[16];
+        tmem_ld16(base + FX_R + 16u * g, v);
+#pragma unroll
+        for (int c = 0; c < 16; c++) acc[16 * g + c] += v[c];
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(rest);
+      const uint32_t row = tile * 128u + warp * 32u + lane, seg = blockIdx.x - fx_cta(uint64_t(tile) * KT, total, gridDim.x);
+      if (row < n) {
+        float4* dst = reinterpret_cast<float4*>(partials + (size_t(seg) * n + row) * R);
+#pragma unroll
+        for (int c = 0; c < 16; c++)
+          if (4u * c < R) dst[c] = make_float4(acc[4 * c], acc[4 * c + 1], acc[4 * c + 2], acc[4 * c + 3]);
+      }
+#pragma unroll
+      for (int c = 0; c < 64; c++) acc[c] = 0.0f;
+      kk = 0;
+      tile++;
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 13) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
+}
+
+__device__ __forceinline__ void block_sum2(double a, double b, double* partials) {
+  __shared__ double sa[32], sb[32];
+  for (int o = 16; o > 0; o >>= 1) { a += __shfl_down_sync(0xffffffffu, a, o); b += __shfl_down_sync(0xffffffffu, b, o); }
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
+  if (l == 0) { sa[w] = a; sb[w] = b; }
+  __syncthreads();
+  if (w == 0) {
+    a = l < nw ? sa[l] : 0.0;
+    b = l < nw ? sb[l] : 0.0;
+    for (int o = 16; o > 0; o >>= 1) { a += __shfl_down_sync(0xffffffffu, a, o); b += __shfl_down_sync(0xffffffffu, b, o); }
+    if (l == 0) { partials[2 * blockIdx.x] = a; partials[2 * blockIdx.x + 1] = b; }
+  }
+}
+
+// A tile of 32 rows of the n x R iterate, in shared memory, to its bf16 parts as K-major rows: Bt (192 x np): row 64 q + c
+// holds part q of column c. A thread splits two neighbours of K: a 32-bit store per part (np is even); c < R
+__device__ __forceinline__ void store_parts(const float (*tile)[65], uint32_t i0, uint32_t R, uint32_t np, uint16_t* __restrict__ Bt) {
+  for (uint32_t q = threadIdx.x; q < R * 16u; q += 256u) {
+    const uint32_t c = q / 16u, k = 2u * (q % 16u);
+    float x0 = tile[k][c], x1 = tile[k + 1u][c];
+    uint32_t* dst = reinterpret_cast<uint32_t*>(Bt + size_t(c) * np + i0 + k);
+    dst[0] = take_bf16x2(x0, x1);
+    dst[size_t(32) * np] = take_bf16x2(x0, x1);
+    dst[size_t(64) * np] = take_bf16x2(x0, x1);
+  }
+}
+__global__ void __launch_bounds__(256) pack_b_f32_kernel(const float* __restrict__ X, uint32_t n, uint32_t R, uint32_t np, uint16_t* __restrict__ Bt) {
+  __shared__ float tile[32][65];
+  const uint32_t i0 = blockIdx.x * 32u;
+  for (uint32_t q = threadIdx.x; q < 32u * R; q += 256u) tile[q / R][q % R] = i0 + q / R < n ? X[size_t(i0) * R + q] : 0.0f;
+  __syncthreads();
+  store_parts(tile, i0, R, np, Bt);
+}
+
+// Y = E + rho (sum of the tile's partials, in CTA order), its parts for the next sweep, and the block's
+// sums of |Y - X|^2 and |Y|^2
+__global__ void __launch_bounds__(256) combine_f32_kernel(const float* __restrict__ part, uint32_t ctas, const float* __restrict__ rho,
+                                                          const float* __restrict__ E, const float* __restrict__ X, float* __restrict__ Y, uint32_t n,
+                                                          uint32_t R, uint32_t np, uint16_t* __restrict__ Bt, double* __restrict__ norms) {
+  __shared__ float tile[32][65];
+  const uint32_t i0 = blockIdx.x * 32u, R4 = R / 4u;
+  const size_t stride = size_t(n) * R4;
+  const float4* P = reinterpret_cast<const float4*>(part);
+  // the CTAs whose runs meet this tile of 128 rows
+  const uint32_t KT = (n + 63u) / 64u;
+  const uint64_t total = uint64_t((n + 127u) / 128u) * KT, g = uint64_t(i0 / 128u) * KT;
+  const uint32_t splits = i0 < n ? fx_cta(g + KT - 1u, total, ctas) - fx_cta(g, total, ctas) + 1u : 0u;
+  double d2 = 0.0, b2 = 0.0;
+  for (uint32_t q = threadIdx.x; q < 32u * R4; q += 256u) {
+    const uint32_t r = q / R4, c = 4u * (q % R4);
+    float4 b = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (i0 + r < n) {
+      const size_t i = size_t(i0) * R4 + q;
+      float4 a = P[i];
+      for (uint32_t s = 1; s < splits; s++) {
+        const float4 v = P[s * stride + i];
+        a.x += v.x; a.y += v.y; a.z += v.z; a.w += v.w;
+      }
+      const float rr = rho[i0 + r];
+      const float4 e = reinterpret_cast<const float4*>(E)[i], x = reinterpret_cast<const float4*>(X)[i];
+      b = make_float4(fmaf(rr, a.x, e.x), fmaf(rr, a.y, e.y), fmaf(rr, a.z, e.z), fmaf(rr, a.w, e.w));
+      reinterpret_cast<float4*>(Y)[i] = b;
+      const double dx = double(b.x) - x.x, dy = double(b.y) - x.y, dz = double(b.z) - x.z, dw = double(b.w) - x.w;
+      d2 += dx * dx + dy * dy + dz * dz + dw * dw;
+      b2 += double(b.x) * b.x + double(b.y) * b.y + double(b.z) * b.z + double(b.w) * b.w;
+    }
+    tile[r][c] = b.x; tile[r][c + 1u] = b.y; tile[r][c + 2u] = b.z; tile[r][c + 3u] = b.w;
+  }
+  __syncthreads();
+  store_parts(tile, i0, R, np, Bt);
+  block_sum2(d2, b2, norms);
+}
+
 // ------------------------------------------------------------------------------------------------ CUDA-core helpers
 __global__ void split_bf16_kernel(const float* __restrict__ F, __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo, size_t count) {
   for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < count; i += size_t(gridDim.x) * blockDim.x) {
@@ -276,20 +594,6 @@ __global__ void pack_b_kernel(const float* __restrict__ X, uint32_t n, uint32_t 
       hi[o] = h;
       if (MODE == TC_BF16X3) lo[o] = __float2bfloat16_rn(x - __bfloat162float(h));
     }
-  }
-}
-
-__device__ __forceinline__ void block_sum2(double a, double b, double* partials) {
-  __shared__ double sa[32], sb[32];
-  for (int o = 16; o > 0; o >>= 1) { a += __shfl_down_sync(0xffffffffu, a, o); b += __shfl_down_sync(0xffffffffu, b, o); }
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
-  if (l == 0) { sa[w] = a; sb[w] = b; }
-  __syncthreads();
-  if (w == 0) {
-    a = l < nw ? sa[l] : 0.0;
-    b = l < nw ? sb[l] : 0.0;
-    for (int o = 16; o > 0; o >>= 1) { a += __shfl_down_sync(0xffffffffu, a, o); b += __shfl_down_sync(0xffffffffu, b, o); }
-    if (l == 0) { partials[2 * blockIdx.x] = a; partials[2 * blockIdx.x + 1] = b; }
   }
 }
 
@@ -374,14 +678,15 @@ EncodeFn encode_fn() {
 
 static_assert(sizeof(CUtensorMap) == sizeof(TcMap), "tensor map size");
 
-bool tc_encode(TcMap* map, const void* base, uint32_t inner, uint32_t rows, uint32_t elt_bytes, uint32_t box_rows, int* code) {
+bool tc_encode(TcMap* map, const void* base, uint32_t inner, uint32_t rows, uint32_t elt_bytes, uint32_t box_rows, int* code, uint32_t pitch) {
   EncodeFn fn = encode_fn();
   if (!fn) { if (code) *code = -1; return false; }
   const cuuint64_t dims[2] = {inner, rows};
-  const cuuint64_t strides[1] = {cuuint64_t(inner) * elt_bytes};
+  const cuuint64_t strides[1] = {cuuint64_t(pitch ? pitch : inner) * elt_bytes};
   const cuuint32_t box[2] = {128u / elt_bytes, box_rows};
   const cuuint32_t estr[2] = {1, 1};
-  const CUresult r = fn(reinterpret_cast<CUtensorMap*>(map), elt_bytes == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8, 2,
+  const CUtensorMapDataType type = elt_bytes == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : elt_bytes == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8;
+  const CUresult r = fn(reinterpret_cast<CUtensorMap*>(map), type, 2,
                         const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (code) *code = int(r);
@@ -395,6 +700,36 @@ void tc_gemm(int mode, const TcMap* A, const TcMap* A2, const TcMap* B, const Tc
   if (mode == TC_BF16) launch_gemm<TC_BF16, 6>(A, A2, B, B2, n, splits, k_tiles, partials, err, st);
   else if (mode == TC_BF16X3) launch_gemm<TC_BF16X3, 4>(A, A2, B, B2, n, splits, k_tiles, partials, err, st);
   else launch_gemm<TC_FP8, 6>(A, A2, B, B2, n, splits, k_tiles, partials, err, st);
+}
+
+size_t tc_f32_parts_bytes(uint32_t n) { return size_t(192) * tc_f32_pad(n) * 2; }
+
+// one CTA per SM, and the most CTAs whose runs meet one tile
+uint32_t tc_f32_ctas(uint32_t n, uint32_t sms) {
+  return uint32_t(std::min<uint64_t>(sms, uint64_t((n + 127u) / 128u) * ((n + 63u) / 64u)));
+}
+uint32_t tc_f32_segments(uint32_t n, uint32_t ctas) {
+  const uint32_t KT = (n + 63u) / 64u;
+  const uint64_t run = uint64_t((n + 127u) / 128u) * KT / ctas;
+  return uint32_t(KT / std::max<uint64_t>(1, run)) + 2u;
+}
+
+void tc_gemm_f32(const TcMap* F, const TcMap* B, uint32_t n, uint32_t R, uint32_t ctas, float* partials, uint32_t* err, cudaStream_t st) {
+  static std::atomic<int> set[MAX_DEVICES];
+  per_device_value(set, [](int) { cudaFuncSetAttribute(tc_gemm_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(FX_SMEM)); return 1; });
+  tc_gemm_f32_kernel<<<ctas, FX_THREADS, FX_SMEM, st>>>(*F, *B, n, R, partials, err);
+}
+
+void tc_pack_b_f32(const float* X, uint32_t n, uint32_t R, uint16_t* Bt, cudaStream_t st) {
+  const uint32_t np = tc_f32_pad(n);
+  pack_b_f32_kernel<<<np / 32, 256, 0, st>>>(X, n, R, np, Bt);
+}
+
+uint32_t tc_combine_f32(const float* part, uint32_t ctas, const float* rho, const float* E, const float* X, float* Y, uint32_t n, uint32_t R, uint16_t* Bt,
+                        double* norms, cudaStream_t st) {
+  const uint32_t np = tc_f32_pad(n);
+  combine_f32_kernel<<<np / 32, 256, 0, st>>>(part, ctas, rho, E, X, Y, n, R, np, Bt, norms);
+  return np / 32;
 }
 
 void tc_split_bf16(const float* F, uint16_t* hi, uint16_t* lo, size_t count, cudaStream_t st) {

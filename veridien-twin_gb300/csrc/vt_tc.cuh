@@ -16,12 +16,25 @@ struct alignas(64) TcMap { unsigned char bytes[128]; };
 // F (n x n, K contiguous) and the transposed right-hand sides Bt (r x n, K contiguous) as TMA tiles:
 // mode BF16 / BF16X3: bf16 elements, boxes of 64 x 128 (F) and 64 x 64 (Bt); FP8: bytes, boxes of 128 x 128 / 128 x 64.
 // Returns false (with the driver's error code in *code) when the map cannot be encoded.
-bool tc_encode(TcMap* map, const void* base, uint32_t inner, uint32_t rows, uint32_t elt_bytes, uint32_t box_rows, int* code);
+// pitch: elements from row to row (0: inner).
+bool tc_encode(TcMap* map, const void* base, uint32_t inner, uint32_t rows, uint32_t elt_bytes, uint32_t box_rows, int* code, uint32_t pitch = 0);
 
 // partials[s][i][c] = sum over split s's K range of A[i][k] B[c][k]  (c < 64), three products for BF16X3
 void tc_gemm(int mode, const TcMap* A, const TcMap* A2, const TcMap* B, const TcMap* B2, uint32_t n, uint32_t splits, uint32_t k_tiles,
              float* partials, uint32_t* err, cudaStream_t st);
 uint32_t tc_k_elems(int mode);   // K elements per pipeline stage (128 bytes of a row)
+
+// FP32 F (n x n, n % 4 == 0, 16-byte aligned rows) times the FP32 columns whose parts tc_pack_b_f32 laid out, by `ctas`
+// CTAs: partials[s][i][c], s < tc_f32_segments, summed over the segments of row i's tile by tc_combine_f32; c < R
+inline uint32_t tc_f32_pad(uint32_t n) { return (n + 63u) / 64u * 64u; }
+size_t tc_f32_parts_bytes(uint32_t n);   // X's parts: 192 rows (h | m | l, 64 columns each) of tc_f32_pad(n) bf16
+uint32_t tc_f32_ctas(uint32_t n, uint32_t sms);
+uint32_t tc_f32_segments(uint32_t n, uint32_t ctas);
+void tc_pack_b_f32(const float* X, uint32_t n, uint32_t R, uint16_t* Bt, cudaStream_t st);
+void tc_gemm_f32(const TcMap* F, const TcMap* B, uint32_t n, uint32_t R, uint32_t ctas, float* partials, uint32_t* err, cudaStream_t st);
+// Y = E + rho (sum of the partials), Y's parts into Bt, norms of Y - X and Y per block; returns the blocks
+uint32_t tc_combine_f32(const float* part, uint32_t ctas, const float* rho, const float* E, const float* X, float* Y, uint32_t n, uint32_t R, uint16_t* Bt,
+                        double* norms, cudaStream_t st);
 
 // F (fp32) -> hi = bf16(F), lo = bf16(F - hi)
 void tc_split_bf16(const float* F, uint16_t* hi, uint16_t* lo, size_t count, cudaStream_t st);
