@@ -74,7 +74,7 @@ vt_status alloc_calib(vt_ctx* ctx) {
   K.max_partials = std::max<uint32_t>(4096, 2 * ((K.n + 7) / 8) + 16);
   const size_t bytes[] = {n * n * 4, n * L * 4, n * 12, n * 12, n * 4, size_t(ctx->S.tri_count) * 4, size_t(ctx->S.tri_count) * 4,
                           kMaxMat * 12, L * 4, n * 12, n * 4, n * 12,
-                          size_t(K.max_partials) * 8, kMaxMat * 24, L * 8, n * 24, n * 8, n * 8, n * 24, vtk::jacobi_t_work(uint32_t(n)), 64,
+                          size_t(K.max_partials) * 8, kMaxMat * 24, L * 8, n * 24, n * 24, n * 24, vtk::jacobi_t_work(uint32_t(n)), 64,
                           ctx->S.cams.size() * 64};
   size_t total = 0;
   for (size_t b : bytes) total += (b + 255) / 256 * 256;
@@ -91,7 +91,7 @@ vt_status alloc_calib(vt_ctx* ctx) {
   K.DL = reinterpret_cast<float*>(take()); K.H = reinterpret_cast<float*>(take());
   K.partials = reinterpret_cast<double*>(take());
   K.g_alb = reinterpret_cast<double*>(take()); K.g_lamp = reinterpret_cast<double*>(take()); K.g_H = reinterpret_cast<double*>(take());
-  K.lam0 = reinterpret_cast<double*>(take()); K.lam1 = reinterpret_cast<double*>(take()); K.lam = reinterpret_cast<double*>(take());
+  K.lam0 = reinterpret_cast<double*>(take()); K.lam1 = reinterpret_cast<double*>(take());
   K.work = reinterpret_cast<double*>(take()); K.loss = reinterpret_cast<double*>(take());
   K.g_K = reinterpret_cast<double*>(take());
   return VT_OK;
@@ -384,22 +384,19 @@ vt_status vt_calib_backward(vt_ctx* ctx, double* g_albedo, double* g_lamp) {
   }
   K.have_k = K.want_k;
   VT_CK(cudaGetLastError());
-  // transposed Jacobi: lambda = F^T (g_H + rho o lambda) per channel, from lambda = 0
-  for (uint32_t c = 0; c < 3; c++) {
-    VT_CK(cudaMemsetAsync(K.lam0, 0, n * 8, ctx->stream));
-    double *cur = K.lam0, *nxt = K.lam1;
-    for (uint32_t it = 0; it < K.iters; it++) {
-      vtk::launch_jacobi_t(K.F, K.g_H + c * n, K.rho + c * n, cur, nxt, uint32_t(n), K.work, ctx->stream);
-      std::swap(cur, nxt);
-    }
-    VT_CK(cudaMemcpyAsync(K.lam + c * n, cur, n * 8, cudaMemcpyDeviceToDevice, ctx->stream));
+  // transposed Jacobi: lambda = F^T (g_H + rho o lambda), the three channels together, from lambda = 0
+  double *cur = K.lam0, *nxt = K.lam1;
+  VT_CK(cudaMemsetAsync(cur, 0, 3 * n * 8, ctx->stream));
+  for (uint32_t it = 0; it < K.iters; it++) {
+    vtk::launch_jacobi_t(K.F, K.g_H, K.rho, cur, nxt, uint32_t(n), K.work, ctx->stream);
+    std::swap(cur, nxt);
   }
   VT_CK(cudaGetLastError());
   std::vector<double> ga(size_t(K.n_mat) * 3), gl(K.n_lamps), lam(3 * n);
   std::vector<float> DL(n), H(3 * n);
   VT_CK(cudaMemcpyAsync(ga.data(), K.g_alb, ga.size() * 8, cudaMemcpyDeviceToHost, ctx->stream));
   VT_CK(cudaMemcpyAsync(gl.data(), K.g_lamp, gl.size() * 8, cudaMemcpyDeviceToHost, ctx->stream));
-  VT_CK(cudaMemcpyAsync(lam.data(), K.lam, lam.size() * 8, cudaMemcpyDeviceToHost, ctx->stream));
+  VT_CK(cudaMemcpyAsync(lam.data(), cur, lam.size() * 8, cudaMemcpyDeviceToHost, ctx->stream));
   VT_CK(cudaMemcpyAsync(DL.data(), K.DL, n * 4, cudaMemcpyDeviceToHost, ctx->stream));
   VT_CK(cudaMemcpyAsync(H.data(), K.H, 3 * n * 4, cudaMemcpyDeviceToHost, ctx->stream));
   VT_CK(cudaStreamSynchronize(ctx->stream));

@@ -637,87 +637,187 @@ __device__ __forceinline__ void df_mac(float f, float2 x, float& sh, float& sl) 
   sl = __fsub_rn(lo, __fsub_rn(sh, t));
 }
 
-// 64 row splits, so that a sweep has blocks enough to fill the SMs several times (16 splits took 2.7x as long under
-// ncu); a thread sums its column's rows in two interleaved float pairs (two independent dependency chains), which
-// meet in FP64
-constexpr uint32_t JT_SPLITS = 64, JT_COLS = 256;
-// partial[split][j] = sum over rows i of the split of F[i][j] (g_i + rho_i lam_i)
-__global__ void __launch_bounds__(JT_COLS) jacobi_t_kernel(const float* __restrict__ F, const double* __restrict__ g, const float* __restrict__ rho,
-                                                          const double* __restrict__ lam, uint32_t n, double* __restrict__ part) {
-  __shared__ float2 w[JT_COLS];
-  const uint32_t j = blockIdx.x * JT_COLS + threadIdx.x;
-  const uint32_t rows = (n + JT_SPLITS - 1) / JT_SPLITS, i0 = blockIdx.y * rows, i1 = min(n, i0 + rows);
-  float sh0 = 0.0f, sl0 = 0.0f, sh1 = 0.0f, sl1 = 0.0f;
-  for (uint32_t ib = i0; ib < i1; ib += JT_COLS) {
-    const uint32_t ii = ib + threadIdx.x;
-    w[threadIdx.x] = ii < i1 ? df_split(g[ii] + double(rho[ii]) * lam[ii]) : make_float2(0.0f, 0.0f);
-    __syncthreads();
-    const uint32_t m = min(JT_COLS, i1 - ib);
-    if (j < n) {
-      const float* Fc = F + size_t(ib) * n + j;
-      uint32_t k = 0;
-      for (; k + 1 < m; k += 2) {
-        const float f0 = Fc[size_t(k) * n], f1 = Fc[size_t(k + 1) * n];
-        df_mac(f0, w[k], sh0, sl0);
-        df_mac(f1, w[k + 1], sh1, sl1);
-      }
-      if (k < m) df_mac(Fc[size_t(k) * n], w[k], sh0, sl0);
-    }
-    __syncthreads();
-  }
-  if (j < n) part[size_t(blockIdx.y) * n + j] = (double(sh0) + double(sl0)) + (double(sh1) + double(sl1));
+// df_mac on two products at once, the pair's sums apart (every element rounded as df_mac's own step; x - y is x + (-y)
+// exactly). f2 and nf2 = -f2; xh, xl the vector's parts.
+struct DfAcc { float2 h, l; };
+__device__ __forceinline__ float2 f2(float a, float b) { return make_float2(a, b); }
+__device__ __forceinline__ void df_mac2(float2 f, float2 nf, float2 xh, float2 xl, DfAcc& s) {
+  const float2 m1 = f2(-1.0f, -1.0f);
+  const float2 np = __fmul2_rn(nf, xh);                              // -p
+  const float2 e = __ffma2_rn(f, xl, __ffma2_rn(f, xh, np));
+  const float2 t = __ffma2_rn(np, m1, s.h);                          // sh + p
+  const float2 nv = __ffma2_rn(t, m1, s.h);                          // -(t - sh)
+  const float2 a = __ffma2_rn(__fadd2_rn(t, nv), m1, s.h);           // sh - (t - v)
+  const float2 b = __ffma2_rn(np, m1, nv);                           // p - v
+  const float2 lo = __fadd2_rn(s.l, __fadd2_rn(__fadd2_rn(a, b), e));
+  s.h = __fadd2_rn(t, lo);
+  s.l = __fadd2_rn(lo, __ffma2_rn(s.h, m1, t));                      // lo - (sh - t)
 }
-__global__ void jacobi_t_combine(const double* __restrict__ part, uint32_t n, double* __restrict__ out) {
-  const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= n) return;
-  double a = 0.0;
-  for (uint32_t s = 0; s < JT_SPLITS; s++) a += part[size_t(s) * n + j];
-  out[j] = a;
+// the sum of two float pairs, renormalised
+__device__ __forceinline__ float2 df_add(float2 x, float2 y) {
+  const float t = __fadd_rn(x.x, y.x), v = __fsub_rn(t, x.x);
+  const float lo = __fadd_rn(__fadd_rn(x.y, y.y), __fadd_rn(__fsub_rn(x.x, __fsub_rn(t, v)), __fsub_rn(y.x, v)));
+  const float h = __fadd_rn(t, lo);
+  return make_float2(h, __fsub_rn(lo, __fsub_rn(h, t)));
 }
 
-// The three channels' B_c,out = rho_c o (DL + F B_c,in) at FP64 accuracy (F in FP32, B as float pairs planar [c][n],
-// the products summed in float pairs), one warp per row reading F once for all three; with `H` set, H_c = F B_c,in
-// (rounded to FP32) instead. Each channel's sums run in the order of a one-channel sweep, so the values are its.
-__global__ void __launch_bounds__(256) radiosity64_kernel(const float* __restrict__ F, const float* __restrict__ rho, const float* __restrict__ DL,
-                                                        const float2* __restrict__ Bin, float2* __restrict__ Bout, float* __restrict__ H,
-                                                        uint32_t n) {
-  const uint32_t row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
-  if (row >= n) return;
-  const float* Fr = F + size_t(row) * n;
-  float sh[3] = {0.0f, 0.0f, 0.0f}, sl[3] = {0.0f, 0.0f, 0.0f};
-  if ((n & 3u) == 0u && ((reinterpret_cast<uintptr_t>(F) | reinterpret_cast<uintptr_t>(Bin)) & 15u) == 0u) {
-    const float4* F4 = reinterpret_cast<const float4*>(Fr);
-    for (uint32_t j = lane; j < (n >> 2); j += 32) {
-      const float4 f = __ldg(F4 + j);
+// Transposed sweep, the three channels in one pass over F: partial[split][c][j] = sum over rows i of the split of F[i][j]
+// (g_c,i + rho_c,i lam_c,i). A thread takes four columns, two float-pair sums a step (f32x2), so a row of F is one 16-byte
+// load for 12 products; the rows' weights lie in shared memory as the pairs the products take. Bound by the FMA pipe: 14
+// operations a product, 18 us at its rate. N = 4096: 38 + 5 us a sweep of three channels with its combine (a channel and a
+// product at a time, one row in flight: 80 + 25 us).
+constexpr uint32_t JT_SPLITS = 64, JT_THREADS = 256, JT_ROWS = 64;
+__global__ void __launch_bounds__(JT_THREADS) jacobi_t_kernel(const float* __restrict__ F, const double* __restrict__ g, const float* __restrict__ rho,
+                                                             const double* __restrict__ lam, uint32_t n, double* __restrict__ part) {
+  __shared__ float4 w[3][JT_ROWS];   // (hi, hi, lo, lo)
+  const uint32_t j = 4u * (blockIdx.x * JT_THREADS + threadIdx.x);
+  const uint32_t rows = (n + JT_SPLITS - 1) / JT_SPLITS, i0 = blockIdx.y * rows, i1 = min(n, i0 + rows);
+  const bool vec = (n & 3u) == 0u;
+  DfAcc s[3][2];
 #pragma unroll
-      for (int c = 0; c < 3; c++) {
-        const float4* B4 = reinterpret_cast<const float4*>(Bin + size_t(c) * n);   // two pairs per float4
-        const float4 b01 = __ldg(B4 + 2 * j), b23 = __ldg(B4 + 2 * j + 1);
-        df_mac(f.x, make_float2(b01.x, b01.y), sh[c], sl[c]);
-        df_mac(f.y, make_float2(b01.z, b01.w), sh[c], sl[c]);
-        df_mac(f.z, make_float2(b23.x, b23.y), sh[c], sl[c]);
-        df_mac(f.w, make_float2(b23.z, b23.w), sh[c], sl[c]);
-      }
+  for (int c = 0; c < 3; c++) s[c][0].h = s[c][0].l = s[c][1].h = s[c][1].l = f2(0.0f, 0.0f);
+  for (uint32_t ib = i0; ib < i1; ib += JT_ROWS) {
+    const uint32_t m = min(JT_ROWS, i1 - ib);
+    __syncthreads();
+    for (uint32_t q = threadIdx.x; q < 3u * m; q += JT_THREADS) {
+      const uint32_t c = q / m, k = q % m;
+      const size_t i = size_t(c) * n + ib + k;
+      const float2 x = df_split(g[i] + double(rho[i]) * lam[i]);
+      w[c][k] = make_float4(x.x, x.x, x.y, x.y);
     }
-  } else {
-    for (uint32_t j = lane; j < n; j += 32) {
-      const float f = __ldg(Fr + j);
+    __syncthreads();
+    if (j < n) {
+      const float* Fc = F + size_t(ib) * n + j;
+      auto load = [&](const float* p) {
+        if (vec) return __ldg(reinterpret_cast<const float4*>(p));
+        return make_float4(p[0], j + 1 < n ? p[1] : 0.0f, j + 2 < n ? p[2] : 0.0f, j + 3 < n ? p[3] : 0.0f);
+      };
+      auto row = [&](float4 f, uint32_t k) {
 #pragma unroll
-      for (int c = 0; c < 3; c++) df_mac(f, Bin[size_t(c) * n + j], sh[c], sl[c]);
+        for (int c = 0; c < 3; c++) {
+          const float4 x = w[c][k];
+          df_mac2(f2(f.x, f.y), f2(-f.x, -f.y), f2(x.x, x.y), f2(x.z, x.w), s[c][0]);
+          df_mac2(f2(f.z, f.w), f2(-f.z, -f.w), f2(x.x, x.y), f2(x.z, x.w), s[c][1]);
+        }
+      };
+      uint32_t k = 0;
+      for (; k + 4u <= m; k += 4u, Fc += size_t(4) * n) {   // four rows in flight
+        float4 f[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) f[q] = load(Fc + size_t(q) * n);
+#pragma unroll
+        for (int q = 0; q < 4; q++) row(f[q], k + q);
+      }
+      for (; k < m; k++, Fc += n) row(load(Fc), k);
     }
   }
 #pragma unroll
   for (int c = 0; c < 3; c++) {
-    double a = double(sh[c]) + double(sl[c]);
-    for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-    if (lane) continue;
-    if (H) H[size_t(c) * n + row] = float(a);
-    else Bout[size_t(c) * n + row] = df_split(double(rho[size_t(c) * n + row]) * (double(DL[row]) + a));
+    double* p = part + (size_t(blockIdx.y) * 3 + c) * n + j;
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+      if (j + 2 * q < n) p[2 * q] = double(s[c][q].h.x) + double(s[c][q].l.x);
+      if (j + 2 * q + 1 < n) p[2 * q + 1] = double(s[c][q].h.y) + double(s[c][q].l.y);
+    }
   }
 }
-__global__ void radiosity64_init(const float* __restrict__ rho, const float* __restrict__ DL, float2* __restrict__ B, uint32_t n) {
+// out = the sum of the partials, 3 n values: a block takes 32 of them, each warp an eighth of the splits, the warps' sums in
+// order
+__global__ void __launch_bounds__(256) jacobi_t_combine(const double* __restrict__ part, uint32_t n3, double* __restrict__ out) {
+  __shared__ double red[8][32];
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, j = blockIdx.x * 32u + lane;
+  double a = 0.0;
+  if (j < n3) {
+#pragma unroll
+    for (uint32_t s = 0; s < JT_SPLITS / 8; s++) a += part[size_t(warp * (JT_SPLITS / 8) + s) * n3 + j];
+  }
+  red[warp][lane] = a;
+  __syncthreads();
+  if (warp || j >= n3) return;
+  for (uint32_t w = 1; w < 8; w++) a += red[w][lane];
+  out[j] = a;
+}
+
+// The three channels' B_c,out = rho_c o (DL + F B_c,in) at FP64 accuracy (F in FP32, B as float pairs, planar [c][hi | lo]
+// [np]), the products summed in float pairs; with `H` set, H_c = F B_c,in (rounded to FP32) instead. A block takes
+// R64_ROWS rows, a thread four columns at a time of each: a load of B serves the rows, and a step is two products (f32x2) in
+// 12 independent sums. Bound by the FMA pipe (14 operations a product, 18 us at its rate). N = 4096: 37 us a sweep; a warp per
+// row with one product a step and B read again for each row took 51 us.
+constexpr uint32_t R64_ROWS = 4, R64_THREADS = 256;
+__global__ void __launch_bounds__(R64_THREADS, 2) radiosity64_kernel(const float* __restrict__ F, const float* __restrict__ rho, const float* __restrict__ DL,
+                                                                    const float* __restrict__ Bin, float* __restrict__ Bout, float* __restrict__ H,
+                                                                    uint32_t n, uint32_t np) {
+  __shared__ float2 red[R64_THREADS / 32][R64_ROWS * 3];
+  const uint32_t row0 = blockIdx.x * R64_ROWS, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const bool vec = (n & 3u) == 0u;
+  DfAcc s[R64_ROWS][3];
+#pragma unroll
+  for (uint32_t r = 0; r < R64_ROWS; r++)
+#pragma unroll
+    for (int c = 0; c < 3; c++) s[r][c].h = s[r][c].l = f2(0.0f, 0.0f);
+  for (uint32_t j = 4u * threadIdx.x; j < n; j += 4u * R64_THREADS) {
+    float4 f[R64_ROWS];
+#pragma unroll
+    for (uint32_t r = 0; r < R64_ROWS; r++) {
+      const float* p = F + size_t(min(row0 + r, n - 1u)) * n + j;
+      if (vec) f[r] = __ldg(reinterpret_cast<const float4*>(p));
+      else f[r] = make_float4(p[0], j + 1 < n ? p[1] : 0.0f, j + 2 < n ? p[2] : 0.0f, j + 3 < n ? p[3] : 0.0f);
+    }
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      const float4 xh = __ldg(reinterpret_cast<const float4*>(Bin + size_t(2 * c) * np + j));
+      const float4 xl = __ldg(reinterpret_cast<const float4*>(Bin + size_t(2 * c + 1) * np + j));
+#pragma unroll
+      for (uint32_t r = 0; r < R64_ROWS; r++) {
+        df_mac2(f2(f[r].x, f[r].y), f2(-f[r].x, -f[r].y), f2(xh.x, xh.y), f2(xl.x, xl.y), s[r][c]);
+        df_mac2(f2(f[r].z, f[r].w), f2(-f[r].z, -f[r].w), f2(xh.z, xh.w), f2(xl.z, xl.w), s[r][c]);
+      }
+    }
+  }
+  // the block's sums, as float pairs over a warp's lanes, then over the warps in FP64. A step over the lanes halves the
+  // values that a lane still adds (lane 2 v ends with value v): 16 additions for the 12 values
+  static_assert(R64_ROWS * 3 <= 16, "values of a lane");
+  float2 v[16];
+#pragma unroll
+  for (uint32_t q = 0; q < 16; q++) {
+    if (q < R64_ROWS * 3) {
+      const DfAcc& a = s[q / 3][q % 3];
+      v[q] = df_add(make_float2(a.h.x, a.l.x), make_float2(a.h.y, a.l.y));
+    } else {
+      v[q] = make_float2(0.0f, 0.0f);
+    }
+  }
+#pragma unroll
+  for (uint32_t half = 8; half > 0; half >>= 1) {
+    const bool up = (lane & (2u * half)) != 0u;
+#pragma unroll
+    for (uint32_t q = 0; q < half; q++) {
+      const float2 mine = up ? v[q + half] : v[q], other = up ? v[q] : v[q + half];
+      v[q] = df_add(mine, make_float2(__shfl_xor_sync(0xffffffffu, other.x, 2 * half), __shfl_xor_sync(0xffffffffu, other.y, 2 * half)));
+    }
+  }
+  v[0] = df_add(v[0], make_float2(__shfl_xor_sync(0xffffffffu, v[0].x, 1), __shfl_xor_sync(0xffffffffu, v[0].y, 1)));
+  if (!(lane & 1u) && lane / 2u < R64_ROWS * 3) red[warp][lane / 2u] = v[0];
+  __syncthreads();
+  const uint32_t q = threadIdx.x, row = row0 + q / 3u, c = q % 3u;
+  if (q >= 3u * R64_ROWS || row >= n) return;
+  double a = 0.0;
+  for (uint32_t w = 0; w < R64_THREADS / 32; w++) a += double(red[w][q].x) + double(red[w][q].y);
+  if (H) { H[size_t(c) * n + row] = float(a); return; }
+  const float2 x = df_split(double(rho[size_t(c) * n + row]) * (double(DL[row]) + a));
+  Bout[size_t(2 * c) * np + row] = x.x;
+  Bout[size_t(2 * c + 1) * np + row] = x.y;
+}
+// the first iterate, and zeros in both arrays' tails
+__global__ void radiosity64_init(const float* __restrict__ rho, const float* __restrict__ DL, float* __restrict__ B, float* __restrict__ other, uint32_t n,
+                                 uint32_t np) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < 3 * n) B[i] = df_split(double(rho[i]) * double(DL[i % n]));
+  if (i >= 3 * np) return;
+  const uint32_t c = i / np, k = i % np;
+  const float2 x = k < n ? df_split(double(rho[size_t(c) * n + k]) * double(DL[k])) : make_float2(0.0f, 0.0f);
+  B[size_t(2 * c) * np + k] = x.x;
+  B[size_t(2 * c + 1) * np + k] = x.y;
+  if (k >= n) other[size_t(2 * c) * np + k] = other[size_t(2 * c + 1) * np + k] = 0.0f;
 }
 
 __global__ void mul_kernel(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ y, uint32_t n) {
@@ -895,12 +995,12 @@ void launch_dl(const float* D, const float* L, uint32_t n, uint32_t n_lamps, flo
   dl_kernel<<<(n + 7) / 8, 256, 0, st>>>(D, L, n, n_lamps, y);
 }
 
-size_t jacobi_t_work(uint32_t n) { return size_t(JT_SPLITS) * n * 8; }
+size_t jacobi_t_work(uint32_t n) { return size_t(JT_SPLITS) * 3 * n * 8; }
 
 void launch_jacobi_t(const float* F, const double* g, const float* rho, const double* lam_in, double* lam_out, uint32_t n, double* work,
                      cudaStream_t st) {
-  jacobi_t_kernel<<<dim3((n + JT_COLS - 1) / JT_COLS, JT_SPLITS), JT_COLS, 0, st>>>(F, g, rho, lam_in, n, work);
-  jacobi_t_combine<<<(n + 255) / 256, 256, 0, st>>>(work, n, lam_out);
+  jacobi_t_kernel<<<dim3((n + 4 * JT_THREADS - 1) / (4 * JT_THREADS), JT_SPLITS), JT_THREADS, 0, st>>>(F, g, rho, lam_in, n, work);
+  jacobi_t_combine<<<(3 * n + 31) / 32, 256, 0, st>>>(work, 3 * n, lam_out);
 }
 
 void launch_sum(const double* p, uint32_t n, double* out, cudaStream_t st) { sum_kernel<<<1, 1024, 0, st>>>(p, n, out); }
@@ -909,16 +1009,17 @@ void launch_mul(const float* a, const float* b, float* y, uint32_t n, cudaStream
 
 void launch_radiosity64(const float* F, const float* rho, const float* DL, uint32_t n, uint32_t iters, void* work, float* H,
                         cudaStream_t st) {
-  // the three channels' iterates as float pairs, two planar 3 x n arrays in `work`
-  float2* p0 = static_cast<float2*>(work);
-  float2* p1 = p0 + size_t(3) * n;
-  radiosity64_init<<<(3 * n + 255) / 256, 256, 0, st>>>(rho, DL, p0, n);
-  float2 *cur = p0, *nxt = p1;
+  // the three channels' iterates as float pairs, two planar arrays in `work`, rows of a multiple of 4
+  const uint32_t np = (n + 3u) / 4u * 4u;
+  float* cur = static_cast<float*>(work);
+  float* nxt = cur + size_t(6) * np;
+  const uint32_t blocks = (n + R64_ROWS - 1) / R64_ROWS;
+  radiosity64_init<<<(3 * np + 255) / 256, 256, 0, st>>>(rho, DL, cur, nxt, n, np);
   for (uint32_t it = 0; it < iters; it++) {
-    radiosity64_kernel<<<(n + 7) / 8, 256, 0, st>>>(F, rho, DL, cur, nxt, nullptr, n);
+    radiosity64_kernel<<<blocks, R64_THREADS, 0, st>>>(F, rho, DL, cur, nxt, nullptr, n, np);
     std::swap(cur, nxt);
   }
-  radiosity64_kernel<<<(n + 7) / 8, 256, 0, st>>>(F, rho, DL, cur, nullptr, H, n);
+  radiosity64_kernel<<<blocks, R64_THREADS, 0, st>>>(F, rho, DL, cur, nullptr, H, n, np);
 }
 
 }  // namespace vtk

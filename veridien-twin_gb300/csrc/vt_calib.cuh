@@ -59,7 +59,8 @@ void launch_direct_transfer(const vtd::Scene& S, const float* centres, const flo
                             uint32_t samples, float* D, cudaStream_t st);
 // y = D L (n x n_lamps times n_lamps)
 void launch_dl(const float* D, const float* L, uint32_t n, uint32_t n_lamps, float* y, cudaStream_t st);
-// one transposed Jacobi sweep of the adjoint: lam_out = F^T (g + rho o lam_in), FP64 vectors; work: splits x n doubles
+// one transposed Jacobi sweep of the adjoint: lam_out = F^T (g + rho o lam_in) per channel, FP64 vectors planar 3 x n; work:
+// jacobi_t_work(n) bytes
 void launch_jacobi_t(const float* F, const double* g, const float* rho, const double* lam_in, double* lam_out, uint32_t n, double* work,
                      cudaStream_t st);
 size_t jacobi_t_work(uint32_t n);
@@ -67,7 +68,7 @@ size_t jacobi_t_work(uint32_t n);
 void launch_mul(const float* a, const float* b, float* y, uint32_t n, cudaStream_t st);
 // the calibration model's node radiosity for the three channels at once: B_c = rho_c o (DL + F B_c) by `iters`
 // Jacobi sweeps from B_c = rho_c o DL, at FP64 accuracy (F in FP32; float-pair products and sums), then H_c = F B_c
-// rounded to FP32; rho and H planar 3 x n; work: at least 48 n bytes, 16-byte aligned
+// rounded to FP32; rho and H planar 3 x n; work: at least 48 (n + 3) bytes, 16-byte aligned
 void launch_radiosity64(const float* F, const float* rho, const float* DL, uint32_t n, uint32_t iters, void* work, float* H, cudaStream_t st);
 // sum of n doubles (deterministic order) into out
 void launch_sum(const double* p, uint32_t n, double* out, cudaStream_t st);

@@ -104,7 +104,7 @@ struct vt_ctx {
     uint32_t *tri_node_d = nullptr, *emit_of_tri_d = nullptr;
     float *albedo = nullptr, *lamp = nullptr, *rho = nullptr /* 3 x n */, *DL = nullptr, *H = nullptr /* 3 x n */;
     double *partials = nullptr, *g_alb = nullptr, *g_lamp = nullptr, *g_H = nullptr, *lam0 = nullptr, *lam1 = nullptr,
-           *lam = nullptr /* 3 x n */, *work = nullptr, *loss = nullptr;
+           *work = nullptr, *loss = nullptr;   // lam0, lam1: 3 x n
     uint32_t max_partials = 0;
     std::vector<float4*> image, target;   // per scene camera (device, w x h)
     std::vector<std::vector<float>> albedo_host;
