@@ -965,7 +965,7 @@ vt_status vt_radiosity_solve(vt_ctx* ctx, vt_solve_req* q) {
   const bool tma = q->precision == VT_PREC_FP32_TMA;
   if (tma && dF && !aligned16(q->F)) return fail(ctx, VT_ERR_ARG, "solve: the bulk-copy matvec needs a 16-byte aligned F");
   const uint32_t max_blocks = std::max<uint32_t>(std::max<uint32_t>((n + 7) / 8, uint32_t((size_t(n) * R / 4 + 255) / 256)),
-                                                 tma ? vtk::jacobi_matvec_tma_blocks(n) : 0u) + 8;
+                                                 tma ? vtk::jacobi_matvec_tma_blocks(n) : R == 1 ? vtk::jacobi_matvec_sweeps_blocks(n) : 0u) + 8;
   // several right-hand sides: the tensor cores where F allows it (a host F is copied to aligned memory)
   bool tc = q->precision == VT_PREC_FP32 && vtk::jacobi_tc_f32_ok(dF ? q->F : nullptr, n, R);
   const size_t gemm_work = R > 1 ? std::max(vtk::jacobi_gemm_fp32_work(n, R), tc ? vtk::jacobi_tc_f32_work(n, R) : 0) : 0;
@@ -999,8 +999,11 @@ vt_status vt_radiosity_solve(vt_ctx* ctx, vt_solve_req* q) {
   };
   if ((s = first_iterate()) != VT_OK) return s;
   vtk::TcMap mF, mB;
-  uint32_t* wait_err = reinterpret_cast<uint32_t*>(norms + 4);   // a bounded wait ran out
-  if (tc) VT_CK(cudaMemsetAsync(wait_err, 0, 4, ctx->stream));
+  uint32_t* wait_err = reinterpret_cast<uint32_t*>(norms + 4);   // a bounded wait ran out; then the grid barrier's counter
+  // one right-hand side of a room whose iterate fits shared memory: the sweeps between two checks in one launch
+  const bool coop = R == 1 && !tma && vtk::jacobi_matvec_sweeps_ok(n);
+  uint32_t arrivals = 0;
+  if (tc || coop) VT_CK(cudaMemsetAsync(wait_err, 0, 8, ctx->stream));
   if (tc) {
     int code = 0;
     const float* Ft = Fd;
@@ -1021,7 +1024,13 @@ vt_status vt_radiosity_solve(vt_ctx* ctx, vt_solve_req* q) {
   VT_CK(cudaEventRecord(ctx->ev0, ctx->stream));
   while (it < max_it) {
     const uint32_t k = std::min(check, max_it - it);
-    for (uint32_t j = 0; j < k; j++) {
+    if (coop) {
+      VT_CK(cudaEventRecord(ctx->ev2, ctx->stream));
+      VT_CK(vtk::launch_jacobi_matvec_sweeps(Fd, rho, E, cur, nxt, n, k, wait_err + 1, &arrivals, wait_err, partials, &np, ctx->stream));
+      VT_CK(cudaEventRecord(ctx->ev3, ctx->stream));
+      if (k & 1u) std::swap(cur, nxt);
+    }
+    for (uint32_t j = 0; j < k && !coop; j++) {
       if (j == 0) VT_CK(cudaEventRecord(ctx->ev2, ctx->stream));
       if (tma) vtk::launch_jacobi_matvec_tma(Fd, rho, E, cur, nxt, n, partials, &np, ctx->stream);
       else if (R == 1) vtk::launch_jacobi_matvec(Fd, rho, E, cur, nxt, n, partials, &np, ctx->stream);
@@ -1030,17 +1039,17 @@ vt_status vt_radiosity_solve(vt_ctx* ctx, vt_solve_req* q) {
       if (j == 0) VT_CK(cudaEventRecord(ctx->ev3, ctx->stream));
       std::swap(cur, nxt);
     }
-    ctx->tim.launches += k * (work ? 2 : 1) + 1;
+    ctx->tim.launches += (coop ? 1 : k * (work ? 2 : 1)) + 1;
     it += k;
     vtk::launch_reduce_partials(partials, np, norms, ctx->stream);
     VT_CK(cudaGetLastError());
     double h[5];   // the norms; wait_err in the first word of h[4]
     VT_CK(cudaMemcpyAsync(h, norms, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
     VT_CK(cudaStreamSynchronize(ctx->stream));
-    if (tc) {
+    if (tc || coop) {
       uint32_t e = 0;
       memcpy(&e, h + 4, 4);
-      if (e) return fail(ctx, VT_ERR_TIMEOUT, "solve: a tensor-core pipeline wait ran out");
+      if (e) return fail(ctx, VT_ERR_TIMEOUT, tc ? "solve: a tensor-core pipeline wait ran out" : "solve: a grid barrier ran out");
     }
     if (tc) {
       if (!std::isfinite(h[0]) || !std::isfinite(h[1])) {
@@ -1054,7 +1063,7 @@ vt_status vt_radiosity_solve(vt_ctx* ctx, vt_solve_req* q) {
     resid = h[1] > 0 ? std::sqrt(h[0] / h[1]) : 0.0;
     float gms = 0;
     cudaEventElapsedTime(&gms, ctx->ev2, ctx->ev3);
-    sweep_sum += gms;
+    sweep_sum += coop ? gms / k : gms;
     sweep_n++;
     if (resid <= q->tol) break;
   }

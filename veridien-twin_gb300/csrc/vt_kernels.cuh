@@ -67,6 +67,12 @@ void launch_sensor_expose_u16(const SensorParams& su, const float4* E, float sca
 // B_out = E + rho (F B_in), n x 1, and per-block partial sums of |B_out - B_in|^2 and |B_out|^2 (doubles)
 void launch_jacobi_matvec(const float* F, const float* rho, const float* E, const float* Bin, float* Bout, uint32_t n,
                           double* partials, uint32_t* n_partials, cudaStream_t st);
+// several such sweeps in one cooperative launch (n within jacobi_matvec_sweeps_ok): the result lies in B1 after an odd
+// number, in B0 after an even one; counter: a word cleared when *arrivals was 0; *err: a wait ran out
+bool jacobi_matvec_sweeps_ok(uint32_t n);
+uint32_t jacobi_matvec_sweeps_blocks(uint32_t n);
+cudaError_t launch_jacobi_matvec_sweeps(const float* F, const float* rho, const float* E, float* B0, float* B1, uint32_t n, uint32_t sweeps,
+                                        uint32_t* counter, uint32_t* arrivals, uint32_t* err, double* partials, uint32_t* n_partials, cudaStream_t st);
 // the same with F's rows fed into shared memory by bulk copies (n % 4 == 0); bounded waits raise matvec_error
 void launch_jacobi_matvec_tma(const float* F, const float* rho, const float* E, const float* Bin, float* Bout, uint32_t n,
                               double* partials, uint32_t* n_partials, cudaStream_t st);

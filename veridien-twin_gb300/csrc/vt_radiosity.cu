@@ -76,6 +76,95 @@ __global__ void __launch_bounds__(MV_THREADS) jacobi_matvec_kernel(const float* 
   block_sum2(d2, b2, partials);
 }
 
+// Several sweeps in one cooperative launch, one block per SM: a warp per row as in jacobi_matvec_kernel (the same sums in
+// the same order, so the same iterates), the iterate in shared memory, a grid barrier between sweeps. A launch per sweep of a
+// small room is mostly its start and its end: n = 4096, 16 sweeps and two checks: 358 us of a solve -> 227 (21.2 -> 8.5 us a
+// sweep under ncu; F, 67 MB, comes from the L2)
+constexpr int MVS_THREADS = 1024;
+constexpr uint32_t MVS_MAX_N = 16384;   // the iterate in shared memory: 64 KB
+
+// wait for every block's arrival (`target` arrivals since the counter was cleared); false in every thread when it runs out
+__device__ __forceinline__ bool grid_barrier(uint32_t* counter, uint32_t target, uint32_t* err) {
+  __shared__ uint32_t ok;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    atomicAdd(counter, 1u);
+    ok = 1u;
+    const unsigned long long t0 = clock64();
+    while (*reinterpret_cast<volatile uint32_t*>(counter) < target)
+      if (clock64() - t0 > async::WAIT_CYCLES) { atomicOr(err, 1u); ok = 0u; break; }
+    __threadfence();
+  }
+  __syncthreads();
+  return ok != 0u;
+}
+
+template <bool KEEP>
+__global__ void __launch_bounds__(MVS_THREADS, 1) jacobi_matvec_sweeps_kernel(const float* __restrict__ F, const float* __restrict__ rho,
+                                                                             const float* __restrict__ E, float* B0, float* B1, uint32_t n,
+                                                                             uint32_t sweeps, uint32_t* counter, uint32_t base, uint32_t* err,
+                                                                             double* __restrict__ partials) {
+  extern __shared__ __align__(16) float xs[];
+  __shared__ double sd[MVS_THREADS / 32], sb[MVS_THREADS / 32];
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const bool vec = (n & 3u) == 0u && (reinterpret_cast<uintptr_t>(F) & 15u) == 0u;
+  double d2 = 0.0, b2 = 0.0;
+  for (uint32_t it = 0; it < sweeps; it++) {
+    const float* Bin = it & 1u ? B1 : B0;
+    float* Bout = it & 1u ? B0 : B1;
+    if (it && !grid_barrier(counter, base + it * gridDim.x, err)) return;
+    for (uint32_t j = threadIdx.x; j < n; j += MVS_THREADS) xs[j] = __ldcg(Bin + j);
+    __syncthreads();
+    d2 = b2 = 0.0;
+    for (uint32_t row = blockIdx.x + gridDim.x * warp; row < n; row += gridDim.x * (MVS_THREADS / 32)) {
+      const float* Fr = F + size_t(row) * n;
+      float acc = 0.0f;
+      if (vec) {
+        const float4* F4 = reinterpret_cast<const float4*>(Fr);
+        const float4* X4 = reinterpret_cast<const float4*>(xs);
+        const uint32_t n4 = n >> 2;
+        uint32_t j = lane;
+        for (; j + 7u * 32u < n4; j += 8u * 32u) {
+          float4 f[8];
+#pragma unroll
+          for (int q = 0; q < 8; q++) f[q] = KEEP ? __ldg(F4 + j + 32 * q) : __ldcs(F4 + j + 32 * q);
+#pragma unroll
+          for (int q = 0; q < 8; q++) {
+            const float4 b = X4[j + 32 * q];
+            acc = fmaf(f[q].x, b.x, acc); acc = fmaf(f[q].y, b.y, acc); acc = fmaf(f[q].z, b.z, acc); acc = fmaf(f[q].w, b.w, acc);
+          }
+        }
+        for (; j < n4; j += 32) {
+          const float4 f = KEEP ? __ldg(F4 + j) : __ldcs(F4 + j);
+          const float4 b = X4[j];
+          acc = fmaf(f.x, b.x, acc); acc = fmaf(f.y, b.y, acc); acc = fmaf(f.z, b.z, acc); acc = fmaf(f.w, b.w, acc);
+        }
+      } else {
+#pragma unroll 8
+        for (uint32_t j = lane; j < n; j += 32) acc = fmaf(KEEP ? __ldg(Fr + j) : __ldcs(Fr + j), xs[j], acc);
+      }
+      for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+      if (lane == 0) {
+        const float b = fmaf(rho[row], acc, E[row]);
+        __stcg(Bout + row, b);
+        if (it + 1u == sweeps) {
+          const double dd = double(b) - double(xs[row]);
+          d2 += dd * dd;
+          b2 += double(b) * double(b);
+        }
+      }
+    }
+  }
+  if (lane == 0) { sd[warp] = d2; sb[warp] = b2; }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < MVS_THREADS / 32; w++) { d2 += sd[w]; b2 += sb[w]; }
+    partials[2 * blockIdx.x] = d2;
+    partials[2 * blockIdx.x + 1] = b2;
+  }
+}
+
 // ------------------------------------------------------------------------------------------ TMA-fed matvec
 // One right-hand side, F rows streamed by the copy engine: thread 0 of each block keeps MVT_STAGES bulk copies
 // (cp.async.bulk, 8 KB chunks of a row) in flight into a shared-memory ring, completing on mbarriers; all threads
@@ -197,6 +286,30 @@ void launch_jacobi_matvec(const float* F, const float* rho, const float* E, cons
   else jacobi_matvec_kernel<false><<<blocks, MV_THREADS, 0, st>>>(F, rho, E, Bin, Bout, n, partials);
 }
 
+
+bool jacobi_matvec_sweeps_ok(uint32_t n) { return n <= MVS_MAX_N; }
+uint32_t jacobi_matvec_sweeps_blocks(uint32_t n) {
+  static std::atomic<int> sms[MAX_DEVICES];   // and the kernels' shared memory, once per device
+  return std::min(n, uint32_t(per_device_value(sms, [](int dev) {
+    cudaFuncSetAttribute(jacobi_matvec_sweeps_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(MVS_MAX_N * 4));
+    cudaFuncSetAttribute(jacobi_matvec_sweeps_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(MVS_MAX_N * 4));
+    return device_sms(dev);
+  })));
+}
+
+// `sweeps` sweeps from B0 (the result in B1 when their number is odd, else in B0); *arrivals counts the barrier's arrivals
+// since `counter` was cleared
+cudaError_t launch_jacobi_matvec_sweeps(const float* F, const float* rho, const float* E, float* B0, float* B1, uint32_t n, uint32_t sweeps,
+                                        uint32_t* counter, uint32_t* arrivals, uint32_t* err, double* partials, uint32_t* n_partials, cudaStream_t st) {
+  const uint32_t blocks = jacobi_matvec_sweeps_blocks(n);
+  uint32_t base = *arrivals;
+  *n_partials = blocks;
+  void* args[] = {&F, &rho, &E, &B0, &B1, &n, &sweeps, &counter, &base, &err, &partials};
+  const void* k = keep_f(n) ? reinterpret_cast<const void*>(jacobi_matvec_sweeps_kernel<true>) : reinterpret_cast<const void*>(jacobi_matvec_sweeps_kernel<false>);
+  const cudaError_t e = cudaLaunchCooperativeKernel(k, dim3(blocks), dim3(MVS_THREADS), args, size_t(n) * 4, st);
+  *arrivals += (sweeps - 1u) * blocks;
+  return e;
+}
 
 // ---------------------------------------------------------------------------------------------- FP32 GEMM sweep
 // 128 x 64 output tile per 256-thread block (8 x 4 outputs per thread), K in 16-wide slices double-buffered through
