@@ -435,7 +435,8 @@ __global__ void __launch_bounds__(WT, 4) calib_shadow_kernel(const Scene S, cons
     j++;
     state = next_sample() ? LANE_NODE : LANE_IDLE;
   };
-  while (serve_lanes(state, exhausted, wb.fetch, n, cp.refill, next, start)) trace_round<true>(S, 0.0f, st, stk, state);
+  const uint32_t lanes = lanes_of(n);
+  while (serve_lanes(state, exhausted, wb.fetch, n, cp.refill, lanes, next, start)) trace_round<true>(S, 0.0f, st, stk, state);
 }
 
 // per pixel: the image value from the records in sub-sample order, its loss partial (forward); or the gradient of

@@ -77,7 +77,8 @@ __global__ void __launch_bounds__(256, VT_NODE_TRACE_BLOCKS) gather_build_kernel
     st.best = Hit{BIG, 0.0f, 0.0f, MISS, MISS};
     state = trace_phase(S, 0u, o, d, 0.0f, 0.5f, 1u, 0u, st, -1) ? LANE_NODE : LANE_WAIT;
   };
-  while (serve_lanes(state, exhausted, head, total, 8u, next, start)) trace_round<false>(S, 0.0f, st, stk, state);
+  const uint32_t lanes = lanes_of(total);
+  while (serve_lanes(state, exhausted, head, total, 8u, lanes, next, start)) trace_round<false>(S, 0.0f, st, stk, state);
 }
 
 // escapes per node (gpu/wgsl/kernels.wgsl.js:326 gatherCount)
@@ -231,7 +232,8 @@ __global__ void __launch_bounds__(256, VT_NODE_TRACE_BLOCKS) node_direct_shadow(
     if (trace_phase(S, 0u, o, d, 0.0f, 0.5f, 3u, skip, st, st.k + 1)) state = LANE_NODE;
     else visible();
   };
-  while (serve_lanes(state, exhausted, b.counts + 1, n, refill, next, start)) trace_round<true>(S, 0.0f, st, stk, state);
+  const uint32_t lanes = lanes_of(n);
+  while (serve_lanes(state, exhausted, b.counts + 1, n, refill, lanes, next, start)) trace_round<true>(S, 0.0f, st, stk, state);
 }
 
 __global__ void node_direct_sum(const Scene S, const uint32_t* __restrict__ active, uint32_t n_active, uint32_t NS, NodeDirectBufs b,

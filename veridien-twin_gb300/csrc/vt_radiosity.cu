@@ -652,7 +652,8 @@ __global__ void __launch_bounds__(FV_THREADS, 4) ff_visibility_kernel(const Scen
     k++;
     if (!next_ray()) finish();
   };
-  while (serve_lanes(state, exhausted, head, total, REFILL, next, start)) trace_round<true>(S, 0.0f, st, stk, state);
+  const uint32_t lanes = lanes_of(total);
+  while (serve_lanes(state, exhausted, head, total, REFILL, lanes, next, start)) trace_round<true>(S, 0.0f, st, stk, state);
 }
 
 __global__ void ff_rows_kernel(uint32_t n, const float* __restrict__ C, const float* __restrict__ N, const float* __restrict__ A,

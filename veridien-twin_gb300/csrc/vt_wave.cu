@@ -198,7 +198,8 @@ __global__ void __launch_bounds__(WAVE_THREADS, VT_TRACE_BLOCKS) wave_extend(con
     if (trace_phase(path_scene<VAR>(S, wb, p), root, xyz(o4), xyz(d4), 0.0f, o4.w, 3u, skip, st, st.k + 1)) state = LANE_NODE;
     else finish();
   };
-  while (serve_lanes(state, exhausted, wb.fetch, n, cp.refill, next, start)) trace_round<false>(S, 0.0f, st, stk, state);
+  const uint32_t lanes = lanes_of(n);
+  while (serve_lanes(state, exhausted, wb.fetch, n, cp.refill, lanes, next, start)) trace_round<false>(S, 0.0f, st, stk, state);
 }
 
 template <int MODE, int VAR>
@@ -445,7 +446,8 @@ __global__ void __launch_bounds__(WAVE_THREADS, VT_TRACE_BLOCKS) wave_shadow(con
     if (next_sample()) state = LANE_NODE;
     else finish_path();
   };
-  while (serve_lanes(state, exhausted, wb.fetch, n, cp.refill, next, start)) trace_round<true>(S0, 0.0f, st, stk, state);
+  const uint32_t lanes = lanes_of(n);
+  while (serve_lanes(state, exhausted, wb.fetch, n, cp.refill, lanes, next, start)) trace_round<true>(S0, 0.0f, st, stk, state);
 }
 
 // per pixel, the wave's sub-samples in order i0..i0+n_i-1 added to the running sum; the last wave writes the pixel
