@@ -470,11 +470,8 @@ vt_status vt_readback(vt_ctx* ctx, uint32_t camera, uint32_t kind, void* out, si
       if (s != VT_OK) return s;
     } else {
       if (bytes < px * 3) return VT_ERR_ARG;
-      std::vector<uint8_t> rgba(px * 4);
-      VT_CK(cudaMemcpyAsync(rgba.data(), C.isp.out, px * 4, cudaMemcpyDeviceToHost, ctx->stream));
-      VT_CK(cudaStreamSynchronize(ctx->stream));
-      uint8_t* o = static_cast<uint8_t*>(out);
-      for (size_t i = 0; i < px; i++) { o[3 * i] = rgba[4 * i]; o[3 * i + 1] = rgba[4 * i + 1]; o[3 * i + 2] = rgba[4 * i + 2]; }
+      vt_status s = rgb8_from_device(ctx, out, C.isp.out, px);
+      if (s != VT_OK) return s;
     }
   } else {
     return fail(ctx, VT_ERR_ARG, "readback kind");

@@ -422,13 +422,8 @@ vt_status vt_lite_readback(vt_ctx* ctx, uint32_t camera, int kind, void* dst, si
     if (!C.displayed) return fail(ctx, VT_ERR_STATE, "lite: 8-bit readback before display");
     const size_t ch = kind == VT_READ_RGBA8 ? 4 : 3;
     if (bytes < n * ch) return fail(ctx, VT_ERR_ARG, "lite readback: buffer too small");
-    std::vector<uint8_t> h(n * 4);
-    VT_CK(cudaMemcpyAsync(h.data(), C.out, n * 4, cudaMemcpyDeviceToHost, ctx->stream));
-    VT_CK(cudaStreamSynchronize(ctx->stream));
-    uint8_t* o = static_cast<uint8_t*>(dst);
-    if (ch == 4) std::memcpy(o, h.data(), n * 4);
-    else for (size_t i = 0; i < n; i++) { o[3 * i] = h[4 * i]; o[3 * i + 1] = h[4 * i + 1]; o[3 * i + 2] = h[4 * i + 2]; }
-    return VT_OK;
+    vt_status s = ch == 4 ? from_device(ctx, dst, C.out, n * 4) : rgb8_from_device(ctx, dst, C.out, n);
+    if (s != VT_OK) return s;
   } else {
     return fail(ctx, VT_ERR_ARG, "lite readback: linear, rgb8 or rgba8 (the raster pass has no raw or YCbCr planes)");
   }

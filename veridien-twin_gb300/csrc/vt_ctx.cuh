@@ -295,6 +295,15 @@ inline vt_status from_device(vt_ctx* ctx, void* dst, const void* src, size_t byt
   return VT_OK;
 }
 
+// n RGBA pixels of the device as packed RGB, by way of the scratch
+inline vt_status rgb8_from_device(vt_ctx* ctx, void* dst, const uchar4* rgba, size_t n) {
+  const vt_status s = ensure_scratch(ctx, n * 3 + 16);
+  if (s != VT_OK) return s;
+  vtk::launch_pack_rgb8(rgba, n, static_cast<uint8_t*>(ctx->d_scratch), ctx->stream);
+  VT_CK(cudaGetLastError());
+  return from_device(ctx, dst, ctx->d_scratch, n * 3);
+}
+
 // launch parameters of one camera dispatch (gpu/renderer.js:888 _packCam)
 inline vtk::CamParams make_cam(const vt_ctx* ctx, uint32_t camera, uint32_t spp, uint32_t n_light, uint32_t seed, uint32_t options, uint32_t mode,
                                uint32_t max_depth, uint32_t root, const float shutter[2], float scale) {

@@ -21,6 +21,9 @@ struct IspBufs {
 // the whole chain for one frame of the uniform's size; returns the number of kernels launched
 int launch_isp(const SensorParams& P, const IspBufs& b, cudaStream_t st);
 
+// n RGBA pixels to packed RGB (3 n bytes; both 4-byte aligned)
+void launch_pack_rgb8(const uchar4* rgba, size_t n, uint8_t* rgb, cudaStream_t st);
+
 // the raster pass's display look (vt_lite_display): du as lite_nodes/renderer.js:892 writes it, the previous frame's
 // statistics; stats receives this frame's (luma sum, count)
 struct LiteDisplay { float du[20]; uint32_t prev[4]; uint32_t W, H; };

@@ -144,10 +144,10 @@ class LiteNodesRenderer:
         c = self._cam(name)
         w, h = self.size(c)
         if kind == "linear":
-            out = np.zeros((h, w, 4), np.float32)
+            out = np.empty((h, w, 4), np.float32)
             check(self.lib.vt_lite_readback(self.tr._ctx, c, A.VT_READ_LINEAR, _p(out), out.nbytes), self.tr._ctx)
         elif kind in ("rgb8", "rgba8"):
-            out = np.zeros((h, w, 3 if kind == "rgb8" else 4), np.uint8)
+            out = np.empty((h, w, 3 if kind == "rgb8" else 4), np.uint8)
             check(self.lib.vt_lite_readback(self.tr._ctx, c, A.VT_READ_RGB8 if kind == "rgb8" else A.VT_READ_RGBA8, _p(out), out.nbytes),
                   self.tr._ctx)
         else:

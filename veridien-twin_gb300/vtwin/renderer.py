@@ -273,17 +273,17 @@ class TwinRenderer:
         c = self._cam(name)
         w, h = self.scene["cameras"][c]["size"]
         if kind == "linear":
-            out = np.zeros((h, w, 4), np.float32)
+            out = np.empty((h, w, 4), np.float32)
             check(self.lib.vt_readback(self._ctx, c, A.VT_READ_LINEAR, _p(out), out.nbytes), self._ctx)
         elif kind == "raw":
-            out = np.zeros((h, w), np.float32)
+            out = np.empty((h, w), np.float32)
             check(self.lib.vt_readback(self._ctx, c, A.VT_READ_RAW, _p(out), out.nbytes), self._ctx)
         elif kind in ("rgb8", "rgba8"):
-            out = np.zeros((h, w, 3 if kind == "rgb8" else 4), np.uint8)
+            out = np.empty((h, w, 3 if kind == "rgb8" else 4), np.uint8)
             check(self.lib.vt_readback(self._ctx, c, A.VT_READ_RGB8 if kind == "rgb8" else A.VT_READ_RGBA8, _p(out), out.nbytes), self._ctx)
         elif kind == "yuv420":
             cw, ch = (w + 1) // 2, (h + 1) // 2
-            buf = np.zeros(w * h + 2 * cw * ch, np.uint8)
+            buf = np.empty(w * h + 2 * cw * ch, np.uint8)
             check(self.lib.vt_readback(self._ctx, c, A.VT_READ_YUV420, _p(buf), buf.nbytes), self._ctx)
             return {"width": w, "height": h, "y": buf[:w * h].reshape(h, w), "cb": buf[w * h:w * h + cw * ch].reshape(ch, cw),
                     "cr": buf[w * h + cw * ch:].reshape(ch, cw)}
