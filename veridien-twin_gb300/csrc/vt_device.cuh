@@ -553,7 +553,8 @@ struct LaneStack {
 enum { LANE_IDLE = 0, LANE_WAIT = 1, LANE_POP = 2, LANE_NODE = 3, LANE_LEAF = 4 };
 // Lanes at a leaf before a warp tests leaves. Few: the leaf code is issued for few lanes; many: lanes stand idle at
 // their leaf. 640x480, 16 spp, depth 4 on the 12k-triangle dome: 16.7 ms at 4, 15.6 at 8, 15.4 at 12 and 14; 1920x1200,
-// 8 spp, depth 6 with six instruments: 148, 139, 136, 136 ms; the same order on the pose batch and the twin frame
+// 8 spp, depth 6 with six instruments: 148, 139, 136, 136 ms; the same order on the pose batch and the twin frame. At most
+// half of the lanes that traverse, where a small queue or its end leaves few (160x120, 1 spp: 0.73 -> 0.67 ms)
 #ifndef VT_LEAF_BATCH
 #define VT_LEAF_BATCH 12
 #endif
@@ -622,14 +623,14 @@ __device__ __forceinline__ uint32_t trace_leaf(const Scene& S, float tmin, Trace
   return trace_pop(st, stk);
 }
 
-// One round of a warp's lanes (all call it): the lanes at a node visit it, until VT_LEAF_BATCH lanes wait at a leaf or
-// none is at a node; then those test their leaves. The warp issues one kind of work at a time: with a visit or a triangle
+// One round of a warp's lanes (all call it): the lanes at a node visit it, until enough lanes wait at a leaf or none is at
+// a node; then those test their leaves. The warp issues one kind of work at a time: with a visit or a triangle
 // per lane in every step, both and the push / pop were issued for some lane in nearly each (328 warp instructions a step,
 // 10.4 lanes in the mean on secondary rays; now 16.3). With serve_lanes below: 640x480, 16 spp, depth 4: 19.6 -> 15.4 ms.
 template <bool ANY>
 __device__ __forceinline__ void trace_round(const Scene& S, float tmin, TraceState& st, LaneStack& stk, uint32_t& state) {
   const uint32_t at_node = __ballot_sync(0xffffffffu, state >= LANE_POP), at_leaf = __ballot_sync(0xffffffffu, state == LANE_LEAF);
-  if (at_node != at_leaf && __popc(at_leaf) < VT_LEAF_BATCH) {
+  if (at_node != at_leaf && __popc(at_leaf) < min(VT_LEAF_BATCH, (__popc(at_node) + 1) / 2)) {
     if (state == LANE_NODE) state = trace_node(S, tmin, st, stk);
     else if (state == LANE_POP) state = trace_pop(st, stk);
   } else {
