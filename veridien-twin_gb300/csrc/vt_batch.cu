@@ -230,7 +230,7 @@ BatchWave batch_carve(void* base, uint32_t P, uint32_t n_pw, uint32_t cap, uint3
   auto take = [&](size_t bytes) { char* r = c; c += (bytes + 255) / 256 * 256; return r; };
   BatchWave b{};
   b.shared = wave_carve(take(wave_bytes(P, n_light, 0)), P, n_light, 0, counts);
-  b.pairs = wave_carve(take(wave_bytes(cap, n_light, 0)), cap, n_light, 0, counts + 4);
+  b.pairs = wave_carve(take(wave_bytes(cap, n_light, 0)), cap, n_light, 0, counts + 32);
   b.dirty = reinterpret_cast<uint64_t*>(take(size_t(P) * 8));
   b.off = reinterpret_cast<uint32_t*>(take(size_t(P) * 4));
   b.blk = reinterpret_cast<uint32_t*>(take(((P + SCAN - 1) / SCAN) * 4));

@@ -436,7 +436,7 @@ __global__ void __launch_bounds__(WT, 4) calib_shadow_kernel(const Scene S, cons
     state = next_sample() ? LANE_NODE : LANE_IDLE;
   };
   const uint32_t lanes = lanes_of(n);
-  while (serve_lanes(state, exhausted, wb.fetch, n, cp.refill, lanes, next, start)) trace_round<true>(S, 0.0f, st, stk, state);
+  while (serve_lanes(state, exhausted, wb.fetch_sh, n, cp.refill, lanes, next, start)) trace_round<true>(S, 0.0f, st, stk, state);
 }
 
 // per pixel: the image value from the records in sub-sample order, its loss partial (forward); or the gradient of
@@ -915,19 +915,12 @@ static void calib_trace(const Scene& S, const CamParams& cp, const CalibDev& C, 
     const int dm = db ? dmode : 0;
     for (uint32_t b = 1; b <= cp.max_depth; b++) {
       WaveBufs w = wb;
-      w.q_in = (b & 1) ? wb.qa : wb.qb;
-      w.q_out = (b & 1) ? wb.qb : wb.qa;
-      w.count_in = wb.counts + ((b & 1) ? 0 : 1);
-      w.count_out = wb.counts + ((b & 1) ? 1 : 0);
-      w.count_sh = wb.counts + 2;
-      cudaMemsetAsync(w.count_out, 0, 4, st);
-      cudaMemsetAsync(w.count_sh, 0, 4, st);
+      begin_bounce(w, b, st);
       if (dm == 2) calib_rehit_kernel<<<std::max(1, blocks), 256, 0, st>>>(S, w, db, b);
       else launch_wave_extend(S, cp, w, blocks, st);
       if (tb) calib_shade_kernel<true><<<calib_shade_grid<true>(), WT, 0, st>>>(S, cp, C, w, rb, tb, b, db, dm);
       else calib_shade_kernel<false><<<calib_shade_grid<false>(), WT, 0, st>>>(S, cp, C, w, rb, nullptr, b, db, dm);
       if (dm == 2) continue;   // the recorded shadow outcomes were applied by the shading
-      cudaMemsetAsync(w.fetch, 0, 4, st);
       if (tb) calib_shadow_kernel<true><<<blocks, WT, 0, st>>>(S, cp, w, rb, tb, db);
       else calib_shadow_kernel<false><<<blocks, WT, 0, st>>>(S, cp, w, rb, nullptr, db);
     }

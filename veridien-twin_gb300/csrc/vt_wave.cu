@@ -447,7 +447,7 @@ __global__ void __launch_bounds__(WAVE_THREADS, VT_TRACE_BLOCKS) wave_shadow(con
     else finish_path();
   };
   const uint32_t lanes = lanes_of(n);
-  while (serve_lanes(state, exhausted, wb.fetch, n, cp.refill, lanes, next, start)) trace_round<true>(S0, 0.0f, st, stk, state);
+  while (serve_lanes(state, exhausted, wb.fetch_sh, n, cp.refill, lanes, next, start)) trace_round<true>(S0, 0.0f, st, stk, state);
 }
 
 // per pixel, the wave's sub-samples in order i0..i0+n_i-1 added to the running sum; the last wave writes the pixel
@@ -577,7 +577,9 @@ WaveBufs wave_carve(void* base, uint32_t paths, uint32_t n_light, uint32_t n_pix
   w.scache = nullptr;
   w.hc_stride = w.hc_cap = 0;
   w.counts = counts;
-  w.fetch = counts + 3;
+  w.count_sh = counts + 1;
+  w.fetch = counts + 2;
+  w.fetch_sh = counts + 3;
   return w;
 }
 
@@ -607,9 +609,20 @@ int shade_grid() {
   });
 }
 
+// The queue of bounce b in (qa | qb), the next bounce's in the other, its count in words 0 and 4 in turn; the words between
+// (shadow paths, entries taken by the two traversal kernels) and the next count are cleared in one piece: a bounce of a
+// small queue is a few launches, and each clearing was one
+void begin_bounce(WaveBufs& w, uint32_t b, cudaStream_t st) {
+  const bool odd = (b & 1u) != 0u;
+  w.q_in = odd ? w.qa : w.qb;
+  w.q_out = odd ? w.qb : w.qa;
+  w.count_in = w.counts + (odd ? 0 : 4);
+  w.count_out = w.counts + (odd ? 4 : 0);
+  cudaMemsetAsync(w.counts + (odd ? 1 : 0), 0, 16, st);
+}
+
 template <int VAR>
 void bounce_kernels(const Scene& S, const CamParams& cp, const WaveBufs& w, int blocks, cudaStream_t st, KernelTimer* timer) {
-  cudaMemsetAsync(w.fetch, 0, 4, st);
   {
     TimedLaunch tl(timer, st, 0);
     if (VAR == WAVE_PLAIN && w.hcache) wave_extend<VAR, true><<<blocks, WAVE_THREADS, 0, st>>>(S, cp, w);
@@ -620,7 +633,6 @@ void bounce_kernels(const Scene& S, const CamParams& cp, const WaveBufs& w, int 
     if (cp.mode == VT_SHADE_TWIN) wave_shade<VT_SHADE_TWIN, VAR><<<shade_grid<VT_SHADE_TWIN, VAR>(), WAVE_THREADS, 0, st>>>(S, cp, w);
     else wave_shade<VT_SHADE_PATH, VAR><<<shade_grid<VT_SHADE_PATH, VAR>(), WAVE_THREADS, 0, st>>>(S, cp, w);
   }
-  cudaMemsetAsync(w.fetch, 0, 4, st);
   {
     TimedLaunch tl(timer, st, 2);
     if (VAR == WAVE_PLAIN && w.scache) wave_shadow<VAR, true><<<blocks, WAVE_THREADS, 0, st>>>(S, cp, w);
@@ -632,14 +644,7 @@ void wave_bounces(const Scene& S, const CamParams& cp, WaveBufs wb, int var, int
   const uint32_t depth = cp.mode == VT_SHADE_TWIN ? 2u : cp.max_depth;
   WaveBufs w = wb;
   for (uint32_t b = 1; b <= depth; b++) {
-    // queue of this bounce in (qa | qb), next bounce's in the other; counters 0/1 alternate, 2 is the shadow count
-    w.q_in = (b & 1) ? wb.qa : wb.qb;
-    w.q_out = (b & 1) ? wb.qb : wb.qa;
-    w.count_in = wb.counts + ((b & 1) ? 0 : 1);
-    w.count_out = wb.counts + ((b & 1) ? 1 : 0);
-    w.count_sh = wb.counts + 2;
-    cudaMemsetAsync(w.count_out, 0, 4, st);
-    cudaMemsetAsync(w.count_sh, 0, 4, st);
+    begin_bounce(w, b, st);
     if (var == WAVE_SHARED) bounce_kernels<WAVE_SHARED>(S, cp, w, blocks, st, timer);
     else if (var == WAVE_PAIRS) bounce_kernels<WAVE_PAIRS>(S, cp, w, blocks, st, timer);
     else bounce_kernels<WAVE_PLAIN>(S, cp, w, blocks, st, timer);
@@ -648,7 +653,6 @@ void wave_bounces(const Scene& S, const CamParams& cp, WaveBufs wb, int var, int
 }
 
 void launch_wave_extend(const Scene& S, const CamParams& cp, const WaveBufs& wb, int blocks, cudaStream_t st) {
-  cudaMemsetAsync(wb.fetch, 0, 4, st);
   wave_extend<WAVE_PLAIN, false><<<blocks, WAVE_THREADS, 0, st>>>(S, cp, wb);
 }
 

@@ -46,14 +46,15 @@ struct WaveBufs {
   float4* acc2;     // per refined pixel: running sum of the refinement waves
   uint32_t* rlist;  // refined pixel ids
   uint32_t* rcount; // their number (refinement only)
-  uint32_t* counts; // queue lengths
+  uint32_t* counts; // WAVE_COUNTS words: queue lengths and entries taken (begin_bounce)
   // the current bounce's view
   uint32_t* q_in;
   uint32_t* q_out;
   uint32_t* count_in;
   uint32_t* count_out;
   uint32_t* count_sh;
-  uint32_t* fetch;  // next queue entry to take, for the persistent traversal kernels (zeroed before each)
+  uint32_t* fetch;  // next queue entry to take, for the persistent traversal kernels: closest hit,
+  uint32_t* fetch_sh;   // and any hit
   // static first-hit cache of a fixed camera (null: off): per (sub-sample i, pixel id) at i * hc_stride + id the
   // closest hit in the static BVH (t, u, v, triangle bits), t = 0 while empty
   float4* hcache;
@@ -71,6 +72,10 @@ struct KernelTimer {
   uint8_t* kind;
   int cap, n;
 };
+
+// words of WaveBufs::counts, and a bounce's view of them and of the queues, cleared where it starts from zero
+constexpr uint32_t WAVE_COUNTS = 5;
+void begin_bounce(WaveBufs& w, uint32_t b, cudaStream_t st);
 
 size_t wave_bytes(uint32_t paths, uint32_t n_light, uint32_t n_pix);
 WaveBufs wave_carve(void* base, uint32_t paths, uint32_t n_light, uint32_t n_pix, uint32_t* counts);
