@@ -157,11 +157,6 @@ __global__ void __launch_bounds__(WAVE_THREADS, VT_TRACE_BLOCKS) wave_extend(con
   auto finish = [&]() {
     wb.hit[p] = make_float4(st.best.t, st.best.u, st.best.v, __uint_as_float(st.best.tri));
     wb.hinst[p] = st.best.inst;
-    if (VAR == WAVE_SHARED) {
-      const uint64_t have = wb.bc.dirty[p];
-      const uint64_t bits = cull_bits(wb.bc, xyz(wb.o[p]), xyz(wb.d[p]), st.best.t, wb.meta[p].w == 1 ? cp.skip : 0u, have);
-      if (bits & ~have) wb.bc.dirty[p] = have | bits;
-    }
     state = LANE_IDLE;
   };
   // static first-hit cache (camera rays of a fixed camera, gpu/wgsl/kernels.wgsl.js:82 staticFirstHit): a cached
@@ -359,10 +354,9 @@ __global__ void __launch_bounds__(WAVE_THREADS, VT_TRACE_BLOCKS) wave_shadow(con
   float4 nee = make_float4(0, 0, 0, 0);
   float3 Ld = f3(0, 0, 0);
   uint32_t p = 0, j = 0;
-  uint64_t have = 0ull, bits = 0ull;
   uint32_t state = LANE_IDLE;
   bool exhausted = false;
-  const float4* rec = nullptr;
+  float4* rec = nullptr;
   // the static-occlusion cache's bookkeeping of the current path (shade.wgsl.js:270-301): lit and visible samples,
   // their luminance range, a posed body blocking one, and the occlusion word to store
   bool cm = false, dyn = false, fill = false;
@@ -371,6 +365,7 @@ __global__ void __launch_bounds__(WAVE_THREADS, VT_TRACE_BLOCKS) wave_shadow(con
   auto visible = [&](uint32_t jj) {
     const float3 c = xyz(rec[3 * jj + 2]);
     Ld = Ld + c;
+    if (VAR == WAVE_SHARED) rec[3 * jj + 1].w = 2.0f;   // cull_shadow_kernel's
     if (SC && cm) {
       nvis++;
       const float y = lum(c);
@@ -388,7 +383,6 @@ __global__ void __launch_bounds__(WAVE_THREADS, VT_TRACE_BLOCKS) wave_shadow(con
       if (trace_phase(S, root, o, d, 0.0f, nee.w, 3u, skip, st, SC && w.w == 5.0f ? 0 : -1)) return true;
       // nothing to traverse: the segment is unoccluded
       visible(j);
-      if (VAR == WAVE_SHARED) bits |= cull_bits(wb.bc, o, d, a.w, skip0, have | bits);
     }
     return false;
   };
@@ -401,7 +395,6 @@ __global__ void __launch_bounds__(WAVE_THREADS, VT_TRACE_BLOCKS) wave_shadow(con
       if (dyn || (nvis > 0u && nvis < nlit) || (nvis > 1u && lmax - lmin > 0.2f * (lmax + lmin) * 0.5f)) key |= 0x20000u;
     }
     wb.L[p] = make_float4(v.x, v.y, v.z, __uint_as_float(key));
-    if (VAR == WAVE_SHARED && bits) wb.bc.dirty[p] = have | bits;
     state = LANE_IDLE;
   };
   auto start = [&](uint32_t idx) {
@@ -411,8 +404,6 @@ __global__ void __launch_bounds__(WAVE_THREADS, VT_TRACE_BLOCKS) wave_shadow(con
     rec = wb.sh + size_t(p) * nl * 3;
     Ld = f3(0, 0, 0);
     j = 0;
-    bits = 0ull;
-    if (VAR == WAVE_SHARED) have = wb.bc.dirty[p];
     cm = fill = dyn = false;
     if (SC && VAR == WAVE_PLAIN) {
       for (uint32_t q = 0; q < nl; q++) {
@@ -437,7 +428,6 @@ __global__ void __launch_bounds__(WAVE_THREADS, VT_TRACE_BLOCKS) wave_shadow(con
     if (st.best.tri == MISS && trace_phase(S, root, o, d, 0.0f, nee.w, 3u, skip, st, st.k + 1)) { state = LANE_NODE; return; }
     if (st.best.tri == MISS) {
       visible(j);
-      if (VAR == WAVE_SHARED) bits |= cull_bits(wb.bc, o, d, rec[3 * j].w, skip0, have | bits);
     } else if (SC && cm) {
       if (st.k < 0) word |= 1u << j;   // the static scene hides it
       else dyn = true;                 // a posed body does
@@ -448,6 +438,35 @@ __global__ void __launch_bounds__(WAVE_THREADS, VT_TRACE_BLOCKS) wave_shadow(con
   };
   const uint32_t lanes = lanes_of(n);
   while (serve_lanes(state, exhausted, wb.fetch_sh, n, cp.refill, lanes, next, start)) trace_round<true>(S0, 0.0f, st, stk, state);
+}
+
+// A batch's shared segments against the other poses, on all lanes of a warp at once (in the traversal's next() a few lanes
+// walked the cull BVH while the rest of the warp waited: the pose batch of three 960x600 cameras, 16 poses: 67.0 ms of traversal -> 56.3 and 7.0 here): the extension
+// segments up to their hit, then the light samples that nothing hides
+__global__ void __launch_bounds__(WAVE_THREADS) cull_extend_kernel(const CamParams cp, WaveBufs wb) {
+  const uint32_t n = *wb.count_in;
+  for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+    const uint32_t p = wb.q_in[k];
+    const uint64_t have = wb.bc.dirty[p];
+    const uint64_t bits = cull_bits(wb.bc, xyz(wb.o[p]), xyz(wb.d[p]), wb.hit[p].x, wb.meta[p].w == 1u ? cp.skip : 0u, have);
+    if (bits & ~have) wb.bc.dirty[p] = have | bits;
+  }
+}
+__global__ void __launch_bounds__(WAVE_THREADS) cull_shadow_kernel(const Scene S, const CamParams cp, WaveBufs wb) {
+  const uint32_t n = *wb.count_sh, nl = cp.n_light, skip = ldu(S.su + 7);
+  for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+    const uint32_t p = wb.q_sh[k];
+    const float4* rec = wb.sh + size_t(p) * nl * 3;
+    const uint64_t have = wb.bc.dirty[p];
+    uint64_t bits = 0ull;
+    for (uint32_t j = 0; j < nl; j++) {
+      const float4 w = rec[3 * j + 1];
+      if (w.w != 2.0f) continue;
+      const float4 a = rec[3 * j];
+      bits |= cull_bits(wb.bc, xyz(a), xyz(w), a.w, skip, have | bits);
+    }
+    if (bits & ~have) wb.bc.dirty[p] = have | bits;
+  }
 }
 
 // per pixel, the wave's sub-samples in order i0..i0+n_i-1 added to the running sum; the last wave writes the pixel
@@ -625,8 +644,10 @@ template <int VAR>
 void bounce_kernels(const Scene& S, const CamParams& cp, const WaveBufs& w, int blocks, cudaStream_t st, KernelTimer* timer) {
   {
     TimedLaunch tl(timer, st, 0);
-    if (VAR == WAVE_PLAIN && w.hcache) wave_extend<VAR, true><<<blocks, WAVE_THREADS, 0, st>>>(S, cp, w);
+    if (VAR == WAVE_PLAIN && w.hcache) wave_extend<VAR, VAR == WAVE_PLAIN><<<blocks, WAVE_THREADS, 0, st>>>(S, cp, w);
     else wave_extend<VAR, false><<<blocks, WAVE_THREADS, 0, st>>>(S, cp, w);
+    // before the shading, which moves the rays on
+    if (VAR == WAVE_SHARED && w.bc.n_nodes) cull_extend_kernel<<<blocks * 2, WAVE_THREADS, 0, st>>>(cp, w);
   }
   {
     TimedLaunch tl(timer, st, 1);
@@ -635,8 +656,9 @@ void bounce_kernels(const Scene& S, const CamParams& cp, const WaveBufs& w, int 
   }
   {
     TimedLaunch tl(timer, st, 2);
-    if (VAR == WAVE_PLAIN && w.scache) wave_shadow<VAR, true><<<blocks, WAVE_THREADS, 0, st>>>(S, cp, w);
+    if (VAR == WAVE_PLAIN && w.scache) wave_shadow<VAR, VAR == WAVE_PLAIN><<<blocks, WAVE_THREADS, 0, st>>>(S, cp, w);
     else wave_shadow<VAR, false><<<blocks, WAVE_THREADS, 0, st>>>(S, cp, w);
+    if (VAR == WAVE_SHARED && w.bc.n_nodes) cull_shadow_kernel<<<blocks * 2, WAVE_THREADS, 0, st>>>(S, cp, w);
   }
 }
 
