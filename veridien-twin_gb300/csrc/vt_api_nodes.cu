@@ -119,7 +119,9 @@ vt_status vt_nodes_build(vt_ctx* ctx, const vt_nodes_opts* opts, vt_nodes_info* 
   N.nbr_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
   if (N.n_active) {
     VT_CK(cudaMemcpyAsync(N.active, N.active_h.data(), size_t(N.n_active) * 4, cudaMemcpyHostToDevice, ctx->stream));
-    VT_CK(cudaMemcpyAsync(N.nbr, nbr.data(), nbr.size() * 4, cudaMemcpyHostToDevice, ctx->stream));
+    if ((s = ensure_scratch(ctx, nbr.size() * 4)) != VT_OK) return s;
+    VT_CK(cudaMemcpyAsync(ctx->d_scratch, nbr.data(), nbr.size() * 4, cudaMemcpyHostToDevice, ctx->stream));
+    vtk::launch_transpose_nbr(static_cast<const uint2*>(ctx->d_scratch), N.n_active, o.nbr_k, N.nbr, ctx->stream);
   }
   vtk::launch_amu(S, n_mat, K, N.amu, ctx->stream);
   VT_CK(cudaGetLastError());
@@ -276,7 +278,13 @@ vt_status vt_nodes_export(vt_ctx* ctx, uint32_t* gtable, uint32_t* active, uint3
   const auto& N = ctx->nodes;
   if (!N.built) return fail(ctx, VT_ERR_ARG, "nodes: vt_nodes_build first");
   if (gtable && N.n) VT_CK(cudaMemcpyAsync(gtable, N.gtable, size_t(N.n) * N.o.gather_k * 4, cudaMemcpyDeviceToHost, ctx->stream));
-  if (nbr && N.n_active) VT_CK(cudaMemcpyAsync(nbr, N.nbr, size_t(N.n_active) * N.o.nbr_k * 8, cudaMemcpyDeviceToHost, ctx->stream));
+  if (nbr && N.n_active) {
+    const size_t bytes = size_t(N.n_active) * N.o.nbr_k * 8;
+    const vt_status s = ensure_scratch(ctx, bytes);
+    if (s != VT_OK) return s;
+    vtk::launch_transpose_nbr(N.nbr, N.o.nbr_k, N.n_active, static_cast<uint2*>(ctx->d_scratch), ctx->stream);
+    VT_CK(cudaMemcpyAsync(nbr, ctx->d_scratch, bytes, cudaMemcpyDeviceToHost, ctx->stream));
+  }
   VT_CK(cudaStreamSynchronize(ctx->stream));
   if (active) std::copy(N.active_h.begin(), N.active_h.end(), active);
   if (misses) std::copy(N.misses.begin(), N.misses.end(), misses);

@@ -290,20 +290,34 @@ __global__ void __launch_bounds__(256) jacobi_gather_kernel(const Scene S, const
   }
 }
 
+constexpr uint32_t UPD_FLY = 4;
 // jacobiUpdate (gpu/wgsl/kernels.wgsl.js:440): E_free = weighted mean of aux over the node's neighbours, and the
-// separable source Ls = (B_dir + E_free V hh) / (pi hh) into slot_out (w = 1 marks a solved node)
+// separable source Ls = (B_dir + E_free V hh) / (pi hh) into slot_out (w = 1 marks a solved node). The neighbours lie in one
+// row per neighbour, so a warp reads 256 bytes of each, UPD_FLY at a time in flight: with lists of 16 (96k nodes) 11.7 us, with a
+// node's pairs in a line of its own and one after another 14.4; with lists of one or two (331k nodes of 15 mm spacing, 6 mm
+// radius) 14 and 17 us. Eight in flight: 11.7 and 16
 __global__ void jacobi_update_kernel(const Scene S, const uint32_t* __restrict__ active, uint32_t n_active, const uint2* __restrict__ nbr,
                                      uint32_t nbr_k, const float4* __restrict__ aux, uint32_t slot_out, float4* __restrict__ nstate) {
   for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n_active; k += gridDim.x * blockDim.x) {
     const uint32_t i = active[k];
     float3 ef = f3(0, 0, 0);
     float ws = 0.0f;
-    for (uint32_t j = 0; j < nbr_k; j++) {
-      const uint2 e = __ldcs(nbr + size_t(k) * nbr_k + j);
-      const float w = __uint_as_float(e.y);
-      if (w <= 0.0f) break;
-      ef = ef + xyz(aux[e.x]) * w;
-      ws += w;
+    bool more = true;   // a weight of 0 ends the list
+    for (uint32_t j0 = 0; j0 < nbr_k && more; j0 += UPD_FLY) {
+      uint2 e[UPD_FLY];
+      float4 a[UPD_FLY];
+#pragma unroll
+      for (uint32_t j = 0; j < UPD_FLY; j++) e[j] = j0 + j < nbr_k ? __ldcs(nbr + size_t(j0 + j) * n_active + k) : make_uint2(0u, 0u);
+#pragma unroll
+      for (uint32_t j = 0; j < UPD_FLY; j++) a[j] = __uint_as_float(e[j].y) > 0.0f ? aux[e[j].x] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+      for (uint32_t j = 0; j < UPD_FLY; j++) {
+        const float w = __uint_as_float(e[j].y);
+        more = more && w > 0.0f;
+        if (!more) continue;
+        ef = ef + xyz(a[j]) * w;
+        ws += w;
+      }
     }
     ef = ws > 0.0f ? ef / ws : xyz(aux[k]);
     const float4 st = nstate[4u * i];
@@ -361,43 +375,60 @@ __global__ void __launch_bounds__(256) transport_fill_kernel(const Scene S, cons
   }
 }
 
-// jacobiGather over the transport table: aux[k] = sum over the row of weight x Ls_h. A half-warp per row, four
-// 16-byte entries per lane in flight (a row of K = 64 rays in one pass), then the landing nodes' Ls; the entry
-// stream is the only DRAM traffic that grows with the rays; it is loaded evict-first, so the node state (21 MB at
-// 331k nodes) stays in L2 for the gathers.
+// jacobiGather over the transport table: aux[k] = sum over the row of weight x Ls_h. Eight lanes per row, eight 16-byte
+// entries per lane in flight (a row of K = 64 rays in one pass), then the landing nodes' Ls; the entry stream is the only
+// DRAM traffic that grows with the rays; it is loaded evict-first, so the node state (21 MB at 331k nodes) stays in L2 for
+// the gathers. Bound by the L1: a landing node is a line of its own, 21.1 M of them are 71 us at a line per cycle and SM
+// (331k nodes). A lane's two sums are those of lanes l and l + 8 of a half-warp per row, whose first step over the lanes is
+// their addition: the order of the sums does not depend on how many lanes a row has.
 __global__ void __launch_bounds__(256) jacobi_gather_table_kernel(const uint32_t* __restrict__ row, const float4* __restrict__ ent, uint32_t n_active,
                                                                   uint32_t slot_in, const float4* __restrict__ nstate, float4* __restrict__ aux) {
-  const uint32_t hl = threadIdx.x & 15u;
-  const uint32_t half = (blockIdx.x * blockDim.x + threadIdx.x) >> 4, halves = (gridDim.x * blockDim.x) >> 4;
-  // whole warps iterate together (the half-warp shuffles need both halves present)
-  const uint32_t rounds = (n_active + halves - 1) / halves;
+  const uint32_t ql = threadIdx.x & 7u;
+  const uint32_t group = (blockIdx.x * blockDim.x + threadIdx.x) >> 3, groups = (gridDim.x * blockDim.x) >> 3;
+  // whole warps iterate together (the shuffles need all groups of a warp present)
+  const uint32_t rounds = (n_active + groups - 1) / groups;
   for (uint32_t it = 0; it < rounds; it++) {
-    const uint32_t k = half + it * halves;
+    const uint32_t k = group + it * groups;
     const bool in = k < n_active;
     const uint32_t e0 = in ? row[k] : 0u, e1 = in ? row[k + 1] : 0u;
-    float3 acc = f3(0, 0, 0);
+    float3 acc[2] = {f3(0, 0, 0), f3(0, 0, 0)};
     for (uint32_t b = e0; b < e1; b += 64) {
-      float4 w[4], l[4];
+      float4 w[8], l[8];
 #pragma unroll
-      for (int q = 0; q < 4; q++) {
-        const uint32_t e = b + hl + 16u * q;
+      for (int q = 0; q < 8; q++) {
+        const uint32_t e = b + ql + 8u * q;
         w[q] = e < e1 ? __ldcs(ent + e) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);   // streamed: keep Ls in L2
       }
 #pragma unroll
-      for (int q = 0; q < 4; q++) {
-        const uint32_t e = b + hl + 16u * q;
+      for (int q = 0; q < 8; q++) {
+        const uint32_t e = b + ql + 8u * q;
         l[q] = e < e1 ? nstate[4u * __float_as_uint(w[q].w) + slot_in] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
       }
 #pragma unroll
-      for (int q = 0; q < 4; q++) acc = acc + xyz(w[q]) * xyz(l[q]);
+      for (int q = 0; q < 8; q++) acc[q & 1] = acc[q & 1] + xyz(w[q]) * xyz(l[q]);
     }
-    for (int o = 8; o > 0; o >>= 1) {
-      acc.x += __shfl_xor_sync(0xffffffffu, acc.x, o);
-      acc.y += __shfl_xor_sync(0xffffffffu, acc.y, o);
-      acc.z += __shfl_xor_sync(0xffffffffu, acc.z, o);
+    float3 s = acc[0] + acc[1];
+    for (int o = 4; o > 0; o >>= 1) {
+      s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
+      s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
+      s.z += __shfl_xor_sync(0xffffffffu, s.z, o);
     }
-    if (in && hl == 0) aux[k] = make_float4(acc.x, acc.y, acc.z, 0.0f);
+    if (in && ql == 0) aux[k] = make_float4(s.x, s.y, s.z, 0.0f);
   }
+}
+
+// the smoothing neighbours, n_active x nbr_k pairs, to one row per neighbour (out[j * n_active + k]) or back
+__global__ void __launch_bounds__(256) transpose_nbr_kernel(const uint2* __restrict__ in, uint32_t rows, uint32_t cols, uint2* __restrict__ out) {
+  __shared__ uint2 tile[32][33];
+  const uint32_t x = threadIdx.x & 31u, y = threadIdx.x >> 5, r0 = blockIdx.x * 32u, c0 = blockIdx.y * 32u;
+  for (uint32_t i = y; i < 32u; i += 8u)
+    if (r0 + i < rows && c0 + x < cols) tile[i][x] = in[size_t(r0 + i) * cols + c0 + x];
+  __syncthreads();
+  for (uint32_t i = y; i < 32u; i += 8u)
+    if (c0 + i < cols && r0 + x < rows) out[size_t(c0 + i) * rows + r0 + x] = tile[x][i];
+}
+void launch_transpose_nbr(const uint2* in, uint32_t rows, uint32_t cols, uint2* out, cudaStream_t st) {
+  if (rows && cols) transpose_nbr_kernel<<<dim3((rows + 31) / 32, (cols + 31) / 32), 256, 0, st>>>(in, rows, cols, out);
 }
 
 static int grid_for(size_t work, int threads) {
@@ -463,7 +494,7 @@ void launch_jacobi_step(const Scene& S, const uint32_t* active, uint32_t n_activ
                         float4* nstate, float4* aux, cudaStream_t st) {
   if (!n_active) return;
   if (ent)
-    jacobi_gather_table_kernel<<<grid_for(size_t(n_active) * 16, 256), 256, 0, st>>>(row, ent, n_active, slot_in, nstate, aux);
+    jacobi_gather_table_kernel<<<grid_for(size_t(n_active) * 8, 256), 256, 0, st>>>(row, ent, n_active, slot_in, nstate, aux);
   else
     jacobi_gather_kernel<<<grid_for(size_t(n_active) * 32, 256), 256, 0, st>>>(S, active, n_active, K, gtable, amu, slot_in, nstate, aux);
   jacobi_update_kernel<<<grid_for(n_active, 128), 128, 0, st>>>(S, active, n_active, nbr, nbr_k, aux, slot_out, nstate);

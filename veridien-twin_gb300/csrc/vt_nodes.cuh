@@ -27,6 +27,8 @@ void launch_transport_fill(const vtd::Scene& S, const uint32_t* active, uint32_t
                            const uint32_t* row, float4* ent, cudaStream_t st);
 // one Jacobi step: gather from slot_in into aux (from the transport table when ent is set, else evaluating each
 // ray's factor), update into slot_out
+// neighbour pairs, rows x cols, transposed (the Jacobi step reads nbr_k rows of n_active)
+void launch_transpose_nbr(const uint2* in, uint32_t rows, uint32_t cols, uint2* out, cudaStream_t st);
 void launch_jacobi_step(const vtd::Scene& S, const uint32_t* active, uint32_t n_active, uint32_t K, const uint32_t* gtable, const float4* amu,
                         const uint32_t* row, const float4* ent, const uint2* nbr, uint32_t nbr_k, uint32_t slot_in, uint32_t slot_out,
                         float4* nstate, float4* aux, cudaStream_t st);
