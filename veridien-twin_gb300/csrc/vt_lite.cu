@@ -285,6 +285,7 @@ __device__ float3 fragment(const Scene& S, const Geo& g, const View& V, const Sh
 #pragma unroll
   for (uint32_t k = 0; k < K_SECT; k++) {
     const float3 ak = k == 0 ? acc0 : k == 1 ? acc1 : k == 2 ? acc2 : acc3;
+    if (dbg != 2u && maxc(ak) <= 0.0f) continue;   // nothing to shadow
     float vk = 1.0f;
     if (dbg != 1u) vk = sm_vis(V, a, off, k, is_static ? V.lo[k][3] : 6e-4f);
     vsum = vsum + vk;
