@@ -63,13 +63,14 @@ vt_status vt_nodes_build(vt_ctx* ctx, const vt_nodes_opts* opts, vt_nodes_info* 
   const uint32_t n = ctx->S.static_verts, K = o.gather_k;
   const uint32_t n_mat = uint32_t(std::max<size_t>(1, ctx->S.mats.size()));
   const size_t b_g = al(size_t(n) * K * 4), b_aux = al(size_t(n) * 16 + 16), b_act = al(size_t(n) * 4 + 4),
-               b_nbr = al(size_t(n) * o.nbr_k * 8 + 8), b_amu = al(size_t(n_mat) * K * 16);
+               b_nbr = al(size_t(n) * o.nbr_k * 8 + 8), b_amu = al(size_t(n_mat) * K * 16),
+               b_hh = al(size_t(n_mat) * 48), b_sums = al(vtk::node_sums_bytes());
   VT_CK(cudaStreamSynchronize(ctx->stream));
   cudaFree(N.mem);
   cudaFree(N.table_mem);
   cudaFree(N.direct_mem);
   N = vt_ctx::Nodes{};
-  if (cudaMalloc(&N.mem, b_g + b_aux + b_act + b_nbr + b_amu) != cudaSuccess) {
+  if (cudaMalloc(&N.mem, b_g + b_aux + b_act + b_nbr + b_amu + b_hh + b_sums) != cudaSuccess) {
     cudaGetLastError();
     N.mem = nullptr;
     return fail(ctx, VT_ERR_OOM, "nodes: gather table allocation failed");
@@ -79,7 +80,9 @@ vt_status vt_nodes_build(vt_ctx* ctx, const vt_nodes_opts* opts, vt_nodes_info* 
   N.aux = reinterpret_cast<float4*>(p); p += b_aux;
   N.active = reinterpret_cast<uint32_t*>(p); p += b_act;
   N.nbr = reinterpret_cast<uint2*>(p); p += b_nbr;
-  N.amu = reinterpret_cast<float4*>(p);
+  N.amu = reinterpret_cast<float4*>(p); p += b_amu;
+  N.hh = reinterpret_cast<double*>(p); p += b_hh;
+  N.sums = reinterpret_cast<double*>(p);
   N.o = o;
   N.n = n;
   N.n_mat = n_mat;
@@ -87,6 +90,13 @@ vt_status vt_nodes_build(vt_ctx* ctx, const vt_nodes_opts* opts, vt_nodes_info* 
   std::vector<float> st(std::max<size_t>(16, size_t(n) * 16), 0.0f);
   for (uint32_t i = 0; i < n; i++) { st[16 * size_t(i) + 3] = 1; st[16 * size_t(i) + 15] = -1; }
   VT_CK(cudaMemcpyAsync(ctx->d_nstate, st.data(), size_t(n) * 64, cudaMemcpyHostToDevice, ctx->stream));
+  std::vector<double> hh(size_t(n_mat) * 6, 1.0);
+  for (size_t m = 0; m < ctx->S.mats.size(); m++)
+    for (int c = 0; c < 3; c++) {
+      hh[6 * m + c] = std::max(1e-4, ctx->S.mats[m].hh[c]);
+      hh[6 * m + 3 + c] = 1.0 / std::max(1e-3, ctx->S.mats[m].hh[c]);
+    }
+  VT_CK(cudaMemcpyAsync(N.hh, hh.data(), hh.size() * 8, cudaMemcpyHostToDevice, ctx->stream));
   ctx->slot = 1;
   vt_status s = write_su(ctx);
   if (s != VT_OK) return s;
@@ -195,22 +205,12 @@ vt_status vt_node_summary(vt_ctx* ctx, double out[13]) {
   if (!ctx) return VT_ERR_ARG;
   auto& N = ctx->nodes;
   if (!N.built) return fail(ctx, VT_ERR_ARG, "nodes: vt_nodes_build first");
-  std::vector<float> st(size_t(N.n) * 16);
-  if (N.n) VT_CK(cudaMemcpyAsync(st.data(), ctx->d_nstate, st.size() * 4, cudaMemcpyDeviceToHost, ctx->stream));
+  vtk::launch_node_sums(dev_scene(ctx), N.active, N.n_active, N.hh, ctx->slot ? ctx->slot : 1, ctx->d_nstate, N.sums, ctx->stream);
+  VT_CK(cudaGetLastError());
+  double sums[10];
+  VT_CK(cudaMemcpyAsync(sums, N.sums, sizeof(sums), cudaMemcpyDeviceToHost, ctx->stream));
   VT_CK(cudaStreamSynchronize(ctx->stream));
-  const uint32_t slot = ctx->slot ? ctx->slot : 1;
-  double A = 0, E[3] = {0, 0, 0}, Ed[3] = {0, 0, 0}, Lo[3] = {0, 0, 0};
-  for (uint32_t i : N.active_h) {
-    const double a = ctx->S.node_area[i], V = st[16 * size_t(i) + 3];
-    A += a;
-    const uint32_t mesh = ctx->S.verts[8 * size_t(i) + 3];
-    const double* hh = ctx->S.mats[ctx->S.meshes[mesh].mat].hh;
-    for (int c = 0; c < 3; c++) {
-      E[c] += a * st[16 * size_t(i) + c] * V;
-      Lo[c] += a * st[16 * size_t(i) + 4 * slot + c] * std::max(1e-4, hh[c]);
-      Ed[c] += a * st[16 * size_t(i) + 12 + c] / std::max(1e-3, hh[c]);
-    }
-  }
+  const double A = sums[0], *E = sums + 1, *Ed = sums + 4, *Lo = sums + 7;
   double r[13] = {A};
   for (int c = 0; c < 3; c++) {
     const double inv = A > 0 ? 1.0 / A : 0.0;

@@ -141,6 +141,7 @@ struct vt_ctx {
     uint32_t* active = nullptr;
     uint2* nbr = nullptr;
     float4* amu = nullptr;
+    double *hh = nullptr, *sums = nullptr;   // the materials' hh for launch_node_sums, and its work
     void* table_mem = nullptr;               // transport table: row offsets, then entries
     void* direct_mem = nullptr;              // the direct light's shadow rays and terms (node_direct_bytes)
     uint32_t* row = nullptr;
