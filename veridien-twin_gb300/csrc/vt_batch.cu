@@ -206,6 +206,7 @@ void batch_camera(const Scene& S, const CamParams& cp, const BatchCull& bc, cons
     wp.bc.px0 = px0;
     wp.bc.pair_src = bw.pair_src;
     wp.bc.pair_pose = bw.pair_pose;
+    cudaMemsetAsync(wp.counts, 0, 16, st);
     scan_blocks_kernel<<<nb, SCAN, 0, st>>>(bw.dirty, P, bw.off, bw.blk);
     scan_top_kernel<<<1, 1024, 0, st>>>(bw.blk, nb, bw.cap, wp.counts, bw.status, bw.stats);
     expand_kernel<<<blocks, T, 0, st>>>(bw.dirty, P, bw.off, bw.blk, bw.cap, bw.pair_src, bw.pair_pose);

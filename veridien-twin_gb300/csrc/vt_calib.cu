@@ -395,6 +395,7 @@ __global__ void __launch_bounds__(WT, 3) calib_shade_kernel(const Scene S, const
 // any hit of the pending light samples on persistent lanes; an occluded sample's contribution is cleared in the record
 template <bool TAN>
 __global__ void __launch_bounds__(WT, 4) calib_shadow_kernel(const Scene S, const CamParams cp, WaveBufs wb, CalPath* rec, CalTan* tan, CalDec* dec) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // the next bounce's closest hits
   const uint32_t n = *wb.count_sh;
   const uint32_t nl = cp.n_light;
   const uint32_t skip = ldu(S.su + 7);
@@ -915,9 +916,10 @@ static void calib_trace(const Scene& S, const CamParams& cp, const CalibDev& C, 
     const int dm = db ? dmode : 0;
     for (uint32_t b = 1; b <= cp.max_depth; b++) {
       WaveBufs w = wb;
-      begin_bounce(w, b, st);
+      bounce_view(w, b);
       if (dm == 2) calib_rehit_kernel<<<std::max(1, blocks), 256, 0, st>>>(S, w, db, b);
-      else launch_wave_extend(S, cp, w, blocks, st);
+      else launch_wave_extend(S, cp, w, blocks, st, b > 1);   // over the light samples' tail
+      clear_next_bounce(w, st);
       if (tb) calib_shade_kernel<true><<<calib_shade_grid<true>(), WT, 0, st>>>(S, cp, C, w, rb, tb, b, db, dm);
       else calib_shade_kernel<false><<<calib_shade_grid<false>(), WT, 0, st>>>(S, cp, C, w, rb, nullptr, b, db, dm);
       if (dm == 2) continue;   // the recorded shadow outcomes were applied by the shading

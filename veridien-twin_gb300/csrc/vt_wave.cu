@@ -195,6 +195,7 @@ __global__ void __launch_bounds__(WAVE_THREADS, VT_TRACE_BLOCKS) wave_extend(con
   };
   const uint32_t lanes = lanes_of(n);
   while (serve_lanes(state, exhausted, wb.fetch, n, cp.refill, lanes, next, start)) trace_round<false>(S, 0.0f, st, stk, state);
+  asm volatile("griddepcontrol.wait;" ::: "memory");   // launched beside the light samples: the next kernel follows both
 }
 
 template <int MODE, int VAR>
@@ -339,6 +340,7 @@ __global__ void __launch_bounds__(WAVE_THREADS, VT_WAVE_SHADE_BLOCKS) wave_shade
 // SC: the static-occlusion cache is on (compiled separately, so the plain kernel keeps its registers)
 template <int VAR, bool SC = false>
 __global__ void __launch_bounds__(WAVE_THREADS, VT_TRACE_BLOCKS) wave_shadow(const Scene S0, const CamParams cp, WaveBufs wb) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // the next bounce's closest hits (wave_bounces_of)
   const uint32_t n = *wb.count_sh;
   if (wb.stats && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(wb.stats + 1, (unsigned long long)n);
   const uint32_t nl = cp.n_light;
@@ -628,54 +630,84 @@ int shade_grid() {
   });
 }
 
-// The queue of bounce b in (qa | qb), the next bounce's in the other, its count in words 0 and 4 in turn; the words between
-// (shadow paths, entries taken by the two traversal kernels) and the next count are cleared in one piece: a bounce of a
-// small queue is a few launches, and each clearing was one
-void begin_bounce(WaveBufs& w, uint32_t b, cudaStream_t st) {
-  const bool odd = (b & 1u) != 0u;
+// The queue of bounce b in (qa | qb), the next bounce's in the other; of the counts four words per bounce in turn: the
+// queue's length, shadow paths, entries taken by the closest-hit and by the any-hit lanes. They are cleared in one piece:
+// a bounce of a small queue is a few launches, and each clearing was one
+void bounce_view(WaveBufs& w, uint32_t b) {
+  const uint32_t odd = b & 1u;
   w.q_in = odd ? w.qa : w.qb;
   w.q_out = odd ? w.qb : w.qa;
   w.count_in = w.counts + (odd ? 0 : 4);
   w.count_out = w.counts + (odd ? 4 : 0);
-  cudaMemsetAsync(w.counts + (odd ? 1 : 0), 0, 16, st);
+  w.count_sh = w.count_in + 1;
+  w.fetch = w.count_in + 2;
+  w.fetch_sh = w.count_in + 3;
+}
+void clear_next_bounce(const WaveBufs& w, cudaStream_t st) { cudaMemsetAsync(w.count_out, 0, 16, st); }
+
+// A bounce's closest hits read nothing that the previous bounce's light samples write, nor the other way round: their
+// kernel is launched over that one's tail (programmatic launch: its blocks start where the other's have ended, and wait
+// for the whole of it before they end themselves, so that what follows in the stream follows both)
+template <int VAR, bool HC>
+void extend_over(const Scene& S, const CamParams& cp, const WaveBufs& w, int blocks, cudaStream_t st, bool over) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t lc{};
+  lc.gridDim = blocks;
+  lc.blockDim = WAVE_THREADS;
+  lc.stream = st;
+  lc.attrs = &attr;
+  lc.numAttrs = over ? 1 : 0;
+  cudaLaunchKernelEx(&lc, wave_extend<VAR, HC>, S, cp, w);
 }
 
 template <int VAR>
-void bounce_kernels(const Scene& S, const CamParams& cp, const WaveBufs& w, int blocks, cudaStream_t st, KernelTimer* timer) {
-  {
-    TimedLaunch tl(timer, st, 0);
-    if (VAR == WAVE_PLAIN && w.hcache) wave_extend<VAR, VAR == WAVE_PLAIN><<<blocks, WAVE_THREADS, 0, st>>>(S, cp, w);
-    else wave_extend<VAR, false><<<blocks, WAVE_THREADS, 0, st>>>(S, cp, w);
-    // before the shading, which moves the rays on
-    if (VAR == WAVE_SHARED && w.bc.n_nodes) cull_extend_kernel<<<blocks * 2, WAVE_THREADS, 0, st>>>(cp, w);
-  }
-  {
-    TimedLaunch tl(timer, st, 1);
-    if (cp.mode == VT_SHADE_TWIN) wave_shade<VT_SHADE_TWIN, VAR><<<shade_grid<VT_SHADE_TWIN, VAR>(), WAVE_THREADS, 0, st>>>(S, cp, w);
-    else wave_shade<VT_SHADE_PATH, VAR><<<shade_grid<VT_SHADE_PATH, VAR>(), WAVE_THREADS, 0, st>>>(S, cp, w);
-  }
-  {
-    TimedLaunch tl(timer, st, 2);
-    if (VAR == WAVE_PLAIN && w.scache) wave_shadow<VAR, VAR == WAVE_PLAIN><<<blocks, WAVE_THREADS, 0, st>>>(S, cp, w);
-    else wave_shadow<VAR, false><<<blocks, WAVE_THREADS, 0, st>>>(S, cp, w);
-    if (VAR == WAVE_SHARED && w.bc.n_nodes) cull_shadow_kernel<<<blocks * 2, WAVE_THREADS, 0, st>>>(S, cp, w);
-  }
-}
-
-void wave_bounces(const Scene& S, const CamParams& cp, WaveBufs wb, int var, int blocks, cudaStream_t st, uint64_t* launches, KernelTimer* timer) {
+void wave_bounces_of(const Scene& S, const CamParams& cp, const WaveBufs& wb, int blocks, cudaStream_t st, uint64_t* launches, KernelTimer* timer) {
   const uint32_t depth = cp.mode == VT_SHADE_TWIN ? 2u : cp.max_depth;
+  constexpr bool PLAIN = VAR == WAVE_PLAIN;
+  const bool cull = VAR == WAVE_SHARED && wb.bc.n_nodes != 0u;
   WaveBufs w = wb;
-  for (uint32_t b = 1; b <= depth; b++) {
-    begin_bounce(w, b, st);
-    if (var == WAVE_SHARED) bounce_kernels<WAVE_SHARED>(S, cp, w, blocks, st, timer);
-    else if (var == WAVE_PAIRS) bounce_kernels<WAVE_PAIRS>(S, cp, w, blocks, st, timer);
-    else bounce_kernels<WAVE_PLAIN>(S, cp, w, blocks, st, timer);
+  for (uint32_t b = 1; b <= depth + 1; b++) {
+    // closest hits of bounce b over the light samples of bounce b - 1
+    if (b <= depth) {
+      bounce_view(w, b);
+      TimedLaunch tl(timer, st, 0);
+      const bool over = b > 1 && !timer;   // the kernels' own times need them apart
+      if (PLAIN && w.hcache) extend_over<VAR, PLAIN>(S, cp, w, blocks, st, over);
+      else extend_over<VAR, false>(S, cp, w, blocks, st, over);
+      // before the shading, which moves the rays on
+      if (cull) cull_extend_kernel<<<blocks * 2, WAVE_THREADS, 0, st>>>(cp, w);
+    }
+    if (cull && b > 1) {
+      bounce_view(w, b - 1);
+      cull_shadow_kernel<<<blocks * 2, WAVE_THREADS, 0, st>>>(S, cp, w);
+    }
+    if (b > depth) break;
+    bounce_view(w, b);
+    clear_next_bounce(w, st);
+    {
+      TimedLaunch tl(timer, st, 1);
+      if (cp.mode == VT_SHADE_TWIN) wave_shade<VT_SHADE_TWIN, VAR><<<shade_grid<VT_SHADE_TWIN, VAR>(), WAVE_THREADS, 0, st>>>(S, cp, w);
+      else wave_shade<VT_SHADE_PATH, VAR><<<shade_grid<VT_SHADE_PATH, VAR>(), WAVE_THREADS, 0, st>>>(S, cp, w);
+    }
+    {
+      TimedLaunch tl(timer, st, 2);
+      if (PLAIN && w.scache) wave_shadow<VAR, PLAIN><<<blocks, WAVE_THREADS, 0, st>>>(S, cp, w);
+      else wave_shadow<VAR, false><<<blocks, WAVE_THREADS, 0, st>>>(S, cp, w);
+    }
     if (launches) *launches += 3;
   }
 }
 
-void launch_wave_extend(const Scene& S, const CamParams& cp, const WaveBufs& wb, int blocks, cudaStream_t st) {
-  wave_extend<WAVE_PLAIN, false><<<blocks, WAVE_THREADS, 0, st>>>(S, cp, wb);
+void wave_bounces(const Scene& S, const CamParams& cp, WaveBufs wb, int var, int blocks, cudaStream_t st, uint64_t* launches, KernelTimer* timer) {
+  if (var == WAVE_SHARED) wave_bounces_of<WAVE_SHARED>(S, cp, wb, blocks, st, launches, timer);
+  else if (var == WAVE_PAIRS) wave_bounces_of<WAVE_PAIRS>(S, cp, wb, blocks, st, launches, timer);
+  else wave_bounces_of<WAVE_PLAIN>(S, cp, wb, blocks, st, launches, timer);
+}
+
+void launch_wave_extend(const Scene& S, const CamParams& cp, const WaveBufs& wb, int blocks, cudaStream_t st, bool over) {
+  extend_over<WAVE_PLAIN, false>(S, cp, wb, blocks, st, over);
 }
 
 void launch_wave_gen(const CamParams& cp, WaveBufs wb, uint32_t i0, uint32_t n_i, uint32_t n_pix, int blocks, cudaStream_t st) {

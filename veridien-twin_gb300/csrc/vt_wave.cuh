@@ -46,7 +46,7 @@ struct WaveBufs {
   float4* acc2;     // per refined pixel: running sum of the refinement waves
   uint32_t* rlist;  // refined pixel ids
   uint32_t* rcount; // their number (refinement only)
-  uint32_t* counts; // WAVE_COUNTS words: queue lengths and entries taken (begin_bounce)
+  uint32_t* counts; // WAVE_COUNTS words: queue lengths and entries taken (bounce_view)
   // the current bounce's view
   uint32_t* q_in;
   uint32_t* q_out;
@@ -73,9 +73,11 @@ struct KernelTimer {
   int cap, n;
 };
 
-// words of WaveBufs::counts, and a bounce's view of them and of the queues, cleared where it starts from zero
-constexpr uint32_t WAVE_COUNTS = 5;
-void begin_bounce(WaveBufs& w, uint32_t b, cudaStream_t st);
+// Words of WaveBufs::counts. A bounce's view of them and of the queues; the next bounce's words cleared, once the closest
+// hits of bounce b and the light samples of bounce b - 1 are traced. The first bounce begins with words 1 to 3 clear.
+constexpr uint32_t WAVE_COUNTS = 8;
+void bounce_view(WaveBufs& w, uint32_t b);
+void clear_next_bounce(const WaveBufs& w, cudaStream_t st);
 
 size_t wave_bytes(uint32_t paths, uint32_t n_light, uint32_t n_pix);
 WaveBufs wave_carve(void* base, uint32_t paths, uint32_t n_light, uint32_t n_pix, uint32_t* counts);
@@ -90,7 +92,8 @@ void wave_bounces(const vtd::Scene& S, const CamParams& cp, WaveBufs wb, int var
                   KernelTimer* timer = nullptr);
 // the closest-hit kernel over wb.qa / counts (plain scene) and the camera rays of sub-samples [i0, i0 + n_i) of all
 // n_pix pixel ids (path p = (i - i0) n_pix + id), queued in wb.qa / counts[0]
-void launch_wave_extend(const vtd::Scene& S, const CamParams& cp, const WaveBufs& wb, int blocks, cudaStream_t st);
+// over: beside the tail of the light-sample kernel launched just before (wave_bounces_of), whose blocks have to trigger it
+void launch_wave_extend(const vtd::Scene& S, const CamParams& cp, const WaveBufs& wb, int blocks, cudaStream_t st, bool over = false);
 void launch_wave_gen(const CamParams& cp, WaveBufs wb, uint32_t i0, uint32_t n_i, uint32_t n_pix, int blocks, cudaStream_t st);
 // camera rays of a batch wave: paths p = i * n_pw + lp, i < spp, pixel id px0 + lp; clears the dirty masks
 void wave_gen_batch(const CamParams& cp, WaveBufs wb, int blocks, cudaStream_t st);
