@@ -917,9 +917,12 @@ static void calib_trace(const Scene& S, const CamParams& cp, const CalibDev& C, 
     for (uint32_t b = 1; b <= cp.max_depth; b++) {
       WaveBufs w = wb;
       bounce_view(w, b);
-      if (dm == 2) calib_rehit_kernel<<<std::max(1, blocks), 256, 0, st>>>(S, w, db, b);
-      else launch_wave_extend(S, cp, w, blocks, st, b > 1);   // over the light samples' tail
-      clear_next_bounce(w, st);
+      if (dm == 2) {
+        cudaMemsetAsync(w.count_out, 0, 16, st);
+        calib_rehit_kernel<<<std::max(1, blocks), 256, 0, st>>>(S, w, db, b);
+      } else {
+        launch_wave_extend(S, cp, w, blocks, st, b > 1);   // over the light samples' tail
+      }
       if (tb) calib_shade_kernel<true><<<calib_shade_grid<true>(), WT, 0, st>>>(S, cp, C, w, rb, tb, b, db, dm);
       else calib_shade_kernel<false><<<calib_shade_grid<false>(), WT, 0, st>>>(S, cp, C, w, rb, nullptr, b, db, dm);
       if (dm == 2) continue;   // the recorded shadow outcomes were applied by the shading

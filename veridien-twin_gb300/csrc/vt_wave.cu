@@ -196,6 +196,8 @@ __global__ void __launch_bounds__(WAVE_THREADS, VT_TRACE_BLOCKS) wave_extend(con
   const uint32_t lanes = lanes_of(n);
   while (serve_lanes(state, exhausted, wb.fetch, n, cp.refill, lanes, next, start)) trace_round<false>(S, 0.0f, st, stk, state);
   asm volatile("griddepcontrol.wait;" ::: "memory");   // launched beside the light samples: the next kernel follows both
+  // theirs, the next bounce's (a batch's cull_shadow_kernel reads them once more)
+  if (VAR != WAVE_SHARED && blockIdx.x == 0 && threadIdx.x == 0) *reinterpret_cast<uint4*>(wb.count_out) = make_uint4(0, 0, 0, 0);
 }
 
 template <int MODE, int VAR>
@@ -206,6 +208,7 @@ template <int MODE, int VAR>
 #define VT_WAVE_SHADE_BLOCKS 3
 #endif
 __global__ void __launch_bounds__(WAVE_THREADS, VT_WAVE_SHADE_BLOCKS) wave_shade(const Scene S0, const CamParams cp, WaveBufs wb) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   const uint32_t n = *wb.count_in;
   const uint32_t nl = cp.n_light;
   const bool no_mis = (cp.options & VT_O_NO_MIS) != 0u;
@@ -340,6 +343,7 @@ __global__ void __launch_bounds__(WAVE_THREADS, VT_WAVE_SHADE_BLOCKS) wave_shade
 // SC: the static-occlusion cache is on (compiled separately, so the plain kernel keeps its registers)
 template <int VAR, bool SC = false>
 __global__ void __launch_bounds__(WAVE_THREADS, VT_TRACE_BLOCKS) wave_shadow(const Scene S0, const CamParams cp, WaveBufs wb) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // the next bounce's closest hits (wave_bounces_of)
   const uint32_t n = *wb.count_sh;
   if (wb.stats && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(wb.stats + 1, (unsigned long long)n);
@@ -631,8 +635,8 @@ int shade_grid() {
 }
 
 // The queue of bounce b in (qa | qb), the next bounce's in the other; of the counts four words per bounce in turn: the
-// queue's length, shadow paths, entries taken by the closest-hit and by the any-hit lanes. They are cleared in one piece:
-// a bounce of a small queue is a few launches, and each clearing was one
+// queue's length, shadow paths, entries taken by the closest-hit and by the any-hit lanes. They are clear for the next
+// bounce once the closest hits of this one and the light samples of the one before are traced
 void bounce_view(WaveBufs& w, uint32_t b) {
   const uint32_t odd = b & 1u;
   w.q_in = odd ? w.qa : w.qb;
@@ -643,13 +647,10 @@ void bounce_view(WaveBufs& w, uint32_t b) {
   w.fetch = w.count_in + 2;
   w.fetch_sh = w.count_in + 3;
 }
-void clear_next_bounce(const WaveBufs& w, cudaStream_t st) { cudaMemsetAsync(w.count_out, 0, 16, st); }
 
-// A bounce's closest hits read nothing that the previous bounce's light samples write, nor the other way round: their
-// kernel is launched over that one's tail (programmatic launch: its blocks start where the other's have ended, and wait
-// for the whole of it before they end themselves, so that what follows in the stream follows both)
-template <int VAR, bool HC>
-void extend_over(const Scene& S, const CamParams& cp, const WaveBufs& w, int blocks, cudaStream_t st, bool over) {
+// launched before the kernel ahead has ended, whose results `kernel` waits for itself (griddepcontrol.wait)
+template <typename... P, typename... A>
+void launch_dependent(void (*kernel)(P...), int blocks, cudaStream_t st, bool dependent, const A&... args) {
   cudaLaunchAttribute attr{};
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
@@ -658,8 +659,16 @@ void extend_over(const Scene& S, const CamParams& cp, const WaveBufs& w, int blo
   lc.blockDim = WAVE_THREADS;
   lc.stream = st;
   lc.attrs = &attr;
-  lc.numAttrs = over ? 1 : 0;
-  cudaLaunchKernelEx(&lc, wave_extend<VAR, HC>, S, cp, w);
+  lc.numAttrs = dependent ? 1 : 0;
+  cudaLaunchKernelEx(&lc, kernel, args...);
+}
+
+// A bounce's closest hits read nothing that the previous bounce's light samples write, nor the other way round: their
+// kernel is launched over that one's tail (programmatic launch: its blocks start where the other's have ended, and wait
+// for the whole of it before they end themselves, so that what follows in the stream follows both)
+template <int VAR, bool HC>
+void extend_over(const Scene& S, const CamParams& cp, const WaveBufs& w, int blocks, cudaStream_t st, bool over) {
+  launch_dependent(wave_extend<VAR, HC>, blocks, st, over, S, cp, w);
 }
 
 template <int VAR>
@@ -685,16 +694,16 @@ void wave_bounces_of(const Scene& S, const CamParams& cp, const WaveBufs& wb, in
     }
     if (b > depth) break;
     bounce_view(w, b);
-    clear_next_bounce(w, st);
+    if (VAR == WAVE_SHARED) cudaMemsetAsync(w.count_out, 0, 16, st);
     {
       TimedLaunch tl(timer, st, 1);
-      if (cp.mode == VT_SHADE_TWIN) wave_shade<VT_SHADE_TWIN, VAR><<<shade_grid<VT_SHADE_TWIN, VAR>(), WAVE_THREADS, 0, st>>>(S, cp, w);
-      else wave_shade<VT_SHADE_PATH, VAR><<<shade_grid<VT_SHADE_PATH, VAR>(), WAVE_THREADS, 0, st>>>(S, cp, w);
+      if (cp.mode == VT_SHADE_TWIN) launch_dependent(wave_shade<VT_SHADE_TWIN, VAR>, shade_grid<VT_SHADE_TWIN, VAR>(), st, !timer, S, cp, w);
+      else launch_dependent(wave_shade<VT_SHADE_PATH, VAR>, shade_grid<VT_SHADE_PATH, VAR>(), st, !timer, S, cp, w);
     }
     {
       TimedLaunch tl(timer, st, 2);
-      if (PLAIN && w.scache) wave_shadow<VAR, PLAIN><<<blocks, WAVE_THREADS, 0, st>>>(S, cp, w);
-      else wave_shadow<VAR, false><<<blocks, WAVE_THREADS, 0, st>>>(S, cp, w);
+      if (PLAIN && w.scache) launch_dependent(wave_shadow<VAR, PLAIN>, blocks, st, !timer, S, cp, w);
+      else launch_dependent(wave_shadow<VAR, false>, blocks, st, !timer, S, cp, w);
     }
     if (launches) *launches += 3;
   }

@@ -73,11 +73,10 @@ struct KernelTimer {
   int cap, n;
 };
 
-// Words of WaveBufs::counts. A bounce's view of them and of the queues; the next bounce's words cleared, once the closest
-// hits of bounce b and the light samples of bounce b - 1 are traced. The first bounce begins with words 1 to 3 clear.
+// Words of WaveBufs::counts, and a bounce's view of them and of the queues. The first bounce begins with words 1 to 3
+// clear; a bounce's closest-hit kernel clears the next one's.
 constexpr uint32_t WAVE_COUNTS = 8;
 void bounce_view(WaveBufs& w, uint32_t b);
-void clear_next_bounce(const WaveBufs& w, cudaStream_t st);
 
 size_t wave_bytes(uint32_t paths, uint32_t n_light, uint32_t n_pix);
 WaveBufs wave_carve(void* base, uint32_t paths, uint32_t n_light, uint32_t n_pix, uint32_t* counts);
