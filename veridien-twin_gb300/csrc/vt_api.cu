@@ -327,20 +327,27 @@ static vt_status render_impl(vt_ctx* ctx, const vt_render_req* q, float* out_rgb
                                 q->options, q->mode, q->max_depth, q->root, q->shutter, q->scale);
   cp2.refine = cp.refine;
   if (q->frame != ctx->frame) { ctx->frame = q->frame; vt_status s = write_su(ctx); if (s != VT_OK) return s; }
-  // wave of up to 8 M paths (whole sub-sample indices): ~1.4 GB of path state at one light sample
-  const uint32_t n_pix = vtk::tiled_pixels(c.width, c.height, cp.tile_w, cp.tile_h);
-  const uint32_t per_wave = std::max(1u, std::min(cp.spp, (8u << 20) / std::max(1u, n_pix)));
-  const uint32_t paths = per_wave * n_pix;
-  const size_t need = vtk::wave_bytes(paths, std::max(cp.n_light, cp2.n_light), n_pix);
-  if (ctx->wave_cap < need) {
+  // wave of up to 8 M paths (whole sub-sample indices): ~1.4 GB of path state at one light sample. The refinement's
+  // sub-samples count too: how many pixels they are taken for is not known here, and in waves of pass 1's (one of
+  // each pixel in the twin's presets) it ran in launches that were mostly tails: twin frame
+  // of three 1280x720 cameras with 6 more sub-samples, 10.8 ms in six waves, 8.95 in one
+  const uint32_t n_pix = vtk::tiled_pixels(c.width, c.height, cp.tile_w, cp.tile_h), nl_max = std::max(cp.n_light, cp2.n_light);
+  const uint32_t per_max = std::max(1u, (8u << 20) / std::max(1u, n_pix));
+  const uint32_t paths_least = std::min(std::max(1u, cp.spp), per_max) * n_pix;
+  uint32_t paths = std::max(paths_least, std::min(cp.refine, per_max) * n_pix);
+  for (;;) {
+    const size_t need = vtk::wave_bytes(paths, nl_max, n_pix);
+    if (ctx->wave_cap >= need) break;
     VT_CK(cudaStreamSynchronize(ctx->stream));
     cudaFree(ctx->d_wave);
     ctx->d_wave = nullptr;
     ctx->wave_cap = 0;
-    if (cudaMalloc(&ctx->d_wave, need) != cudaSuccess) { cudaGetLastError(); return fail(ctx, VT_ERR_OOM, "wavefront state allocation failed"); }
-    ctx->wave_cap = need;
+    if (cudaMalloc(&ctx->d_wave, need) == cudaSuccess) { ctx->wave_cap = need; break; }
+    cudaGetLastError();
+    if (paths == paths_least) return fail(ctx, VT_ERR_OOM, "wavefront state allocation failed");
+    paths = paths_least;   // the refinement in smaller waves
   }
-  vtk::WaveBufs wb = vtk::wave_carve(ctx->d_wave, paths, std::max(cp.n_light, cp2.n_light), n_pix, ctx->d_work);
+  vtk::WaveBufs wb = vtk::wave_carve(ctx->d_wave, paths, nl_max, n_pix, ctx->d_work);
   wb.rcount = ctx->d_work + 12;
   if (q->options & (VT_O_CACHE_WRITE | VT_O_CACHE_READ)) {
     // the cache stays valid while what decides a camera ray's static hit holds (its time does not: the static
