@@ -213,6 +213,10 @@ __global__ void __launch_bounds__(WAVE_THREADS, VT_WAVE_SHADE_BLOCKS) wave_shade
   const uint32_t nl = cp.n_light;
   const bool no_mis = (cp.options & VT_O_NO_MIS) != 0u;
   const float emit_area = __ldg(S0.su + 3);
+  // a batch's pairs have a pose each
+  constexpr bool ONE_POSE = MODE == VT_SHADE_TWIN && VAR != WAVE_PAIRS;
+  __shared__ Capsules caps;
+  if (ONE_POSE) load_capsules(S0, caps);
   for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
     const uint32_t p = wb.q_in[k];
     const Scene S = path_scene<VAR>(S0, wb, p);
@@ -266,8 +270,14 @@ __global__ void __launch_bounds__(WAVE_THREADS, VT_WAVE_SHADE_BLOCKS) wave_shade
           }
         }
       } else {
-        const Mat M = load_mat(S, s.mat);
         const float3 n = shading_normal(S, s, cp.options);
+        // the node radiosity first: its nodes and weights are not held over the light samples
+        if (MODE == VT_SHADE_TWIN && is_static && !(cp.options & (VT_O_NO_INDIRECT | VT_O_DIRECT_ONLY))) {
+          float3 E = node_slot(S, s, 0u, ldu(S.su + 18));
+          if (!(cp.options & VT_O_NO_CAPSULE)) E = E * (ONE_POSE ? capsule_vis(caps, s.p, n) : capsule_vis(S, s.p, n));
+          L = L + E * INV_PI_F * albedo(S, s.mat, fmaxf(dot(n, wo), 0.0f));
+        }
+        const Mat M = load_mat(S, s.mat);
         const bool mis = !no_mis && (MODE == VT_SHADE_PATH || !is_static);
         const float sh0 = b == 1 ? u01(pcg(hs + 3u)) : bounce_shift(hs, b, 0);
         const float sh1 = b == 1 ? u01(pcg(hs + 4u)) : bounce_shift(hs, b, 1);
@@ -302,18 +312,7 @@ __global__ void __launch_bounds__(WAVE_THREADS, VT_WAVE_SHADE_BLOCKS) wave_shade
         // key bit 0x20000: a first-hit light sample needs its shadow ray (shade.wgsl.js:177, no shadow culling); with
         // the static-occlusion cache the shadow kernel decides it (a body blocks a sample, a penumbra, uneven samples)
         if (b == 1 && shadow && !cached) L4.w = __uint_as_float(__float_as_uint(L4.w) | 0x20000u);
-        bool bounce;
-        if (MODE == VT_SHADE_TWIN) {
-          bounce = !is_static;
-          if (is_static && !(cp.options & (VT_O_NO_INDIRECT | VT_O_DIRECT_ONLY))) {
-            float3 E = node_slot(S, s, 0u, ldu(S.su + 18));
-            if (!(cp.options & VT_O_NO_CAPSULE)) E = E * capsule_vis(S, s.p, n);
-            L = L + E * INV_PI_F * albedo(S, s.mat, fmaxf(dot(n, wo), 0.0f));
-          }
-        } else {
-          bounce = b < cp.max_depth;
-        }
-        if (bounce) {
+        if (MODE == VT_SHADE_TWIN ? !is_static : b < cp.max_depth) {
           const float3 ub = b == 1 ? f3(kr(i, KB0, u01(pcg(hs + 6u))), kr(i, KB1, u01(pcg(hs + 7u))), kr(i, KB2, u01(pcg(hs + 8u))))
                                    : f3(kr(i, KB0, bounce_shift(hs, b, 3)), kr(i, KB1, bounce_shift(hs, b, 4)), kr(i, KB2, bounce_shift(hs, b, 5)));
           float3 l;
