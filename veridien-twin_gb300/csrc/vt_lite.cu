@@ -114,16 +114,32 @@ __global__ void vertex_shadow_kernel(const Scene S, const Geo g, const View V, u
 }
 
 // ---------------------------------------------------------------------------------------------- fragment stage
-__device__ __forceinline__ uint32_t sm_less(const uint32_t* m, uint32_t res, uint32_t k, int x, int y, float dref) {
-  x = min(max(x, 0), int(res) - 1);
-  y = min(max(y, 0), int(res) - 1);
-  const uint32_t b = __ldg(m + (size_t(k) * res + y) * res + x);
-  return dref < (b == 0xffffffffu ? 1.0f : __uint_as_float(b)) ? 1u : 0u;
+// of the 4 x 4 texels from (x0, y0), clamped to the map: bit 4 j + i set where dref < depth. A texel is the bits of a
+// depth in [0, 1), or ~0u (empty: depth 1), so that dref's bits are compared; a negative dref lies before every depth.
+__device__ __forceinline__ uint32_t sm_less(const uint32_t* m, uint32_t res, int x0, int y0, float dref) {
+  if (dref < 0.0f) return 0xffffu;
+  const uint32_t r = __float_as_uint(dref + 0.0f);   // -0 as 0; a NaN's bits are above every depth's
+  uint32_t bits = 0;
+  if (x0 >= 0 && y0 >= 0 && x0 + 3 < int(res) && y0 + 3 < int(res)) {
+    const uint32_t* row = m + size_t(y0) * res + x0;
+#pragma unroll
+    for (int j = 0; j < 4; j++, row += res)
+#pragma unroll
+      for (int i = 0; i < 4; i++) bits |= r < min(__ldg(row + i), 0x3f800000u) ? 1u << (4 * j + i) : 0u;
+  } else {
+    for (int j = 0; j < 4; j++)
+      for (int i = 0; i < 4; i++) {
+        const int x = min(max(x0 + i, 0), int(res) - 1), y = min(max(y0 + j, 0), int(res) - 1);
+        bits |= r < min(__ldg(m + size_t(y) * res + x), 0x3f800000u) ? 1u << (4 * j + i) : 0u;
+      }
+  }
+  return bits;
 }
 // smVis (lite_nodes/renderer.js:267): 3x3 taps one texel apart of textureSampleCompareLevel ('less' comparison,
 // linear filtering, clamp to edge: the 2x2 texels around a tap compare dref < depth and blend bilinearly), min of
 // the static and dynamic maps per tap. The taps share the bilinear fraction of the centre tap (they sit exactly one
-// texel apart), so the 4x4 texels under them are compared once per map.
+// texel apart), so the 4x4 texels under them are compared once per map; where either map hides all of them, or both
+// none, the taps are known. Four 1280x720 views: shading 1.45 -> 1.36 ms.
 __device__ float sm_vis(const View& V, const ShadeArgs& a, float3 pw, uint32_t k, float bias) {
   const float3 q = sm_project(V, pw, k);
   if (fabsf(q.x) >= 1.0f || fabsf(q.y) >= 1.0f) return 1.0f;
@@ -134,27 +150,29 @@ __device__ float sm_vis(const View& V, const ShadeArgs& a, float3 pw, uint32_t k
   const float fx0 = floorf(tx), fy0 = floorf(ty);
   const float fx = tx - fx0, fy = ty - fy0;
   const int x0 = int(fx0) - 1, y0 = int(fy0) - 1;
-  uint32_t ms = 0, md = 0;
-#pragma unroll
-  for (int j = 0; j < 4; j++)
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-      ms |= sm_less(a.sm_static, a.sm_res, k, x0 + i, y0 + j, dref) << (4 * j + i);
-      md |= sm_less(a.sm_dyn, a.sm_res, k, x0 + i, y0 + j, dref) << (4 * j + i);
-    }
+  const size_t layer = size_t(k) * a.sm_res * a.sm_res;
+  const uint32_t ms = sm_less(a.sm_static + layer, a.sm_res, x0, y0, dref);
+  if (!ms) return 0.0f;
+  const uint32_t md = sm_less(a.sm_dyn + layer, a.sm_res, x0, y0, dref);
+  if (!md) return 0.0f;
   const float w00 = (1.0f - fx) * (1.0f - fy), w10 = fx * (1.0f - fy), w01 = (1.0f - fx) * fy, w11 = fx * fy;
   float s = 0.0f;
+  if ((ms & md) == 0xffffu) {   // all taps alike
+    const float c = w00 + w10 + w01 + w11;
 #pragma unroll
-  for (int j = 0; j < 3; j++)
+    for (int i = 0; i < 9; i++) s = s + c;
+  } else {
 #pragma unroll
-    for (int i = 0; i < 3; i++) {
-      const int b = 4 * j + i;
-      const float cs = w00 * float((ms >> b) & 1u) + w10 * float((ms >> (b + 1)) & 1u) + w01 * float((ms >> (b + 4)) & 1u) +
-                       w11 * float((ms >> (b + 5)) & 1u);
-      const float cd = w00 * float((md >> b) & 1u) + w10 * float((md >> (b + 1)) & 1u) + w01 * float((md >> (b + 4)) & 1u) +
-                       w11 * float((md >> (b + 5)) & 1u);
-      s = s + fminf(cs, cd);
-    }
+    for (int j = 0; j < 3; j++)
+#pragma unroll
+      for (int i = 0; i < 3; i++) {
+        const int b = 4 * j + i;
+        auto tap = [&](uint32_t m) {
+          return ((m >> b) & 1u ? w00 : 0.0f) + ((m >> (b + 1)) & 1u ? w10 : 0.0f) + ((m >> (b + 4)) & 1u ? w01 : 0.0f) + ((m >> (b + 5)) & 1u ? w11 : 0.0f);
+        };
+        s = s + fminf(tap(ms), tap(md));
+      }
+  }
   return s / 9.0f;
 }
 
@@ -197,7 +215,7 @@ __device__ __forceinline__ float3 eval_bsdf_v(const Mat& M, const BsdfView& B, f
 }
 
 // fsCam (lite_nodes/renderer.js:284) for triangle `tri` at the centre of pixel (px, py); radiance x outScale
-__device__ float3 fragment(const Scene& S, const Geo& g, const View& V, const ShadeArgs& a, uint32_t tri, uint32_t px, uint32_t py) {
+__device__ float3 fragment(const Scene& S, const Geo& g, const View& V, const ShadeArgs& a, const Capsules& caps, uint32_t tri, uint32_t px, uint32_t py) {
   uint4 va[3], vb[3];
   float4 c[3];
   for (int j = 0; j < 3; j++) {
@@ -299,7 +317,7 @@ __device__ float3 fragment(const Scene& S, const Geo& g, const View& V, const Sh
   if (is_static) {
     float3 E = f3(0.0f, 0.0f, 0.0f);
     if (ew.w > 1e-6f) E = f3(ew.x, ew.y, ew.z) / ew.w;
-    E = E * capsule_vis(S, p, ns);
+    E = E * capsule_vis(caps, p, ns);
     L = L + E * INV_PI_F * Al;
   } else {
     L = L + v3(V.env) * Al;
@@ -368,10 +386,12 @@ __global__ void __launch_bounds__(128, VT_SHADE_BLOCKS) shade_frag_kernel(const 
                                                          uint32_t cap, const uint32_t* __restrict__ counts, uint2* __restrict__ colors) {
   const uint32_t ns = counts[0], nd = counts[1];
   const uint32_t W = uint32_t(V.size[0]);
+  __shared__ Capsules caps;
+  load_capsules(S, caps);
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < ns + nd; i += gridDim.x * blockDim.x) {
-    const uint32_t fi = i < ns ? i : cap - nd + (i - ns);
+    const uint32_t fi = i < nd ? cap - nd + i : i - nd;   // the longer ones first
     const uint2 fr = frags[fi];
-    const float3 c = fragment(S, g, V, a, fr.y, fr.x % W, fr.x / W);
+    const float3 c = fragment(S, g, V, a, caps, fr.y, fr.x % W, fr.x / W);
     const __half2 rg = __floats2half2_rn(c.x, c.y), bz = __floats2half2_rn(c.z, 0.0f);
     colors[fi] = make_uint2(*reinterpret_cast<const uint32_t*>(&rg), *reinterpret_cast<const uint32_t*>(&bz));
   }
