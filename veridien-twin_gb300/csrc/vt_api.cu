@@ -777,30 +777,14 @@ vt_status vt_timings_get(const vt_ctx* ctx, vt_timings* out) {
 //   r = E + rho F B - B            F = F_hi + F_lo and B = B_hi + B_lo in bf16, three tcgen05 products, FP64 epilogue
 //   d <- r + rho F_lp d            BF16 or FP8 (per-row / per-column scales) sweeps until the update stalls
 //   B <- B + d
-// Splits of K are chosen so the grid of 128-row tiles x splits fills whole waves of the SMs.
-namespace {
-uint32_t choose_splits(uint32_t mtiles, uint32_t ktiles, int sms) {
-  uint32_t best = 1;
-  double best_eff = 0;
-  for (uint32_t s = 1; s <= 8 && s <= ktiles; s++) {
-    const double ctas = double(mtiles) * s, waves = std::ceil(ctas / sms);
-    const double eff = ctas / (waves * sms);
-    if (eff > best_eff + 0.02) { best_eff = eff; best = s; }
-  }
-  return best;
-}
-}  // namespace
-
 static vt_status tc_solve(vt_ctx* ctx, vt_solve_req* q) {
   const uint32_t n = q->n, R = q->n_rhs;
   if (n % 16) return fail(ctx, VT_ERR_ARG, "solve: BF16/FP8 need n % 16 == 0");
   const bool fp8 = q->precision == VT_PREC_FP8;
   int sms = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
-  const uint32_t mtiles = (n + 127) / 128;
-  const uint32_t kt_bf = (n + 63) / 64, kt_q = (n + 127) / 128;
-  const uint32_t sp_bf = choose_splits(mtiles, kt_bf, sms), sp_q = choose_splits(mtiles, kt_q, sms);
-  const uint32_t sp_max = std::max(sp_bf, sp_q);
+  const uint32_t c_bf = vtk::tc_ctas(vtk::TC_BF16, n, sms), c_q = vtk::tc_ctas(vtk::TC_FP8, n, sms);
+  const uint32_t segs = std::max(vtk::tc_segments(vtk::TC_BF16, n, c_bf), vtk::tc_segments(vtk::TC_FP8, n, c_q));
   const size_t nn = size_t(n) * n, nr = size_t(n) * R;
   const bool dF = is_device_ptr(q->F);
   // layout of the context's mixed-precision block (each piece 256-byte aligned)
@@ -808,9 +792,9 @@ static vt_status tc_solve(vt_ctx* ctx, vt_solve_req* q) {
   auto place = [&](size_t bytes) { const size_t o = off; off += (bytes + 255) / 256 * 256; return o; };
   const size_t o_f32 = dF ? 0 : place(nn * 4), o_hi = place(nn * 2), o_lo = place(nn * 2), o_q = fp8 ? place(nn) : 0;
   const size_t o_rs = place(size_t(n) * 4), o_bhi = place(size_t(64) * n * 2), o_blo = place(size_t(64) * n * 2),
-               o_bq = place(size_t(64) * n), o_cs = place(256), o_cm = place(256), o_part = place(size_t(sp_max) * n * 64 * 4),
+               o_bq = place(size_t(64) * n), o_cs = place(256), o_cm = place(256), o_part = place(size_t(segs) * n * 64 * 4),
                o_E = place(nr * 4), o_rho = place(size_t(n) * 4), o_B = place(nr * 4), o_r = place(nr * 4), o_d = place(nr * 4),
-               o_d2 = place(nr * 4), o_np = place((nr / 256 + 2) * 16), o_err = place(64);
+               o_d2 = place(nr * 4), o_np = place((size_t(n) / 32 + 2) * 16), o_err = place(64);
   auto& T = ctx->tc;
   const bool same_f = q->reuse_f && T.f_src == q->F && T.n == n && T.mem;
   if (T.bytes < off) {
@@ -882,8 +866,8 @@ static vt_status tc_solve(vt_ctx* ctx, vt_solve_req* q) {
   for (;;) {
     // accurate residual of the current iterate
     vtk::tc_pack_b(vtk::TC_BF16X3, B, n, R, Bhi, Blo, nullptr, nullptr, nullptr, ctx->stream);
-    vtk::tc_gemm(vtk::TC_BF16X3, &mhi, &mlo, &mbhi, &mblo, n, sp_bf, (kt_bf + sp_bf - 1) / sp_bf, part, err, ctx->stream);
-    vtk::tc_combine_residual(part, sp_bf, n, R, rho, E, B, r, np, &npart, ctx->stream);
+    vtk::tc_gemm(vtk::TC_BF16X3, &mhi, &mlo, &mbhi, &mblo, n, R, c_bf, part, err, ctx->stream);
+    npart = vtk::tc_combine_residual(part, c_bf, n, R, rho, E, B, r, fp8 ? nullptr : Bhi, np, ctx->stream);
     ctx->tim.launches += 3;
     double h[2];
     if ((s = read_norms(h)) != VT_OK) return s;
@@ -893,7 +877,7 @@ static vt_status tc_solve(vt_ctx* ctx, vt_solve_req* q) {
     // correction: (I - diag(rho) F_lp) d = r by Jacobi sweeps from d = r, to the accuracy the next residual needs to
     // fall under tol with a margin of 4 (an inexact correction), never finer than the low precision's floor
     const double inner_goal = std::min(0.1, std::max(inner_tol, 0.25 * q->tol / resid));
-    VT_CK(cudaMemcpyAsync(d, r, nr * 4, cudaMemcpyDeviceToDevice, ctx->stream));
+    const float* x = r;
     // The sweeps' relative change falls geometrically. Each host check costs a stream synchronisation, about as
     // much as a sweep at small n, so the observed rate (from two checked sweeps, or the previous correction's)
     // predicts how many more sweeps reach the goal; they run back to back and one check follows (then one per
@@ -902,19 +886,19 @@ static vt_status tc_solve(vt_ctx* ctx, vt_solve_req* q) {
     double c_prev = -1.0;
     for (uint32_t k = 0; k < inner_max && sweeps < max_it; k++) {
       if (fp8) {
-        vtk::tc_pack_b(vtk::TC_FP8, d, n, R, nullptr, nullptr, Bq, cs, cm, ctx->stream);
+        vtk::tc_pack_b(vtk::TC_FP8, x, n, R, nullptr, nullptr, Bq, cs, cm, ctx->stream);
         VT_CK(cudaEventRecord(ctx->ev2, ctx->stream));
-        vtk::tc_gemm(vtk::TC_FP8, &mq, nullptr, &mbq, nullptr, n, sp_q, (kt_q + sp_q - 1) / sp_q, part, err, ctx->stream);
+        vtk::tc_gemm(vtk::TC_FP8, &mq, nullptr, &mbq, nullptr, n, R, c_q, part, err, ctx->stream);
         VT_CK(cudaEventRecord(ctx->ev3, ctx->stream));
-        vtk::tc_combine_sweep(part, sp_q, n, R, rho, r, d, d2, rs, cs, np, &npart, ctx->stream);
-      } else {
-        vtk::tc_pack_b(vtk::TC_BF16, d, n, R, Bhi, nullptr, nullptr, nullptr, nullptr, ctx->stream);
+        npart = vtk::tc_combine_sweep(vtk::TC_FP8, part, c_q, n, R, rho, r, x, d, rs, cs, nullptr, np, ctx->stream);
+      } else {   // x's columns are in Bhi: the kernel that made x put them there
         VT_CK(cudaEventRecord(ctx->ev2, ctx->stream));
-        vtk::tc_gemm(vtk::TC_BF16, &mhi, nullptr, &mbhi, nullptr, n, sp_bf, (kt_bf + sp_bf - 1) / sp_bf, part, err, ctx->stream);
+        vtk::tc_gemm(vtk::TC_BF16, &mhi, nullptr, &mbhi, nullptr, n, R, c_bf, part, err, ctx->stream);
         VT_CK(cudaEventRecord(ctx->ev3, ctx->stream));
-        vtk::tc_combine_sweep(part, sp_bf, n, R, rho, r, d, d2, nullptr, nullptr, np, &npart, ctx->stream);
+        npart = vtk::tc_combine_sweep(vtk::TC_BF16, part, c_bf, n, R, rho, r, x, d, nullptr, nullptr, Bhi, np, ctx->stream);
       }
-      ctx->tim.launches += 3;
+      ctx->tim.launches += fp8 ? 3 : 2;
+      x = d;
       std::swap(d, d2);
       sweeps++;
       if (++in_batch < batch && k + 1 < inner_max && sweeps < max_it) continue;
@@ -934,7 +918,7 @@ static vt_status tc_solve(vt_ctx* ctx, vt_solve_req* q) {
       k_prev = k + 1;
       in_batch = 0;
     }
-    vtk::tc_axpy(B, d, nr, ctx->stream);
+    vtk::tc_axpy(B, x, nr, ctx->stream);
   }
   VT_CK(cudaEventRecord(ctx->ev1, ctx->stream));
   uint32_t herr = 0;

@@ -1,10 +1,10 @@
 // Multi-right-hand-side node radiosity sweeps on the 5th-generation tensor cores (tcgen05) of sm_103a.
 //
-// tc_gemm_kernel: one CTA computes a 128-row x 64-column FP32 accumulator in tensor memory (TMEM) over one split of
-// the K range. Warp 0 lane 0 feeds a ring of shared-memory stages with TMA (cp.async.bulk.tensor, 128-byte
-// swizzle; a stage is 128 rows x 128 B of F and 64 rows x 128 B of the transposed right-hand sides Bt), warp 1
-// lane 0 issues tcgen05.mma (M = 128, N = 64, K = 16 bf16 / 32 e4m3 per instruction) and releases each stage with
-// tcgen05.commit, and all four warps read the accumulator back with tcgen05.ld into per-split partial sums. The
+// tc_gemm_kernel: one CTA per SM takes a run of the (128 rows, 128 bytes of K) tiles of F. One warp feeds a ring of
+// shared-memory stages with TMA (cp.async.bulk.tensor, 128-byte swizzle; a stage is 128 rows x 128 B of F and 64 rows x 128 B
+// of the transposed right-hand sides Bt), one issues tcgen05.mma (M = 128, N = 64, K = 16 bf16 / 32 e4m3 per instruction)
+// into two accumulators in tensor memory (TMEM) in turn and releases each stage with tcgen05.commit, and four read the
+// accumulators back with tcgen05.ld and sum them in registers, into a partial per row tile that the run meets. The
 // combine kernels (CUDA cores, HBM-bound and small) apply the Jacobi epilogue or the accurate residual in FP64.
 //
 // The sweep streams F once: 2 B per element in BF16, 1 B in FP8, so it is HBM-bound (64 flop/B at 64 right-hand
@@ -26,7 +26,6 @@ namespace vtk {
 
 namespace {
 
-constexpr int TC_THREADS = 128;
 constexpr uint32_t A_BYTES = 128 * 128;   // 128 rows x 128 B
 constexpr uint32_t B_BYTES = 64 * 128;    // 64 rows x 128 B
 using namespace async;
@@ -82,40 +81,71 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
   for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
 }
 
+__device__ __forceinline__ bool elect_one() {
+  uint32_t r;
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(r));
+  return r != 0u;
+}
+// two floats' bf16 parts, packed (the first in the low half); x becomes the remainder
+__device__ __forceinline__ uint32_t take_bf16x2(float& x0, float& x1) {
+  uint32_t w;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(w) : "f"(x1), "f"(x0));
+  x0 -= __uint_as_float(w << 16);
+  x1 -= __uint_as_float(w & 0xffff0000u);
+  return w;
+}
+
+// One CTA per SM takes an equal run of the (row tile, K stage) pairs in tile order, across tiles without a break in the
+// pipeline (a CTA's start and end cost ~5 us); a tile's sum is then that of the few CTAs whose runs meet it, each in a
+// partial of its own. Stage g belongs to CTA run_cta(g).
+__host__ __device__ inline uint32_t run_cta(uint64_t g, uint64_t total, uint32_t ctas) { return uint32_t(((g + 1u) * ctas - 1u) / total); }
+// the CTAs whose runs meet row tile `tile` of KT stages
+__device__ __forceinline__ uint32_t run_segments(uint32_t tile, uint32_t KT, uint32_t n, uint32_t ctas) {
+  const uint64_t total = uint64_t((n + 127u) / 128u) * KT, g = uint64_t(tile) * KT;
+  return run_cta(g + KT - 1u, total, ctas) - run_cta(g, total, ctas) + 1u;
+}
+
+// Bound: F from HBM. n = 32768, 64 columns: 323 us a BF16 sweep, 2.1 GB of F at 0.98 of the measured copy rate, and 640 us the accurate
+// product's 4.3 GB (0.99); 361 and 660 by a CTA per row tile and quarter of K, whose starts and ends lay bare.
+//
+// The accumulation of the tensor cores drops what lies below the accumulator's last bit: an accumulator takes TC_CHAIN stages
+// at most, the rest of a row's sum is in FP32 registers, rounded to nearest.
+constexpr uint32_t TC_CHAIN = 2;
+constexpr int TC_THREADS = 192;   // warps 0-3 drain, 4 TMA, 5 MMA
+
 template <int MODE, int STAGES>
 __global__ void __launch_bounds__(TC_THREADS, 1)
     tc_gemm_kernel(const __grid_constant__ TcMap mA, const __grid_constant__ TcMap mA2, const __grid_constant__ TcMap mB,
-                   const __grid_constant__ TcMap mB2, uint32_t n, uint32_t k_tiles, float* __restrict__ partials, uint32_t* err) {
+                   const __grid_constant__ TcMap mB2, uint32_t n, uint32_t R, float* __restrict__ partials, uint32_t* err) {
   constexpr bool X3 = MODE == TC_BF16X3;
   constexpr uint32_t STAGE_BYTES = (X3 ? 2 : 1) * (A_BYTES + B_BYTES);
   constexpr uint32_t K_ELEMS = MODE == TC_FP8 ? 128 : 64;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);   // full[STAGES], empty[STAGES], done
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 1);
-  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-  const uint32_t m0 = blockIdx.x * 128u;
-  const uint32_t split = blockIdx.y;
-  const uint32_t total_kt = (n + K_ELEMS - 1) / K_ELEMS;
-  const uint32_t kt0 = split * k_tiles;
-  const uint32_t kt1 = min(total_kt, kt0 + k_tiles);
-  const uint32_t nkt = kt1 > kt0 ? kt1 - kt0 : 0u;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
+  // full[s]: a stage's tiles landed; empty[s]: its MMAs are done; ready[b]: accumulator b's MMAs are done; read[b]: it is
+  // read back; fin: the last MMA is done
   auto full = [&](uint32_t s) { return smem_u32(bars + s); };
   auto empty = [&](uint32_t s) { return smem_u32(bars + STAGES + s); };
-  const uint32_t done = smem_u32(bars + 2 * STAGES);
-  auto sA = [&](uint32_t s) { return smem_u32(smem + s * STAGE_BYTES); };
-  auto sA2 = [&](uint32_t s) { return smem_u32(smem + s * STAGE_BYTES + A_BYTES); };
-  auto sB = [&](uint32_t s) { return smem_u32(smem + s * STAGE_BYTES + (X3 ? 2 : 1) * A_BYTES); };
-  auto sB2 = [&](uint32_t s) { return smem_u32(smem + s * STAGE_BYTES + 2 * A_BYTES + B_BYTES); };
+  auto ready = [&](uint32_t b) { return smem_u32(bars + 2 * STAGES + b); };
+  auto read = [&](uint32_t b) { return smem_u32(bars + 2 * STAGES + 2 + b); };
+  const uint32_t fin = smem_u32(bars + 2 * STAGES + 4);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 5);
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+  const uint32_t KT = (n + K_ELEMS - 1u) / K_ELEMS;
+  const uint64_t total = uint64_t((n + 127u) / 128u) * KT;
+  const uint64_t g0 = uint64_t(blockIdx.x) * total / gridDim.x;
+  const uint32_t nkt = uint32_t((uint64_t(blockIdx.x) + 1u) * total / gridDim.x - g0);
+  uint32_t tile = uint32_t(g0 / KT), kk = uint32_t(g0 % KT);   // of the role's next stage
 
   if (threadIdx.x == 0) {
     for (uint32_t s = 0; s < STAGES; s++) { mbar_init(full(s), 1); mbar_init(empty(s), 1); }
-    mbar_init(done, 1);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    for (uint32_t b = 0; b < 2; b++) { mbar_init(ready(b), 1); mbar_init(read(b), 4); }
+    mbar_init(fin, 1);
+    mbar_fence_init();
   }
-  if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 64;" ::"r"(smem_u32(tmem_slot)) : "memory");
+  if (warp == 5) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 128;" ::"r"(smem_u32(tmem_slot)) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   tc_fence_before();
@@ -123,79 +153,115 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
 
-  if (warp == 0 && lane == 0) {
-    // TMA producer
-    uint32_t issued = 0;
-    for (uint32_t kt = 0; kt < nkt; kt++) {
-      const uint32_t s = kt % STAGES;
-      if (kt >= STAGES && !mbar_wait(empty(s), ((kt / STAGES) & 1u) ^ 1u, err)) break;
-      mbar_expect_tx(full(s), STAGE_BYTES);
-      const int32_t kx = int32_t((kt0 + kt) * K_ELEMS);
-      tma_load_2d(sA(s), &mA, kx, int32_t(m0), full(s));
-      if (X3) tma_load_2d(sA2(s), &mA2, kx, int32_t(m0), full(s));
-      tma_load_2d(sB(s), &mB, kx, 0, full(s));
-      if (X3) tma_load_2d(sB2(s), &mB2, kx, 0, full(s));
-      issued++;
-    }
-    // drain: every stage this thread filled must have landed before the CTA may exit
-    for (uint32_t kt = issued > STAGES ? issued - STAGES : 0; kt < issued; kt++) mbar_wait(full(kt % STAGES), (kt / STAGES) & 1u, err);
-  } else if (warp == 1 && lane == 0) {
-    // MMA issuer
-    bool ok = true;
-    for (uint32_t kt = 0; kt < nkt && ok; kt++) {
-      const uint32_t s = kt % STAGES;
-      ok = mbar_wait(full(s), (kt / STAGES) & 1u, err);
-      if (!ok) break;
-      tc_fence_after();
-#pragma unroll
-      for (uint32_t k = 0; k < 4; k++) {   // 4 MMAs of 32 bytes of K each
-        const uint64_t a = sw128_desc(sA(s) + 32 * k), b = sw128_desc(sB(s) + 32 * k);
-        mma<MODE>(tmem, a, b, (kt | k) != 0u);
-        if (X3) {
-          mma<MODE>(tmem, a, sw128_desc(sB2(s) + 32 * k), 1u);
-          mma<MODE>(tmem, sw128_desc(sA2(s) + 32 * k), b, 1u);
-        }
+  if (warp == 4) {
+    if (lane == 0) {
+      uint32_t issued = 0;
+      for (uint32_t kt = 0; kt < nkt; kt++) {
+        const uint32_t s = kt % STAGES;
+        if (kt >= STAGES && !mbar_wait(empty(s), ((kt / STAGES) & 1u) ^ 1u, err)) break;
+        mbar_expect_tx(full(s), STAGE_BYTES);
+        const int32_t kx = int32_t(kk * K_ELEMS), m0 = int32_t(tile * 128u);
+        const uint32_t at = smem_u32(smem + s * STAGE_BYTES), bt = at + (X3 ? 2 : 1) * A_BYTES;
+        tma_load_2d(at, &mA, kx, m0, full(s));
+        if (X3) tma_load_2d(at + A_BYTES, &mA2, kx, m0, full(s));
+        tma_load_2d(bt, &mB, kx, 0, full(s));
+        if (X3) tma_load_2d(bt + B_BYTES, &mB2, kx, 0, full(s));
+        if (++kk == KT) { kk = 0; tile++; }
+        issued++;
       }
-      mma_commit(empty(s));
+      // drain: every stage this thread filled must have landed before the CTA may exit
+      for (uint32_t kt = issued > STAGES ? issued - STAGES : 0; kt < issued; kt++) mbar_wait(full(kt % STAGES), (kt / STAGES) & 1u, err);
     }
-    if (nkt > 0 && ok) mma_commit(done);
-    else mbar_arrive(done);
-  }
-  __syncwarp();
-  // epilogue: warp w reads accumulator rows 32 w .. 32 w + 31 (TMEM lanes), 64 columns
-  const bool have = mbar_wait(done, 0, err) && nkt > 0;
-  __syncwarp();   // tcgen05.ld is warp-collective
-  tc_fence_after();
-  float v[64];
+  } else if (warp == 5) {
+    // The whole warp runs the loop, so that the descriptors stay in uniform registers, and one elected lane issues
+    const bool el = elect_one();
+    const uint64_t A0 = sw128_desc(smem_u32(smem)), B0 = sw128_desc(smem_u32(smem + (X3 ? 2 : 1) * A_BYTES));
+    uint32_t chain = 0;   // accumulators begun before this one
+    for (uint32_t kt = 0; kt < nkt; kt++) {
+      const uint32_t s = kt % STAGES, b = chain & 1u;
+      const bool first = kt == 0u || kk % TC_CHAIN == 0u;
+      bool ok = mbar_wait(full(s), (kt / STAGES) & 1u, err);
+      if (first && chain >= 2u) ok = ok && mbar_wait(read(b), ((chain >> 1) - 1u) & 1u, err);
+      if (++kk == KT) kk = 0;
+      const bool last = kk % TC_CHAIN == 0u || kt + 1u == nkt;
+      if (!__all_sync(0xffffffffu, ok)) break;
+      tc_fence_after();
+      const uint64_t A = A0 + ((s * STAGE_BYTES) >> 4), B = B0 + ((s * STAGE_BYTES) >> 4);
+      const uint32_t d = tmem + 64u * b;
+      if (el) {
 #pragma unroll
-  for (int c = 0; c < 4; c++) tmem_ld16(tmem + ((warp * 32u) << 16) + 16u * c, v + 16 * c);
-  const uint32_t row = m0 + warp * 32u + lane;
-  if (row < n) {
-    float4* dst = reinterpret_cast<float4*>(partials + (size_t(split) * n + row) * 64);
+        for (uint32_t k = 0; k < 4; k++) {   // 32 bytes of K each
+          mma<MODE>(d, A + 2 * k, B + 2 * k, k || !first);
+          if (X3) {
+            mma<MODE>(d, A + 2 * k, B + (B_BYTES >> 4) + 2 * k, 1u);
+            mma<MODE>(d, A + (A_BYTES >> 4) + 2 * k, B + 2 * k, 1u);
+          }
+        }
+        mma_commit(empty(s));
+        if (last) mma_commit(ready(b));
+      }
+      __syncwarp();
+      if (last) chain++;
+    }
+    if (el) mma_commit(fin);
+    mbar_wait(fin, 0, err);   // no MMA in flight when the TMEM is given back
+  } else {
+    // warp w reads accumulator rows 32 w .. 32 w + 31 (TMEM lanes)
+    float acc[64];
 #pragma unroll
-    for (int c = 0; c < 16; c++)
-      dst[c] = have ? make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]) : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int c = 0; c < 64; c++) acc[c] = 0.0f;
+    uint32_t chain = 0;
+    for (uint32_t kt = 0; kt < nkt; kt++) {
+      const bool end = ++kk == KT || kt + 1u == nkt;
+      if (!end && kk % TC_CHAIN) continue;
+      const uint32_t b = chain & 1u;
+      if (!__all_sync(0xffffffffu, mbar_wait(ready(b), (chain >> 1) & 1u, err))) break;
+      tc_fence_after();
+      chain++;
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        float v[16];
+        tmem_ld16(tmem + ((warp * 32u) << 16) + 64u * b + 16u * q, v);
+#pragma unroll
+        for (int c = 0; c < 16; c++) acc[16 * q + c] += v[c];
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(read(b));
+      if (!end) continue;
+      // the tile's end, or the run's: this CTA's partial of it
+      const uint32_t row = tile * 128u + warp * 32u + lane, seg = blockIdx.x - run_cta(uint64_t(tile) * KT, total, gridDim.x);
+      if (row < n) {
+        float4* dst = reinterpret_cast<float4*>(partials + (size_t(seg) * n + row) * 64);
+#pragma unroll
+        for (int c = 0; c < 16; c++)
+          if (4u * c < R) dst[c] = make_float4(acc[4 * c], acc[4 * c + 1], acc[4 * c + 2], acc[4 * c + 3]);
+      }
+#pragma unroll
+      for (int c = 0; c < 64; c++) acc[c] = 0.0f;
+      kk = 0;
+      tile++;
+    }
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 64;" ::"r"(tmem) : "memory");
+  if (warp == 5) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 128;" ::"r"(tmem) : "memory");
 }
 
 template <int MODE, int STAGES>
 constexpr size_t smem_bytes() {
-  return size_t(STAGES) * (MODE == TC_BF16X3 ? 2 : 1) * (A_BYTES + B_BYTES) + 1024 + 8 * (2 * STAGES + 1) + 16;
+  return size_t(STAGES) * (MODE == TC_BF16X3 ? 2 : 1) * (A_BYTES + B_BYTES) + 1024 + 8 * (2 * STAGES + 5) + 16;
 }
 
 template <int MODE, int STAGES>
-void launch_gemm(const TcMap* A, const TcMap* A2, const TcMap* B, const TcMap* B2, uint32_t n, uint32_t splits, uint32_t k_tiles,
-                 float* partials, uint32_t* err, cudaStream_t st) {
-  static std::once_flag once;
-  std::call_once(once, [] {
+void launch_gemm(const TcMap* A, const TcMap* A2, const TcMap* B, const TcMap* B2, uint32_t n, uint32_t R, uint32_t ctas, float* partials,
+                 uint32_t* err, cudaStream_t st) {
+  static std::atomic<int> set[MAX_DEVICES];
+  per_device_value(set, [](int) {
     cudaFuncSetAttribute(tc_gemm_kernel<MODE, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem_bytes<MODE, STAGES>()));
+    return 1;
   });
-  const dim3 grid((n + 127) / 128, splits);
-  tc_gemm_kernel<MODE, STAGES><<<grid, TC_THREADS, smem_bytes<MODE, STAGES>(), st>>>(*A, A2 ? *A2 : *A, *B, B2 ? *B2 : *B, n, k_tiles,
-                                                                                    partials, err);
+  tc_gemm_kernel<MODE, STAGES><<<ctas, TC_THREADS, smem_bytes<MODE, STAGES>(), st>>>(*A, A2 ? *A2 : *A, *B, B2 ? *B2 : *B, n, R, partials, err);
 }
 
 // ------------------------------------------------------------------------------------------------ FP32 sweeps
@@ -235,11 +301,6 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
       "r"(r[14]), "r"(r[15])
       : "memory");
 }
-__device__ __forceinline__ bool elect_one() {
-  uint32_t r;
-  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(r));
-  return r != 0u;
-}
 // 16 columns of two neighbouring accumulators of 64
 __device__ __forceinline__ void tmem_ld16x2(uint32_t taddr, float* v) {
   uint32_t r[32];
@@ -256,20 +317,6 @@ __device__ __forceinline__ void tmem_ld16x2(uint32_t taddr, float* v) {
 #pragma unroll
   for (int i = 0; i < 32; i++) v[i] = __uint_as_float(r[i]);
 }
-// two floats' bf16 parts, packed (the first in the low half); x becomes the remainder
-__device__ __forceinline__ uint32_t take_bf16x2(float& x0, float& x1) {
-  uint32_t w;
-  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(w) : "f"(x1), "f"(x0));
-  x0 -= __uint_as_float(w << 16);
-  x1 -= __uint_as_float(w & 0xffff0000u);
-  return w;
-}
-
-// One CTA per SM takes an equal run of the (row tile, K stage) pairs in tile order, across tiles without a break in the
-// pipeline (a CTA's start and end cost ~5 us); a tile's sum is then that of the few CTAs whose runs meet it, each in a
-// partial of its own. Stage g belongs to CTA fx_cta(g).
-__host__ __device__ inline uint32_t fx_cta(uint64_t g, uint64_t total, uint32_t ctas) { return uint32_t(((g + 1u) * ctas - 1u) / total); }
-
 __global__ void __launch_bounds__(FX_THREADS, 1)
     tc_gemm_f32_kernel(const __grid_constant__ TcMap mF, const __grid_constant__ TcMap mB, uint32_t n, uint32_t R, float* __restrict__ partials,
                        uint32_t* err) {
@@ -424,7 +471,7 @@ __global__ void __launch_bounds__(FX_THREADS, 1)
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(rest);
-      const uint32_t row = tile * 128u + warp * 32u + lane, seg = blockIdx.x - fx_cta(uint64_t(tile) * KT, total, gridDim.x);
+      const uint32_t row = tile * 128u + warp * 32u + lane, seg = blockIdx.x - run_cta(uint64_t(tile) * KT, total, gridDim.x);
       if (row < n) {
         float4* dst = reinterpret_cast<float4*>(partials + (size_t(seg) * n + row) * R);
 #pragma unroll
@@ -485,10 +532,7 @@ __global__ void __launch_bounds__(256) combine_f32_kernel(const float* __restric
   const uint32_t i0 = blockIdx.x * 32u, R4 = R / 4u;
   const size_t stride = size_t(n) * R4;
   const float4* P = reinterpret_cast<const float4*>(part);
-  // the CTAs whose runs meet this tile of 128 rows
-  const uint32_t KT = (n + 63u) / 64u;
-  const uint64_t total = uint64_t((n + 127u) / 128u) * KT, g = uint64_t(i0 / 128u) * KT;
-  const uint32_t splits = i0 < n ? fx_cta(g + KT - 1u, total, ctas) - fx_cta(g, total, ctas) + 1u : 0u;
+  const uint32_t splits = i0 < n ? run_segments(i0 / 128u, (n + 63u) / 64u, n, ctas) : 0u;
   double d2 = 0.0, b2 = 0.0;
   for (uint32_t q = threadIdx.x; q < 32u * R4; q += 256u) {
     const uint32_t r = q / R4, c = 4u * (q % R4);
@@ -592,7 +636,7 @@ __global__ void pack_b_kernel(const float* __restrict__ X, uint32_t n, uint32_t 
     } else {
       const __nv_bfloat16 h = __float2bfloat16_rn(x);
       hi[o] = h;
-      if (MODE == TC_BF16X3) lo[o] = __float2bfloat16_rn(x - __bfloat162float(h));
+      lo[o] = __float2bfloat16_rn(x - __bfloat162float(h));
     }
   }
 }
@@ -614,43 +658,90 @@ __device__ __forceinline__ void block_sum2f(float a, float b, double* partials) 
   }
 }
 
-// thread per (row, column < R); splits summed in order s = 0, 1, ... (deterministic)
-__global__ void __launch_bounds__(CB_THREADS) combine_sweep_kernel(const float* __restrict__ P, uint32_t splits, uint32_t n, uint32_t R,
+// a block's 32 rows of the iterate, in shared memory, to the next sweep's right-hand sides in BF16 (c < R; the other rows of
+// Bt stay zero): two neighbours of K a store (n is a multiple of 16)
+__device__ __forceinline__ void store_hi(const float (*tile)[65], uint32_t i0, uint32_t n, uint32_t R, uint16_t* __restrict__ Bt) {
+  for (uint32_t q = threadIdx.x; q < R * 16u; q += CB_THREADS) {
+    const uint32_t c = q / 16u, k = 2u * (q % 16u);
+    if (i0 + k >= n) continue;
+    float x0 = tile[k][c], x1 = tile[k + 1u][c];
+    *reinterpret_cast<uint32_t*>(Bt + size_t(c) * n + i0 + k) = take_bf16x2(x0, x1);
+  }
+}
+
+// Y = rhs + rho (sum of the row tile's partials, in CTA order), 32 rows a block; Bt: also the next sweep's right-hand sides
+// (null: none). Norms of Y - Xin and Y in FP32 per thread. W: columns a thread takes at a time, 4 where R is a multiple (n =
+// 32768, 64 columns: 12 us, 20 a column at a time; with a pack launch of its own 35)
+template <int W>
+__global__ void __launch_bounds__(CB_THREADS) combine_sweep_kernel(const float* __restrict__ P, uint32_t ctas, uint32_t KT, uint32_t n, uint32_t R,
                                                                    const float* __restrict__ rho, const float* __restrict__ rhs,
                                                                    const float* __restrict__ Xin, float* __restrict__ Y,
                                                                    const float* __restrict__ rs, const float* __restrict__ cs,
-                                                                   double* __restrict__ parts) {
-  const size_t idx = size_t(blockIdx.x) * CB_THREADS + threadIdx.x;
+                                                                   uint16_t* __restrict__ Bt, double* __restrict__ parts) {
+  __shared__ float tile[32][65];
+  const uint32_t i0 = blockIdx.x * 32u, rows = min(32u, n - i0), RW = R / W, segs = run_segments(i0 / 128u, KT, n, ctas);
+  auto load = [](const float* p, float* v) {
+    if (W == 4) {
+      const float4 x = *reinterpret_cast<const float4*>(p);
+      v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+    } else {
+      v[0] = *p;
+    }
+  };
   float d2 = 0.0f, y2 = 0.0f;
-  if (idx < size_t(n) * R) {
-    const uint32_t i = uint32_t(idx / R), c = uint32_t(idx % R);
-    float acc = 0.0f;
-    for (uint32_t s = 0; s < splits; s++) acc += P[(size_t(s) * n + i) * 64 + c];
-    if (rs) acc *= rs[i] * cs[c];
-    const float y = fmaf(rho[i], acc, rhs[idx]);
-    Y[idx] = y;
-    const float dd = y - Xin[idx];
-    d2 = dd * dd;
-    y2 = y * y;
+#pragma unroll 2
+  for (uint32_t q = threadIdx.x; q < rows * RW; q += CB_THREADS) {
+    const uint32_t r = q / RW, c = W * (q % RW), i = i0 + r;
+    const size_t idx = size_t(i) * R + c;
+    float acc[W], v[W], e[W], x[W];
+    load(rhs + idx, e);
+    load(Xin + idx, x);
+    load(P + size_t(i) * 64 + c, acc);
+    for (uint32_t s = 1; s < segs; s++) {
+      load(P + (size_t(s) * n + i) * 64 + c, v);
+#pragma unroll
+      for (int k = 0; k < W; k++) acc[k] += v[k];
+    }
+#pragma unroll
+    for (int k = 0; k < W; k++) {
+      if (rs) acc[k] *= rs[i] * cs[c + k];
+      acc[k] = fmaf(rho[i], acc[k], e[k]);
+      tile[r][c + k] = acc[k];
+      const float dd = acc[k] - x[k];
+      d2 = fmaf(dd, dd, d2);
+      y2 = fmaf(acc[k], acc[k], y2);
+    }
+    if (W == 4) *reinterpret_cast<float4*>(Y + idx) = make_float4(acc[0], acc[1 % W], acc[2 % W], acc[3 % W]);
+    else Y[idx] = acc[0];
   }
+  __syncthreads();
+  if (Bt) store_hi(tile, i0, n, R, Bt);
   block_sum2f(d2, y2, parts);
 }
 
-__global__ void __launch_bounds__(CB_THREADS) combine_residual_kernel(const float* __restrict__ P, uint32_t splits, uint32_t n, uint32_t R,
+// r = E + rho (sum of the partials) - B in FP64, and r's BF16 columns (Bt, null: none)
+__global__ void __launch_bounds__(CB_THREADS) combine_residual_kernel(const float* __restrict__ P, uint32_t ctas, uint32_t KT, uint32_t n, uint32_t R,
                                                                       const float* __restrict__ rho, const float* __restrict__ E,
-                                                                      const float* __restrict__ B, float* __restrict__ r,
+                                                                      const float* __restrict__ B, float* __restrict__ r, uint16_t* __restrict__ Bt,
                                                                       double* __restrict__ parts) {
-  const size_t idx = size_t(blockIdx.x) * CB_THREADS + threadIdx.x;
+  __shared__ float tile[32][65];
+  const uint32_t i0 = blockIdx.x * 32u, rows = min(32u, n - i0), segs = run_segments(i0 / 128u, KT, n, ctas);
   double r2 = 0.0, b2 = 0.0;
-  if (idx < size_t(n) * R) {
-    const uint32_t i = uint32_t(idx / R), c = uint32_t(idx % R);
-    float acc = 0.0f;
-    for (uint32_t s = 0; s < splits; s++) acc += P[(size_t(s) * n + i) * 64 + c];
-    const double rr = double(E[idx]) + double(rho[i]) * double(acc) - double(B[idx]);
-    r[idx] = float(rr);
-    r2 = rr * rr;
-    b2 = double(B[idx]) * double(B[idx]);
+#pragma unroll 4
+  for (uint32_t q = threadIdx.x; q < rows * R; q += CB_THREADS) {
+    const uint32_t k = q / R, c = q % R, i = i0 + k;
+    const size_t idx = size_t(i0) * R + q;
+    float acc = P[size_t(i) * 64 + c];
+    for (uint32_t s = 1; s < segs; s++) acc += P[(size_t(s) * n + i) * 64 + c];
+    const double b = double(B[idx]), rr = double(E[idx]) + double(rho[i]) * double(acc) - b;
+    const float x = float(rr);
+    r[idx] = x;
+    tile[k][c] = x;
+    r2 += rr * rr;
+    b2 += b * b;
   }
+  __syncthreads();
+  if (Bt) store_hi(tile, i0, n, R, Bt);
   block_sum2(r2, b2, parts);
 }
 
@@ -693,13 +784,21 @@ bool tc_encode(TcMap* map, const void* base, uint32_t inner, uint32_t rows, uint
   return r == CUDA_SUCCESS;
 }
 
-uint32_t tc_k_elems(int mode) { return mode == TC_FP8 ? 128u : 64u; }
+// One CTA per SM; runs of an eighth of a row tile at least, so that few of them meet a tile
+uint32_t tc_ctas(int mode, uint32_t n, uint32_t sms) {
+  const uint32_t ke = mode == TC_FP8 ? 128u : 64u, KT = (n + ke - 1u) / ke;
+  return uint32_t(std::max<uint64_t>(1, std::min<uint64_t>(sms, uint64_t((n + 127u) / 128u) * KT / ((KT + 7u) / 8u))));
+}
+uint32_t tc_segments(int mode, uint32_t n, uint32_t ctas) {
+  const uint32_t ke = mode == TC_FP8 ? 128u : 64u, KT = (n + ke - 1u) / ke;
+  return uint32_t(KT / std::max<uint64_t>(1, uint64_t((n + 127u) / 128u) * KT / ctas)) + 2u;
+}
 
-void tc_gemm(int mode, const TcMap* A, const TcMap* A2, const TcMap* B, const TcMap* B2, uint32_t n, uint32_t splits, uint32_t k_tiles,
-             float* partials, uint32_t* err, cudaStream_t st) {
-  if (mode == TC_BF16) launch_gemm<TC_BF16, 6>(A, A2, B, B2, n, splits, k_tiles, partials, err, st);
-  else if (mode == TC_BF16X3) launch_gemm<TC_BF16X3, 4>(A, A2, B, B2, n, splits, k_tiles, partials, err, st);
-  else launch_gemm<TC_FP8, 6>(A, A2, B, B2, n, splits, k_tiles, partials, err, st);
+void tc_gemm(int mode, const TcMap* A, const TcMap* A2, const TcMap* B, const TcMap* B2, uint32_t n, uint32_t R, uint32_t ctas, float* partials,
+             uint32_t* err, cudaStream_t st) {
+  if (mode == TC_BF16) launch_gemm<TC_BF16, 6>(A, A2, B, B2, n, R, ctas, partials, err, st);
+  else if (mode == TC_BF16X3) launch_gemm<TC_BF16X3, 4>(A, A2, B, B2, n, R, ctas, partials, err, st);
+  else launch_gemm<TC_FP8, 6>(A, A2, B, B2, n, R, ctas, partials, err, st);
 }
 
 size_t tc_f32_parts_bytes(uint32_t n) { return size_t(192) * tc_f32_pad(n) * 2; }
@@ -747,26 +846,25 @@ void tc_pack_b(int mode, const float* X, uint32_t n, uint32_t R, uint16_t* hi, u
     cudaMemsetAsync(col_max, 0, 64 * sizeof(uint32_t), st);
     col_max_kernel<<<304, 256, 0, st>>>(X, n, R, col_max);
     pack_b_kernel<TC_FP8><<<grid, block, 0, st>>>(X, n, R, nullptr, nullptr, q8, col_max, col_scale);
-  } else if (mode == TC_BF16X3) {
+  } else {
     pack_b_kernel<TC_BF16X3><<<grid, block, 0, st>>>(X, n, R, reinterpret_cast<__nv_bfloat16*>(hi), reinterpret_cast<__nv_bfloat16*>(lo),
                                                      nullptr, nullptr, nullptr);
-  } else {
-    pack_b_kernel<TC_BF16><<<grid, block, 0, st>>>(X, n, R, reinterpret_cast<__nv_bfloat16*>(hi), nullptr, nullptr, nullptr, nullptr);
   }
 }
 
-void tc_combine_sweep(const float* partials, uint32_t splits, uint32_t n, uint32_t R, const float* rho, const float* rhs, const float* Xin,
-                      float* Y, const float* row_scale, const float* col_scale, double* norm_partials, uint32_t* n_partials, cudaStream_t st) {
-  const uint32_t blocks = uint32_t((size_t(n) * R + CB_THREADS - 1) / CB_THREADS);
-  *n_partials = blocks;
-  combine_sweep_kernel<<<blocks, CB_THREADS, 0, st>>>(partials, splits, n, R, rho, rhs, Xin, Y, row_scale, col_scale, norm_partials);
+uint32_t tc_combine_sweep(int mode, const float* partials, uint32_t ctas, uint32_t n, uint32_t R, const float* rho, const float* rhs, const float* Xin,
+                          float* Y, const float* row_scale, const float* col_scale, uint16_t* Bt, double* norm_partials, cudaStream_t st) {
+  const uint32_t blocks = (n + 31u) / 32u, ke = mode == TC_FP8 ? 128u : 64u;
+  const auto kernel = R % 4u ? combine_sweep_kernel<1> : combine_sweep_kernel<4>;
+  kernel<<<blocks, CB_THREADS, 0, st>>>(partials, ctas, (n + ke - 1u) / ke, n, R, rho, rhs, Xin, Y, row_scale, col_scale, Bt, norm_partials);
+  return blocks;
 }
 
-void tc_combine_residual(const float* partials, uint32_t splits, uint32_t n, uint32_t R, const float* rho, const float* E, const float* B,
-                         float* r, double* norm_partials, uint32_t* n_partials, cudaStream_t st) {
-  const uint32_t blocks = uint32_t((size_t(n) * R + CB_THREADS - 1) / CB_THREADS);
-  *n_partials = blocks;
-  combine_residual_kernel<<<blocks, CB_THREADS, 0, st>>>(partials, splits, n, R, rho, E, B, r, norm_partials);
+uint32_t tc_combine_residual(const float* partials, uint32_t ctas, uint32_t n, uint32_t R, const float* rho, const float* E, const float* B, float* r,
+                             uint16_t* Bt, double* norm_partials, cudaStream_t st) {
+  const uint32_t blocks = (n + 31u) / 32u;
+  combine_residual_kernel<<<blocks, CB_THREADS, 0, st>>>(partials, ctas, (n + 63u) / 64u, n, R, rho, E, B, r, Bt, norm_partials);
+  return blocks;
 }
 
 void tc_axpy(float* B, const float* d, size_t count, cudaStream_t st) { axpy_kernel<<<1216, 256, 0, st>>>(B, d, count); }
