@@ -231,7 +231,7 @@ vt_status vt_calib_forward(vt_ctx* ctx, const vt_calib_req* q, double* loss) {
   for (uint32_t c = 0; c < q->n_cameras; c++) {
     cps.push_back(calib_cam(ctx, q->cameras[c], q->spp, q->light_samples, q->seed, q->max_depth));
     K.rec_off.push_back(rec_total);
-    rec_total += size_t(vtk::tiled_pixels(cps[c].w, cps[c].h, cps[c].tile_w, cps[c].tile_h)) * cps[c].spp;
+    rec_total += vtk::calib_records(size_t(vtk::tiled_pixels(cps[c].w, cps[c].h, cps[c].tile_w, cps[c].tile_h)) * cps[c].spp);
   }
   K.stored = false;
   K.use_dec = false;
@@ -286,8 +286,9 @@ vt_status vt_calib_forward(vt_ctx* ctx, const vt_calib_req* q, double* loss) {
     K.chunk = uint32_t(std::max<size_t>(1, std::min<size_t>({size_t(cap), size_t(q->spp), (fr / 4) / std::max<size_t>(per_sub, 1)})));
     const size_t chunk_paths = n_pix_max * K.chunk;
     K.wave_paths = uint32_t(std::min<size_t>(8u << 20, chunk_paths));
-    const size_t rec_bytes = vtk::calib_record_bytes(uint32_t(chunk_paths));
-    const size_t tan_bytes = K.want_k ? vtk::calib_tan_bytes(uint32_t(chunk_paths)) : 0;
+    const uint32_t chunk_records = uint32_t(vtk::calib_records(chunk_paths));
+    const size_t rec_bytes = vtk::calib_record_bytes(chunk_records);
+    const size_t tan_bytes = K.want_k ? vtk::calib_tan_bytes(chunk_records) : 0;
     const size_t wave_need = vtk::wave_bytes(K.wave_paths, cps[0].n_light, 0);
     auto grow = [&](void*& ptr, size_t& cap_bytes, size_t need) -> bool {
       if (cap_bytes >= need) return true;

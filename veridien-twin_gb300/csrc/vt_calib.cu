@@ -43,37 +43,53 @@ __device__ __forceinline__ uint32_t warp_append_c(uint32_t* count, bool want) {
   return base + __popc(mask & ((1u << lane) - 1u));
 }
 
-struct CalVertex {
-  uint32_t mat;
-  uint32_t lamp[CAL_MAX_NL];
-  float q[CAL_MAX_NL];   // contribution per unit emitter radiance, per unit albedo (0: no contribution)
+// Path records, in 32-bit words. 32 paths' records lie together, word by word (word k of record r at 32 k + r % 32 of its
+// group), so that a warp's accesses to a word are one or two lines: with a record to itself each was a line per lane, and
+// calib_shade, whose bound that was, took 971 us for 2.3 M paths (now 357; a calibration step of three 480 x 300 cameras, 16 sub-samples:
+// 31.6 -> 27.1 ms)
+template <typename Word>
+struct RecordOf {
+  Word* w;
+  __device__ __forceinline__ uint32_t get(uint32_t k) const { return w[32u * k]; }
+  __device__ __forceinline__ float getf(uint32_t k) const { return __uint_as_float(w[32u * k]); }
+  __device__ __forceinline__ float3 get3(uint32_t k) const { return f3(getf(k), getf(k + 1u), getf(k + 2u)); }
+  __device__ __forceinline__ void put(uint32_t k, uint32_t v) const { w[32u * k] = v; }
+  __device__ __forceinline__ void putf(uint32_t k, float v) const { w[32u * k] = __float_as_uint(v); }
+  __device__ __forceinline__ void put3(uint32_t k, float3 v) const { putf(k, v.x); putf(k + 1u, v.y); putf(k + 2u, v.z); }
 };
-struct CalPath {
-  uint32_t n;            // shading vertices
-  CalVertex v[CAL_MAX_DEPTH];
-  uint32_t emit_lamp;    // emitter hit after the n shading vertices (~0: none)
-  float emit_a;          // its MIS weight x profile
-  uint32_t node;         // node term at the last shading vertex (~0: none)
-};
+using Record = RecordOf<uint32_t>;
+using ConstRecord = RecordOf<const uint32_t>;
+template <typename Word>
+__device__ __forceinline__ RecordOf<Word> record_at(Word* base, uint32_t words, size_t r) { return {base + (r >> 5) * 32u * words + (r & 31u)}; }
+
+// a path: its shading vertices, the emitter hit after them (~0: none) with its MIS weight x profile, the node term at the
+// last of them (~0: none); per vertex the material, and per light sample the lamp and the contribution per unit emitter
+// radiance, per unit albedo (0: no contribution)
+constexpr uint32_t CP_N = 0, CP_EMIT_LAMP = 1, CP_EMIT_A = 2, CP_NODE = 3, CP_VERTEX = 4, CP_VERTEX_WORDS = 1 + 2 * CAL_MAX_NL;
+constexpr uint32_t CP_WORDS = CP_VERTEX + CAL_MAX_DEPTH * CP_VERTEX_WORDS;
+__device__ __forceinline__ uint32_t cp_mat(uint32_t k) { return CP_VERTEX + k * CP_VERTEX_WORDS; }
+__device__ __forceinline__ uint32_t cp_lamp(uint32_t k, uint32_t j) { return cp_mat(k) + 1u + j; }
+__device__ __forceinline__ uint32_t cp_q(uint32_t k, uint32_t j) { return cp_mat(k) + 1u + CAL_MAX_NL + j; }
 
 // the derivative record of a path in d0 (stored form, kept only when the intrinsics' derivative is asked for): each
-// light sample's dq (per unit emitter radiance and albedo; cleared with q when the sample is occluded), the emitter
-// hit's d a, the ray's tangents between bounces, and the triangle each bounce hit (~0: none)
-struct CalTan {
-  float dq[CAL_MAX_DEPTH][CAL_MAX_NL][3];
-  float de[3];
-  Tan3 Jo, Jd;
-  float3 dpb;
-  uint32_t tri[CAL_MAX_DEPTH], inst[CAL_MAX_DEPTH];
-};
+// light sample's dq (per unit emitter radiance and albedo; meant where the path's q is not 0), the emitter hit's d a (meant
+// where it has one), the ray's tangents between bounces, and the triangle and instance each bounce hit (~0: none)
+constexpr uint32_t CT_DQ = 0, CT_DE = CAL_MAX_DEPTH * CAL_MAX_NL * 3, CT_JO = CT_DE + 3, CT_JD = CT_JO + 9, CT_DPB = CT_JD + 9, CT_TRI = CT_DPB + 3,
+                   CT_INST = CT_TRI + CAL_MAX_DEPTH, CT_WORDS = CT_INST + CAL_MAX_DEPTH;
+__device__ __forceinline__ uint32_t ct_dq(uint32_t k, uint32_t j) { return CT_DQ + (k * CAL_MAX_NL + j) * 3u; }
+__device__ __forceinline__ Tan3 get_tan(const Record& G, uint32_t k) {
+  Tan3 J;
+  for (uint32_t c = 0; c < 3; c++) J.c[c] = G.get3(k + 3u * c);
+  return J;
+}
+__device__ __forceinline__ void put_tan(const Record& G, uint32_t k, const Tan3& J) {
+  for (uint32_t c = 0; c < 3; c++) G.put3(k + 3u * c, J.c[c]);
+}
 
-// a path's discrete decisions (replay form): per bounce the triangle and instance its extension ray met (~0 and 0xff:
-// none), and one bit per vertex and light sample, set when that sample's shadow ray was occluded
-struct CalDec {
-  uint32_t tri[CAL_MAX_DEPTH];
-  uint8_t inst[CAL_MAX_DEPTH];
-  uint32_t occ;
-};
+// a path's discrete decisions (replay form): per bounce the triangle its extension ray met (~0: none) and, a byte each, the
+// instance (0xff: none), and one bit per vertex and light sample, set when that sample's shadow ray was occluded
+constexpr uint32_t CD_TRI = 0, CD_INST = CAL_MAX_DEPTH, CD_OCC = CD_INST + 1, CD_WORDS = CD_OCC + 1;
+static_assert(CAL_MAX_DEPTH <= 4, "a word of instance bytes");
 static_assert(CAL_MAX_DEPTH * CAL_MAX_NL <= 32, "one occlusion bit per vertex and light sample");
 static_assert(VT_MAX_INST < 0xff, "instances fit a byte");
 
@@ -132,21 +148,25 @@ __device__ __forceinline__ float3 tan_emitter_hit(const Scene& S, const Hit& h, 
 }
 
 // radiance of a recorded path
-__device__ __forceinline__ float3 path_value(const CalibDev& C, const CalPath& P, uint32_t nl) {
+__device__ __forceinline__ float3 path_value(const CalibDev& C, const ConstRecord& P, uint32_t nl) {
+  const uint32_t n = P.get(CP_N), node = P.get(CP_NODE), lamp = P.get(CP_EMIT_LAMP);
   float3 L = f3(0, 0, 0), T = f3(1, 1, 1);
-  for (uint32_t k = 0; k < P.n; k++) {
-    const float3 rho = alb(C, P.v[k].mat);
+  for (uint32_t k = 0; k < n; k++) {
+    const float3 rho = alb(C, P.get(cp_mat(k)));
     float s = 0.0f;
-    for (uint32_t j = 0; j < nl; j++) if (P.v[k].q[j] != 0.0f) s += __ldg(C.lamp + P.v[k].lamp[j]) * P.v[k].q[j];
+    for (uint32_t j = 0; j < nl; j++) {
+      const float q = P.getf(cp_q(k, j));
+      if (q != 0.0f) s += __ldg(C.lamp + P.get(cp_lamp(k, j))) * q;
+    }
     const float3 Tr = T * rho;
     L = L + Tr * (s / float(nl));
-    if (k + 1 == P.n && P.node != MISS) {
-      const float3 Hn = f3(__ldg(C.H + P.node), __ldg(C.H + C.n_nodes + P.node), __ldg(C.H + 2 * C.n_nodes + P.node));
+    if (k + 1 == n && node != MISS) {
+      const float3 Hn = f3(__ldg(C.H + node), __ldg(C.H + C.n_nodes + node), __ldg(C.H + 2 * C.n_nodes + node));
       L = L + Tr * Hn * INV_PI_F;
     }
     T = Tr;
   }
-  if (P.emit_lamp != MISS) L = L + T * (P.emit_a * __ldg(C.lamp + P.emit_lamp));
+  if (lamp != MISS) L = L + T * (P.getf(CP_EMIT_A) * __ldg(C.lamp + lamp));
   return L;
 }
 
@@ -158,7 +178,9 @@ struct AlbGrad {
   bool on[CAL_MAX_DEPTH];
 };
 
-__device__ __forceinline__ void path_grad(const CalibDev& C, const CalPath& P, uint32_t nl, float3 g, double* sh_lamp, AlbGrad& ag) {
+__device__ __forceinline__ void path_grad(const CalibDev& C, const ConstRecord& P, uint32_t nl, float3 g, double* sh_lamp, AlbGrad& ag) {
+  const uint32_t n = P.get(CP_N), node = P.get(CP_NODE), lamp = P.get(CP_EMIT_LAMP);
+  const float emit_a = P.getf(CP_EMIT_A);
   // Each term is formed in FP32 and added to the FP64 accumulators (FP64 arithmetic runs at a small fraction of
   // this part's FP32 rate; the reductions stay FP64). A term whose albedo product ends at vertex k adds
   // g o value / rho_l to every vertex l <= k: D[k] gathers the g-weighted values of the terms ending at k, and vertex
@@ -170,42 +192,42 @@ __device__ __forceinline__ void path_grad(const CalibDev& C, const CalPath& P, u
   for (uint32_t k = 0; k < CAL_MAX_DEPTH; k++) {
     D[k] = f3(0, 0, 0);
     rho[k] = f3(1, 1, 1);
-    if (k >= P.n) continue;
-    rho[k] = alb(C, P.v[k].mat);
+    if (k >= n) continue;
+    rho[k] = alb(C, P.get(cp_mat(k)));
     T = T * rho[k];
     float s = 0.0f;
     for (uint32_t j = 0; j < nl; j++) {
-      const float q = P.v[k].q[j];
+      const float q = P.getf(cp_q(k, j));
       if (q == 0.0f) continue;
-      atomicAdd(sh_lamp + P.v[k].lamp[j], double(dot(g, T) * q / fnl));
-      s += __ldg(C.lamp + P.v[k].lamp[j]) * q;
+      atomicAdd(sh_lamp + P.get(cp_lamp(k, j)), double(dot(g, T) * q / fnl));
+      s += __ldg(C.lamp + P.get(cp_lamp(k, j))) * q;
     }
     if (s != 0.0f) D[k] = D[k] + g * T * (s / fnl);
-    if (k + 1 == P.n && P.node != MISS) {
+    if (k + 1 == n && node != MISS) {
       const float ip = 0.318309886183790672f;
-      const float3 Hn = f3(__ldg(C.H + P.node), __ldg(C.H + C.n_nodes + P.node), __ldg(C.H + 2 * C.n_nodes + P.node));
-      atomicAdd(C.g_H + P.node, double(g.x * T.x * ip));
-      atomicAdd(C.g_H + C.n_nodes + P.node, double(g.y * T.y * ip));
-      atomicAdd(C.g_H + 2 * C.n_nodes + P.node, double(g.z * T.z * ip));
+      const float3 Hn = f3(__ldg(C.H + node), __ldg(C.H + C.n_nodes + node), __ldg(C.H + 2 * C.n_nodes + node));
+      atomicAdd(C.g_H + node, double(g.x * T.x * ip));
+      atomicAdd(C.g_H + C.n_nodes + node, double(g.y * T.y * ip));
+      atomicAdd(C.g_H + 2 * C.n_nodes + node, double(g.z * T.z * ip));
       D[k] = D[k] + g * T * Hn * ip;
     }
   }
-  if (P.emit_lamp != MISS && P.emit_a != 0.0f) {
-    atomicAdd(sh_lamp + P.emit_lamp, double(dot(g, T) * P.emit_a));
-    if (P.n) {
-      const float Le = P.emit_a * __ldg(C.lamp + P.emit_lamp);
+  if (lamp != MISS && emit_a != 0.0f) {
+    atomicAdd(sh_lamp + lamp, double(dot(g, T) * emit_a));
+    if (n) {
+      const float Le = emit_a * __ldg(C.lamp + lamp);
 #pragma unroll
       for (uint32_t k = 0; k < CAL_MAX_DEPTH; k++)
-        if (k + 1 == P.n) D[k] = D[k] + g * T * Le;
+        if (k + 1 == n) D[k] = D[k] + g * T * Le;
     }
   }
   float3 acc = f3(0, 0, 0);
 #pragma unroll
   for (int k = CAL_MAX_DEPTH - 1; k >= 0; k--) {
-    ag.on[k] = uint32_t(k) < P.n;
+    ag.on[k] = uint32_t(k) < n;
     if (!ag.on[k]) continue;
     acc = acc + D[k];
-    ag.mat[k] = P.v[k].mat;
+    ag.mat[k] = P.get(cp_mat(k));
     ag.val[k] = f3(acc.x / rho[k].x, acc.y / rho[k].y, acc.z / rho[k].z);
   }
 }
@@ -240,56 +262,54 @@ __device__ __forceinline__ void warp_key_add3(double* sh, uint32_t key, float3 v
 // The estimator split like the path tracer: the closest-hit kernel of the wavefront, then calib_shade (one vertex:
 // the record of the vertex, its light samples' unshadowed contributions and shadow segments, the cosine
 // continuation), then calib_shadow (any hit per light sample; an occluded sample's contribution is cleared in the
-// record). Each path's record (CalPath) stays in HBM, so the backward evaluates path_grad on the records without
-// tracing again. Records of path (i, id) of a camera's sub-samples [i0, i1) sit at rec[(i - i0) n_pix + id].
+// record). Each path's record stays in HBM, so the backward evaluates path_grad on the records without
+// tracing again. The record of path (i, id) of a camera's sub-samples [i0, i1) is record (i - i0) n_pix + id; a wave's
+// begin at r0.
 constexpr int WT = 256;
 
 template <bool TAN>
-__global__ void __launch_bounds__(WT, 3) calib_shade_kernel(const Scene S, const CamParams cp, const CalibDev C, WaveBufs wb, CalPath* rec,
-                                                        CalTan* tan, uint32_t b, CalDec* dec, int dmode) {
+__global__ void __launch_bounds__(WT, 3) calib_shade_kernel(const Scene S, const CamParams cp, const CalibDev C, WaveBufs wb, uint32_t* rec,
+                                                        uint32_t* tan, size_t r0, uint32_t b, uint32_t* dec, size_t d0, int dmode) {
   const uint32_t n = *wb.count_in;
   const uint32_t nl = cp.n_light;
   const float fnl = float(nl);
   const float area = __ldg(S.su + 3);
   for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
     const uint32_t p = wb.q_in[k];
-    CalPath& P = rec[p];
-    if (b == 1) { P.n = 0; P.emit_lamp = MISS; P.emit_a = 0.0f; P.node = MISS; }
+    const Record P = record_at(rec, CP_WORDS, r0 + p);
+    if (b == 1) { P.put(CP_N, 0u); P.put(CP_EMIT_LAMP, MISS); P.putf(CP_EMIT_A, 0.0f); P.put(CP_NODE, MISS); }
     const uint4 meta = wb.meta[p];
     const uint32_t i = meta.y, hs = meta.z;
     const float4 o4 = wb.o[p], d4 = wb.d[p], hv = wb.hit[p];
     const float3 o = xyz(o4), d = xyz(d4);
     const float tt = o4.w, pb_prev = d4.w;
     const Hit h{hv.x, hv.y, hv.z, __float_as_uint(hv.w), wb.hinst[p]};
+    const Record D = record_at(dec, CD_WORDS, d0 + p);
     if (dmode == 1) {
-      CalDec& D = dec[p];
       // every bounce of the path starts as none: a replay whose path continues where the recorded one stopped (its
       // rays can differ from the recorded ones in the last bits) meets nothing there, never a stale triangle
       if (b == 1) {
-        D.occ = 0u;
-        for (uint32_t a = 0; a < CAL_MAX_DEPTH; a++) { D.tri[a] = MISS; D.inst[a] = uint8_t(0xff); }
+        D.put(CD_OCC, 0u);
+        for (uint32_t a = 1; a < CAL_MAX_DEPTH; a++) D.put(CD_TRI + a, MISS);
       }
-      D.tri[b - 1] = h.tri;
-      D.inst[b - 1] = h.inst == MISS ? uint8_t(0xff) : uint8_t(h.inst);
+      D.put(CD_TRI + b - 1, h.tri);
+      const uint32_t at = 8u * (b - 1u), inst = h.inst == MISS ? 0xffu : h.inst;
+      D.put(CD_INST, ((b == 1 ? MISS : D.get(CD_INST)) & ~(0xffu << at)) | inst << at);
     }
-    const uint32_t occ = dmode == 2 ? dec[p].occ : 0u;
+    const uint32_t occ = dmode == 2 ? D.get(CD_OCC) : 0u;
     bool cont = false, shadow = false;
+    const Record G = record_at(tan, CT_WORDS, r0 + p);
     Tan3 Jo, Jd, Jx;
     float3 dpb, dt;
     if (TAN) {
-      CalTan& G = tan[p];
       if (b == 1) {
-        for (uint32_t a = 0; a < CAL_MAX_DEPTH; a++) {
-          G.tri[a] = MISS; G.inst[a] = MISS;
-          for (uint32_t j = 0; j < CAL_MAX_NL; j++) G.dq[a][j][0] = G.dq[a][j][1] = G.dq[a][j][2] = 0.0f;
-        }
-        G.de[0] = G.de[1] = G.de[2] = 0.0f;
+        for (uint32_t a = 1; a < cp.max_depth; a++) { G.put(CT_TRI + a, MISS); G.put(CT_INST + a, MISS); }
         Jo = tan_zero(); Jd = tan_identity(); dpb = f3(0, 0, 0);
       } else {
-        Jo = G.Jo; Jd = G.Jd; dpb = G.dpb;
+        Jo = get_tan(G, CT_JO); Jd = get_tan(G, CT_JD); dpb = G.get3(CT_DPB);
       }
-      G.tri[b - 1] = h.tri;
-      G.inst[b - 1] = h.inst;
+      G.put(CT_TRI + b - 1, h.tri);
+      G.put(CT_INST + b - 1, h.inst);
     }
     if (h.tri != MISS) {
       const Surf s = surface(S, h, o, d, tt);
@@ -304,18 +324,17 @@ __global__ void __launch_bounds__(WT, 3) calib_shade_kernel(const Scene S, const
             const float pL = h.t * h.t / (cosE * area);
             w = pb_prev * pb_prev / (pb_prev * pb_prev + fnl * fnl * pL * pL);
           }
-          P.emit_lamp = __ldg(C.emit_of_tri + h.tri);
-          P.emit_a = w * prof;
+          P.put(CP_EMIT_LAMP, __ldg(C.emit_of_tri + h.tri));
+          P.putf(CP_EMIT_A, w * prof);
           if (TAN) {
             const float3 de = tan_emitter_hit(S, h, s, d, tt, b, pb_prev, dpb, fnl, area, Jd, Jx, dt);
-            tan[p].de[0] = de.x; tan[p].de[1] = de.y; tan[p].de[2] = de.z;
+            G.put3(CT_DE, de);
           }
         }
       } else {
-        const uint32_t vk = P.n;
-        CalVertex& V = P.v[vk];
-        V.mat = s.mat;
-        P.n = vk + 1;
+        const uint32_t vk = b == 1 ? 0u : P.get(CP_N);
+        P.put(cp_mat(vk), s.mat);
+        P.put(CP_N, vk + 1u);
         const float3 nrm = s.ns, wo = -d;
         Tan3 Jn;
         if (TAN) Jn = tan_shading_normal(S, h, s, tt, Jx);
@@ -326,8 +345,8 @@ __global__ void __launch_bounds__(WT, 3) calib_shade_kernel(const Scene S, const
         for (uint32_t j = 0; j < nl; j++) {
           const float3 u = f3(kr(i * nl + j, KL0, sh0), kr(i * nl + j, KL1, sh1), kr(i * nl + j, KL2, sh2));
           float3 lp, ln, la;
-          V.lamp[j] = sample_emitter_idx(S, u, tt, lp, ln, la);
-          V.q[j] = 0.0f;
+          P.put(cp_lamp(vk, j), sample_emitter_idx(S, u, tt, lp, ln, la));
+          P.putf(cp_q(vk, j), 0.0f);
           srec[3 * j + 1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
           float3 wi = lp - s.p;
           const float d2 = dot(wi, wi), dist = sqrtf(d2);
@@ -338,19 +357,11 @@ __global__ void __launch_bounds__(WT, 3) calib_shade_kernel(const Scene S, const
           if (prof <= 0.0f) continue;
           const float pdfW = d2 / (cosE * area), pb = cosS * INV_PI_F;
           const float w = fnl * fnl * pdfW * pdfW / (fnl * fnl * pdfW * pdfW + pb * pb);
-          V.q[j] = prof * cosS * w * INV_PI_F / pdfW;
-          if (TAN) {
-            const float3 dq = tan_light(S, s.p, nrm, lp, ln, la, area, fnl, V.q[j], Jx, Jn);
-            tan[p].dq[vk][j][0] = dq.x; tan[p].dq[vk][j][1] = dq.y; tan[p].dq[vk][j][2] = dq.z;
-          }
-          if (dmode == 2) {
-            // the recorded shadow ray's outcome: an occluded sample is cleared as calib_shadow_kernel clears it
-            if ((occ >> (vk * CAL_MAX_NL + j)) & 1u) {
-              V.q[j] = 0.0f;
-              if (TAN) tan[p].dq[vk][j][0] = tan[p].dq[vk][j][1] = tan[p].dq[vk][j][2] = 0.0f;
-            }
-            continue;
-          }
+          const float q = prof * cosS * w * INV_PI_F / pdfW;
+          if (TAN) G.put3(ct_dq(vk, j), tan_light(S, s.p, nrm, lp, ln, la, area, fnl, q, Jx, Jn));
+          // the recorded shadow ray's outcome: an occluded sample stays as calib_shadow_kernel clears it
+          if (!((occ >> (vk * CAL_MAX_NL + j)) & 1u)) P.putf(cp_q(vk, j), q);
+          if (dmode == 2) continue;
           const float3 so = offset_ray(s.p, s.ng, wi);
           srec[3 * j] = make_float4(so.x, so.y, so.z, dist - 2e-5f);
           srec[3 * j + 1] = make_float4(wi.x, wi.y, wi.z, 1.0f);
@@ -359,7 +370,7 @@ __global__ void __launch_bounds__(WT, 3) calib_shade_kernel(const Scene S, const
         }
         if (shadow) wb.nee[p] = make_float4(0.0f, 0.0f, 0.0f, tt);
         if (b == cp.max_depth) {
-          if (h.inst == MISS && h.tri < C.n_static_tris) P.node = __ldg(C.tri_node + h.tri);
+          if (h.inst == MISS && h.tri < C.n_static_tris) P.put(CP_NODE, __ldg(C.tri_node + h.tri));
         } else if (dot(nrm, wo) > 0.0f) {
           const float u1 = b == 1 ? kr(i, KB1, u01(pcg(hs + 7u))) : kr(i, KB1, bounce_shift(hs, b, 4));
           const float u2 = b == 1 ? kr(i, KB2, u01(pcg(hs + 8u))) : kr(i, KB2, bounce_shift(hs, b, 5));
@@ -377,9 +388,9 @@ __global__ void __launch_bounds__(WT, 3) calib_shade_kernel(const Scene S, const
             cont = true;
             if (TAN) {
               const Tan3 Jl = tan_continue(nrm, Jn, r, cpz, sp, sqrtf(fmaxf(0.0f, 1.0f - u1)));
-              tan[p].dpb = (tan_dot(l, Jn) + tan_dot(nrm, Jl)) * INV_PI_F;
-              tan[p].Jo = Jx;
-              tan[p].Jd = Jl;
+              G.put3(CT_DPB, (tan_dot(l, Jn) + tan_dot(nrm, Jl)) * INV_PI_F);
+              put_tan(G, CT_JO, Jx);
+              put_tan(G, CT_JD, Jl);
             }
           }
         }
@@ -393,8 +404,8 @@ __global__ void __launch_bounds__(WT, 3) calib_shade_kernel(const Scene S, const
 }
 
 // any hit of the pending light samples on persistent lanes; an occluded sample's contribution is cleared in the record
-template <bool TAN>
-__global__ void __launch_bounds__(WT, 4) calib_shadow_kernel(const Scene S, const CamParams cp, WaveBufs wb, CalPath* rec, CalTan* tan, CalDec* dec) {
+__global__ void __launch_bounds__(WT, 4) calib_shadow_kernel(const Scene S, const CamParams cp, WaveBufs wb, uint32_t* rec, size_t r0, uint32_t* dec,
+                                                             size_t d0) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // the next bounce's closest hits
   const uint32_t n = *wb.count_sh;
   const uint32_t nl = cp.n_light;
@@ -429,9 +440,11 @@ __global__ void __launch_bounds__(WT, 4) calib_shadow_kernel(const Scene S, cons
     if (st.best.tri == MISS && trace_phase(S, cp.root, o, d, 0.0f, tt, 3u, skip, st, st.k + 1)) { state = LANE_NODE; return; }
     if (st.best.tri != MISS) {
       const uint32_t vk = __float_as_uint(srec[3 * j + 2].z);
-      rec[p].v[vk].q[j] = 0.0f;
-      if (TAN) tan[p].dq[vk][j][0] = tan[p].dq[vk][j][1] = tan[p].dq[vk][j][2] = 0.0f;
-      if (dec) dec[p].occ |= 1u << (vk * CAL_MAX_NL + j);
+      record_at(rec, CP_WORDS, r0 + p).putf(cp_q(vk, j), 0.0f);
+      if (dec) {
+        const Record D = record_at(dec, CD_WORDS, d0 + p);
+        D.put(CD_OCC, D.get(CD_OCC) | 1u << (vk * CAL_MAX_NL + j));
+      }
     }
     j++;
     state = next_sample() ? LANE_NODE : LANE_IDLE;
@@ -443,19 +456,20 @@ __global__ void __launch_bounds__(WT, 4) calib_shadow_kernel(const Scene S, cons
 // per pixel: the image value from the records in sub-sample order, its loss partial (forward); or the gradient of
 // every record (backward)
 // the derivative in d0 of a recorded path's radiance, per channel, from its derivative record
-__device__ __forceinline__ void path_tangent(const CalibDev& C, const CalPath& P, const CalTan& G, uint32_t nl, float3* dL) {
+__device__ __forceinline__ void path_tangent(const CalibDev& C, const ConstRecord& P, const ConstRecord& G, uint32_t nl, float3* dL) {
+  const uint32_t n = P.get(CP_N), lamp = P.get(CP_EMIT_LAMP);
   dL[0] = dL[1] = dL[2] = f3(0, 0, 0);
   float3 T = f3(1, 1, 1);
-  for (uint32_t k = 0; k < P.n; k++) {
-    T = mul3(T, alb(C, P.v[k].mat));
+  for (uint32_t k = 0; k < n; k++) {
+    T = mul3(T, alb(C, P.get(cp_mat(k))));
     for (uint32_t j = 0; j < nl; j++) {
-      if (P.v[k].q[j] == 0.0f) continue;
-      const float3 dq = f3(G.dq[k][j][0], G.dq[k][j][1], G.dq[k][j][2]) * (__ldg(C.lamp + P.v[k].lamp[j]) / float(nl));
+      if (P.getf(cp_q(k, j)) == 0.0f) continue;
+      const float3 dq = G.get3(ct_dq(k, j)) * (__ldg(C.lamp + P.get(cp_lamp(k, j))) / float(nl));
       dL[0] = dL[0] + dq * T.x; dL[1] = dL[1] + dq * T.y; dL[2] = dL[2] + dq * T.z;
     }
   }
-  if (P.emit_lamp != MISS) {
-    const float3 de = f3(G.de[0], G.de[1], G.de[2]) * __ldg(C.lamp + P.emit_lamp);
+  if (lamp != MISS) {
+    const float3 de = G.get3(CT_DE) * __ldg(C.lamp + lamp);
     dL[0] = dL[0] + de * T.x; dL[1] = dL[1] + de * T.y; dL[2] = dL[2] + de * T.z;
   }
 }
@@ -481,8 +495,8 @@ __device__ __forceinline__ void add_intrinsics_grad(const CamParams& cp, uint32_
 // per pixel over the records of sub-samples [i0, i1): backward 0 adds their values to the pixel's running sum (kept in
 // the image between chunks; the chunk that ends at spp writes the image and the loss partials), 1 / 2 accumulate the
 // gradients (2: with the intrinsics' derivative)
-__global__ void __launch_bounds__(CT) calib_records_kernel(const CamParams cp, const CalibDev C, const CalPath* __restrict__ rec,
-                                                          const CalTan* __restrict__ tan, uint32_t n_pix, int backward, uint32_t i0,
+__global__ void __launch_bounds__(CT) calib_records_kernel(const CamParams cp, const CalibDev C, const uint32_t* __restrict__ rec,
+                                                          const uint32_t* __restrict__ tan, uint32_t n_pix, int backward, uint32_t i0,
                                                           uint32_t i1) {
   extern __shared__ double sm[];
   double* sh_alb = sm;
@@ -520,12 +534,12 @@ __global__ void __launch_bounds__(CT) calib_records_kernel(const CamParams cp, c
         AlbGrad ag;
 #pragma unroll
         for (uint32_t k = 0; k < CAL_MAX_DEPTH; k++) { ag.on[k] = false; ag.mat[k] = 0u; ag.val[k] = f3(0, 0, 0); }
-        if (valid) path_grad(C, rec[r], cp.n_light, gf, sh_lamp, ag);
+        if (valid) path_grad(C, record_at(rec, CP_WORDS, r), cp.n_light, gf, sh_lamp, ag);
 #pragma unroll
         for (uint32_t k = 0; k < CAL_MAX_DEPTH; k++) warp_key_add3(sh_alb, ag.mat[k], ag.val[k], ag.on[k]);
         if (backward == 2 && valid) {
           float3 dL[3];
-          path_tangent(C, rec[r], tan[r], cp.n_light, dL);
+          path_tangent(C, record_at(rec, CP_WORDS, r), record_at(tan, CT_WORDS, r), cp.n_light, dL);
           add_intrinsics_grad(cp, id, i, dL, g, kacc);
         }
       }
@@ -534,7 +548,7 @@ __global__ void __launch_bounds__(CT) calib_records_kernel(const CamParams cp, c
       // the sum over sub-samples in order, carried across chunks exactly (a float in the image)
       float3 s = f3(0, 0, 0);
       if (i0 > 0) s = xyz(C.image[px]);
-      for (uint32_t i = i0; i < i1; i++) s = s + path_value(C, rec[size_t(i - i0) * n_pix + id], cp.n_light);
+      for (uint32_t i = i0; i < i1; i++) s = s + path_value(C, record_at(rec, CP_WORDS, size_t(i - i0) * n_pix + id), cp.n_light);
       if (i1 < cp.spp) {
         C.image[px] = make_float4(s.x, s.y, s.z, 0.0f);
         continue;
@@ -852,11 +866,11 @@ int calib_shade_grid() {
 }
 }  // namespace
 
-size_t calib_record_bytes(uint32_t paths) { return size_t(paths) * sizeof(CalPath); }
+size_t calib_record_bytes(uint32_t paths) { return size_t(paths) * CP_WORDS * 4; }
 
-size_t calib_tan_bytes(uint32_t paths) { return size_t(paths) * sizeof(CalTan); }
+size_t calib_tan_bytes(uint32_t paths) { return size_t(paths) * CT_WORDS * 4; }
 
-// the paths of sub-samples [i0, i1) of the camera through the wavefront, their records at rec[(i - i0) n_pix + id]
+// the paths of sub-samples [i0, i1) of the camera through the wavefront, their records (i - i0) n_pix + id
 // tri_hit's arithmetic without its range checks: for a hit tri_hit accepted, the same t, u, v; a recorded hit is met
 // again even when the ray moved by rounding (the derivative-record kernel's ray can differ from the plain kernel's
 // in its last bits)
@@ -875,11 +889,12 @@ __device__ __forceinline__ void tri_uvt(const Scene& S, uint32_t k, float3 o, fl
 
 // the extension rays of a replayed bounce meet the triangles the traced bounce recorded: the traversal's frame (the
 // world, or the instance's pose at the path's time) and its triangle arithmetic, so t, u, v are the traced hit's
-__global__ void __launch_bounds__(256) calib_rehit_kernel(const Scene S, WaveBufs wb, const CalDec* __restrict__ dec, uint32_t b) {
+__global__ void __launch_bounds__(256) calib_rehit_kernel(const Scene S, WaveBufs wb, const uint32_t* __restrict__ dec, size_t d0, uint32_t b) {
   const uint32_t n = *wb.count_in;
   for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
     const uint32_t p = wb.q_in[k];
-    const uint32_t tri = dec[p].tri[b - 1], inst = dec[p].inst[b - 1];
+    const ConstRecord D = record_at(dec, CD_WORDS, d0 + p);
+    const uint32_t tri = D.get(CD_TRI + b - 1), inst = (D.get(CD_INST) >> (8u * (b - 1u))) & 0xffu;
     float4 hit = make_float4(BIG, 0.0f, 0.0f, __uint_as_float(MISS));
     uint32_t hinst = MISS;
     if (tri != MISS) {
@@ -902,32 +917,30 @@ __global__ void __launch_bounds__(256) calib_rehit_kernel(const Scene S, WaveBuf
   }
 }
 
-static void calib_trace(const Scene& S, const CamParams& cp, const CalibDev& C, WaveBufs wb, uint32_t wave_paths, CalPath* rec, CalTan* tan,
-                        uint32_t i0, uint32_t i1, int blocks, cudaStream_t st, CalDec* dec, int dmode) {
+static void calib_trace(const Scene& S, const CamParams& cp, const CalibDev& C, WaveBufs wb, uint32_t wave_paths, uint32_t* rec, uint32_t* tan,
+                        uint32_t i0, uint32_t i1, int blocks, cudaStream_t st, uint32_t* dec, int dmode) {
   const uint32_t n_pix = tiled_pixels(cp.w, cp.h, cp.tile_w, cp.tile_h);
   const uint32_t per_wave = std::max(1u, std::min(i1 - i0, wave_paths / std::max(1u, n_pix)));
   for (uint32_t w0 = i0; w0 < i1; w0 += per_wave) {
     const uint32_t n_i = std::min(per_wave, i1 - w0);
     cudaMemsetAsync(wb.counts, 0, 16, st);
     launch_wave_gen(cp, wb, w0, n_i, n_pix, blocks, st);
-    CalPath* rb = rec + size_t(w0 - i0) * n_pix;
-    CalTan* tb = tan ? tan + size_t(w0 - i0) * n_pix : nullptr;
-    CalDec* db = dec && dmode ? dec + size_t(w0) * n_pix : nullptr;
-    const int dm = db ? dmode : 0;
+    const size_t r0 = size_t(w0 - i0) * n_pix, d0 = size_t(w0) * n_pix;
+    const int dm = dec ? dmode : 0;
+    uint32_t* db = dm ? dec : nullptr;
     for (uint32_t b = 1; b <= cp.max_depth; b++) {
       WaveBufs w = wb;
       bounce_view(w, b);
       if (dm == 2) {
         cudaMemsetAsync(w.count_out, 0, 16, st);
-        calib_rehit_kernel<<<std::max(1, blocks), 256, 0, st>>>(S, w, db, b);
+        calib_rehit_kernel<<<std::max(1, blocks), 256, 0, st>>>(S, w, db, d0, b);
       } else {
         launch_wave_extend(S, cp, w, blocks, st, b > 1);   // over the light samples' tail
       }
-      if (tb) calib_shade_kernel<true><<<calib_shade_grid<true>(), WT, 0, st>>>(S, cp, C, w, rb, tb, b, db, dm);
-      else calib_shade_kernel<false><<<calib_shade_grid<false>(), WT, 0, st>>>(S, cp, C, w, rb, nullptr, b, db, dm);
+      if (tan) calib_shade_kernel<true><<<calib_shade_grid<true>(), WT, 0, st>>>(S, cp, C, w, rec, tan, r0, b, db, d0, dm);
+      else calib_shade_kernel<false><<<calib_shade_grid<false>(), WT, 0, st>>>(S, cp, C, w, rec, nullptr, r0, b, db, d0, dm);
       if (dm == 2) continue;   // the recorded shadow outcomes were applied by the shading
-      if (tb) calib_shadow_kernel<true><<<blocks, WT, 0, st>>>(S, cp, w, rb, tb, db);
-      else calib_shadow_kernel<false><<<blocks, WT, 0, st>>>(S, cp, w, rb, nullptr, db);
+      calib_shadow_kernel<<<blocks, WT, 0, st>>>(S, cp, w, rec, r0, db, d0);
     }
   }
 }
@@ -937,13 +950,12 @@ uint32_t calib_wave_forward(const Scene& S, const CamParams& cp, const CalibDev&
   return calib_wave_chunk(S, cp, C, wb, wave_paths, records, tangents, 0, cp.spp, 0, blocks, st);
 }
 
-size_t calib_dec_bytes(uint32_t paths) { return size_t(paths) * sizeof(CalDec); }
+size_t calib_dec_bytes(uint32_t paths) { return size_t(paths) * CD_WORDS * 4; }
 
 uint32_t calib_wave_chunk(const Scene& S, const CamParams& cp, const CalibDev& C, WaveBufs wb, uint32_t wave_paths, void* records, void* tangents,
                           uint32_t i0, uint32_t i1, int mode, int blocks, cudaStream_t st, void* decisions, int dec_mode) {
-  CalPath* rec = static_cast<CalPath*>(records);
-  CalTan* tan = static_cast<CalTan*>(tangents);
-  calib_trace(S, cp, C, wb, wave_paths, rec, tan, i0, i1, blocks, st, static_cast<CalDec*>(decisions), dec_mode);
+  uint32_t *rec = static_cast<uint32_t*>(records), *tan = static_cast<uint32_t*>(tangents);
+  calib_trace(S, cp, C, wb, wave_paths, rec, tan, i0, i1, blocks, st, static_cast<uint32_t*>(decisions), dec_mode);
   const uint32_t n_pix = tiled_pixels(cp.w, cp.h, cp.tile_w, cp.tile_h);
   const uint32_t grid = std::max(1u, std::min(uint32_t(blocks), (n_pix + CT - 1) / CT));
   const size_t smem = mode ? size_t(3 * C.n_mat + C.n_lamps) * 8 : 0;
@@ -954,32 +966,33 @@ uint32_t calib_wave_chunk(const Scene& S, const CamParams& cp, const CalibDev& C
 void calib_records_backward(const CamParams& cp, const CalibDev& C, const void* records, const void* tangents, int blocks, cudaStream_t st) {
   const uint32_t n_pix = tiled_pixels(cp.w, cp.h, cp.tile_w, cp.tile_h);
   const uint32_t grid = std::max(1u, std::min(uint32_t(blocks), (n_pix + CT - 1) / CT));
-  calib_records_kernel<<<grid, CT, size_t(3 * C.n_mat + C.n_lamps) * 8, st>>>(cp, C, static_cast<const CalPath*>(records),
-                                                                             static_cast<const CalTan*>(tangents), n_pix, tangents ? 2 : 1,
+  calib_records_kernel<<<grid, CT, size_t(3 * C.n_mat + C.n_lamps) * 8, st>>>(cp, C, static_cast<const uint32_t*>(records),
+                                                                             static_cast<const uint32_t*>(tangents), n_pix, tangents ? 2 : 1,
                                                                              0, cp.spp);
 }
 
 // per path of the camera's records, in (row, column, sub-sample) order: the triangle and instance of each bounce
 // (~0: none) and each vertex's light samples' q (0: occluded or no contribution)
-__global__ void calib_export_paths_kernel(const CamParams cp, const CalPath* __restrict__ rec, const CalTan* __restrict__ tan, uint32_t n_pix,
+__global__ void calib_export_paths_kernel(const CamParams cp, const uint32_t* __restrict__ rec, const uint32_t* __restrict__ tan, uint32_t n_pix,
                                           uint32_t* __restrict__ tri_inst, float* __restrict__ q) {
   const uint32_t id = blockIdx.x * blockDim.x + threadIdx.x;
   uint32_t x, y;
   if (id >= n_pix || !pixel_xy(cp, id, x, y)) return;
   for (uint32_t i = 0; i < cp.spp; i++) {
     const size_t r = size_t(i) * n_pix + id, o = (size_t(y) * cp.w + x) * cp.spp + i;
-    const CalPath& P = rec[r];
+    const ConstRecord P = record_at(rec, CP_WORDS, r), G = record_at(tan, CT_WORDS, r);
+    const uint32_t n = P.get(CP_N);
     for (uint32_t b = 0; b < CAL_MAX_DEPTH; b++) {
-      tri_inst[(o * CAL_MAX_DEPTH + b) * 2] = tan[r].tri[b];
-      tri_inst[(o * CAL_MAX_DEPTH + b) * 2 + 1] = tan[r].inst[b];
-      for (uint32_t j = 0; j < CAL_MAX_NL; j++) q[(o * CAL_MAX_DEPTH + b) * CAL_MAX_NL + j] = b < P.n && j < cp.n_light ? P.v[b].q[j] : 0.0f;
+      tri_inst[(o * CAL_MAX_DEPTH + b) * 2] = b < cp.max_depth ? G.get(CT_TRI + b) : MISS;
+      tri_inst[(o * CAL_MAX_DEPTH + b) * 2 + 1] = b < cp.max_depth ? G.get(CT_INST + b) : MISS;
+      for (uint32_t j = 0; j < CAL_MAX_NL; j++) q[(o * CAL_MAX_DEPTH + b) * CAL_MAX_NL + j] = b < n && j < cp.n_light ? P.getf(cp_q(b, j)) : 0.0f;
     }
   }
 }
 
 void calib_export_paths(const CamParams& cp, const void* records, const void* tangents, uint32_t* tri_inst, float* q, cudaStream_t st) {
   const uint32_t n_pix = tiled_pixels(cp.w, cp.h, cp.tile_w, cp.tile_h);
-  calib_export_paths_kernel<<<(n_pix + 127) / 128, 128, 0, st>>>(cp, static_cast<const CalPath*>(records), static_cast<const CalTan*>(tangents),
+  calib_export_paths_kernel<<<(n_pix + 127) / 128, 128, 0, st>>>(cp, static_cast<const uint32_t*>(records), static_cast<const uint32_t*>(tangents),
                                                                 n_pix, tri_inst, q);
 }
 

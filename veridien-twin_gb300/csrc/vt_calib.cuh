@@ -27,9 +27,11 @@ struct CalibDev {
 };
 
 // stored-path form: the wavefront forward of one camera (records of all its paths kept, path (i, id) at
-// records[i n_pix + id]), the image and per-block loss partials (returns their number); and the backward from the
+// record i n_pix + id of `records`), the image and per-block loss partials (returns their number); and the backward from the
 // records, without tracing
 size_t calib_record_bytes(uint32_t paths);
+// records lie in groups of 32: what `paths` of them take, and where the next camera's may begin
+inline size_t calib_records(size_t paths) { return (paths + 31) / 32 * 32; }
 // with `tangents` (calib_tan_bytes per path, NULL: none) the forward also keeps each path's derivative record in its
 // primary direction, and the backward then adds the derivative in the camera's intrinsics (C.g_K)
 size_t calib_tan_bytes(uint32_t paths);
@@ -40,12 +42,12 @@ void calib_records_backward(const CamParams& cp, const CalibDev& C, const void* 
 // (triangle, instance) and CAL_MAX_DEPTH x CAL_MAX_NL light-sample weights q (0: occluded or no contribution)
 void calib_export_paths(const CamParams& cp, const void* records, const void* tangents, uint32_t* tri_inst, float* q, cudaStream_t st);
 // replay form: the paths of the camera's sub-samples [i0, i1) traced into `records` (and `tangents`, NULL: none) at
-// records[(i - i0) n_pix + id], then mode 0 adds their values to the image (the chunk ending at spp writes the image
+// record (i - i0) n_pix + id, then mode 0 adds their values to the image (the chunk ending at spp writes the image
 // and the per-block loss partials, whose number it returns), 1 accumulates the gradients of the image loss
 // (albedos, emitter radiances, node light), 2 also the derivative in the camera's intrinsics (C.g_K). The image of
 // the forward's chunks is the stored form's image bit for bit.
 //
-// `decisions` (calib_dec_bytes per path of the camera, at decisions[i n_pix + id]; NULL: none) keeps each path's
+// `decisions` (calib_dec_bytes per path of the camera, the path's at i n_pix + id; NULL: none) keeps each path's
 // discrete decisions: per bounce the triangle and instance the extension ray met, per vertex and light sample
 // whether the shadow ray was occluded. dec_mode 1 records them while tracing; dec_mode 2 replays them: the extension
 // rays meet the recorded triangles (one intersection each, the traversal's own arithmetic) and the occluded samples
