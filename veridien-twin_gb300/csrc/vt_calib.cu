@@ -178,9 +178,22 @@ struct AlbGrad {
   bool on[CAL_MAX_DEPTH];
 };
 
-__device__ __forceinline__ void path_grad(const CalibDev& C, const ConstRecord& P, uint32_t nl, float3 g, double* sh_lamp, AlbGrad& ag) {
+__device__ __forceinline__ void path_grad(const CalibDev& C, const ConstRecord& P, uint32_t depth, uint32_t nl, float3 g, double* sh_lamp, AlbGrad& ag) {
   const uint32_t n = P.get(CP_N), node = P.get(CP_NODE), lamp = P.get(CP_EMIT_LAMP);
   const float emit_a = P.getf(CP_EMIT_A);
+  // the vertices' words at once, before it is known how many there are: the records come from HBM
+  uint32_t mat[CAL_MAX_DEPTH], lamps[CAL_MAX_DEPTH][CAL_MAX_NL];
+  float qs[CAL_MAX_DEPTH][CAL_MAX_NL];
+#pragma unroll
+  for (uint32_t k = 0; k < CAL_MAX_DEPTH; k++) {
+    mat[k] = k < depth ? P.get(cp_mat(k)) : 0u;
+#pragma unroll
+    for (uint32_t j = 0; j < CAL_MAX_NL; j++) {
+      const bool on = k < depth && j < nl;
+      qs[k][j] = on ? P.getf(cp_q(k, j)) : 0.0f;
+      lamps[k][j] = on ? P.get(cp_lamp(k, j)) : 0u;
+    }
+  }
   // Each term is formed in FP32 and added to the FP64 accumulators (FP64 arithmetic runs at a small fraction of
   // this part's FP32 rate; the reductions stay FP64). A term whose albedo product ends at vertex k adds
   // g o value / rho_l to every vertex l <= k: D[k] gathers the g-weighted values of the terms ending at k, and vertex
@@ -193,14 +206,15 @@ __device__ __forceinline__ void path_grad(const CalibDev& C, const ConstRecord& 
     D[k] = f3(0, 0, 0);
     rho[k] = f3(1, 1, 1);
     if (k >= n) continue;
-    rho[k] = alb(C, P.get(cp_mat(k)));
+    rho[k] = alb(C, mat[k]);
     T = T * rho[k];
     float s = 0.0f;
-    for (uint32_t j = 0; j < nl; j++) {
-      const float q = P.getf(cp_q(k, j));
-      if (q == 0.0f) continue;
-      atomicAdd(sh_lamp + P.get(cp_lamp(k, j)), double(dot(g, T) * q / fnl));
-      s += __ldg(C.lamp + P.get(cp_lamp(k, j))) * q;
+#pragma unroll
+    for (uint32_t j = 0; j < CAL_MAX_NL; j++) {
+      const float q = qs[k][j];
+      if (j >= nl || q == 0.0f) continue;
+      atomicAdd(sh_lamp + lamps[k][j], double(dot(g, T) * q / fnl));
+      s += __ldg(C.lamp + lamps[k][j]) * q;
     }
     if (s != 0.0f) D[k] = D[k] + g * T * (s / fnl);
     if (k + 1 == n && node != MISS) {
@@ -227,7 +241,7 @@ __device__ __forceinline__ void path_grad(const CalibDev& C, const ConstRecord& 
     ag.on[k] = uint32_t(k) < n;
     if (!ag.on[k]) continue;
     acc = acc + D[k];
-    ag.mat[k] = P.get(cp_mat(k));
+    ag.mat[k] = mat[k];
     ag.val[k] = f3(acc.x / rho[k].x, acc.y / rho[k].y, acc.z / rho[k].z);
   }
 }
@@ -249,11 +263,7 @@ __device__ __forceinline__ void warp_key_add3(double* sh, uint32_t key, float3 v
       b += __shfl_xor_sync(0xffffffffu, b, o);
       c += __shfl_xor_sync(0xffffffffu, c, o);
     }
-    if (lane == leader) {
-      atomicAdd(sh + 3 * k0, double(a));
-      atomicAdd(sh + 3 * k0 + 1, double(b));
-      atomicAdd(sh + 3 * k0 + 2, double(c));
-    }
+    if (lane < 3u) atomicAdd(sh + 3 * k0 + lane, double(lane == 0u ? a : lane == 1u ? b : c));   // one compare-and-swap loop, not three
     if (in) on = false;
   }
 }
@@ -534,7 +544,7 @@ __global__ void __launch_bounds__(CT) calib_records_kernel(const CamParams cp, c
         AlbGrad ag;
 #pragma unroll
         for (uint32_t k = 0; k < CAL_MAX_DEPTH; k++) { ag.on[k] = false; ag.mat[k] = 0u; ag.val[k] = f3(0, 0, 0); }
-        if (valid) path_grad(C, record_at(rec, CP_WORDS, r), cp.n_light, gf, sh_lamp, ag);
+        if (valid) path_grad(C, record_at(rec, CP_WORDS, r), cp.max_depth, cp.n_light, gf, sh_lamp, ag);
 #pragma unroll
         for (uint32_t k = 0; k < CAL_MAX_DEPTH; k++) warp_key_add3(sh_alb, ag.mat[k], ag.val[k], ag.on[k]);
         if (backward == 2 && valid) {
