@@ -147,26 +147,54 @@ __device__ __forceinline__ float3 tan_emitter_hit(const Scene& S, const Hit& h, 
   return f3(out[0], out[1], out[2]);
 }
 
+// a path's vertices at once, before it is known how many there are: the records come from HBM
+struct PathWords {
+  uint32_t mat[CAL_MAX_DEPTH], lamp[CAL_MAX_DEPTH][CAL_MAX_NL];
+  float q[CAL_MAX_DEPTH][CAL_MAX_NL];
+};
+__device__ __forceinline__ PathWords path_words(const ConstRecord& P, uint32_t depth, uint32_t nl) {
+  PathWords W;
+#pragma unroll
+  for (uint32_t k = 0; k < CAL_MAX_DEPTH; k++) {
+    W.mat[k] = k < depth ? P.get(cp_mat(k)) : 0u;
+#pragma unroll
+    for (uint32_t j = 0; j < CAL_MAX_NL; j++) {
+      const bool on = k < depth && j < nl;
+      W.q[k][j] = on ? P.getf(cp_q(k, j)) : 0.0f;
+      W.lamp[k][j] = on ? P.get(cp_lamp(k, j)) : 0u;
+    }
+  }
+  return W;
+}
+
+// one rounding each, whatever the compiler knows of the operands in an unrolled loop
+__device__ __forceinline__ float3 mac3(float3 a, float b, float3 c) { return f3(__fmaf_rn(a.x, b, c.x), __fmaf_rn(a.y, b, c.y), __fmaf_rn(a.z, b, c.z)); }
+
 // radiance of a recorded path
-__device__ __forceinline__ float3 path_value(const CalibDev& C, const ConstRecord& P, uint32_t nl) {
+__device__ __forceinline__ float3 path_value(const CalibDev& C, const ConstRecord& P, uint32_t depth, uint32_t nl) {
   const uint32_t n = P.get(CP_N), node = P.get(CP_NODE), lamp = P.get(CP_EMIT_LAMP);
+  const PathWords W = path_words(P, depth, nl);
+  const float emit_a = P.getf(CP_EMIT_A);
   float3 L = f3(0, 0, 0), T = f3(1, 1, 1);
-  for (uint32_t k = 0; k < n; k++) {
-    const float3 rho = alb(C, P.get(cp_mat(k)));
+#pragma unroll
+  for (uint32_t k = 0; k < CAL_MAX_DEPTH; k++) {
+    if (k >= n) continue;
+    const float3 rho = alb(C, W.mat[k]);
     float s = 0.0f;
-    for (uint32_t j = 0; j < nl; j++) {
-      const float q = P.getf(cp_q(k, j));
-      if (q != 0.0f) s += __ldg(C.lamp + P.get(cp_lamp(k, j))) * q;
+#pragma unroll
+    for (uint32_t j = 0; j < CAL_MAX_NL; j++) {
+      const float q = W.q[k][j];
+      if (j < nl && q != 0.0f) s += __ldg(C.lamp + W.lamp[k][j]) * q;
     }
     const float3 Tr = T * rho;
-    L = L + Tr * (s / float(nl));
+    L = mac3(Tr, s / float(nl), L);
     if (k + 1 == n && node != MISS) {
       const float3 Hn = f3(__ldg(C.H + node), __ldg(C.H + C.n_nodes + node), __ldg(C.H + 2 * C.n_nodes + node));
-      L = L + Tr * Hn * INV_PI_F;
+      L = mac3(Tr * Hn, INV_PI_F, L);
     }
     T = Tr;
   }
-  if (lamp != MISS) L = L + T * (P.getf(CP_EMIT_A) * __ldg(C.lamp + lamp));
+  if (lamp != MISS) L = mac3(T, emit_a * __ldg(C.lamp + lamp), L);
   return L;
 }
 
@@ -181,19 +209,7 @@ struct AlbGrad {
 __device__ __forceinline__ void path_grad(const CalibDev& C, const ConstRecord& P, uint32_t depth, uint32_t nl, float3 g, double* sh_lamp, AlbGrad& ag) {
   const uint32_t n = P.get(CP_N), node = P.get(CP_NODE), lamp = P.get(CP_EMIT_LAMP);
   const float emit_a = P.getf(CP_EMIT_A);
-  // the vertices' words at once, before it is known how many there are: the records come from HBM
-  uint32_t mat[CAL_MAX_DEPTH], lamps[CAL_MAX_DEPTH][CAL_MAX_NL];
-  float qs[CAL_MAX_DEPTH][CAL_MAX_NL];
-#pragma unroll
-  for (uint32_t k = 0; k < CAL_MAX_DEPTH; k++) {
-    mat[k] = k < depth ? P.get(cp_mat(k)) : 0u;
-#pragma unroll
-    for (uint32_t j = 0; j < CAL_MAX_NL; j++) {
-      const bool on = k < depth && j < nl;
-      qs[k][j] = on ? P.getf(cp_q(k, j)) : 0.0f;
-      lamps[k][j] = on ? P.get(cp_lamp(k, j)) : 0u;
-    }
-  }
+  const PathWords W = path_words(P, depth, nl);
   // Each term is formed in FP32 and added to the FP64 accumulators (FP64 arithmetic runs at a small fraction of
   // this part's FP32 rate; the reductions stay FP64). A term whose albedo product ends at vertex k adds
   // g o value / rho_l to every vertex l <= k: D[k] gathers the g-weighted values of the terms ending at k, and vertex
@@ -206,15 +222,15 @@ __device__ __forceinline__ void path_grad(const CalibDev& C, const ConstRecord& 
     D[k] = f3(0, 0, 0);
     rho[k] = f3(1, 1, 1);
     if (k >= n) continue;
-    rho[k] = alb(C, mat[k]);
+    rho[k] = alb(C, W.mat[k]);
     T = T * rho[k];
     float s = 0.0f;
 #pragma unroll
     for (uint32_t j = 0; j < CAL_MAX_NL; j++) {
-      const float q = qs[k][j];
+      const float q = W.q[k][j];
       if (j >= nl || q == 0.0f) continue;
-      atomicAdd(sh_lamp + lamps[k][j], double(dot(g, T) * q / fnl));
-      s += __ldg(C.lamp + lamps[k][j]) * q;
+      atomicAdd(sh_lamp + W.lamp[k][j], double(dot(g, T) * q / fnl));
+      s += __ldg(C.lamp + W.lamp[k][j]) * q;
     }
     if (s != 0.0f) D[k] = D[k] + g * T * (s / fnl);
     if (k + 1 == n && node != MISS) {
@@ -241,7 +257,7 @@ __device__ __forceinline__ void path_grad(const CalibDev& C, const ConstRecord& 
     ag.on[k] = uint32_t(k) < n;
     if (!ag.on[k]) continue;
     acc = acc + D[k];
-    ag.mat[k] = mat[k];
+    ag.mat[k] = W.mat[k];
     ag.val[k] = f3(acc.x / rho[k].x, acc.y / rho[k].y, acc.z / rho[k].z);
   }
 }
@@ -558,7 +574,7 @@ __global__ void __launch_bounds__(CT) calib_records_kernel(const CamParams cp, c
       // the sum over sub-samples in order, carried across chunks exactly (a float in the image)
       float3 s = f3(0, 0, 0);
       if (i0 > 0) s = xyz(C.image[px]);
-      for (uint32_t i = i0; i < i1; i++) s = s + path_value(C, record_at(rec, CP_WORDS, size_t(i - i0) * n_pix + id), cp.n_light);
+      for (uint32_t i = i0; i < i1; i++) s = s + path_value(C, record_at(rec, CP_WORDS, size_t(i - i0) * n_pix + id), cp.max_depth, cp.n_light);
       if (i1 < cp.spp) {
         C.image[px] = make_float4(s.x, s.y, s.z, 0.0f);
         continue;
