@@ -42,11 +42,11 @@ W_, H_, SPP, DEPTH, NL = 640, 480, 16, 4, 1
 WORKLOAD = "C0 synthetic dome path tracer: 640x480 KB4 camera, 16 spp, depth 4, 1 light sample, ~12.4k tris"
 # DRAM bytes (read + write) of wave_extend per extension ray and its issue rate, measured by ncu on this workload:
 # `ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum,sm__inst_executed.avg.per_cycle_active ... -k regex:wave_extend`
-# over the four launches of one frame of `bench.py --case render:640:480:16` (1339.5 MB for 19,248,063 rays)
-EXTEND_DRAM_PER_RAY = 1339544576.0 / 19248063.0
-EXTEND_IPC = 2.755
+# over the four launches of one frame of `bench.py --case render:640:480:16` (1353.9 MB for 19,248,063 rays)
+EXTEND_DRAM_PER_RAY = 1353893888.0 / 19248063.0
+EXTEND_IPC = 2.618
 TRAFFIC_SOURCE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of the 4 wave_extend launches of one 640x480x16 frame, "
-                  "per extension ray (69.6 B), times this run's rays per launch")
+                  "per extension ray (70.3 B), times this run's rays per launch")
 
 
 def bench_config(world):

@@ -936,8 +936,8 @@ static vt_status tc_solve(vt_ctx* ctx, vt_solve_req* q) {
 }
 
 // ------------------------------------------------------------------------------------------------ radiosity solve
-// Plain FP32: Jacobi sweeps B <- E + rho F B on CUDA cores (the matvec for one right-hand side, the FP32 GEMM
-// for several), the relative update checked every `check_every` sweeps. BF16 / FP8: see vt_tc.cu.
+// Plain FP32: Jacobi sweeps B <- E + rho F B (the matvec for one right-hand side; for several the tensor cores by bf16
+// parts, or the CUDA-core GEMM where those do not apply), the relative update checked every `check_every` sweeps. BF16 / FP8: see vt_tc.cu.
 vt_status vt_radiosity_solve(vt_ctx* ctx, vt_solve_req* q) {
   if (!ctx || !q || !q->n || !q->n_rhs || !q->F || !q->rho || !q->E || !q->B) return VT_ERR_ARG;
   if (q->n_rhs > 64) return fail(ctx, VT_ERR_ARG, "solve: at most 64 right-hand sides");
