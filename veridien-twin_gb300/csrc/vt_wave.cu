@@ -15,6 +15,7 @@
 #include <algorithm>
 
 #include "vt_camera.cuh"
+#include "vt_queue.cuh"
 #include "vt_wave.cuh"
 
 namespace vtk {
@@ -101,30 +102,48 @@ __device__ __forceinline__ uint64_t cull_bits(const BatchCull& C, float3 o, floa
 // paths of the wave: sub-sample index i in [i0, i0 + n_i), pixel id in [0, n_pix); path p = (i - i0) * n_pix + id
 __global__ void __launch_bounds__(WAVE_THREADS) wave_gen(const CamParams cp, WaveBufs wb, uint32_t i0, uint32_t n_i, uint32_t n_pix) {
   const uint32_t total = n_i * n_pix;
-  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < total; p += gridDim.x * blockDim.x) {
-    const uint32_t id = p % n_pix, i = i0 + p / n_pix;
-    float4 o4, d4;
-    uint32_t hs;
-    const bool valid = camera_path(cp, id, i, o4, d4, hs);
-    init_path(wb, p, o4, d4, id, i, hs, valid);
-    const uint32_t slot = warp_append(wb.count_in, valid);
-    if (valid) wb.q_in[slot] = p;
-  }
+  __shared__ uint32_t queued[WAVE_THREADS / 32][WQ_CAP];
+  WarpQueue queue(queued[threadIdx.x >> 5]);
+  const WarpShare share(total);
+  for (uint32_t p0 = share.first; p0 < total; p0 += share.stride)
+    for (uint32_t r = 0; r < share.runs && p0 + r < total; r += 32u) {
+      const uint32_t p = p0 + r + (threadIdx.x & 31u);
+      bool valid = false;
+      if (p < total) {
+        const uint32_t id = p % n_pix, i = i0 + p / n_pix;
+        float4 o4, d4;
+        uint32_t hs;
+        valid = camera_path(cp, id, i, o4, d4, hs);
+        init_path(wb, p, o4, d4, id, i, hs, valid);
+      }
+      __syncwarp();
+      queue.push(valid, p, wb.count_in, wb.q_in);
+    }
+  queue.flush(wb.count_in, wb.q_in);
 }
 
 // a batch wave: paths p = i * n_pw + lp (all sub-samples i < spp of pixels px0 + lp)
 __global__ void __launch_bounds__(WAVE_THREADS) wave_gen_batch_kernel(const CamParams cp, WaveBufs wb) {
   const uint32_t n_pw = wb.bc.n_pw, total = cp.spp * n_pw;
-  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < total; p += gridDim.x * blockDim.x) {
-    const uint32_t id = wb.bc.px0 + p % n_pw, i = p / n_pw;
-    float4 o4, d4;
-    uint32_t hs;
-    const bool valid = camera_path(cp, id, i, o4, d4, hs);
-    init_path(wb, p, o4, d4, id, i, hs, valid);
-    wb.bc.dirty[p] = 0ull;
-    const uint32_t slot = warp_append(wb.count_in, valid);
-    if (valid) wb.q_in[slot] = p;
-  }
+  __shared__ uint32_t queued[WAVE_THREADS / 32][WQ_CAP];
+  WarpQueue queue(queued[threadIdx.x >> 5]);
+  const WarpShare share(total);
+  for (uint32_t p0 = share.first; p0 < total; p0 += share.stride)
+    for (uint32_t r = 0; r < share.runs && p0 + r < total; r += 32u) {
+      const uint32_t p = p0 + r + (threadIdx.x & 31u);
+      bool valid = false;
+      if (p < total) {
+        const uint32_t id = wb.bc.px0 + p % n_pw, i = p / n_pw;
+        float4 o4, d4;
+        uint32_t hs;
+        valid = camera_path(cp, id, i, o4, d4, hs);
+        init_path(wb, p, o4, d4, id, i, hs, valid);
+        wb.bc.dirty[p] = 0ull;
+      }
+      __syncwarp();
+      queue.push(valid, p, wb.count_in, wb.q_in);
+    }
+  queue.flush(wb.count_in, wb.q_in);
 }
 
 // pair paths: pair j repeats shared path pair_src[j] (same pixel and sub-sample) under its own pose
@@ -512,45 +531,66 @@ __device__ __forceinline__ uint32_t pixel_id(const CamParams& cp, uint32_t x, ui
 }
 
 __global__ void __launch_bounds__(WAVE_THREADS) refine_select(const CamParams cp, const Scene S, WaveBufs wb, uint32_t n_pix, float4* __restrict__ out) {
-  for (uint32_t id = blockIdx.x * blockDim.x + threadIdx.x; id < n_pix; id += gridDim.x * blockDim.x) {
-    uint32_t x, y;
-    bool want = false;
-    if (pixel_xy(cp, id, x, y)) {
-      const float4 a = wb.acc[id];
-      const uint32_t k = __float_as_uint(a.w);
-      want = (k & 0x50000u) != 0u || ((k & 0x20000u) != 0u && (cp.options & VT_O_REFINE_SHADOW) != 0u);
-      for (int dy = -1; dy <= 1 && !want; dy++)
-        for (int dx = -1; dx <= 1; dx++) {
-          const uint32_t xx = uint32_t(min(max(int(x) + dx, 0), int(cp.w) - 1)), yy = uint32_t(min(max(int(y) + dy, 0), int(cp.h) - 1));
-          if ((__float_as_uint(wb.acc[pixel_id(cp, xx, yy)].w) & 0xffffu) != (k & 0xffffu)) { want = true; break; }
+  __shared__ uint32_t queued[WAVE_THREADS / 32][WQ_CAP];
+  WarpQueue queue(queued[threadIdx.x >> 5]);
+  uint32_t tally[4] = {0u, 0u, 0u, 0u};   // refined pixels; posed body, shadow, sub-sample mesh change among them
+  const WarpShare share(n_pix);
+  for (uint32_t p0 = share.first; p0 < n_pix; p0 += share.stride)
+    for (uint32_t r = 0; r < share.runs && p0 + r < n_pix; r += 32u) {
+      const uint32_t id = p0 + r + (threadIdx.x & 31u);
+      uint32_t x, y;
+      bool want = false;
+      if (id < n_pix && pixel_xy(cp, id, x, y)) {
+        const float4 a = wb.acc[id];
+        const uint32_t k = __float_as_uint(a.w);
+        want = (k & 0x50000u) != 0u || ((k & 0x20000u) != 0u && (cp.options & VT_O_REFINE_SHADOW) != 0u);
+        for (int dy = -1; dy <= 1 && !want; dy++)
+          for (int dx = -1; dx <= 1; dx++) {
+            const uint32_t xx = uint32_t(min(max(int(x) + dx, 0), int(cp.w) - 1)), yy = uint32_t(min(max(int(y) + dy, 0), int(cp.h) - 1));
+            if ((__float_as_uint(wb.acc[pixel_id(cp, xx, yy)].w) & 0xffffu) != (k & 0xffffu)) { want = true; break; }
+          }
+        if (want) {
+          tally[0]++;
+          tally[1] += (k >> 16) & 1u;
+          tally[2] += (k >> 17) & 1u;
+          tally[3] += (k >> 18) & 1u;
+        } else {
+          const float sc = cp.scale / float(cp.spp);
+          out[size_t(y) * cp.w + x] = make_float4(a.x * sc, a.y * sc, a.z * sc, k == 0xfffeu ? 0.0f : 1.0f);
         }
-      if (want) {
-        atomicAdd(S.dbg + 2, 1u);
-        if (k & 0x10000u) atomicAdd(S.dbg + 3, 1u);
-        if (k & 0x20000u) atomicAdd(S.dbg + 4, 1u);
-        if (k & 0x40000u) atomicAdd(S.dbg + 5, 1u);
-      } else {
-        const float sc = cp.scale / float(cp.spp);
-        out[size_t(y) * cp.w + x] = make_float4(a.x * sc, a.y * sc, a.z * sc, k == 0xfffeu ? 0.0f : 1.0f);
       }
+      __syncwarp();
+      queue.push(want, id, wb.rcount, wb.rlist);
     }
-    const uint32_t slot = warp_append(wb.rcount, want);
-    if (want) wb.rlist[slot] = id;
+  queue.flush(wb.rcount, wb.rlist);
+#pragma unroll
+  for (int c = 0; c < 4; c++) {
+    const uint32_t sum = __reduce_add_sync(0xffffffffu, tally[c]);
+    if ((threadIdx.x & 31u) == 0u && sum) atomicAdd(S.dbg + 2 + c, sum);
   }
 }
 
 // refinement paths p = e * n_list + l: sub-sample spp + e0 + e of listed pixel l
 __global__ void __launch_bounds__(WAVE_THREADS) refine_gen(const CamParams cp, WaveBufs wb, uint32_t spp1, uint32_t e0, uint32_t n_e) {
   const uint32_t n_list = *wb.rcount, total = n_list * n_e;
-  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < total; p += gridDim.x * blockDim.x) {
-    const uint32_t l = p % n_list, i = spp1 + e0 + p / n_list, id = wb.rlist[l];
-    float4 o4, d4;
-    uint32_t hs;
-    const bool valid = camera_path(cp, id, i, o4, d4, hs);
-    init_path(wb, p, o4, d4, id, i, hs, valid);
-    const uint32_t slot = warp_append(wb.count_in, valid);
-    if (valid) wb.q_in[slot] = p;
-  }
+  __shared__ uint32_t queued[WAVE_THREADS / 32][WQ_CAP];
+  WarpQueue queue(queued[threadIdx.x >> 5]);
+  const WarpShare share(total);
+  for (uint32_t p0 = share.first; p0 < total; p0 += share.stride)
+    for (uint32_t r = 0; r < share.runs && p0 + r < total; r += 32u) {
+      const uint32_t p = p0 + r + (threadIdx.x & 31u);
+      bool valid = false;
+      if (p < total) {
+        const uint32_t l = p % n_list, i = spp1 + e0 + p / n_list, id = wb.rlist[l];
+        float4 o4, d4;
+        uint32_t hs;
+        valid = camera_path(cp, id, i, o4, d4, hs);
+        init_path(wb, p, o4, d4, id, i, hs, valid);
+      }
+      __syncwarp();
+      queue.push(valid, p, wb.count_in, wb.q_in);
+    }
+  queue.flush(wb.count_in, wb.q_in);
 }
 
 __global__ void __launch_bounds__(WAVE_THREADS) refine_finalize(const CamParams cp, WaveBufs wb, uint32_t spp1, uint32_t e0, uint32_t n_e,
