@@ -167,8 +167,9 @@ __device__ __forceinline__ PathWords path_words(const ConstRecord& P, uint32_t d
   return W;
 }
 
-// one rounding each, whatever the compiler knows of the operands in an unrolled loop
+// one rounding each in this order, whatever the compiler knows of the operands in an unrolled loop
 __device__ __forceinline__ float3 mac3(float3 a, float b, float3 c) { return f3(__fmaf_rn(a.x, b, c.x), __fmaf_rn(a.y, b, c.y), __fmaf_rn(a.z, b, c.z)); }
+__device__ __forceinline__ float dot_fma(float3 a, float3 b) { return __fmaf_rn(a.z, b.z, __fmaf_rn(a.x, b.x, __fmul_rn(a.y, b.y))); }
 
 // radiance of a recorded path
 __device__ __forceinline__ float3 path_value(const CalibDev& C, const ConstRecord& P, uint32_t depth, uint32_t nl) {
@@ -229,7 +230,7 @@ __device__ __forceinline__ void path_grad(const CalibDev& C, const ConstRecord& 
     for (uint32_t j = 0; j < CAL_MAX_NL; j++) {
       const float q = W.q[k][j];
       if (j >= nl || q == 0.0f) continue;
-      atomicAdd(sh_lamp + W.lamp[k][j], double(dot(g, T) * q / fnl));
+      atomicAdd(sh_lamp + W.lamp[k][j], double(dot_fma(g, T) * q / fnl));
       s += __ldg(C.lamp + W.lamp[k][j]) * q;
     }
     if (s != 0.0f) D[k] = D[k] + g * T * (s / fnl);
@@ -243,7 +244,7 @@ __device__ __forceinline__ void path_grad(const CalibDev& C, const ConstRecord& 
     }
   }
   if (lamp != MISS && emit_a != 0.0f) {
-    atomicAdd(sh_lamp + lamp, double(dot(g, T) * emit_a));
+    atomicAdd(sh_lamp + lamp, double(dot_fma(g, T) * emit_a));
     if (n) {
       const float Le = emit_a * __ldg(C.lamp + lamp);
 #pragma unroll
