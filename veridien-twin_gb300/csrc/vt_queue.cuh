@@ -5,6 +5,23 @@
 
 namespace vtk {
 
+// A path with a next ray, with light samples or both to the next bounce's queue and the bounce's shadow queue (WaveBufs, whose
+// counts of the two are neighbours): one atomic a warp for both. A warp waits for its answer at the end of each 32 paths, and the
+// counter's line takes one in ~1.3 ns (one for each queue, 640x480, 16 spp: 14.42 ms, pose batch
+// 83.9; now 14.32, 83.2)
+template <typename Bufs>
+__device__ __forceinline__ void append_path(const Bufs& wb, uint32_t p, bool cont, bool shadow) {
+  const uint32_t act = __activemask(), lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
+  const uint32_t mc = __ballot_sync(act, cont), ms = __ballot_sync(act, shadow);
+  if (!(mc | ms)) return;
+  const uint32_t leader = __ffs(act) - 1;
+  unsigned long long base = 0;
+  if (lane == leader) base = atomicAdd(reinterpret_cast<unsigned long long*>(wb.count_out), (unsigned long long)__popc(ms) << 32 | uint32_t(__popc(mc)));
+  const uint32_t b0 = __shfl_sync(act, uint32_t(base), leader), b1 = __shfl_sync(act, uint32_t(base >> 32), leader);
+  if (cont) wb.q_out[b0 + __popc(mc & below)] = p;
+  if (shadow) wb.q_sh[b1 + __popc(ms & below)] = p;
+}
+
 // A warp's entries for a queue, kept in shared memory and appended by one atomic when they are many (or at the end): for the
 // short kernels, which with an atomic a warp for each 32 paths were bound by the counter's line, ~1.3 ns each (camera rays
 // of 4.3 M paths 176 us, now 97; bytes 50). In the shading the queue's state costs more registers than the atomics time

@@ -27,19 +27,6 @@ constexpr int WAVE_THREADS = 256;
 #define VT_TRACE_BLOCKS 4
 #endif
 
-// append `want` lanes' items to a queue with one atomic per warp; returns the slot of this lane (if want)
-__device__ __forceinline__ uint32_t warp_append(uint32_t* count, bool want) {
-  const uint32_t act = __activemask();
-  const uint32_t mask = __ballot_sync(act, want);
-  if (!mask) return 0;
-  const uint32_t lane = threadIdx.x & 31u;
-  const uint32_t leader = __ffs(mask) - 1;
-  uint32_t base = 0;
-  if (lane == leader) base = atomicAdd(count, uint32_t(__popc(mask)));
-  base = __shfl_sync(act, base, leader);
-  return base + __popc(mask & ((1u << lane) - 1u));
-}
-
 __device__ __forceinline__ void init_path(const WaveBufs& wb, uint32_t p, float4 o4, float4 d4, uint32_t id, uint32_t i, uint32_t hs, bool valid) {
   wb.o[p] = o4;
   wb.d[p] = d4;
@@ -215,8 +202,7 @@ __global__ void __launch_bounds__(WAVE_THREADS, VT_TRACE_BLOCKS) wave_extend(con
   const uint32_t lanes = lanes_of(n);
   while (serve_lanes(state, exhausted, wb.fetch, n, cp.refill, lanes, next, start)) trace_round<false>(S, 0.0f, st, stk, state);
   asm volatile("griddepcontrol.wait;" ::: "memory");   // launched beside the light samples: the next kernel follows both
-  // theirs, the next bounce's (a batch's cull_shadow_kernel reads them once more)
-  if (VAR != WAVE_SHARED && blockIdx.x == 0 && threadIdx.x == 0) *reinterpret_cast<uint4*>(wb.count_out) = make_uint4(0, 0, 0, 0);
+  if (blockIdx.x == 0 && threadIdx.x == 0) *reinterpret_cast<uint4*>(wb.count_out) = make_uint4(0, 0, 0, 0);   // the next bounce's
 }
 
 template <int MODE, int VAR>
@@ -349,10 +335,7 @@ __global__ void __launch_bounds__(WAVE_THREADS, VT_WAVE_SHADE_BLOCKS) wave_shade
       }
     }
     wb.L[p] = make_float4(L.x, L.y, L.z, L4.w);
-    const uint32_t qs = warp_append(wb.count_out, cont);
-    if (cont) wb.q_out[qs] = p;
-    const uint32_t ss = warp_append(wb.count_sh, shadow);
-    if (shadow) wb.q_sh[ss] = p;
+    append_path(wb, p, cont, shadow);
   }
 }
 
@@ -674,17 +657,18 @@ int shade_grid() {
 }
 
 // The queue of bounce b in (qa | qb), the next bounce's in the other; of the counts four words per bounce in turn: the
-// queue's length, shadow paths, entries taken by the closest-hit and by the any-hit lanes. They are clear for the next
-// bounce once the closest hits of this one and the light samples of the one before are traced
+// queue's length and the previous bounce's shadow paths (one shading kernel fills both: append_path), and what the closest-hit
+// and the any-hit lanes have taken of them. They are clear for the next bounce once the closest hits of this one and the
+// light samples of the one before are traced
 void bounce_view(WaveBufs& w, uint32_t b) {
   const uint32_t odd = b & 1u;
   w.q_in = odd ? w.qa : w.qb;
   w.q_out = odd ? w.qb : w.qa;
   w.count_in = w.counts + (odd ? 0 : 4);
   w.count_out = w.counts + (odd ? 4 : 0);
-  w.count_sh = w.count_in + 1;
+  w.count_sh = w.count_out + 1;
   w.fetch = w.count_in + 2;
-  w.fetch_sh = w.count_in + 3;
+  w.fetch_sh = w.count_out + 3;
 }
 
 // launched before the kernel ahead has ended, whose results `kernel` waits for itself (griddepcontrol.wait)
@@ -733,7 +717,6 @@ void wave_bounces_of(const Scene& S, const CamParams& cp, const WaveBufs& wb, in
     }
     if (b > depth) break;
     bounce_view(w, b);
-    if (VAR == WAVE_SHARED) cudaMemsetAsync(w.count_out, 0, 16, st);
     {
       TimedLaunch tl(timer, st, 1);
       if (cp.mode == VT_SHADE_TWIN) launch_dependent(wave_shade<VT_SHADE_TWIN, VAR>, shade_grid<VT_SHADE_TWIN, VAR>(), st, !timer, S, cp, w);
