@@ -858,39 +858,6 @@ __device__ __forceinline__ float capsule_vis(const Scene& S, float3 p, float3 n)
   }
   return clampf(v, 0.0f, 1.0f);
 }
-// The frame's capsules, laid out once per block: their axes are a square root, three divisions and nine words a point else
-// (the seven bodies' occlusions were 39 % of the twin's shading: frame of three cameras with refinement 8.95 -> 8.54 ms,
-// with the shading's shorter live ranges)
-struct Capsules {
-  float4 ar[VT_MAX_INST], el[VT_MAX_INST];   // a, r; e, L
-  float hides[VT_MAX_INST];
-  uint32_t n;
-};
-__device__ __forceinline__ void load_capsules(const Scene& S, Capsules& C) {   // the whole block calls it
-  static_assert(VT_MAX_INST <= 32, "a lane per body");
-  if (threadIdx.x < 32u) {
-    float3 a, e;
-    float r, L, hides;
-    const bool have = threadIdx.x < min(ldu(S.su + 16), uint32_t(VT_MAX_INST)) && load_capsule(S, threadIdx.x, a, r, e, L, hides);
-    const uint32_t mask = __ballot_sync(0xffffffffu, have);
-    if (have) {
-      const uint32_t k = __popc(mask & ((1u << threadIdx.x) - 1u));
-      C.ar[k] = make_float4(a.x, a.y, a.z, r);
-      C.el[k] = make_float4(e.x, e.y, e.z, L);
-      C.hides[k] = hides;
-    }
-    if (threadIdx.x == 0) C.n = __popc(mask);
-  }
-  __syncthreads();
-}
-__device__ __forceinline__ float capsule_vis(const Capsules& C, float3 p, float3 n) {
-  float v = 1.0f;
-  for (uint32_t i = 0; i < C.n; i++) {
-    const float4 ar = C.ar[i], el = C.el[i];
-    v = v - capsule_occ(p, n, xyz(ar), ar.w, xyz(el), el.w) * C.hides[i];
-  }
-  return clampf(v, 0.0f, 1.0f);
-}
 // barycentrics renormalised over the triangle's active nodes (gpu/wgsl/shade.wgsl.js:194-209)
 __device__ __forceinline__ float3 node_weights(const Scene& S, const Surf& s, uint32_t slot) {
   const float3 w = s.b * f3(__ldg(S.nstate + 4u * s.vi0 + slot).w, __ldg(S.nstate + 4u * s.vi1 + slot).w, __ldg(S.nstate + 4u * s.vi2 + slot).w);

@@ -215,7 +215,7 @@ __device__ __forceinline__ float3 eval_bsdf_v(const Mat& M, const BsdfView& B, f
 }
 
 // fsCam (lite_nodes/renderer.js:284) for triangle `tri` at the centre of pixel (px, py); radiance x outScale
-__device__ float3 fragment(const Scene& S, const Geo& g, const View& V, const ShadeArgs& a, const Capsules& caps, uint32_t tri, uint32_t px, uint32_t py) {
+__device__ float3 fragment(const Scene& S, const Geo& g, const View& V, const ShadeArgs& a, uint32_t tri, uint32_t px, uint32_t py) {
   uint4 va[3], vb[3];
   float4 c[3];
   for (int j = 0; j < 3; j++) {
@@ -317,7 +317,7 @@ __device__ float3 fragment(const Scene& S, const Geo& g, const View& V, const Sh
   if (is_static) {
     float3 E = f3(0.0f, 0.0f, 0.0f);
     if (ew.w > 1e-6f) E = f3(ew.x, ew.y, ew.z) / ew.w;
-    E = E * capsule_vis(caps, p, ns);
+    E = E * capsule_vis(S, p, ns);
     L = L + E * INV_PI_F * Al;
   } else {
     L = L + v3(V.env) * Al;
@@ -386,12 +386,10 @@ __global__ void __launch_bounds__(128, VT_SHADE_BLOCKS) shade_frag_kernel(const 
                                                          uint32_t cap, const uint32_t* __restrict__ counts, uint2* __restrict__ colors) {
   const uint32_t ns = counts[0], nd = counts[1];
   const uint32_t W = uint32_t(V.size[0]);
-  __shared__ Capsules caps;
-  load_capsules(S, caps);
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < ns + nd; i += gridDim.x * blockDim.x) {
     const uint32_t fi = i < nd ? cap - nd + i : i - nd;   // the longer ones first
     const uint2 fr = frags[fi];
-    const float3 c = fragment(S, g, V, a, caps, fr.y, fr.x % W, fr.x / W);
+    const float3 c = fragment(S, g, V, a, fr.y, fr.x % W, fr.x / W);
     const __half2 rg = __floats2half2_rn(c.x, c.y), bz = __floats2half2_rn(c.z, 0.0f);
     colors[fi] = make_uint2(*reinterpret_cast<const uint32_t*>(&rg), *reinterpret_cast<const uint32_t*>(&bz));
   }

@@ -218,10 +218,6 @@ __global__ void __launch_bounds__(WAVE_THREADS, VT_WAVE_SHADE_BLOCKS) wave_shade
   const uint32_t nl = cp.n_light;
   const bool no_mis = (cp.options & VT_O_NO_MIS) != 0u;
   const float emit_area = __ldg(S0.su + 3);
-  // a batch's pairs have a pose each
-  constexpr bool ONE_POSE = MODE == VT_SHADE_TWIN && VAR != WAVE_PAIRS;
-  __shared__ Capsules caps;
-  if (ONE_POSE) load_capsules(S0, caps);
   for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
     const uint32_t p = wb.q_in[k];
     const Scene S = path_scene<VAR>(S0, wb, p);
@@ -279,7 +275,7 @@ __global__ void __launch_bounds__(WAVE_THREADS, VT_WAVE_SHADE_BLOCKS) wave_shade
         // the node radiosity first: its nodes and weights are not held over the light samples
         if (MODE == VT_SHADE_TWIN && is_static && !(cp.options & (VT_O_NO_INDIRECT | VT_O_DIRECT_ONLY))) {
           float3 E = node_slot(S, s, 0u, ldu(S.su + 18));
-          if (!(cp.options & VT_O_NO_CAPSULE)) E = E * (ONE_POSE ? capsule_vis(caps, s.p, n) : capsule_vis(S, s.p, n));
+          if (!(cp.options & VT_O_NO_CAPSULE)) E = E * capsule_vis(S, s.p, n);
           L = L + E * INV_PI_F * albedo(S, s.mat, fmaxf(dot(n, wo), 0.0f));
         }
         const Mat M = load_mat(S, s.mat);
