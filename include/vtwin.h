@@ -540,6 +540,12 @@ vt_status vt_get_node_state(vt_ctx* ctx, float* state, uint32_t* slot);
  * browser's). */
 vt_status vt_wait_check(vt_ctx* ctx, uint64_t cycles, int arrive);
 
+/* What the host has been refused, on purpose, so that a program or a test sees what a call does then: allocations of more
+ * than `limit` bytes of a kind are refused on the host, as a device without the memory refuses them (UINT64_MAX: none).
+ * WAVE: the path tracer's wavefront state (a render with refinement then takes it in smaller waves, or VT_ERR_OOM). */
+enum { VT_REFUSE_WAVE = 0 };
+vt_status vt_refuse(vt_ctx* ctx, uint32_t what, uint64_t limit);
+
 /* ------------------------------------------------------------------- lite_nodes: the raster camera pass */
 
 /* lite_nodes/renderer.js: a raster live renderer that keeps the node radiosity (vt_nodes_*) and replaces the camera

@@ -137,7 +137,7 @@ vt_status vt_destroy(vt_ctx* ctx) {
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
   for (auto& c : ctx->cams) { cudaFree(c.radiance); cudaFree(c.raw); cudaFree(c.ri); cudaFree(c.isp_mem); cudaFree(c.hcache); cudaFree(c.scache); }
   cudaFree(ctx->d_nodes); cudaFree(ctx->d_tris); cudaFree(ctx->d_verts); cudaFree(ctx->d_params); cudaFree(ctx->d_nstate);
-  cudaFree(ctx->d_su); cudaFree(ctx->d_dbg); cudaFree(ctx->d_work); cudaFree(ctx->d_scratch); cudaFree(ctx->d_wave); cudaFree(ctx->tc.mem);
+  cudaFree(ctx->d_su); cudaFree(ctx->d_dbg); cudaFree(ctx->d_work); cudaFree(ctx->d_scratch); cudaFree(ctx->wave.p); cudaFree(ctx->tc.mem);
   cudaFree(ctx->batch.su); cudaFree(ctx->batch.cull); cudaFree(ctx->batch.ctr); cudaFree(ctx->batch.sensor); cudaFree(ctx->batch.mem);
   cudaFree(ctx->batch.rad); cudaFree(ctx->batch.raw);
   if (ctx->batch.exec) cudaGraphExecDestroy(ctx->batch.exec);
@@ -328,26 +328,20 @@ static vt_status render_impl(vt_ctx* ctx, const vt_render_req* q, float* out_rgb
   cp2.refine = cp.refine;
   if (q->frame != ctx->frame) { ctx->frame = q->frame; vt_status s = write_su(ctx); if (s != VT_OK) return s; }
   // wave of up to 8 M paths (whole sub-sample indices): ~1.4 GB of path state at one light sample. The refinement's
-  // sub-samples count too: how many pixels they are taken for is not known here, and in waves of pass 1's (one of
-  // each pixel in the twin's presets) it ran in launches that were mostly tails: twin frame
-  // of three 1280x720 cameras with 6 more sub-samples, 10.8 ms in six waves, 8.95 in one
-  const uint32_t n_pix = vtk::tiled_pixels(c.width, c.height, cp.tile_w, cp.tile_h), nl_max = std::max(cp.n_light, cp2.n_light);
+  // sub-samples in one wave too, of their own light samples: how many pixels they are taken for is not known here, and in
+  // waves of pass 1's (one of each pixel in the twin's presets) it ran in launches that were mostly tails: twin frame
+  // of three 1280x720 cameras with 6 more sub-samples, 10.8 ms in six waves, 8.95 in one. Without the memory for that
+  // (0.97 GB a 1280x720 camera), in the waves that what there is holds.
+  const uint32_t n_pix = vtk::tiled_pixels(c.width, c.height, cp.tile_w, cp.tile_h);
   const uint32_t per_max = std::max(1u, (8u << 20) / std::max(1u, n_pix));
-  const uint32_t paths_least = std::min(std::max(1u, cp.spp), per_max) * n_pix;
-  uint32_t paths = std::max(paths_least, std::min(cp.refine, per_max) * n_pix);
-  for (;;) {
-    const size_t need = vtk::wave_bytes(paths, nl_max, n_pix);
-    if (ctx->wave_cap >= need) break;
-    VT_CK(cudaStreamSynchronize(ctx->stream));
-    cudaFree(ctx->d_wave);
-    ctx->d_wave = nullptr;
-    ctx->wave_cap = 0;
-    if (cudaMalloc(&ctx->d_wave, need) == cudaSuccess) { ctx->wave_cap = need; break; }
-    cudaGetLastError();
-    if (paths == paths_least) return fail(ctx, VT_ERR_OOM, "wavefront state allocation failed");
-    paths = paths_least;   // the refinement in smaller waves
-  }
-  vtk::WaveBufs wb = vtk::wave_carve(ctx->d_wave, paths, nl_max, n_pix, ctx->d_work);
+  const uint32_t paths = std::min(std::max(1u, cp.spp), per_max) * n_pix;
+  uint32_t per2 = std::min(cp.refine, per_max);
+  const size_t least = std::max(vtk::wave_bytes(paths, cp.n_light, n_pix), cp.refine ? vtk::wave_bytes(n_pix, cp2.n_light, n_pix) : 0);
+  WaveMemory mem{ctx};
+  if (!ctx->wave.try_grow(mem, std::max(least, cp.refine ? vtk::wave_bytes(per2 * n_pix, cp2.n_light, n_pix) : 0)) && !ctx->wave.grow(mem, least))
+    return fail(ctx, VT_ERR_OOM, "wavefront state allocation failed");
+  while (per2 > 1 && vtk::wave_bytes(per2 * n_pix, cp2.n_light, n_pix) > ctx->wave.cap) per2--;
+  vtk::WaveBufs wb = vtk::wave_carve(ctx->wave.p, paths, cp.n_light, n_pix, ctx->d_work);
   wb.rcount = ctx->d_work + 12;
   if (q->options & (VT_O_CACHE_WRITE | VT_O_CACHE_READ)) {
     // the cache stays valid while what decides a camera ray's static hit holds (its time does not: the static
@@ -399,8 +393,11 @@ static vt_status render_impl(vt_ctx* ctx, const vt_render_req* q, float* out_rgb
   vtk::KernelTimer timer{ctx->kev.data(), ctx->kkind.data(), int(ctx->kev.size() / 2), 0};
   if (ctx->kprof) wb.stats = reinterpret_cast<unsigned long long*>(ctx->d_work + 16);
   VT_CK(cudaEventRecord(ctx->ev0, ctx->stream));
+  // the refinement's view of the buffer: its paths, pass 1's sums and queue of pixels
+  vtk::WaveBufs wb2 = vtk::wave_carve(ctx->wave.p, per2 * n_pix, cp2.n_light, n_pix, ctx->d_work);
+  wb2.rcount = wb.rcount; wb2.hcache = wb.hcache; wb2.hc_stride = wb.hc_stride; wb2.hc_cap = wb.hc_cap; wb2.scache = wb.scache; wb2.stats = wb.stats;
   vtk::wave_render(dev_scene(ctx), cp, wb, paths, ctx->cams[q->camera].radiance, ctx->wave_blocks, ctx->stream, &ctx->tim.launches,
-                   ctx->kprof ? &timer : nullptr, &cp2);
+                   ctx->kprof ? &timer : nullptr, cp2, wb2, per2);
   VT_CK(cudaGetLastError());
   VT_CK(cudaEventRecord(ctx->ev1, ctx->stream));
   ctx->cams[q->camera].rendered = true;
@@ -755,6 +752,13 @@ vt_status vt_wait_check(vt_ctx* ctx, uint64_t cycles, int arrive) {
   VT_CK(cudaMemcpyAsync(&e, err, 4, cudaMemcpyDeviceToHost, ctx->stream));
   VT_CK(cudaStreamSynchronize(ctx->stream));
   return e ? fail(ctx, VT_ERR_TIMEOUT, "wait check: the barrier phase did not complete within the limit") : VT_OK;
+}
+
+vt_status vt_refuse(vt_ctx* ctx, uint32_t what, uint64_t limit) {
+  if (!ctx) return VT_ERR_ARG;
+  if (what != VT_REFUSE_WAVE) return fail(ctx, VT_ERR_ARG, "refuse: unknown resource");
+  ctx->refuse_wave = size_t(limit);
+  return VT_OK;
 }
 
 vt_status vt_timings_get(const vt_ctx* ctx, vt_timings* out) {

@@ -238,6 +238,7 @@ vt_status vt_calib_forward(vt_ctx* ctx, const vt_calib_req* q, double* loss) {
   K.want_k = q->intrinsics != 0;
   K.have_k = false;
   uint32_t wave_paths = 0;
+  WaveMemory mem{ctx};
   if (!q->replay) {
     size_t fr = 0, tot = 0;
     cudaMemGetInfo(&fr, &tot);
@@ -245,7 +246,7 @@ vt_status vt_calib_forward(vt_ctx* ctx, const vt_calib_req* q, double* loss) {
     const size_t tan_bytes = K.want_k ? vtk::calib_tan_bytes(uint32_t(std::min<size_t>(rec_total, 0xffffffffu))) : 0;
     wave_paths = uint32_t(std::min<size_t>(8u << 20, rec_total));
     const size_t wave_need = vtk::wave_bytes(wave_paths, cps[0].n_light, 0);
-    if (rec_total < 0xffffffffu && rec_bytes + tan_bytes + (ctx->wave_cap >= wave_need ? 0 : wave_need) <= fr / 2) {
+    if (rec_total < 0xffffffffu && rec_bytes + tan_bytes + (ctx->wave.cap >= wave_need ? 0 : wave_need) <= fr / 2) {
       vt_status st = VT_OK;
       if (K.rec_cap < rec_bytes) {
         VT_CK(cudaStreamSynchronize(ctx->stream));
@@ -263,14 +264,7 @@ vt_status vt_calib_forward(vt_ctx* ctx, const vt_calib_req* q, double* loss) {
         if (cudaMalloc(&K.tan, tan_bytes) != cudaSuccess) { cudaGetLastError(); st = VT_ERR_OOM; }
         else K.tan_cap = tan_bytes;
       }
-      if (st == VT_OK && ctx->wave_cap < wave_need) {
-        VT_CK(cudaStreamSynchronize(ctx->stream));
-        cudaFree(ctx->d_wave);
-        ctx->d_wave = nullptr;
-        ctx->wave_cap = 0;
-        if (cudaMalloc(&ctx->d_wave, wave_need) != cudaSuccess) { cudaGetLastError(); st = VT_ERR_OOM; }
-        else ctx->wave_cap = wave_need;
-      }
+      if (st == VT_OK && !ctx->wave.grow(mem, wave_need)) st = VT_ERR_OOM;
       K.stored = st == VT_OK;
     }
   }
@@ -300,11 +294,7 @@ vt_status vt_calib_forward(vt_ctx* ctx, const vt_calib_req* q, double* loss) {
       cap_bytes = need;
       return true;
     };
-    void* wave = ctx->d_wave;
-    size_t wave_cap = ctx->wave_cap;
-    const bool ok = grow(K.records, K.rec_cap, rec_bytes) && (!tan_bytes || grow(K.tan, K.tan_cap, tan_bytes)) && grow(wave, wave_cap, wave_need);
-    ctx->d_wave = wave;
-    ctx->wave_cap = wave_cap;
+    const bool ok = grow(K.records, K.rec_cap, rec_bytes) && (!tan_bytes || grow(K.tan, K.tan_cap, tan_bytes)) && ctx->wave.grow(mem, wave_need);
     if (!ok) return fail(ctx, VT_ERR_OOM, "calib: replay buffers (one chunk of path records and the wave state)");
     // the paths' decisions (24 B each) when they fit in a quarter of what is left; otherwise the backward traces
     // again. VT_CALIB_RETRACE=1 makes it trace again regardless.
@@ -325,12 +315,12 @@ vt_status vt_calib_forward(vt_ctx* ctx, const vt_calib_req* q, double* loss) {
     const int blocks = std::min<int>(ctx->wave_blocks * 2, int(K.max_partials));
     uint32_t nb;
     if (K.stored) {
-      const vtk::WaveBufs wb = vtk::wave_carve(ctx->d_wave, wave_paths, cp.n_light, 0, ctx->d_work);
+      const vtk::WaveBufs wb = vtk::wave_carve(ctx->wave.p, wave_paths, cp.n_light, 0, ctx->d_work);
       nb = vtk::calib_wave_forward(dev_scene(ctx), cp, C, wb, wave_paths, static_cast<char*>(K.records) + K.rec_off[c] * vtk::calib_record_bytes(1),
                                    K.want_k ? static_cast<char*>(K.tan) + K.rec_off[c] * vtk::calib_tan_bytes(1) : nullptr,
                                    std::min<int>(ctx->wave_blocks, int(K.max_partials)), ctx->stream);
     } else {
-      const vtk::WaveBufs wb = vtk::wave_carve(ctx->d_wave, K.wave_paths, cp.n_light, 0, ctx->d_work);
+      const vtk::WaveBufs wb = vtk::wave_carve(ctx->wave.p, K.wave_paths, cp.n_light, 0, ctx->d_work);
       const int wblocks = std::min<int>(ctx->wave_blocks, int(K.max_partials));
       nb = 0;
       for (uint32_t i0 = 0; i0 < cp.spp; i0 += K.chunk)
@@ -366,6 +356,10 @@ vt_status vt_calib_backward(vt_ctx* ctx, double* g_albedo, double* g_lamp) {
   VT_CK(cudaMemsetAsync(K.g_lamp, 0, size_t(K.n_lamps) * 8, ctx->stream));
   VT_CK(cudaMemsetAsync(K.g_H, 0, n * 24, ctx->stream));
   VT_CK(cudaMemsetAsync(K.g_K, 0, ctx->S.cams.size() * 64, ctx->stream));
+  // a call since the forward may have left a smaller wave buffer than the replay's
+  WaveMemory mem{ctx};
+  const uint32_t nl = calib_cam(ctx, K.cams[0], K.spp, K.nl, K.seed, K.depth).n_light;
+  if (!K.stored && !ctx->wave.grow(mem, vtk::wave_bytes(K.wave_paths, nl, 0))) return fail(ctx, VT_ERR_OOM, "calib: the replay's wave state");
   // every camera of the forward: from the kept records, or by tracing each path again
   for (size_t c = 0; c < K.cams.size(); c++) {
     const uint32_t cam = K.cams[c];
@@ -375,7 +369,7 @@ vt_status vt_calib_backward(vt_ctx* ctx, double* g_albedo, double* g_lamp) {
                                   K.want_k ? static_cast<char*>(K.tan) + K.rec_off[c] * vtk::calib_tan_bytes(1) : nullptr,
                                   ctx->wave_blocks * 2, ctx->stream);
     else {
-      const vtk::WaveBufs wb = vtk::wave_carve(ctx->d_wave, K.wave_paths, cp.n_light, 0, ctx->d_work);
+      const vtk::WaveBufs wb = vtk::wave_carve(ctx->wave.p, K.wave_paths, cp.n_light, 0, ctx->d_work);
       const int wblocks = std::min<int>(ctx->wave_blocks, int(K.max_partials));
       for (uint32_t i0 = 0; i0 < cp.spp; i0 += K.chunk)
         vtk::calib_wave_chunk(dev_scene(ctx), cp, calib_dev(ctx, cam), wb, K.wave_paths, K.records, K.want_k ? K.tan : nullptr, i0,

@@ -11,6 +11,7 @@
 #include <string>
 #include <vector>
 
+#include "vt_grow.h"
 #include "vt_host.h"
 #include "vt_kernels.cuh"
 #include "vt_isp.cuh"
@@ -36,8 +37,9 @@ struct vt_ctx {
   uint32_t* d_dbg = nullptr;
   uint32_t* d_work = nullptr;   // queue counters of the wavefront path tracer
   int wave_blocks = 0;
-  void* d_wave = nullptr;       // wavefront path state (grown on demand)
-  size_t wave_cap = 0;
+  vtapi::GrowBuffer wave;       // wavefront path state of renders and calibrations
+  // what tests have the host refuse (vt_refuse): bytes of the wavefront's state
+  size_t refuse_wave = SIZE_MAX;
   struct Cam {
     float4* radiance = nullptr;
     float* raw = nullptr;
@@ -259,6 +261,24 @@ inline vt_status ensure_scratch(vt_ctx* ctx, size_t bytes) {
   ctx->scratch_bytes = bytes;
   return VT_OK;
 }
+
+// the device side of ctx->wave's growth
+struct WaveMemory {
+  vt_ctx* ctx;
+  void* alloc(size_t bytes) {
+    void* p = nullptr;
+    if (bytes > ctx->refuse_wave || cudaMalloc(&p, bytes) == cudaSuccess) return p;
+    cudaGetLastError();
+    return nullptr;
+  }
+  void free(void* p) { cudaFree(p); }
+  void sync() { cudaStreamSynchronize(ctx->stream); }
+  size_t room() {
+    size_t free_bytes = 0, total = 0;
+    if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) { cudaGetLastError(); return 0; }
+    return std::min(free_bytes, ctx->refuse_wave);
+  }
+};
 
 inline vtd::Scene dev_scene(vt_ctx* ctx) {
   vtd::Scene S;

@@ -600,6 +600,9 @@ WaveBufs wave_carve(void* base, uint32_t paths, uint32_t n_light, uint32_t n_pix
   auto take = [&](size_t bytes) { char* r = c; c += (bytes + 255) / 256 * 256; return r; };
   const size_t P = paths;
   WaveBufs w{};
+  w.acc = reinterpret_cast<float4*>(take(size_t(n_pix) * 16));   // first: the same of one base for any number of paths
+  w.acc2 = reinterpret_cast<float4*>(take(size_t(n_pix) * 16));
+  w.rlist = reinterpret_cast<uint32_t*>(take(size_t(n_pix) * 4));
   w.o = reinterpret_cast<float4*>(take(P * 16));
   w.d = reinterpret_cast<float4*>(take(P * 16));
   w.thr = reinterpret_cast<float4*>(take(P * 16));
@@ -612,9 +615,6 @@ WaveBufs wave_carve(void* base, uint32_t paths, uint32_t n_light, uint32_t n_pix
   w.qb = reinterpret_cast<uint32_t*>(take(P * 4));
   w.q_sh = reinterpret_cast<uint32_t*>(take(P * 4));
   w.sh = reinterpret_cast<float4*>(take(P * size_t(n_light) * 48));
-  w.acc = reinterpret_cast<float4*>(take(size_t(n_pix) * 16));
-  w.acc2 = reinterpret_cast<float4*>(take(size_t(n_pix) * 16));
-  w.rlist = reinterpret_cast<uint32_t*>(take(size_t(n_pix) * 4));
   w.rcount = nullptr;
   w.hcache = nullptr;
   w.scache = nullptr;
@@ -757,7 +757,7 @@ void wave_gen_pairs(const CamParams& cp, WaveBufs wb, int blocks, cudaStream_t s
 
 // one camera: waves of whole sub-sample indices, each bounce extend -> shade -> shadow over compacted queues
 void wave_render(const Scene& S, const CamParams& cp, WaveBufs wb, uint32_t wave_paths, float4* out, int blocks, cudaStream_t st,
-                 uint64_t* launches, KernelTimer* timer, const CamParams* cp2) {
+                 uint64_t* launches, KernelTimer* timer, const CamParams& cp2, const WaveBufs& wb2, uint32_t per2) {
   const uint32_t n_pix = tiled_pixels(cp.w, cp.h, cp.tile_w, cp.tile_h);
   const uint32_t per_wave = std::max(1u, std::min(cp.spp, wave_paths / n_pix));
   uint64_t nlaunch = 0;
@@ -769,23 +769,22 @@ void wave_render(const Scene& S, const CamParams& cp, WaveBufs wb, uint32_t wave
     wave_gen<<<blocks, WAVE_THREADS, 0, st>>>(cp, w, i0, n_i, n_pix);
     nlaunch++;
     wave_bounces(S, cp, wb, WAVE_PLAIN, blocks, st, &nlaunch, timer);
-    const int last = i0 + n_i >= cp.spp && !(cp.refine && cp2 && wb.rcount);
+    const int last = i0 + n_i >= cp.spp && !cp.refine;
     wave_finalize<<<blocks, WAVE_THREADS, 0, st>>>(cp, wb, i0, n_i, n_pix, wb.acc, out, last);
     nlaunch++;
   }
-  if (cp.refine && cp2 && wb.rcount) {
+  if (cp.refine) {
     cudaMemsetAsync(wb.rcount, 0, 4, st);
     refine_select<<<blocks, WAVE_THREADS, 0, st>>>(cp, S, wb, n_pix, out);
     nlaunch++;
-    const uint32_t per = std::max(1u, std::min(cp.refine, wave_paths / n_pix));
-    for (uint32_t e0 = 0; e0 < cp.refine; e0 += per) {
-      const uint32_t n_e = std::min(per, cp.refine - e0);
-      cudaMemsetAsync(wb.counts, 0, 16, st);
-      WaveBufs w = wb;
-      w.q_in = wb.qa; w.count_in = wb.counts + 0;
-      refine_gen<<<blocks, WAVE_THREADS, 0, st>>>(*cp2, w, cp.spp, e0, n_e);
-      wave_bounces(S, *cp2, wb, WAVE_PLAIN, blocks, st, &nlaunch, timer);
-      refine_finalize<<<blocks, WAVE_THREADS, 0, st>>>(cp, wb, cp.spp, e0, n_e, out, e0 + n_e >= cp.refine);
+    for (uint32_t e0 = 0; e0 < cp.refine; e0 += per2) {
+      const uint32_t n_e = std::min(per2, cp.refine - e0);
+      cudaMemsetAsync(wb2.counts, 0, 16, st);
+      WaveBufs w = wb2;
+      w.q_in = wb2.qa; w.count_in = wb2.counts + 0;
+      refine_gen<<<blocks, WAVE_THREADS, 0, st>>>(cp2, w, cp.spp, e0, n_e);
+      wave_bounces(S, cp2, wb2, WAVE_PLAIN, blocks, st, &nlaunch, timer);
+      refine_finalize<<<blocks, WAVE_THREADS, 0, st>>>(cp, wb2, cp.spp, e0, n_e, out, e0 + n_e >= cp.refine);
       nlaunch += 2;
     }
   }

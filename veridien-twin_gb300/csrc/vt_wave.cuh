@@ -81,9 +81,10 @@ void bounce_view(WaveBufs& w, uint32_t b);
 size_t wave_bytes(uint32_t paths, uint32_t n_light, uint32_t n_pix);
 WaveBufs wave_carve(void* base, uint32_t paths, uint32_t n_light, uint32_t n_pix, uint32_t* counts);
 // one camera: pass 1 (cp.spp sub-samples per pixel), then when cp.refine > 0 pass 2 over the selected pixels with
-// cp2 (the refinement's light samples) continuing the sub-sample sequences
+// cp2 (the refinement's light samples) continuing the sub-sample sequences, per2 of them at a time in wb2: a view of wb's
+// buffer for its own number of paths and light samples, with the same acc, acc2 and rlist
 void wave_render(const vtd::Scene& S, const CamParams& cp, WaveBufs wb, uint32_t wave_paths, float4* out, int blocks, cudaStream_t st,
-                 uint64_t* launches, KernelTimer* timer = nullptr, const CamParams* cp2 = nullptr);
+                 uint64_t* launches, KernelTimer* timer, const CamParams& cp2, const WaveBufs& wb2, uint32_t per2);
 int wave_blocks_per_sm();
 
 // one wave's bounces (extend, shade, shadow per bounce) over the paths queued in wb.qa / counts[0]
