@@ -16,7 +16,7 @@ PROGRAM = r'''
 #include "vt_grow.h"
 
 struct Dev {
-  size_t total, used = 0, asked = 0, freed = 0, synced = 0;
+  size_t total = 0, used = 0, asked = 0, freed = 0, synced = 0;
   std::map<void*, size_t> held;
   void* alloc(size_t n) {
     asked++;
@@ -38,7 +38,8 @@ struct Dev {
 };
 
 int main() {
-  Dev d{1000};
+  Dev d;
+  d.total = 1000;
   vtapi::GrowBuffer b;
   assert(b.grow(d, 300) && b.cap == 300 && d.used == 300);
   void* const p = b.p;
