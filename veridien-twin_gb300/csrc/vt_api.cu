@@ -791,16 +791,17 @@ static vt_status tc_solve(vt_ctx* ctx, vt_solve_req* q) {
   const uint32_t segs = std::max(vtk::tc_segments(vtk::TC_BF16, n, c_bf), vtk::tc_segments(vtk::TC_FP8, n, c_q));
   const size_t nn = size_t(n) * n, nr = size_t(n) * R;
   const bool dF = is_device_ptr(q->F);
+  auto& T = ctx->tc;
+  const bool same_f = q->reuse_f && T.f_src == q->F && T.n == n && T.mem;
+  const bool hold_q = fp8 || (same_f && T.have_q);   // a BF16 solve between two FP8 ones leaves the E4M3 copy where it is
   // layout of the context's mixed-precision block (each piece 256-byte aligned)
   size_t off = 0;
   auto place = [&](size_t bytes) { const size_t o = off; off += (bytes + 255) / 256 * 256; return o; };
-  const size_t o_f32 = dF ? 0 : place(nn * 4), o_hi = place(nn * 2), o_lo = place(nn * 2), o_q = fp8 ? place(nn) : 0;
+  const size_t o_f32 = dF ? 0 : place(nn * 4), o_hi = place(nn * 2), o_lo = place(nn * 2), o_q = hold_q ? place(nn) : 0;
   const size_t o_rs = place(size_t(n) * 4), o_bhi = place(size_t(64) * n * 2), o_blo = place(size_t(64) * n * 2),
                o_bq = place(size_t(64) * n), o_cs = place(256), o_cm = place(256), o_part = place(size_t(segs) * n * 64 * 4),
                o_E = place(nr * 4), o_rho = place(size_t(n) * 4), o_B = place(nr * 4), o_r = place(nr * 4), o_d = place(nr * 4),
                o_d2 = place(nr * 4), o_np = place((size_t(n) / 32 + 2) * 16), o_err = place(64);
-  auto& T = ctx->tc;
-  const bool same_f = q->reuse_f && T.f_src == q->F && T.n == n && T.mem;
   if (T.bytes < off) {
     VT_CK(cudaStreamSynchronize(ctx->stream));
     cudaFree(T.mem);
