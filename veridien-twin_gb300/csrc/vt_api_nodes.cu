@@ -283,6 +283,7 @@ vt_status vt_nodes_export(vt_ctx* ctx, uint32_t* gtable, uint32_t* active, uint3
     const vt_status s = ensure_scratch(ctx, bytes);
     if (s != VT_OK) return s;
     vtk::launch_transpose_nbr(N.nbr, N.o.nbr_k, N.n_active, static_cast<uint2*>(ctx->d_scratch), ctx->stream);
+    VT_CK(cudaGetLastError());
     VT_CK(cudaMemcpyAsync(nbr, ctx->d_scratch, bytes, cudaMemcpyDeviceToHost, ctx->stream));
   }
   VT_CK(cudaStreamSynchronize(ctx->stream));

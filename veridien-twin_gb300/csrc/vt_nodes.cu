@@ -417,10 +417,11 @@ __global__ void __launch_bounds__(256) jacobi_gather_table_kernel(const uint32_t
   }
 }
 
-// the smoothing neighbours, n_active x nbr_k pairs, to one row per neighbour (out[j * n_active + k]) or back
+// the smoothing neighbours, n_active x nbr_k pairs, to one row per neighbour (out[j * n_active + k]) or back; a block per tile of
+// 32 x 32, all on the grid's x, since either side may be the long one (y ends at 65535 blocks, 2.1 M pairs)
 __global__ void __launch_bounds__(256) transpose_nbr_kernel(const uint2* __restrict__ in, uint32_t rows, uint32_t cols, uint2* __restrict__ out) {
   __shared__ uint2 tile[32][33];
-  const uint32_t x = threadIdx.x & 31u, y = threadIdx.x >> 5, r0 = blockIdx.x * 32u, c0 = blockIdx.y * 32u;
+  const uint32_t x = threadIdx.x & 31u, y = threadIdx.x >> 5, across = (cols + 31u) / 32u, r0 = blockIdx.x / across * 32u, c0 = blockIdx.x % across * 32u;
   for (uint32_t i = y; i < 32u; i += 8u)
     if (r0 + i < rows && c0 + x < cols) tile[i][x] = in[size_t(r0 + i) * cols + c0 + x];
   __syncthreads();
@@ -428,7 +429,7 @@ __global__ void __launch_bounds__(256) transpose_nbr_kernel(const uint2* __restr
     if (c0 + i < cols && r0 + x < rows) out[size_t(c0 + i) * rows + r0 + x] = tile[x][i];
 }
 void launch_transpose_nbr(const uint2* in, uint32_t rows, uint32_t cols, uint2* out, cudaStream_t st) {
-  if (rows && cols) transpose_nbr_kernel<<<dim3((rows + 31) / 32, (cols + 31) / 32), 256, 0, st>>>(in, rows, cols, out);
+  if (rows && cols) transpose_nbr_kernel<<<((rows + 31) / 32) * ((cols + 31) / 32), 256, 0, st>>>(in, rows, cols, out);
 }
 
 static int grid_for(size_t work, int threads) {
