@@ -195,8 +195,12 @@ vt_status vt_trace_rays(vt_ctx* ctx, const float* o4, const float* d4, uint32_t 
  *                    a material index beyond the scene's gives NaN
  *   VT_UNIT_CAPSULE  in 4n: p, n, (a, r), b; out n: (capsuleOcc, 0, 0, 0)
  *   VT_UNIT_PROFILE  in n: (theta, -, -, -); out n: (p(theta) of the scene's emitter, 0, 0, 0)
+ *   VT_UNIT_TREE     in 4n: the nodes of a BVH over the scene's triangles (gpu/bvh.js's records: c0.lo|ref, c0.hi|count,
+ *                    c1.lo|ref, c1.hi|count), n >= 2, every child a node below n or a leaf of the scene's triangles, else
+ *                    VT_ERR_ARG; the closest hit of the ray lens[0..2] + t lens[3..5] from node 0; out n: slot 0 by the
+ *                    persistent lanes, slot 1 by the plain descent: (t, triangle bits, corruptTree, traversalCap), then 0
  * Buffers are host or device; n <= 2^24. traceTest is vt_trace_rays. */
-enum { VT_UNIT_LENS = 0, VT_UNIT_BSDF = 1, VT_UNIT_CAPSULE = 2, VT_UNIT_PROFILE = 3 };
+enum { VT_UNIT_LENS = 0, VT_UNIT_BSDF = 1, VT_UNIT_CAPSULE = 2, VT_UNIT_PROFILE = 3, VT_UNIT_TREE = 4 };
 typedef struct {
   uint32_t kind, n;
   float lens[12];

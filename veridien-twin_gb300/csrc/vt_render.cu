@@ -9,12 +9,20 @@ using namespace vtd;
 
 // Traversal layout of a node (64 B): per axis the planes (child 0 lo, child 1 lo, child 0 hi, child 1 hi), then the
 // children's words (child 0 ref, count, child 1 ref, count), so that a load leaves the two children's planes as the
-// register pairs of slab_pair's f32x2 operations
+// register pairs of slab_pair's f32x2 operations. gpu/bvh.js numbers a child above its parent; an interior child that is not gets
+// the count BAD_CHILD, and a leaf beside it comes first (traverse tests a node's leaves before it descends)
 __global__ void pack_nodes_kernel(float4* __restrict__ nodes, uint32_t n) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   float4* nb = nodes + size_t(4) * i;
-  const float4 a0 = nb[0], a1 = nb[1], a2 = nb[2], a3 = nb[3];   // c0.lo|ref, c0.hi|count, c1.lo|ref, c1.hi|count
+  float4 a0 = nb[0], a1 = nb[1], a2 = nb[2], a3 = nb[3];   // c0.lo|ref, c0.hi|count, c1.lo|ref, c1.hi|count
+  const bool bad0 = fu(a1.w) == 0u && fu(a0.w) <= i, bad1 = fu(a3.w) == 0u && fu(a2.w) <= i;
+  if (bad0) a1.w = __uint_as_float(BAD_CHILD);
+  if (bad1) a3.w = __uint_as_float(BAD_CHILD);
+  if (bad0 && !bad1 && fu(a3.w) != 0u) {
+    const float4 lo = a0, hi = a1;
+    a0 = a2; a1 = a3; a2 = lo; a3 = hi;
+  }
   nb[0] = make_float4(a0.x, a2.x, a1.x, a3.x);
   nb[1] = make_float4(a0.y, a2.y, a1.y, a3.y);
   nb[2] = make_float4(a0.z, a2.z, a1.z, a3.z);

@@ -65,6 +65,37 @@ __global__ void profile_test_kernel(const Scene S, const float4* __restrict__ in
   out[i] = make_float4(profile(S, in[i].x), 0.0f, 0.0f, 0.0f);
 }
 
+// the two forms of the traversal on a caller's nodes (packed), one ray; dbg: 8 counters of each form. Bounded by MAX_VISITS,
+// whatever the nodes say
+__global__ void tree_test_kernel(Scene S, float3 o, float3 d, uint32_t* dbg, float4* __restrict__ out) {
+  __shared__ uint2 stack_sh[SH_DEPTH * 32];
+  LaneStack stk;
+  stk.sh = stack_sh; stk.lane = threadIdx.x; stk.stride = 32;
+  TraceState st;
+  st.best = Hit{BIG, 0.0f, 0.0f, MISS, MISS};
+  uint32_t state = LANE_IDLE;
+  S.dbg = dbg;
+  if (threadIdx.x == 0 && trace_phase(S, 0u, o, d, 0.0f, 0.5f, 1u, 0u, st, -1)) state = LANE_NODE;
+  while (__any_sync(0xffffffffu, state >= LANE_POP)) trace_round<false>(S, 0.0f, st, stk, state);
+  if (threadIdx.x) return;
+  out[0] = make_float4(st.best.t, __uint_as_float(st.best.tri), float(dbg[DBG_CORRUPT]), float(dbg[DBG_VISITS]));
+  S.dbg = dbg + 8;
+  Hit best{BIG, 0.0f, 0.0f, MISS, MISS};
+  traverse<false>(S, 0u, o, d, 0.0f, best, MISS);
+  out[1] = make_float4(best.t, __uint_as_float(best.tri), float(dbg[8 + DBG_CORRUPT]), float(dbg[8 + DBG_VISITS]));
+}
+
+// every child a node of the n, or a leaf of the scene's triangles
+bool tree_in_range(const float* nodes, uint32_t n, uint32_t n_tris) {
+  for (uint32_t c = 0; c < 2 * n; c++) {
+    uint32_t ref, count;
+    std::memcpy(&ref, nodes + 8 * size_t(c) + 3, 4);
+    std::memcpy(&count, nodes + 8 * size_t(c) + 7, 4);
+    if (count ? size_t(ref) + std::min(count, MAX_LEAF) > n_tris : ref >= n) return false;
+  }
+  return true;
+}
+
 // float4 slots in and out per case of each kind
 void unit_slots(uint32_t kind, uint32_t* in, uint32_t* out) {
   switch (kind) {
@@ -72,6 +103,7 @@ void unit_slots(uint32_t kind, uint32_t* in, uint32_t* out) {
     case VT_UNIT_BSDF: *in = 4; *out = 3; return;
     case VT_UNIT_CAPSULE: *in = 4; *out = 1; return;
     case VT_UNIT_PROFILE: *in = 1; *out = 1; return;
+    case VT_UNIT_TREE: *in = 4; *out = 1; return;
     default: *in = 0; *out = 0; return;
   }
 }
@@ -113,6 +145,19 @@ vt_status vt_unit_test(vt_ctx* ctx, const vt_unit_req* q, const float* in, float
     case VT_UNIT_CAPSULE:
       vtk::capsule_test_kernel<<<blocks, vtk::UT_THREADS, 0, ctx->stream>>>(dIn, dOut, q->n);
       break;
+    case VT_UNIT_TREE: {
+      std::vector<float> nodes(size_t(q->n) * 16);
+      VT_CK(cudaMemcpyAsync(nodes.data(), dIn, bin, cudaMemcpyDeviceToHost, ctx->stream));
+      VT_CK(cudaStreamSynchronize(ctx->stream));
+      if (q->n < 2 || !vtk::tree_in_range(nodes.data(), q->n, ctx->S.tri_count)) return fail(ctx, VT_ERR_ARG, "unit test: a child out of range");
+      VT_CK(cudaMemsetAsync(dOut, 0, bout + 64, ctx->stream));
+      vtk::pack_nodes(dIn, q->n, ctx->stream);
+      vtd::Scene T = S;
+      T.nodes = dIn;
+      vtk::tree_test_kernel<<<1, 32, 0, ctx->stream>>>(T, make_float3(q->lens[0], q->lens[1], q->lens[2]), make_float3(q->lens[3], q->lens[4], q->lens[5]),
+                                                       reinterpret_cast<uint32_t*>(dOut + size_t(q->n) * so), dOut);
+      break;
+    }
     default:
       vtk::profile_test_kernel<<<blocks, vtk::UT_THREADS, 0, ctx->stream>>>(S, dIn, dOut, q->n);
       break;

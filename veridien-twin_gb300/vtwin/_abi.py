@@ -82,7 +82,7 @@ class vt_blas_info(C.Structure):
                 ("kind", C.c_int32)]
 
 
-VT_UNIT_LENS, VT_UNIT_BSDF, VT_UNIT_CAPSULE, VT_UNIT_PROFILE = 0, 1, 2, 3
+VT_UNIT_LENS, VT_UNIT_BSDF, VT_UNIT_CAPSULE, VT_UNIT_PROFILE, VT_UNIT_TREE = 0, 1, 2, 3, 4
 
 
 class vt_unit_req(C.Structure):
