@@ -430,9 +430,11 @@ enum { VT_PREC_FP32 = 0, VT_PREC_BF16 = 1, VT_PREC_FP8 = 2,
 
 /* Dense node radiosity B = E + diag(rho) F B (the lite_nodes / TwinRenderer Jacobi, gpu/wgsl/kernels.wgsl.js
  * :416-461 jacobiGather + jacobiUpdate with Lambertian nodes, gpu/renderer.js:729 _submitJacobi, :804 converge).
- * FP32: plain Jacobi sweeps at FP32 accuracy: one right-hand side on CUDA cores, several on the tensor cores (each number as
- * three bf16 parts, F itself stays FP32), or on CUDA cores where n < 1536, the rows are not 16-byte aligned and there is no
- * room for a copy, or a value leaves bf16's range. BF16 / FP8 (E4M3, per-row scales of F, per-column scales of the iterate):
+ * FP32: plain Jacobi sweeps at FP32 accuracy: one right-hand side on CUDA cores (multiply-adds), several on the tensor cores
+ * (F stays FP32 in memory; each number as three bf16 parts that hold all its bits, six of their nine products, which leaves 2^-26
+ * of a product, sums of 32 products in the tensor cores' truncating accumulators and of those in FP32: the error against FP64 is
+ * measured to be no larger than the multiply-adds'), or on CUDA cores where n < 1536, where a device F is not 16-byte aligned
+ * (n % 4 == 0) or there is no room for its copy in aligned rows (n % 4 != 0), and where a sum passes 2^96 or a value 2^112. BF16 / FP8 (E4M3, per-row scales of F, per-column scales of the iterate):
  * tcgen05 GEMM sweeps with FP32 accumulation solve for a correction, recovered by iterative refinement on an accurate
  * residual r = E + rho F B - B (F and B split into bf16 high and low parts, FP64 epilogue). BF16/FP8 need n % 16 == 0
  * and keep converted copies of F in the context (2 x n^2 x 2 B, plus n^2 B for FP8). `iters` counts low-precision

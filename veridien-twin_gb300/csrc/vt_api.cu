@@ -1046,7 +1046,7 @@ vt_status vt_radiosity_solve(vt_ctx* ctx, vt_solve_req* q) {
     }
     if (tc) {
       if (!std::isfinite(h[0]) || !std::isfinite(h[1])) {
-        // an infinity or NaN (or a value past bf16's range) has no parts: the CUDA-core sweeps from the start
+        // an infinity, a NaN, or what the parts' scale takes past float32's range: the CUDA-core sweeps from the start
         tc = false;
         if ((s = first_iterate()) != VT_OK) return s;
         cur = B0; nxt = B1; it = 0; sweep_n = 0; sweep_sum = 0;

@@ -95,6 +95,14 @@ __device__ __forceinline__ uint32_t take_bf16x2(float& x0, float& x1) {
   return w;
 }
 
+// the same of a pair (x - h as one f32x2 multiply-add, exact as the two differences are)
+__device__ __forceinline__ uint32_t take_bf16x2(float2& x) {
+  uint32_t w;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(w) : "f"(x.y), "f"(x.x));
+  x = __ffma2_rn(make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)), make_float2(-1.0f, -1.0f), x);
+  return w;
+}
+
 // One CTA per SM takes an equal run of the (row tile, K stage) pairs in tile order, across tiles without a break in the
 // pipeline (a CTA's start and end cost ~5 us); a tile's sum is then that of the few CTAs whose runs meet it, each in a
 // partial of its own. Stage g belongs to CTA run_cta(g).
@@ -278,10 +286,15 @@ void launch_gemm(const TcMap* A, const TcMap* A2, const TcMap* B, const TcMap* B
 // entries; the FMA chain of jacobi_gemm_fp32_kernel in brackets): n = 1540 6.3e-8 (6.9e-8), 4096 5.9e-8 (8.0e-8), 16384
 // 1.6e-7 (1.9e-7); signed entries 9.3e-8 (2.0e-7) to 2.5e-7 (7.3e-7).
 //
+// A part reaches down to 2^-133, a float's last bit to 2^-149: F and B are taken FX_SCALE times each, so that the parts hold
+// every bit of every float (without it 8 times the FMA chain's error where B is 2^-118), and the sums are scaled back. A
+// sum past 2^96 (or a value past 2^112) overflows and takes the FMA kernel as an infinity does.
+//
 // Bound: F from HBM. n = 32768, 64 columns: 755 us a sweep with its combine, 4.3 GB of F in ~725 us (0.87 of the measured
 // copy rate), against 3197 us on the FMA pipes. A stage is 32 KB of F, 1450 cycles of an SM's share of the bandwidth; its 24
 // MMAs take 768. What held it back on the way there: one lane's MMA code (72 cycles an MMA), two waits of the MMA warp
 // for each 32 of K (890 us), CTAs per tile and K split instead of one run each (a start and an end of ~5 us per 70 us).
+constexpr float FX_SCALE = 65536.0f;
 constexpr int FX_THREADS = 448;          // warps 0-3 drain, 4-11 convert, 12 TMA, 13 MMA
 constexpr int FX_STAGES = 4;
 constexpr uint32_t FX_F = 2 * 128 * 128, FX_B = 192 * 128, FX_STAGE = FX_F + FX_B;
@@ -426,10 +439,12 @@ __global__ void __launch_bounds__(FX_THREADS, 1)
       uint32_t h[16], m[16], l[16];
 #pragma unroll
       for (uint32_t c = 0; c < 8; c++) {
-        float4 x = src[c ^ (row & 7u)];   // 128-byte swizzle
-        h[2 * c] = take_bf16x2(x.x, x.y); h[2 * c + 1] = take_bf16x2(x.z, x.w);
-        m[2 * c] = take_bf16x2(x.x, x.y); m[2 * c + 1] = take_bf16x2(x.z, x.w);
-        l[2 * c] = take_bf16x2(x.x, x.y); l[2 * c + 1] = take_bf16x2(x.z, x.w);
+        const float4 f = src[c ^ (row & 7u)];   // 128-byte swizzle
+        float2 x = __fmul2_rn(make_float2(f.x, f.y), make_float2(FX_SCALE, FX_SCALE));
+        float2 y = __fmul2_rn(make_float2(f.z, f.w), make_float2(FX_SCALE, FX_SCALE));
+        h[2 * c] = take_bf16x2(x); h[2 * c + 1] = take_bf16x2(y);
+        m[2 * c] = take_bf16x2(x); m[2 * c + 1] = take_bf16x2(y);
+        l[2 * c] = take_bf16x2(x); l[2 * c + 1] = take_bf16x2(y);
       }
       tmem_st16(taddr, h);
       tmem_st16(taddr + 32, m);
@@ -503,12 +518,12 @@ __device__ __forceinline__ void block_sum2(double a, double b, double* partials)
   }
 }
 
-// A tile of 32 rows of the n x R iterate, in shared memory, to its bf16 parts as K-major rows: Bt (192 x np): row 64 q + c
+// A tile of 32 rows of the n x R iterate, in shared memory, to the bf16 parts of FX_SCALE times it as K-major rows: Bt (192 x np): row 64 q + c
 // holds part q of column c. A thread splits two neighbours of K: a 32-bit store per part (np is even); c < R
 __device__ __forceinline__ void store_parts(const float (*tile)[65], uint32_t i0, uint32_t R, uint32_t np, uint16_t* __restrict__ Bt) {
   for (uint32_t q = threadIdx.x; q < R * 16u; q += 256u) {
     const uint32_t c = q / 16u, k = 2u * (q % 16u);
-    float x0 = tile[k][c], x1 = tile[k + 1u][c];
+    float x0 = tile[k][c] * FX_SCALE, x1 = tile[k + 1u][c] * FX_SCALE;
     uint32_t* dst = reinterpret_cast<uint32_t*>(Bt + size_t(c) * np + i0 + k);
     dst[0] = take_bf16x2(x0, x1);
     dst[size_t(32) * np] = take_bf16x2(x0, x1);
@@ -544,6 +559,8 @@ __global__ void __launch_bounds__(256) combine_f32_kernel(const float* __restric
         const float4 v = P[s * stride + i];
         a.x += v.x; a.y += v.y; a.z += v.z; a.w += v.w;
       }
+      constexpr float back = 1.0f / (FX_SCALE * FX_SCALE);
+      a.x *= back; a.y *= back; a.z *= back; a.w *= back;
       const float rr = rho[i0 + r];
       const float4 e = reinterpret_cast<const float4*>(E)[i], x = reinterpret_cast<const float4*>(X)[i];
       b = make_float4(fmaf(rr, a.x, e.x), fmaf(rr, a.y, e.y), fmaf(rr, a.z, e.z), fmaf(rr, a.w, e.w));
