@@ -548,8 +548,9 @@ vt_status vt_wait_check(vt_ctx* ctx, uint64_t cycles, int arrive);
 
 /* What the host has been refused, on purpose, so that a program or a test sees what a call does then: allocations of more
  * than `limit` bytes of a kind are refused on the host, as a device without the memory refuses them (UINT64_MAX: none).
- * WAVE: the path tracer's wavefront state (a render with refinement then takes it in smaller waves, or VT_ERR_OOM). */
-enum { VT_REFUSE_WAVE = 0 };
+ * WAVE: the path tracer's wavefront state (a render with refinement then takes it in smaller waves, or VT_ERR_OOM).
+ * COOPERATIVE: with limit 0, cooperative launches (the FP32 solve of one column then launches its sweeps one by one). */
+enum { VT_REFUSE_WAVE = 0, VT_REFUSE_COOPERATIVE = 1 };
 vt_status vt_refuse(vt_ctx* ctx, uint32_t what, uint64_t limit);
 
 /* ------------------------------------------------------------------- lite_nodes: the raster camera pass */

@@ -756,8 +756,9 @@ vt_status vt_wait_check(vt_ctx* ctx, uint64_t cycles, int arrive) {
 
 vt_status vt_refuse(vt_ctx* ctx, uint32_t what, uint64_t limit) {
   if (!ctx) return VT_ERR_ARG;
-  if (what != VT_REFUSE_WAVE) return fail(ctx, VT_ERR_ARG, "refuse: unknown resource");
-  ctx->refuse_wave = size_t(limit);
+  if (what == VT_REFUSE_WAVE) ctx->refuse_wave = size_t(limit);
+  else if (what == VT_REFUSE_COOPERATIVE) ctx->refuse_coop = limit == 0;
+  else return fail(ctx, VT_ERR_ARG, "refuse: unknown resource");
   return VT_OK;
 }
 
@@ -994,7 +995,7 @@ vt_status vt_radiosity_solve(vt_ctx* ctx, vt_solve_req* q) {
   vtk::TcMap mF, mB;
   uint32_t* wait_err = reinterpret_cast<uint32_t*>(norms + 4);   // a bounded wait ran out; then the grid barrier's counter
   // one right-hand side of a room whose iterate fits shared memory: the sweeps between two checks in one launch
-  const bool coop = R == 1 && !tma && vtk::jacobi_matvec_sweeps_ok(n);
+  bool coop = R == 1 && !tma && vtk::jacobi_matvec_sweeps_ok(n);
   uint32_t arrivals = 0;
   if (tc || coop) VT_CK(cudaMemsetAsync(wait_err, 0, 8, ctx->stream));
   if (tc) {
@@ -1019,9 +1020,18 @@ vt_status vt_radiosity_solve(vt_ctx* ctx, vt_solve_req* q) {
     const uint32_t k = std::min(check, max_it - it);
     if (coop) {
       VT_CK(cudaEventRecord(ctx->ev2, ctx->stream));
-      VT_CK(vtk::launch_jacobi_matvec_sweeps(Fd, rho, E, cur, nxt, n, k, wait_err + 1, &arrivals, wait_err, partials, &np, ctx->stream));
-      VT_CK(cudaEventRecord(ctx->ev3, ctx->stream));
-      if (k & 1u) std::swap(cur, nxt);
+      const cudaError_t e = ctx->refuse_coop ? cudaErrorCooperativeLaunchTooLarge
+                                             : vtk::launch_jacobi_matvec_sweeps(Fd, rho, E, cur, nxt, n, k, wait_err + 1, &arrivals, wait_err, partials,
+                                                                                &np, ctx->stream);
+      if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported || e == cudaErrorLaunchOutOfResources) {
+        // fewer SMs for this process than the device has: a launch per sweep
+        cudaGetLastError();
+        coop = false;
+      } else {
+        VT_CK(e);
+        VT_CK(cudaEventRecord(ctx->ev3, ctx->stream));
+        if (k & 1u) std::swap(cur, nxt);
+      }
     }
     for (uint32_t j = 0; j < k && !coop; j++) {
       if (j == 0) VT_CK(cudaEventRecord(ctx->ev2, ctx->stream));

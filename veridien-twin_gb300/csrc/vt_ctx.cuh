@@ -38,8 +38,9 @@ struct vt_ctx {
   uint32_t* d_work = nullptr;   // queue counters of the wavefront path tracer
   int wave_blocks = 0;
   vtapi::GrowBuffer wave;       // wavefront path state of renders and calibrations
-  // what tests have the host refuse (vt_refuse): bytes of the wavefront's state
+  // what tests have the host refuse (vt_refuse): bytes of the wavefront's state, cooperative launches
   size_t refuse_wave = SIZE_MAX;
+  bool refuse_coop = false;
   struct Cam {
     float4* radiance = nullptr;
     float* raw = nullptr;
