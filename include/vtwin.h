@@ -546,6 +546,11 @@ vt_status vt_get_node_state(vt_ctx* ctx, float* state, uint32_t* slot);
  * browser's). */
 vt_status vt_wait_check(vt_ctx* ctx, uint64_t cycles, int arrive);
 
+/* The same of the grid barrier between the sweeps of one launch (the FP32 solve of one column): a cooperative launch of 24 blocks
+ * meets six times, its counter of arrivals at `start`, and the last `missing` blocks never arrive: VT_OK, or VT_ERR_TIMEOUT after at
+ * most `cycles` SM clocks (1 .. 2^36). */
+vt_status vt_barrier_check(vt_ctx* ctx, uint64_t cycles, uint32_t start, uint32_t missing);
+
 /* What the host has been refused, on purpose, so that a program or a test sees what a call does then: allocations of more
  * than `limit` bytes of a kind are refused on the host, as a device without the memory refuses them (UINT64_MAX: none).
  * WAVE: the path tracer's wavefront state (a render with refinement then takes it in smaller waves, or VT_ERR_OOM).

@@ -754,6 +754,20 @@ vt_status vt_wait_check(vt_ctx* ctx, uint64_t cycles, int arrive) {
   return e ? fail(ctx, VT_ERR_TIMEOUT, "wait check: the barrier phase did not complete within the limit") : VT_OK;
 }
 
+vt_status vt_barrier_check(vt_ctx* ctx, uint64_t cycles, uint32_t start, uint32_t missing) {
+  if (!ctx || cycles == 0 || cycles > (1ull << 36) || missing > vtk::BARRIER_CHECK_BLOCKS) return VT_ERR_ARG;
+  uint32_t h[8 + vtk::BARRIER_CHECK_BLOCKS] = {start};
+  vt_status s = ensure_scratch(ctx, sizeof(h));
+  if (s != VT_OK) return s;
+  uint32_t* work = static_cast<uint32_t*>(ctx->d_scratch);
+  VT_CK(cudaMemcpyAsync(work, h, sizeof(h), cudaMemcpyHostToDevice, ctx->stream));
+  VT_CK(vtk::launch_barrier_check(start, 3, missing, cycles, work, ctx->stream));
+  VT_CK(cudaMemcpyAsync(h, work, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
+  VT_CK(cudaStreamSynchronize(ctx->stream));
+  if (h[2]) return fail(ctx, VT_ERR_TIMEOUT, "barrier check: the blocks did not arrive within the limit");
+  return h[1] ? fail(ctx, VT_ERR_CUDA, "barrier check: a block passed before the others had arrived") : VT_OK;
+}
+
 vt_status vt_refuse(vt_ctx* ctx, uint32_t what, uint64_t limit) {
   if (!ctx) return VT_ERR_ARG;
   if (what == VT_REFUSE_WAVE) ctx->refuse_wave = size_t(limit);

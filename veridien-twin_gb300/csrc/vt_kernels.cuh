@@ -73,6 +73,9 @@ bool jacobi_matvec_sweeps_ok(uint32_t n);
 uint32_t jacobi_matvec_sweeps_blocks(uint32_t n);
 cudaError_t launch_jacobi_matvec_sweeps(const float* F, const float* rho, const float* E, float* B0, float* B1, uint32_t n, uint32_t sweeps,
                                         uint32_t* counter, uint32_t* arrivals, uint32_t* err, double* partials, uint32_t* n_partials, cudaStream_t st);
+// vt_barrier_check's kernel; work: the counter (at `start`), what was seen wrong, *err, and from word 8 a word a block, cleared
+constexpr uint32_t BARRIER_CHECK_BLOCKS = 24;
+cudaError_t launch_barrier_check(uint32_t start, uint32_t rounds, uint32_t missing, uint64_t cycles, uint32_t* work, cudaStream_t st);
 // the same with F's rows fed into shared memory by bulk copies (n % 4 == 0); bounded waits raise matvec_error
 void launch_jacobi_matvec_tma(const float* F, const float* rho, const float* E, const float* Bin, float* Bout, uint32_t n,
                               double* partials, uint32_t* n_partials, cudaStream_t st);

@@ -83,8 +83,9 @@ __global__ void __launch_bounds__(MV_THREADS) jacobi_matvec_kernel(const float* 
 constexpr int MVS_THREADS = 1024;
 constexpr uint32_t MVS_MAX_N = 16384;   // the iterate in shared memory: 64 KB
 
-// wait for every block's arrival (`target` arrivals since the counter was cleared); false in every thread when it runs out
-__device__ __forceinline__ bool grid_barrier(uint32_t* counter, uint32_t target, uint32_t* err) {
+// wait for every block's arrival (`target` arrivals since the counter was cleared, counted modulo 2^32: blocks are at most a
+// barrier apart); false in every thread when it runs out
+__device__ __forceinline__ bool grid_barrier(uint32_t* counter, uint32_t target, uint32_t* err, unsigned long long limit = async::WAIT_CYCLES) {
   __shared__ uint32_t ok;
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -92,8 +93,8 @@ __device__ __forceinline__ bool grid_barrier(uint32_t* counter, uint32_t target,
     atomicAdd(counter, 1u);
     ok = 1u;
     const unsigned long long t0 = clock64();
-    while (*reinterpret_cast<volatile uint32_t*>(counter) < target)
-      if (clock64() - t0 > async::WAIT_CYCLES) { atomicOr(err, 1u); ok = 0u; break; }
+    while (int32_t(*reinterpret_cast<volatile uint32_t*>(counter) - target) < 0)
+      if (clock64() - t0 > limit) { atomicOr(err, 1u); ok = 0u; break; }
     __threadfence();
   }
   __syncthreads();
@@ -163,6 +164,26 @@ __global__ void __launch_bounds__(MVS_THREADS, 1) jacobi_matvec_sweeps_kernel(co
     partials[2 * blockIdx.x] = d2;
     partials[2 * blockIdx.x + 1] = b2;
   }
+}
+
+// vt_barrier_check: `rounds` barriers from a counter that stands at `start`; before each the blocks leave their round's number, after
+// each they count those that lack it, and a second barrier keeps the next round's from being seen. The last `missing` blocks never arrive.
+__global__ void barrier_check_kernel(uint32_t* counter, uint32_t start, uint32_t rounds, uint32_t missing, unsigned long long cycles, uint32_t* left,
+                                     uint32_t* wrong, uint32_t* err) {
+  if (blockIdx.x + missing >= gridDim.x) return;
+  uint32_t target = start;
+  for (uint32_t r = 1; r <= rounds; r++) {
+    if (threadIdx.x == 0) __stcg(left + blockIdx.x, r);
+    if (!grid_barrier(counter, target += gridDim.x, err, cycles)) return;
+    if (threadIdx.x < gridDim.x && __ldcg(left + threadIdx.x) != r) atomicAdd(wrong, 1u);
+    if (!grid_barrier(counter, target += gridDim.x, err, cycles)) return;
+  }
+}
+cudaError_t launch_barrier_check(uint32_t start, uint32_t rounds, uint32_t missing, uint64_t cycles, uint32_t* work, cudaStream_t st) {
+  uint32_t *counter = work, *wrong = work + 1, *err = work + 2, *left = work + 8;
+  unsigned long long limit = cycles;
+  void* args[] = {&counter, &start, &rounds, &missing, &limit, &left, &wrong, &err};
+  return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(barrier_check_kernel), dim3(BARRIER_CHECK_BLOCKS), dim3(64), args, 0, st);
 }
 
 // ------------------------------------------------------------------------------------------ TMA-fed matvec
