@@ -816,7 +816,7 @@ static vt_status tc_solve(vt_ctx* ctx, vt_solve_req* q) {
   const size_t o_rs = place(size_t(n) * 4), o_bhi = place(size_t(64) * n * 2), o_blo = place(size_t(64) * n * 2),
                o_bq = place(size_t(64) * n), o_cs = place(256), o_cm = place(256), o_part = place(size_t(segs) * n * 64 * 4),
                o_E = place(nr * 4), o_rho = place(size_t(n) * 4), o_B = place(nr * 4), o_r = place(nr * 4), o_d = place(nr * 4),
-               o_d2 = place(nr * 4), o_np = place((size_t(n) / 32 + 2) * 16), o_err = place(64);
+               o_d2 = place(nr * 4), o_np = place((size_t(n) / 8 + 2) * 16), o_err = place(64);
   if (T.bytes < off) {
     VT_CK(cudaStreamSynchronize(ctx->stream));
     cudaFree(T.mem);

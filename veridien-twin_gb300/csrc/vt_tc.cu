@@ -105,11 +105,12 @@ __device__ __forceinline__ uint32_t take_bf16x2(float2& x) {
 
 // One CTA per SM takes an equal run of the (row tile, K stage) pairs in tile order, across tiles without a break in the
 // pipeline (a CTA's start and end cost ~5 us); a tile's sum is then that of the few CTAs whose runs meet it, each in a
-// partial of its own. Stage g belongs to CTA run_cta(g).
-__host__ __device__ inline uint32_t run_cta(uint64_t g, uint64_t total, uint32_t ctas) { return uint32_t(((g + 1u) * ctas - 1u) / total); }
+// partial of its own. Stage g belongs to CTA run_cta(g). Stages x CTAs stay below 2^32 (run_ctas; n = 480,000 and more): the
+// divisions of 64 bits took up to 1 us of a small sweep's kernels.
+__device__ __forceinline__ uint32_t run_cta(uint32_t g, uint32_t total, uint32_t ctas) { return ((g + 1u) * ctas - 1u) / total; }
 // the CTAs whose runs meet row tile `tile` of KT stages
 __device__ __forceinline__ uint32_t run_segments(uint32_t tile, uint32_t KT, uint32_t n, uint32_t ctas) {
-  const uint64_t total = uint64_t((n + 127u) / 128u) * KT, g = uint64_t(tile) * KT;
+  const uint32_t total = (n + 127u) / 128u * KT, g = tile * KT;
   return run_cta(g + KT - 1u, total, ctas) - run_cta(g, total, ctas) + 1u;
 }
 
@@ -141,10 +142,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 5);
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
   const uint32_t KT = (n + K_ELEMS - 1u) / K_ELEMS;
-  const uint64_t total = uint64_t((n + 127u) / 128u) * KT;
-  const uint64_t g0 = uint64_t(blockIdx.x) * total / gridDim.x;
-  const uint32_t nkt = uint32_t((uint64_t(blockIdx.x) + 1u) * total / gridDim.x - g0);
-  uint32_t tile = uint32_t(g0 / KT), kk = uint32_t(g0 % KT);   // of the role's next stage
+  const uint32_t total = (n + 127u) / 128u * KT;
+  const uint32_t g0 = blockIdx.x * total / gridDim.x, nkt = (blockIdx.x + 1u) * total / gridDim.x - g0;
+  uint32_t tile = g0 / KT, kk = g0 % KT;   // of the role's next stage
 
   if (threadIdx.x == 0) {
     for (uint32_t s = 0; s < STAGES; s++) { mbar_init(full(s), 1); mbar_init(empty(s), 1); }
@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
       if (lane == 0) mbar_arrive(read(b));
       if (!end) continue;
       // the tile's end, or the run's: this CTA's partial of it
-      const uint32_t row = tile * 128u + warp * 32u + lane, seg = blockIdx.x - run_cta(uint64_t(tile) * KT, total, gridDim.x);
+      const uint32_t row = tile * 128u + warp * 32u + lane, seg = blockIdx.x - run_cta(tile * KT, total, gridDim.x);
       if (row < n) {
         float4* dst = reinterpret_cast<float4*>(partials + (size_t(seg) * n + row) * 64);
 #pragma unroll
@@ -348,10 +348,9 @@ __global__ void __launch_bounds__(FX_THREADS, 1)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * FX_STAGES + 8);
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
   const uint32_t KT = (n + 63u) / 64u;
-  const uint64_t total = uint64_t((n + 127u) / 128u) * KT;
-  const uint64_t g0 = uint64_t(blockIdx.x) * total / gridDim.x;
-  const uint32_t nkt = uint32_t((uint64_t(blockIdx.x) + 1u) * total / gridDim.x - g0);
-  uint32_t tile = uint32_t(g0 / KT), kk = uint32_t(g0 % KT);   // of the role's next stage
+  const uint32_t total = (n + 127u) / 128u * KT;
+  const uint32_t g0 = blockIdx.x * total / gridDim.x, nkt = (blockIdx.x + 1u) * total / gridDim.x - g0;
+  uint32_t tile = g0 / KT, kk = g0 % KT;   // of the role's next stage
   if (threadIdx.x == 0) {
     for (uint32_t s = 0; s < FX_STAGES; s++) { mbar_init(full(s), 1); mbar_init(empty(s), 1); }
     for (uint32_t b = 0; b < 2; b++) { mbar_init(ready(b), 8); mbar_init(done(b), 1); mbar_init(drained(b), 4); }
@@ -486,7 +485,7 @@ __global__ void __launch_bounds__(FX_THREADS, 1)
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(rest);
-      const uint32_t row = tile * 128u + warp * 32u + lane, seg = blockIdx.x - run_cta(uint64_t(tile) * KT, total, gridDim.x);
+      const uint32_t row = tile * 128u + warp * 32u + lane, seg = blockIdx.x - run_cta(tile * KT, total, gridDim.x);
       if (row < n) {
         float4* dst = reinterpret_cast<float4*>(partials + (size_t(seg) * n + row) * R);
 #pragma unroll
@@ -675,28 +674,36 @@ __device__ __forceinline__ void block_sum2f(float a, float b, double* partials) 
   }
 }
 
-// a block's 32 rows of the iterate, in shared memory, to the next sweep's right-hand sides in BF16 (c < R; the other rows of
+// Rows that a block of the combining kernels takes: 32, but 8 where blocks of 32 would be fewer than the SMs and there are columns
+// enough for the threads. The residual's FP64 (few units an SM) and the reads of up to nine partials then lie on four times the SMs:
+// FP8 with 64 columns, n = 512, 1024, 2048, 3008 a solve: 703, 767, 769, 847 us with 32 rows, 669, 733, 731, 797 with 8; from n =
+// 4864 on, and with 4 columns, 32 take the same or less (n = 4096, BF16: 595 us, 614 with 8)
+constexpr uint32_t CB_FEW = 8, CB_MANY = 32;
+uint32_t combine_rows(uint32_t n, uint32_t R) { return n < CB_MANY * 152u && R > 16u ? CB_FEW : CB_MANY; }
+
+// a block's rows of the iterate, in shared memory, to the next sweep's right-hand sides in BF16 (c < R; the other rows of
 // Bt stay zero): two neighbours of K a store (n is a multiple of 16)
+template <uint32_t ROWS>
 __device__ __forceinline__ void store_hi(const float (*tile)[65], uint32_t i0, uint32_t n, uint32_t R, uint16_t* __restrict__ Bt) {
-  for (uint32_t q = threadIdx.x; q < R * 16u; q += CB_THREADS) {
-    const uint32_t c = q / 16u, k = 2u * (q % 16u);
+  for (uint32_t q = threadIdx.x; q < R * (ROWS / 2u); q += CB_THREADS) {
+    const uint32_t c = q / (ROWS / 2u), k = 2u * (q % (ROWS / 2u));
     if (i0 + k >= n) continue;
     float x0 = tile[k][c], x1 = tile[k + 1u][c];
     *reinterpret_cast<uint32_t*>(Bt + size_t(c) * n + i0 + k) = take_bf16x2(x0, x1);
   }
 }
 
-// Y = rhs + rho (sum of the row tile's partials, in CTA order), 32 rows a block; Bt: also the next sweep's right-hand sides
+// Y = rhs + rho (sum of the row tile's partials, in CTA order), ROWS rows a block; Bt: also the next sweep's right-hand sides
 // (null: none). Norms of Y - Xin and Y in FP32 per thread. W: columns a thread takes at a time, 4 where R is a multiple (n =
 // 32768, 64 columns: 12 us, 20 a column at a time; with a pack launch of its own 35)
-template <int W>
+template <int W, uint32_t ROWS>
 __global__ void __launch_bounds__(CB_THREADS) combine_sweep_kernel(const float* __restrict__ P, uint32_t ctas, uint32_t KT, uint32_t n, uint32_t R,
                                                                    const float* __restrict__ rho, const float* __restrict__ rhs,
                                                                    const float* __restrict__ Xin, float* __restrict__ Y,
                                                                    const float* __restrict__ rs, const float* __restrict__ cs,
                                                                    uint16_t* __restrict__ Bt, double* __restrict__ parts) {
-  __shared__ float tile[32][65];
-  const uint32_t i0 = blockIdx.x * 32u, rows = min(32u, n - i0), RW = R / W, segs = run_segments(i0 / 128u, KT, n, ctas);
+  __shared__ float tile[ROWS][65];
+  const uint32_t i0 = blockIdx.x * ROWS, rows = min(ROWS, n - i0), RW = R / W, segs = run_segments(i0 / 128u, KT, n, ctas);
   auto load = [](const float* p, float* v) {
     if (W == 4) {
       const float4 x = *reinterpret_cast<const float4*>(p);
@@ -714,6 +721,7 @@ __global__ void __launch_bounds__(CB_THREADS) combine_sweep_kernel(const float* 
     load(rhs + idx, e);
     load(Xin + idx, x);
     load(P + size_t(i) * 64 + c, acc);
+#pragma unroll 4
     for (uint32_t s = 1; s < segs; s++) {
       load(P + (size_t(s) * n + i) * 64 + c, v);
 #pragma unroll
@@ -732,23 +740,25 @@ __global__ void __launch_bounds__(CB_THREADS) combine_sweep_kernel(const float* 
     else Y[idx] = acc[0];
   }
   __syncthreads();
-  if (Bt) store_hi(tile, i0, n, R, Bt);
+  if (Bt) store_hi<ROWS>(tile, i0, n, R, Bt);
   block_sum2f(d2, y2, parts);
 }
 
 // r = E + rho (sum of the partials) - B in FP64, and r's BF16 columns (Bt, null: none)
+template <uint32_t ROWS>
 __global__ void __launch_bounds__(CB_THREADS) combine_residual_kernel(const float* __restrict__ P, uint32_t ctas, uint32_t KT, uint32_t n, uint32_t R,
                                                                       const float* __restrict__ rho, const float* __restrict__ E,
                                                                       const float* __restrict__ B, float* __restrict__ r, uint16_t* __restrict__ Bt,
                                                                       double* __restrict__ parts) {
-  __shared__ float tile[32][65];
-  const uint32_t i0 = blockIdx.x * 32u, rows = min(32u, n - i0), segs = run_segments(i0 / 128u, KT, n, ctas);
+  __shared__ float tile[ROWS][65];
+  const uint32_t i0 = blockIdx.x * ROWS, rows = min(ROWS, n - i0), segs = run_segments(i0 / 128u, KT, n, ctas);
   double r2 = 0.0, b2 = 0.0;
 #pragma unroll 4
   for (uint32_t q = threadIdx.x; q < rows * R; q += CB_THREADS) {
     const uint32_t k = q / R, c = q % R, i = i0 + k;
     const size_t idx = size_t(i0) * R + q;
     float acc = P[size_t(i) * 64 + c];
+#pragma unroll 4
     for (uint32_t s = 1; s < segs; s++) acc += P[(size_t(s) * n + i) * 64 + c];
     const double b = double(B[idx]), rr = double(E[idx]) + double(rho[i]) * double(acc) - b;
     const float x = float(rr);
@@ -758,7 +768,7 @@ __global__ void __launch_bounds__(CB_THREADS) combine_residual_kernel(const floa
     b2 += b * b;
   }
   __syncthreads();
-  if (Bt) store_hi(tile, i0, n, R, Bt);
+  if (Bt) store_hi<ROWS>(tile, i0, n, R, Bt);
   block_sum2(r2, b2, parts);
 }
 
@@ -801,10 +811,13 @@ bool tc_encode(TcMap* map, const void* base, uint32_t inner, uint32_t rows, uint
   return r == CUDA_SUCCESS;
 }
 
+// `ctas` CTAs at most for `total` stages
+static uint32_t run_ctas(uint64_t ctas, uint64_t total) { return uint32_t(std::max<uint64_t>(1, std::min<uint64_t>(ctas, 0xffffffffu / total))); }
 // One CTA per SM; runs of an eighth of a row tile at least, so that few of them meet a tile
 uint32_t tc_ctas(int mode, uint32_t n, uint32_t sms) {
   const uint32_t ke = mode == TC_FP8 ? 128u : 64u, KT = (n + ke - 1u) / ke;
-  return uint32_t(std::max<uint64_t>(1, std::min<uint64_t>(sms, uint64_t((n + 127u) / 128u) * KT / ((KT + 7u) / 8u))));
+  const uint64_t total = uint64_t((n + 127u) / 128u) * KT;
+  return run_ctas(std::min<uint64_t>(sms, total / ((KT + 7u) / 8u)), total);
 }
 uint32_t tc_segments(int mode, uint32_t n, uint32_t ctas) {
   const uint32_t ke = mode == TC_FP8 ? 128u : 64u, KT = (n + ke - 1u) / ke;
@@ -822,7 +835,8 @@ size_t tc_f32_parts_bytes(uint32_t n) { return size_t(192) * tc_f32_pad(n) * 2; 
 
 // one CTA per SM, and the most CTAs whose runs meet one tile
 uint32_t tc_f32_ctas(uint32_t n, uint32_t sms) {
-  return uint32_t(std::min<uint64_t>(sms, uint64_t((n + 127u) / 128u) * ((n + 63u) / 64u)));
+  const uint64_t total = uint64_t((n + 127u) / 128u) * ((n + 63u) / 64u);
+  return run_ctas(std::min<uint64_t>(sms, total), total);
 }
 uint32_t tc_f32_segments(uint32_t n, uint32_t ctas) {
   const uint32_t KT = (n + 63u) / 64u;
@@ -871,16 +885,18 @@ void tc_pack_b(int mode, const float* X, uint32_t n, uint32_t R, uint16_t* hi, u
 
 uint32_t tc_combine_sweep(int mode, const float* partials, uint32_t ctas, uint32_t n, uint32_t R, const float* rho, const float* rhs, const float* Xin,
                           float* Y, const float* row_scale, const float* col_scale, uint16_t* Bt, double* norm_partials, cudaStream_t st) {
-  const uint32_t blocks = (n + 31u) / 32u, ke = mode == TC_FP8 ? 128u : 64u;
-  const auto kernel = R % 4u ? combine_sweep_kernel<1> : combine_sweep_kernel<4>;
+  const uint32_t rows = combine_rows(n, R), blocks = (n + rows - 1u) / rows, ke = mode == TC_FP8 ? 128u : 64u;
+  const auto kernel = rows == CB_FEW ? (R % 4u ? combine_sweep_kernel<1, CB_FEW> : combine_sweep_kernel<4, CB_FEW>)
+                                     : (R % 4u ? combine_sweep_kernel<1, CB_MANY> : combine_sweep_kernel<4, CB_MANY>);
   kernel<<<blocks, CB_THREADS, 0, st>>>(partials, ctas, (n + ke - 1u) / ke, n, R, rho, rhs, Xin, Y, row_scale, col_scale, Bt, norm_partials);
   return blocks;
 }
 
 uint32_t tc_combine_residual(const float* partials, uint32_t ctas, uint32_t n, uint32_t R, const float* rho, const float* E, const float* B, float* r,
                              uint16_t* Bt, double* norm_partials, cudaStream_t st) {
-  const uint32_t blocks = (n + 31u) / 32u;
-  combine_residual_kernel<<<blocks, CB_THREADS, 0, st>>>(partials, ctas, (n + 63u) / 64u, n, R, rho, E, B, r, Bt, norm_partials);
+  const uint32_t rows = combine_rows(n, R), blocks = (n + rows - 1u) / rows;
+  const auto kernel = rows == CB_FEW ? combine_residual_kernel<CB_FEW> : combine_residual_kernel<CB_MANY>;
+  kernel<<<blocks, CB_THREADS, 0, st>>>(partials, ctas, (n + 63u) / 64u, n, R, rho, E, B, r, Bt, norm_partials);
   return blocks;
 }
 
