@@ -22,6 +22,7 @@
 #include "vt_calib.cuh"
 #include "vt_calib_tan.cuh"
 #include "vt_camera.cuh"
+#include "vt_float_pair.h"
 #include "vt_wave.cuh"
 
 namespace vtk {
@@ -786,18 +787,49 @@ __global__ void __launch_bounds__(256) jacobi_t_combine(const double* __restrict
 // R64_ROWS rows, a thread four columns at a time of each: a load of B serves the rows, and a step is two products (f32x2) in
 // 12 independent sums. Bound by the FMA pipe (14 operations a product, 18 us at its rate). N = 4096: 37 us a sweep; a warp per
 // row with one product a step and B read again for each row took 51 us.
+// A row's sums over the lanes are float pairs where a thread has more than four of its columns: with chains of n / 512 products
+// their error against exact sums stays below that of a warp per row, 32 chains of n / 32 that meet in FP64 (positive terms, rms: n =
+// 1025 4.8e-16, there 6.8e-16; 4096 4.6e-16, there 1.3e-15). A shorter row's error would be the tree's (n = 512 6.7e-16, there 5.4e-16; 31
+// 1.5e-15 and 3.0e-16), so there (SHORT) every product is a sum of its own and the tree takes Df3 (9.9e-17, and 3.0e-16).
 constexpr uint32_t R64_ROWS = 4, R64_THREADS = 256;
-__global__ void __launch_bounds__(R64_THREADS, 2) radiosity64_kernel(const float* __restrict__ F, const float* __restrict__ rho, const float* __restrict__ DL,
-                                                                    const float* __restrict__ Bin, float* __restrict__ Bout, float* __restrict__ H,
-                                                                    uint32_t n, uint32_t np) {
-  __shared__ float2 red[R64_THREADS / 32][R64_ROWS * 3];
+constexpr uint32_t R64_SHORT = 4 * R64_THREADS;   // nodes
+__device__ __forceinline__ float2 df_shfl(float2 v, uint32_t mask) {
+  return make_float2(__shfl_xor_sync(0xffffffffu, v.x, mask), __shfl_xor_sync(0xffffffffu, v.y, mask));
+}
+__device__ __forceinline__ Df3 df_shfl(Df3 v, uint32_t mask) {
+  return {__shfl_xor_sync(0xffffffffu, v.h, mask), __shfl_xor_sync(0xffffffffu, v.m, mask), __shfl_xor_sync(0xffffffffu, v.l, mask)};
+}
+__device__ __forceinline__ double df_double(float2 v) { return double(v.x) + double(v.y); }
+// the sums over a warp's lanes of 16 values a lane: lane 2 v ends with value v. A step halves the values that a lane still adds
+template <typename V>
+__device__ __forceinline__ V df_warp_sum16(V* v, uint32_t lane) {
+#pragma unroll
+  for (uint32_t half = 8; half > 0; half >>= 1) {
+    const bool up = (lane & (2u * half)) != 0u;
+#pragma unroll
+    for (uint32_t q = 0; q < half; q++) {
+      const V mine = up ? v[q + half] : v[q], other = up ? v[q] : v[q + half];
+      v[q] = df_add(mine, df_shfl(other, 2 * half));
+    }
+  }
+  return df_add(v[0], df_shfl(v[0], 1));
+}
+template <bool SHORT>
+__global__ void __launch_bounds__(R64_THREADS, SHORT ? 1 : 2) radiosity64_kernel(const float* __restrict__ F, const float* __restrict__ rho,
+                                                                               const float* __restrict__ DL, const float* __restrict__ Bin,
+                                                                               float* __restrict__ Bout, float* __restrict__ H, uint32_t n, uint32_t np) {
+  constexpr int SUMS = SHORT ? 2 : 1;
+  __shared__ double red[R64_THREADS / 32][R64_ROWS * 3];
   const uint32_t row0 = blockIdx.x * R64_ROWS, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const bool vec = (n & 3u) == 0u;
-  DfAcc s[R64_ROWS][3];
+  DfAcc s[R64_ROWS][3][SUMS];
 #pragma unroll
   for (uint32_t r = 0; r < R64_ROWS; r++)
 #pragma unroll
-    for (int c = 0; c < 3; c++) s[r][c].h = s[r][c].l = f2(0.0f, 0.0f);
+    for (int c = 0; c < 3; c++) {
+      s[r][c][0].h = s[r][c][0].l = f2(0.0f, 0.0f);
+      s[r][c][SUMS - 1] = s[r][c][0];
+    }
   for (uint32_t j = 4u * threadIdx.x; j < n; j += 4u * R64_THREADS) {
     float4 f[R64_ROWS];
 #pragma unroll
@@ -812,40 +844,44 @@ __global__ void __launch_bounds__(R64_THREADS, 2) radiosity64_kernel(const float
       const float4 xl = __ldg(reinterpret_cast<const float4*>(Bin + size_t(2 * c + 1) * np + j));
 #pragma unroll
       for (uint32_t r = 0; r < R64_ROWS; r++) {
-        df_mac2(f2(f[r].x, f[r].y), f2(-f[r].x, -f[r].y), f2(xh.x, xh.y), f2(xl.x, xl.y), s[r][c]);
-        df_mac2(f2(f[r].z, f[r].w), f2(-f[r].z, -f[r].w), f2(xh.z, xh.w), f2(xl.z, xl.w), s[r][c]);
+        df_mac2(f2(f[r].x, f[r].y), f2(-f[r].x, -f[r].y), f2(xh.x, xh.y), f2(xl.x, xl.y), s[r][c][0]);
+        df_mac2(f2(f[r].z, f[r].w), f2(-f[r].z, -f[r].w), f2(xh.z, xh.w), f2(xl.z, xl.w), s[r][c][SUMS - 1]);
       }
     }
+    if (SHORT) break;   // n is R64_SHORT at most
   }
-  // the block's sums, as float pairs over a warp's lanes, then over the warps in FP64. A step over the lanes halves the
-  // values that a lane still adds (lane 2 v ends with value v): 16 additions for the 12 values
+  // the block's sums over a warp's lanes, then over the warps in FP64
   static_assert(R64_ROWS * 3 <= 16, "values of a lane");
-  float2 v[16];
+  double sum = 0.0;
+  if (SHORT) {
+    if (128u * warp < n) {
+      Df3 v[16];
 #pragma unroll
-  for (uint32_t q = 0; q < 16; q++) {
-    if (q < R64_ROWS * 3) {
-      const DfAcc& a = s[q / 3][q % 3];
-      v[q] = df_add(make_float2(a.h.x, a.l.x), make_float2(a.h.y, a.l.y));
-    } else {
+      for (uint32_t q = 0; q < 16; q++) {
+        v[q] = {0.0f, 0.0f, 0.0f};
+        if (q >= R64_ROWS * 3) continue;
+        const DfAcc &a = s[q / 3][q % 3][0], &b = s[q / 3][q % 3][SUMS - 1];
+        v[q] = df_add(df_add(Df3{a.h.x, a.l.x, 0.0f}, Df3{a.h.y, a.l.y, 0.0f}), df_add(Df3{b.h.x, b.l.x, 0.0f}, Df3{b.h.y, b.l.y, 0.0f}));
+      }
+      sum = df_double(df_warp_sum16(v, lane));
+    }
+  } else {
+    float2 v[16];
+#pragma unroll
+    for (uint32_t q = 0; q < 16; q++) {
       v[q] = make_float2(0.0f, 0.0f);
+      if (q >= R64_ROWS * 3) continue;
+      const DfAcc& a = s[q / 3][q % 3][0];
+      v[q] = df_add(make_float2(a.h.x, a.l.x), make_float2(a.h.y, a.l.y));
     }
+    sum = df_double(df_warp_sum16(v, lane));
   }
-#pragma unroll
-  for (uint32_t half = 8; half > 0; half >>= 1) {
-    const bool up = (lane & (2u * half)) != 0u;
-#pragma unroll
-    for (uint32_t q = 0; q < half; q++) {
-      const float2 mine = up ? v[q + half] : v[q], other = up ? v[q] : v[q + half];
-      v[q] = df_add(mine, make_float2(__shfl_xor_sync(0xffffffffu, other.x, 2 * half), __shfl_xor_sync(0xffffffffu, other.y, 2 * half)));
-    }
-  }
-  v[0] = df_add(v[0], make_float2(__shfl_xor_sync(0xffffffffu, v[0].x, 1), __shfl_xor_sync(0xffffffffu, v[0].y, 1)));
-  if (!(lane & 1u) && lane / 2u < R64_ROWS * 3) red[warp][lane / 2u] = v[0];
+  if (!(lane & 1u) && lane / 2u < R64_ROWS * 3) red[warp][lane / 2u] = sum;
   __syncthreads();
   const uint32_t q = threadIdx.x, row = row0 + q / 3u, c = q % 3u;
   if (q >= 3u * R64_ROWS || row >= n) return;
   double a = 0.0;
-  for (uint32_t w = 0; w < R64_THREADS / 32; w++) a += double(red[w][q].x) + double(red[w][q].y);
+  for (uint32_t w = 0; w < R64_THREADS / 32; w++) a += red[w][q];
   if (H) { H[size_t(c) * n + row] = float(a); return; }
   const float2 x = df_split(double(rho[size_t(c) * n + row]) * (double(DL[row]) + a));
   Bout[size_t(2 * c) * np + row] = x.x;
@@ -1054,11 +1090,12 @@ void launch_radiosity64(const float* F, const float* rho, const float* DL, uint3
   float* nxt = cur + size_t(6) * np;
   const uint32_t blocks = (n + R64_ROWS - 1) / R64_ROWS;
   radiosity64_init<<<(3 * np + 255) / 256, 256, 0, st>>>(rho, DL, cur, nxt, n, np);
+  const auto kernel = n <= R64_SHORT ? radiosity64_kernel<true> : radiosity64_kernel<false>;
   for (uint32_t it = 0; it < iters; it++) {
-    radiosity64_kernel<<<blocks, R64_THREADS, 0, st>>>(F, rho, DL, cur, nxt, nullptr, n, np);
+    kernel<<<blocks, R64_THREADS, 0, st>>>(F, rho, DL, cur, nxt, nullptr, n, np);
     std::swap(cur, nxt);
   }
-  radiosity64_kernel<<<blocks, R64_THREADS, 0, st>>>(F, rho, DL, cur, nullptr, H, n, np);
+  kernel<<<blocks, R64_THREADS, 0, st>>>(F, rho, DL, cur, nullptr, H, n, np);
 }
 
 }  // namespace vtk
