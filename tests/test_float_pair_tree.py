@@ -60,7 +60,7 @@ static V tree(V* v, Add plus) {
 // radiosity64_kernel
 static double block(const Row& r) {
   const int n = int(r.F.size());
-  const bool is_short = n <= 1024;
+  const bool is_short = n <= 768;
   double sum = 0;
   for (int w = 0; w < 8; w++) {
     P p[32];
@@ -88,7 +88,7 @@ int main() {
   std::uniform_real_distribution<double> U(0, 1);
   int worse = 0;
   for (int sign = 0; sign < 2; sign++)
-    for (int n : {1, 2, 3, 5, 16, 31, 64, 100, 130, 257, 512, 1000, 1024, 1025, 1500, 2048, 3000, 4096}) {
+    for (int n : {1, 2, 3, 5, 16, 31, 64, 100, 130, 257, 512, 700, 768, 769, 1000, 1025, 1500, 2048, 3000, 4096}) {
       double a2 = 0, b2 = 0;
       for (int rep = 0; rep < 1500; rep++) {
         Row r;

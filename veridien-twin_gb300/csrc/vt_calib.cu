@@ -787,12 +787,12 @@ __global__ void __launch_bounds__(256) jacobi_t_combine(const double* __restrict
 // R64_ROWS rows, a thread four columns at a time of each: a load of B serves the rows, and a step is two products (f32x2) in
 // 12 independent sums. Bound by the FMA pipe (14 operations a product, 18 us at its rate). N = 4096: 37 us a sweep; a warp per
 // row with one product a step and B read again for each row took 51 us.
-// A row's sums over the lanes are float pairs where a thread has more than four of its columns: with chains of n / 512 products
+// A row's sums over the lanes are float pairs where its length allows it: with chains of n / 512 products
 // their error against exact sums stays below that of a warp per row, 32 chains of n / 32 that meet in FP64 (positive terms, rms: n =
-// 1025 4.8e-16, there 6.8e-16; 4096 4.6e-16, there 1.3e-15). A shorter row's error would be the tree's (n = 512 6.7e-16, there 5.4e-16; 31
-// 1.5e-15 and 3.0e-16), so there (SHORT) every product is a sum of its own and the tree takes Df3 (9.9e-17, and 3.0e-16).
+// 769 6.1e-16, there 6.3e-16; 1025 4.8e-16 and 6.8e-16; 4096 4.6e-16 and 1.3e-15). A shorter row's error would be the tree's (n = 512 6.7e-16, there
+// 5.4e-16; 31 1.5e-15 and 3.0e-16), so there (SHORT) every product is a sum of its own and the tree takes Df3 (9.9e-17, and 3.0e-16).
 constexpr uint32_t R64_ROWS = 4, R64_THREADS = 256;
-constexpr uint32_t R64_SHORT = 4 * R64_THREADS;   // nodes
+constexpr uint32_t R64_SHORT = 768;   // nodes, at most four a thread
 __device__ __forceinline__ float2 df_shfl(float2 v, uint32_t mask) {
   return make_float2(__shfl_xor_sync(0xffffffffu, v.x, mask), __shfl_xor_sync(0xffffffffu, v.y, mask));
 }
