@@ -705,21 +705,24 @@ __device__ __forceinline__ float2 df_add(float2 x, float2 y) {
   return make_float2(h, __fsub_rn(lo, __fsub_rn(h, t)));
 }
 
-// Transposed sweep, the three channels in one pass over F: partial[split][c][j] = sum over rows i of the split of F[i][j]
-// (g_c,i + rho_c,i lam_c,i). A thread takes four columns, two float-pair sums a step (f32x2), so a row of F is one 16-byte
-// load for 12 products; the rows' weights lie in shared memory as the pairs the products take. Bound by the FMA pipe: 14
-// operations a product, 18 us at its rate. N = 4096: 38 + 5 us a sweep of three channels with its combine (a channel and a
-// product at a time, one row in flight: 80 + 25 us).
+// Transposed sweep, the three channels in one pass over F: partial[split][c][part][j] = sum over rows i of the split of F[i][j]
+// (g_c,i + rho_c,i lam_c,i), three float parts (Df3), rows of np. A thread takes four columns, two float-pair sums a step (f32x2), so a row of
+// F is one 16-byte load for 12 products; the rows' weights lie in shared memory as the pairs the products take. The even and the odd
+// rows are chains of their own (one chain for both had 1.3 to 1.8 times the error, n = 512 to 8192), which meet as three parts, like the
+// splits. FP64 there, at two operations a cycle and SM, took up to 4 us a sweep: a small calibration step (100 x 100) 3.31 ms with
+// 1000 nodes, 4.17 with FP64; 4.31 and 4.92 with 2048; 8.23 and 8.72 with 4096. Bound by the FMA pipe: 14 operations a product, 18 us of
+// 37 with 4096 nodes, its combine 5 (a channel and a product at a time, one row in flight: 80 and 25).
 constexpr uint32_t JT_SPLITS = 64, JT_THREADS = 256, JT_ROWS = 64;
+__host__ __device__ constexpr uint32_t jt_pitch(uint32_t n) { return (n + 3u) / 4u * 4u; }
 __global__ void __launch_bounds__(JT_THREADS) jacobi_t_kernel(const float* __restrict__ F, const double* __restrict__ g, const float* __restrict__ rho,
-                                                             const double* __restrict__ lam, uint32_t n, double* __restrict__ part) {
+                                                             const double* __restrict__ lam, uint32_t n, float* __restrict__ part) {
   __shared__ float4 w[3][JT_ROWS];   // (hi, hi, lo, lo)
   const uint32_t j = 4u * (blockIdx.x * JT_THREADS + threadIdx.x);
   const uint32_t rows = (n + JT_SPLITS - 1) / JT_SPLITS, i0 = blockIdx.y * rows, i1 = min(n, i0 + rows);
   const bool vec = (n & 3u) == 0u;
-  DfAcc s[3][2];
+  DfAcc s[2][3][2];
 #pragma unroll
-  for (int c = 0; c < 3; c++) s[c][0].h = s[c][0].l = s[c][1].h = s[c][1].l = f2(0.0f, 0.0f);
+  for (int q = 0; q < 12; q++) s[q / 6][q / 2 % 3][q % 2].h = s[q / 6][q / 2 % 3][q % 2].l = f2(0.0f, 0.0f);
   for (uint32_t ib = i0; ib < i1; ib += JT_ROWS) {
     const uint32_t m = min(JT_ROWS, i1 - ib);
     __syncthreads();
@@ -736,12 +739,12 @@ __global__ void __launch_bounds__(JT_THREADS) jacobi_t_kernel(const float* __res
         if (vec) return __ldg(reinterpret_cast<const float4*>(p));
         return make_float4(p[0], j + 1 < n ? p[1] : 0.0f, j + 2 < n ? p[2] : 0.0f, j + 3 < n ? p[3] : 0.0f);
       };
-      auto row = [&](float4 f, uint32_t k) {
+      auto row = [&](float4 f, uint32_t k, DfAcc (&a)[3][2]) {
 #pragma unroll
         for (int c = 0; c < 3; c++) {
           const float4 x = w[c][k];
-          df_mac2(f2(f.x, f.y), f2(-f.x, -f.y), f2(x.x, x.y), f2(x.z, x.w), s[c][0]);
-          df_mac2(f2(f.z, f.w), f2(-f.z, -f.w), f2(x.x, x.y), f2(x.z, x.w), s[c][1]);
+          df_mac2(f2(f.x, f.y), f2(-f.x, -f.y), f2(x.x, x.y), f2(x.z, x.w), a[c][0]);
+          df_mac2(f2(f.z, f.w), f2(-f.z, -f.w), f2(x.x, x.y), f2(x.z, x.w), a[c][1]);
         }
       };
       uint32_t k = 0;
@@ -750,36 +753,49 @@ __global__ void __launch_bounds__(JT_THREADS) jacobi_t_kernel(const float* __res
 #pragma unroll
         for (int q = 0; q < 4; q++) f[q] = load(Fc + size_t(q) * n);
 #pragma unroll
-        for (int q = 0; q < 4; q++) row(f[q], k + q);
+        for (int q = 0; q < 4; q++) row(f[q], k + q, s[q & 1]);
       }
-      for (; k < m; k++, Fc += n) row(load(Fc), k);
+      if (k < m) row(load(Fc), k, s[0]);
+      if (k + 1u < m) row(load(Fc + n), k + 1u, s[1]);
+      if (k + 2u < m) row(load(Fc + size_t(2) * n), k + 2u, s[0]);
     }
   }
+  if (j >= n) return;
+  const size_t np = jt_pitch(n);
 #pragma unroll
   for (int c = 0; c < 3; c++) {
-    double* p = part + (size_t(blockIdx.y) * 3 + c) * n + j;
+    Df3 v[4];
 #pragma unroll
     for (int q = 0; q < 2; q++) {
-      if (j + 2 * q < n) p[2 * q] = double(s[c][q].h.x) + double(s[c][q].l.x);
-      if (j + 2 * q + 1 < n) p[2 * q + 1] = double(s[c][q].h.y) + double(s[c][q].l.y);
+      const DfAcc &a = s[0][c][q], &b = s[1][c][q];
+      v[2 * q] = df_add(Df3{a.h.x, a.l.x, 0.0f}, Df3{b.h.x, b.l.x, 0.0f});
+      v[2 * q + 1] = df_add(Df3{a.h.y, a.l.y, 0.0f}, Df3{b.h.y, b.l.y, 0.0f});
     }
+    float* p = part + (size_t(blockIdx.y) * 3 + c) * 3 * np + j;
+    *reinterpret_cast<float4*>(p) = make_float4(v[0].h, v[1].h, v[2].h, v[3].h);
+    *reinterpret_cast<float4*>(p + np) = make_float4(v[0].m, v[1].m, v[2].m, v[3].m);
+    *reinterpret_cast<float4*>(p + 2 * np) = make_float4(v[0].l, v[1].l, v[2].l, v[3].l);
   }
 }
 // out = the sum of the partials, 3 n values: a block takes 32 of them, each warp an eighth of the splits, the warps' sums in
 // order
-__global__ void __launch_bounds__(256) jacobi_t_combine(const double* __restrict__ part, uint32_t n3, double* __restrict__ out) {
-  __shared__ double red[8][32];
-  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, j = blockIdx.x * 32u + lane;
-  double a = 0.0;
-  if (j < n3) {
+__global__ void __launch_bounds__(256) jacobi_t_combine(const float* __restrict__ part, uint32_t n, double* __restrict__ out) {
+  __shared__ Df3 red[8][32];
+  const uint32_t np = jt_pitch(n), lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, j = blockIdx.x * 32u + lane, c = j / np, k = j % np;
+  Df3 a{0.0f, 0.0f, 0.0f};
+  if (c < 3u) {
+    const float* p = part + (size_t(warp * (JT_SPLITS / 8)) * 3 + c) * 3 * np + k;
+    Df3 x[JT_SPLITS / 8];
 #pragma unroll
-    for (uint32_t s = 0; s < JT_SPLITS / 8; s++) a += part[size_t(warp * (JT_SPLITS / 8) + s) * n3 + j];
+    for (uint32_t s = 0; s < JT_SPLITS / 8; s++, p += size_t(9) * np) x[s] = {p[0], p[np], p[2 * size_t(np)]};
+#pragma unroll
+    for (uint32_t s = 0; s < JT_SPLITS / 8; s++) a = df_add(a, x[s]);
   }
   red[warp][lane] = a;
   __syncthreads();
-  if (warp || j >= n3) return;
-  for (uint32_t w = 1; w < 8; w++) a += red[w][lane];
-  out[j] = a;
+  if (warp || c >= 3u || k >= n) return;
+  for (uint32_t w = 1; w < 8; w++) a = df_add(a, red[w][lane]);
+  out[size_t(c) * n + k] = df_double(a);
 }
 
 // The three channels' B_c,out = rho_c o (DL + F B_c,in) at FP64 accuracy (F in FP32, B as float pairs, planar [c][hi | lo]
@@ -1070,12 +1086,13 @@ void launch_dl(const float* D, const float* L, uint32_t n, uint32_t n_lamps, flo
   dl_kernel<<<(n + 7) / 8, 256, 0, st>>>(D, L, n, n_lamps, y);
 }
 
-size_t jacobi_t_work(uint32_t n) { return size_t(JT_SPLITS) * 3 * n * 8; }
+size_t jacobi_t_work(uint32_t n) { return size_t(JT_SPLITS) * 9 * jt_pitch(n) * 4; }
 
 void launch_jacobi_t(const float* F, const double* g, const float* rho, const double* lam_in, double* lam_out, uint32_t n, double* work,
                      cudaStream_t st) {
-  jacobi_t_kernel<<<dim3((n + 4 * JT_THREADS - 1) / (4 * JT_THREADS), JT_SPLITS), JT_THREADS, 0, st>>>(F, g, rho, lam_in, n, work);
-  jacobi_t_combine<<<(3 * n + 31) / 32, 256, 0, st>>>(work, 3 * n, lam_out);
+  float* part = reinterpret_cast<float*>(work);   // the arena's places are 256-byte aligned
+  jacobi_t_kernel<<<dim3((n + 4 * JT_THREADS - 1) / (4 * JT_THREADS), JT_SPLITS), JT_THREADS, 0, st>>>(F, g, rho, lam_in, n, part);
+  jacobi_t_combine<<<(3 * jt_pitch(n) + 31) / 32, 256, 0, st>>>(part, n, lam_out);
 }
 
 void launch_sum(const double* p, uint32_t n, double* out, cudaStream_t st) { sum_kernel<<<1, 1024, 0, st>>>(p, n, out); }
