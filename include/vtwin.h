@@ -434,7 +434,7 @@ enum { VT_PREC_FP32 = 0, VT_PREC_BF16 = 1, VT_PREC_FP8 = 2,
  * (F stays FP32 in memory; each number as three bf16 parts that hold all its bits, six of their nine products, which leaves 2^-26
  * of a product, sums of 32 products in the tensor cores' truncating accumulators and of those in FP32: the error against FP64 is
  * measured to be no larger than the multiply-adds'), or on CUDA cores where n < 1536, where a device F is not 16-byte aligned
- * (n % 4 == 0) or there is no room for its copy in aligned rows (n % 4 != 0), and where a sum passes 2^96 or a value 2^112. BF16 / FP8 (E4M3, per-row scales of F, per-column scales of the iterate):
+ * (n % 4 == 0) or there is no room for the parts and its copy in aligned rows (n % 4 != 0), and where a sum passes 2^96 or a value 2^112. BF16 / FP8 (E4M3, per-row scales of F, per-column scales of the iterate):
  * tcgen05 GEMM sweeps with FP32 accumulation solve for a correction, recovered by iterative refinement on an accurate
  * residual r = E + rho F B - B (F and B split into bf16 high and low parts, FP64 epilogue). BF16/FP8 need n % 16 == 0
  * and keep converted copies of F in the context (2 x n^2 x 2 B, plus n^2 B for FP8). `iters` counts low-precision
@@ -554,8 +554,9 @@ vt_status vt_barrier_check(vt_ctx* ctx, uint64_t cycles, uint32_t start, uint32_
 /* What the host has been refused, on purpose, so that a program or a test sees what a call does then: allocations of more
  * than `limit` bytes of a kind are refused on the host, as a device without the memory refuses them (UINT64_MAX: none).
  * WAVE: the path tracer's wavefront state (a render with refinement then takes it in smaller waves, or VT_ERR_OOM).
- * COOPERATIVE: with limit 0, cooperative launches (the FP32 solve of one column then launches its sweeps one by one). */
-enum { VT_REFUSE_WAVE = 0, VT_REFUSE_COOPERATIVE = 1 };
+ * COOPERATIVE: with limit 0, cooperative launches (the FP32 solve of one column then launches its sweeps one by one).
+ * SCRATCH: the context's scratch (the FP32 solve of several columns then runs on CUDA cores; others end with VT_ERR_OOM). */
+enum { VT_REFUSE_WAVE = 0, VT_REFUSE_COOPERATIVE = 1, VT_REFUSE_SCRATCH = 2 };
 vt_status vt_refuse(vt_ctx* ctx, uint32_t what, uint64_t limit);
 
 /* ------------------------------------------------------------------- lite_nodes: the raster camera pass */

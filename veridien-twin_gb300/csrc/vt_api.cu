@@ -772,6 +772,7 @@ vt_status vt_refuse(vt_ctx* ctx, uint32_t what, uint64_t limit) {
   if (!ctx) return VT_ERR_ARG;
   if (what == VT_REFUSE_WAVE) ctx->refuse_wave = size_t(limit);
   else if (what == VT_REFUSE_COOPERATIVE) ctx->refuse_coop = limit == 0;
+  else if (what == VT_REFUSE_SCRATCH) ctx->refuse_scratch = size_t(limit);
   else return fail(ctx, VT_ERR_ARG, "refuse: unknown resource");
   return VT_OK;
 }
@@ -976,17 +977,19 @@ vt_status vt_radiosity_solve(vt_ctx* ctx, vt_solve_req* q) {
                                                  tma ? vtk::jacobi_matvec_tma_blocks(n) : R == 1 ? vtk::jacobi_matvec_sweeps_blocks(n) : 0u) + 8;
   // several right-hand sides: the tensor cores where F allows it (a host F is copied to aligned memory)
   bool tc = q->precision == VT_PREC_FP32 && vtk::jacobi_tc_f32_ok(dF ? q->F : nullptr, n, R);
-  const size_t gemm_work = R > 1 ? std::max(vtk::jacobi_gemm_fp32_work(n, R), tc ? vtk::jacobi_tc_f32_work(n, R) : 0) : 0;
+  const size_t fma_work = R > 1 ? vtk::jacobi_gemm_fp32_work(n, R) : 0;
+  size_t gemm_work = tc ? std::max(fma_work, vtk::jacobi_tc_f32_work(n, R)) : fma_work;
   const uint32_t pitch = vtk::jacobi_tc_f32_pitch(n);
   size_t nfp = tc && pitch != n ? size_t(n) * pitch * 4 : 0;   // F's copy in aligned rows
-  const size_t need = (dF ? 0 : nf) + 3 * nb + size_t(n) * 4 + size_t(max_blocks) * 16 + gemm_work + 64 + 2048 + 512;
-  vt_status s = ensure_scratch(ctx, need + nfp);
-  if (s != VT_OK && nfp) {   // no room for the copy
-    tc = false;
+  const size_t need = (dF ? 0 : nf) + 3 * nb + size_t(n) * 4 + size_t(max_blocks) * 16 + 64 + 2048 + 512;
+  vt_status s;
+  if (tc && (s = try_scratch(ctx, need + gemm_work + nfp)) != VT_OK) {
+    if (s != VT_ERR_OOM) return s;
+    tc = false;   // no room for the parts or the copy
     nfp = 0;
-    s = ensure_scratch(ctx, need);
+    gemm_work = fma_work;
   }
-  if (s != VT_OK) return s;
+  if ((s = ensure_scratch(ctx, need + gemm_work + nfp)) != VT_OK) return s;
   char* base = static_cast<char*>(ctx->d_scratch);
   auto take = [&](size_t bytes) { char* p = base; base += (bytes + 255) / 256 * 256; return p; };
   const float* Fd = dF ? q->F : reinterpret_cast<float*>(take(nf));

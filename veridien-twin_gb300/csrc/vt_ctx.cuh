@@ -38,8 +38,8 @@ struct vt_ctx {
   uint32_t* d_work = nullptr;   // queue counters of the wavefront path tracer
   int wave_blocks = 0;
   vtapi::GrowBuffer wave;       // wavefront path state of renders and calibrations
-  // what tests have the host refuse (vt_refuse): bytes of the wavefront's state, cooperative launches
-  size_t refuse_wave = SIZE_MAX;
+  // what tests have the host refuse (vt_refuse): bytes of the wavefront's state and of the scratch, cooperative launches
+  size_t refuse_wave = SIZE_MAX, refuse_scratch = SIZE_MAX;
   bool refuse_coop = false;
   struct Cam {
     float4* radiance = nullptr;
@@ -254,13 +254,18 @@ inline vt_status upload(vt_ctx* ctx, T** dst, const void* src, size_t bytes) {
   return VT_OK;
 }
 
-inline vt_status ensure_scratch(vt_ctx* ctx, size_t bytes) {
+// the scratch for a caller that has another way where it is refused (VT_ERR_OOM, without a message)
+inline vt_status try_scratch(vt_ctx* ctx, size_t bytes) {
   if (ctx->scratch_bytes >= bytes) return VT_OK;
   if (ctx->d_scratch) { VT_CK(cudaStreamSynchronize(ctx->stream)); VT_CK(cudaFree(ctx->d_scratch)); ctx->d_scratch = nullptr; ctx->scratch_bytes = 0; }
-  cudaError_t e = cudaMalloc(&ctx->d_scratch, bytes);
-  if (e != cudaSuccess) { cudaGetLastError(); return fail(ctx, VT_ERR_OOM, "scratch allocation of " + std::to_string(bytes) + " bytes failed"); }
+  if (bytes > ctx->refuse_scratch) return VT_ERR_OOM;
+  if (cudaMalloc(&ctx->d_scratch, bytes) != cudaSuccess) { cudaGetLastError(); ctx->d_scratch = nullptr; return VT_ERR_OOM; }
   ctx->scratch_bytes = bytes;
   return VT_OK;
+}
+inline vt_status ensure_scratch(vt_ctx* ctx, size_t bytes) {
+  const vt_status s = try_scratch(ctx, bytes);
+  return s == VT_ERR_OOM ? fail(ctx, s, "scratch allocation of " + std::to_string(bytes) + " bytes failed") : s;
 }
 
 // the device side of ctx->wave's growth
