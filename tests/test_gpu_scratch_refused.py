@@ -67,3 +67,18 @@ def test_no_scratch_at_all_is_an_error():
     B, info = r.solve_radiosity(np.zeros((64, 64), np.float32), np.zeros(64, np.float32), np.ones((64, 1), np.float32))
     assert info["status"] == A.VT_OK and np.array_equal(B, np.ones((64, 1), np.float32))
     r.destroy()
+
+
+@pytest.mark.parametrize("size", [(16, 9), (19, 2), (640, 480)])
+def test_8_bit_readbacks(size):
+    r = _renderer(*size)
+    r.set_pose_array(A.identity_poses(1))
+    r.renderCamera(0, spp=1, lightSamples=1, mode=A.VT_SHADE_PATH, max_depth=2)
+    r.sensor(0, exposure_s=2e-3, gain=1.0)
+    assert r.lib.vt_refuse(r._ctx, SCRATCH, 0) == A.VT_OK
+    got, left = r.readback(0, "rgb8"), r.lib.vt_last_error(r._ctx)
+    r.lib.vt_refuse(r._ctx, SCRATCH, NONE)
+    rgba = r.readback(0, "rgba8")
+    assert rgba[..., :3].std() > 0 and left == b""
+    assert np.array_equal(got, rgba[..., :3]) and np.array_equal(r.readback(0, "rgb8"), got)
+    r.destroy()

@@ -322,10 +322,18 @@ inline vt_status from_device(vt_ctx* ctx, void* dst, const void* src, size_t byt
   return VT_OK;
 }
 
-// n RGBA pixels of the device as packed RGB, by way of the scratch
+// n RGBA pixels of the device as packed RGB, by way of the scratch; where that is refused, packed on the host
 inline vt_status rgb8_from_device(vt_ctx* ctx, void* dst, const uchar4* rgba, size_t n) {
-  const vt_status s = ensure_scratch(ctx, n * 3 + 16);
-  if (s != VT_OK) return s;
+  const vt_status s = try_scratch(ctx, n * 3 + 16);
+  if (s == VT_ERR_OOM && ptr_kind(dst) == PTR_HOST) {
+    std::vector<uint8_t> h(n * 4);
+    VT_CK(cudaMemcpyAsync(h.data(), rgba, n * 4, cudaMemcpyDeviceToHost, ctx->stream));
+    VT_CK(cudaStreamSynchronize(ctx->stream));
+    uint8_t* o = static_cast<uint8_t*>(dst);
+    for (size_t i = 0; i < n; i++, o += 3) std::copy(&h[4 * i], &h[4 * i] + 3, o);
+    return VT_OK;
+  }
+  if (s != VT_OK) return fail(ctx, s, "readback: no scratch for the packed image");
   vtk::launch_pack_rgb8(rgba, n, static_cast<uint8_t*>(ctx->d_scratch), ctx->stream);
   VT_CK(cudaGetLastError());
   return from_device(ctx, dst, ctx->d_scratch, n * 3);
