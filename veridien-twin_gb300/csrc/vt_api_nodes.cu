@@ -52,6 +52,14 @@ void snapshot(vt_ctx* ctx) {
 
 }  // namespace
 
+// launch_transpose_nbr on the host, for want of scratch
+static std::vector<uint32_t> transposed_pairs(const std::vector<uint32_t>& in, size_t rows, size_t cols) {
+  std::vector<uint32_t> out(in.size());
+  for (size_t r = 0; r < rows; r++)
+    for (size_t c = 0; c < cols; c++) std::copy(&in[2 * (r * cols + c)], &in[2 * (r * cols + c)] + 2, &out[2 * (c * rows + r)]);
+  return out;
+}
+
 vt_status vt_nodes_build(vt_ctx* ctx, const vt_nodes_opts* opts, vt_nodes_info* info) {
   if (!ctx) return VT_ERR_ARG;
   vt_nodes_opts o = opts ? *opts : default_opts();
@@ -129,9 +137,16 @@ vt_status vt_nodes_build(vt_ctx* ctx, const vt_nodes_opts* opts, vt_nodes_info* 
   N.nbr_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
   if (N.n_active) {
     VT_CK(cudaMemcpyAsync(N.active, N.active_h.data(), size_t(N.n_active) * 4, cudaMemcpyHostToDevice, ctx->stream));
-    if ((s = ensure_scratch(ctx, nbr.size() * 4)) != VT_OK) return s;
-    VT_CK(cudaMemcpyAsync(ctx->d_scratch, nbr.data(), nbr.size() * 4, cudaMemcpyHostToDevice, ctx->stream));
-    vtk::launch_transpose_nbr(static_cast<const uint2*>(ctx->d_scratch), N.n_active, o.nbr_k, N.nbr, ctx->stream);
+    s = try_scratch(ctx, nbr.size() * 4);
+    if (s == VT_ERR_OOM) {
+      nbr = transposed_pairs(nbr, N.n_active, o.nbr_k);
+      VT_CK(cudaMemcpyAsync(N.nbr, nbr.data(), nbr.size() * 4, cudaMemcpyHostToDevice, ctx->stream));
+    } else if (s != VT_OK) {
+      return s;
+    } else {
+      VT_CK(cudaMemcpyAsync(ctx->d_scratch, nbr.data(), nbr.size() * 4, cudaMemcpyHostToDevice, ctx->stream));
+      vtk::launch_transpose_nbr(static_cast<const uint2*>(ctx->d_scratch), N.n_active, o.nbr_k, N.nbr, ctx->stream);
+    }
   }
   vtk::launch_amu(S, n_mat, K, N.amu, ctx->stream);
   VT_CK(cudaGetLastError());
@@ -280,11 +295,20 @@ vt_status vt_nodes_export(vt_ctx* ctx, uint32_t* gtable, uint32_t* active, uint3
   if (gtable && N.n) VT_CK(cudaMemcpyAsync(gtable, N.gtable, size_t(N.n) * N.o.gather_k * 4, cudaMemcpyDeviceToHost, ctx->stream));
   if (nbr && N.n_active) {
     const size_t bytes = size_t(N.n_active) * N.o.nbr_k * 8;
-    const vt_status s = ensure_scratch(ctx, bytes);
-    if (s != VT_OK) return s;
-    vtk::launch_transpose_nbr(N.nbr, N.o.nbr_k, N.n_active, static_cast<uint2*>(ctx->d_scratch), ctx->stream);
-    VT_CK(cudaGetLastError());
-    VT_CK(cudaMemcpyAsync(nbr, ctx->d_scratch, bytes, cudaMemcpyDeviceToHost, ctx->stream));
+    const vt_status s = try_scratch(ctx, bytes);
+    if (s == VT_ERR_OOM) {
+      std::vector<uint32_t> rows(bytes / 4);
+      VT_CK(cudaMemcpyAsync(rows.data(), N.nbr, bytes, cudaMemcpyDeviceToHost, ctx->stream));
+      VT_CK(cudaStreamSynchronize(ctx->stream));
+      rows = transposed_pairs(rows, N.o.nbr_k, N.n_active);
+      std::copy(rows.begin(), rows.end(), nbr);
+    } else if (s != VT_OK) {
+      return s;
+    } else {
+      vtk::launch_transpose_nbr(N.nbr, N.o.nbr_k, N.n_active, static_cast<uint2*>(ctx->d_scratch), ctx->stream);
+      VT_CK(cudaGetLastError());
+      VT_CK(cudaMemcpyAsync(nbr, ctx->d_scratch, bytes, cudaMemcpyDeviceToHost, ctx->stream));
+    }
   }
   VT_CK(cudaStreamSynchronize(ctx->stream));
   if (active) std::copy(N.active_h.begin(), N.active_h.end(), active);
