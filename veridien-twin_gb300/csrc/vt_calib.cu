@@ -200,7 +200,6 @@ __device__ __forceinline__ float3 path_value(const CalibDev& C, const ConstRecor
   return L;
 }
 
-// d loss / d parameters of one recorded path, given g = d loss / d (path radiance); FP64 into shared accumulators
 // a path's albedo gradient: per vertex its material and g-weighted value (on: the vertex exists)
 struct AlbGrad {
   uint32_t mat[CAL_MAX_DEPTH];
@@ -208,6 +207,7 @@ struct AlbGrad {
   bool on[CAL_MAX_DEPTH];
 };
 
+// d loss / d parameters of one recorded path, given g = d loss / d (path radiance); FP64 into shared accumulators
 __device__ __forceinline__ void path_grad(const CalibDev& C, const ConstRecord& P, uint32_t depth, uint32_t nl, float3 g, double* sh_lamp, AlbGrad& ag) {
   const uint32_t n = P.get(CP_N), node = P.get(CP_NODE), lamp = P.get(CP_EMIT_LAMP);
   const float emit_a = P.getf(CP_EMIT_A);
@@ -481,8 +481,6 @@ __global__ void __launch_bounds__(WT, 4) calib_shadow_kernel(const Scene S, cons
   while (serve_lanes(state, exhausted, wb.fetch_sh, n, cp.refill, lanes, next, start)) trace_round<true>(S, 0.0f, st, stk, state);
 }
 
-// per pixel: the image value from the records in sub-sample order, its loss partial (forward); or the gradient of
-// every record (backward)
 // the derivative in d0 of a recorded path's radiance, per channel, from its derivative record
 __device__ __forceinline__ void path_tangent(const CalibDev& C, const ConstRecord& P, const ConstRecord& G, uint32_t nl, float3* dL) {
   const uint32_t n = P.get(CP_N), lamp = P.get(CP_EMIT_LAMP);
@@ -520,7 +518,7 @@ __device__ __forceinline__ void add_intrinsics_grad(const CamParams& cp, uint32_
   for (int k = 0; k < 8; k++) kacc[k] += G[0] * J[0][k] + G[1] * J[1][k] + G[2] * J[2][k];
 }
 
-// per pixel over the records of sub-samples [i0, i1): backward 0 adds their values to the pixel's running sum (kept in
+// Per pixel over the records of sub-samples [i0, i1): backward 0 adds their values to the pixel's running sum (kept in
 // the image between chunks; the chunk that ends at spp writes the image and the loss partials), 1 / 2 accumulate the
 // gradients (2: with the intrinsics' derivative)
 __global__ void __launch_bounds__(CT) calib_records_kernel(const CamParams cp, const CalibDev C, const uint32_t* __restrict__ rec,
@@ -670,19 +668,11 @@ __device__ __forceinline__ float2 df_split(double x) {
   const float h = float(x);
   return make_float2(h, float(x - double(h)));
 }
-// each step rounded on its own (the _rn intrinsics are never contracted into a multiply-add)
-__device__ __forceinline__ void df_mac(float f, float2 x, float& sh, float& sl) {
-  const float p = __fmul_rn(f, x.x);
-  const float e = __fmaf_rn(f, x.y, __fmaf_rn(f, x.x, -p));
-  const float t = __fadd_rn(sh, p);
-  const float v = __fsub_rn(t, sh);
-  const float lo = __fadd_rn(sl, __fadd_rn(__fadd_rn(__fsub_rn(sh, __fsub_rn(t, v)), __fsub_rn(p, v)), e));
-  sh = __fadd_rn(t, lo);                    // renormalised, so that lo stays below an ulp of the sum
-  sl = __fsub_rn(lo, __fsub_rn(sh, t));
-}
-
-// df_mac on two products at once, the pair's sums apart (every element rounded as df_mac's own step; x - y is x + (-y)
-// exactly). f2 and nf2 = -f2; xh, xl the vector's parts.
+// A step of two products at once, the pair's sums apart; every product, difference and sum is rounded on its own (the _rn
+// intrinsics are never contracted; x - y is x + (-y) exactly):
+//   p = f xh   e = f xl + (f xh - p)   t = sh + p   v = t - sh   lo = sl + (((sh - (t - v)) + (p - v)) + e)
+//   sh' = t + lo   sl' = lo - (sh' - t)       (renormalised, so that lo stays below an ulp of the sum)
+// f2 and nf2 = -f2; xh, xl the vector's parts.
 struct DfAcc { float2 h, l; };
 __device__ __forceinline__ float2 f2(float a, float b) { return make_float2(a, b); }
 __device__ __forceinline__ void df_mac2(float2 f, float2 nf, float2 xh, float2 xl, DfAcc& s) {
@@ -949,7 +939,6 @@ size_t calib_record_bytes(uint32_t paths) { return size_t(paths) * CP_WORDS * 4;
 
 size_t calib_tan_bytes(uint32_t paths) { return size_t(paths) * CT_WORDS * 4; }
 
-// the paths of sub-samples [i0, i1) of the camera through the wavefront, their records (i - i0) n_pix + id
 // tri_hit's arithmetic without its range checks: for a hit tri_hit accepted, the same t, u, v; a recorded hit is met
 // again even when the ray moved by rounding (the derivative-record kernel's ray can differ from the plain kernel's
 // in its last bits)
@@ -996,6 +985,7 @@ __global__ void __launch_bounds__(256) calib_rehit_kernel(const Scene S, WaveBuf
   }
 }
 
+// the paths of sub-samples [i0, i1) of the camera through the wavefront, their records (i - i0) n_pix + id
 static void calib_trace(const Scene& S, const CamParams& cp, const CalibDev& C, WaveBufs wb, uint32_t wave_paths, uint32_t* rec, uint32_t* tan,
                         uint32_t i0, uint32_t i1, int blocks, cudaStream_t st, uint32_t* dec, int dmode) {
   const uint32_t n_pix = tiled_pixels(cp.w, cp.h, cp.tile_w, cp.tile_h);

@@ -80,7 +80,7 @@ struct vt_ctx {
   struct Batch {
     float* su = nullptr;            // VT_BATCH_MAX_POSES scene uniforms
     float4* cull = nullptr;         // nodes, then items
-    uint32_t* ctr = nullptr;        // queue counters [0..4] and [32..36], status [8], stats (u64) at [16]
+    uint32_t* ctr = nullptr;        // queue counters [0..7] and [32..39], status [8], stats (u64) at [16]
     uint32_t* sensor = nullptr;     // 64 words per camera
     void* mem = nullptr;            // wave buffers
     size_t mem_bytes = 0;

@@ -796,8 +796,12 @@ __device__ __forceinline__ float3 emitter_normal(const Scene& S, const Hit& h, c
 // come from the angles' tangents instead of sin(): with f = atan(t), sin 2f = 2t / (1 + t^2) and sin^2 f = t^2 /
 // (1 + t^2); an end clamped to f0 -+ pi/2 (f0 = atan2(na, np)) has sin 2f = -sin 2f0 = -2 na np / rho^2 and sin^2 f =
 // cos^2 f0 = np^2 / rho^2, rho^2 = na^2 + np^2. The same integral to float rounding, four sines fewer per capsule.
-// The cylinder from a along the unit vector e, length L, radius r.
-__device__ __forceinline__ float capsule_occ(float3 p, float3 n, float3 a, float r, float3 e, float L) {
+// The cylinder from a to bb, radius r.
+__device__ __forceinline__ float capsule_occ(float3 p, float3 n, float3 a, float3 bb, float r) {
+  const float3 ab = bb - a;
+  const float L = length(ab);
+  if (L < 1e-9f || r <= 0.0f) return 0.0f;
+  const float3 e = ab / L;
   const float3 ap = p - a;
   const float s0 = dot(ap, e);
   const float3 perp = ap - e * s0;
@@ -833,35 +837,13 @@ __device__ __forceinline__ float capsule_occ(float3 p, float3 n, float3 a, float
   const float I = np * (0.5f * (f2 - f1) + 0.25f * (s2b - s2a)) + na * 0.5f * (sqb - sqa);
   return clampf(INV_PI_F * (2.0f * r / h) * I, 0.0f, 1.0f);
 }
-// the axis of the cylinder from a to bb; false when it hides nothing
-__device__ __forceinline__ bool capsule_axis(float3 a, float3 bb, float r, float3& e, float& L) {
-  const float3 ab = bb - a;
-  L = length(ab);
-  if (L < 1e-9f || r <= 0.0f) return false;
-  e = ab / L;
-  return true;
-}
-__device__ __forceinline__ float capsule_occ(float3 p, float3 n, float3 a, float3 bb, float r) {
-  float3 e;
-  float L;
-  return capsule_axis(a, bb, r, e, L) ? capsule_occ(p, n, a, r, e, L) : 0.0f;
-}
-// a posed body's, and the share of the light behind it that it hides; false when it hides nothing
-__device__ __forceinline__ bool load_capsule(const Scene& S, uint32_t i, float3& a, float& r, float3& e, float& L, float& hides) {
-  const float* I = inst_rec(S, i);
-  if (ldu(I + 15) & 2u) return false;
-  a = ld3(I + 24);
-  r = __ldg(I + 27);
-  hides = 1.0f - __ldg(I + 31);
-  return capsule_axis(a, ld3(I + 28), r, e, L);
-}
 __device__ __forceinline__ float capsule_vis(const Scene& S, float3 p, float3 n) {
   float v = 1.0f;
   const uint32_t cnt = min(ldu(S.su + 16), uint32_t(VT_MAX_INST));
   for (uint32_t i = 0; i < cnt; i++) {
-    float3 a, e;
-    float r, L, hides;
-    if (load_capsule(S, i, a, r, e, L, hides)) v = v - capsule_occ(p, n, a, r, e, L) * hides;
+    const float* I = inst_rec(S, i);
+    if (ldu(I + 15) & 2u) continue;
+    v = v - capsule_occ(p, n, ld3(I + 24), ld3(I + 28), __ldg(I + 27)) * (1.0f - __ldg(I + 31));
   }
   return clampf(v, 0.0f, 1.0f);
 }

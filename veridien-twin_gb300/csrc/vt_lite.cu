@@ -139,7 +139,7 @@ __device__ __forceinline__ uint32_t sm_less(const uint32_t* m, uint32_t res, int
 // linear filtering, clamp to edge: the 2x2 texels around a tap compare dref < depth and blend bilinearly), min of
 // the static and dynamic maps per tap. The taps share the bilinear fraction of the centre tap (they sit exactly one
 // texel apart), so the 4x4 texels under them are compared once per map; where either map hides all of them, or both
-// none, the taps are known. Four 1280x720 views: shading 1.45 -> 1.36 ms.
+// none, the taps are known (a frame of four 1280x720 views 3.57 -> 3.54 ms).
 __device__ float sm_vis(const View& V, const ShadeArgs& a, float3 pw, uint32_t k, float bias) {
   const float3 q = sm_project(V, pw, k);
   if (fabsf(q.x) >= 1.0f || fabsf(q.y) >= 1.0f) return 1.0f;

@@ -25,8 +25,6 @@ void launch_node_direct(const vtd::Scene& S, const uint32_t* active, uint32_t n_
 void launch_transport_count(const uint32_t* active, uint32_t n_active, uint32_t K, const uint32_t* gtable, uint32_t* cnt, cudaStream_t st);
 void launch_transport_fill(const vtd::Scene& S, const uint32_t* active, uint32_t n_active, uint32_t K, const uint32_t* gtable, const float4* amu,
                            const uint32_t* row, float4* ent, cudaStream_t st);
-// one Jacobi step: gather from slot_in into aux (from the transport table when ent is set, else evaluating each
-// ray's factor), update into slot_out
 // the sums of nodeSummary over the active nodes, 10 doubles at the start of `work` (node_sums_bytes): area, then rgb of area x
 // E_free V, area x B_dir / hh, area x Ls hh; hh: 6 doubles per material, max(1e-4, hh) and 1 / max(1e-3, hh)
 size_t node_sums_bytes();
@@ -34,6 +32,8 @@ void launch_node_sums(const vtd::Scene& S, const uint32_t* active, uint32_t n_ac
                       const float4* nstate, double* work, cudaStream_t st);
 // neighbour pairs, rows x cols, transposed (the Jacobi step reads nbr_k rows of n_active)
 void launch_transpose_nbr(const uint2* in, uint32_t rows, uint32_t cols, uint2* out, cudaStream_t st);
+// one Jacobi step: gather from slot_in into aux (from the transport table when ent is set, else evaluating each
+// ray's factor), update into slot_out
 void launch_jacobi_step(const vtd::Scene& S, const uint32_t* active, uint32_t n_active, uint32_t K, const uint32_t* gtable, const float4* amu,
                         const uint32_t* row, const float4* ent, const uint2* nbr, uint32_t nbr_k, uint32_t slot_in, uint32_t slot_out,
                         float4* nstate, float4* aux, cudaStream_t st);

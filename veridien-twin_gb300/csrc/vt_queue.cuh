@@ -8,7 +8,7 @@ namespace vtk {
 // A path with a next ray, with light samples or both to the next bounce's queue and the bounce's shadow queue (WaveBufs, whose
 // counts of the two are neighbours): one atomic a warp for both. A warp waits for its answer at the end of each 32 paths, and the
 // counter's line takes one in ~1.3 ns (one for each queue, 640x480, 16 spp: 14.42 ms, pose batch
-// 83.9; now 14.32, 83.2)
+// 83.9; now 14.32, 83.0)
 template <typename Bufs>
 __device__ __forceinline__ void append_path(const Bufs& wb, uint32_t p, bool cont, bool shadow) {
   const uint32_t act = __activemask(), lane = threadIdx.x & 31u, below = (1u << lane) - 1u;

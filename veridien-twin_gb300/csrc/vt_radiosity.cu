@@ -81,7 +81,9 @@ __global__ void __launch_bounds__(MV_THREADS) jacobi_matvec_kernel(const float* 
 // small room is mostly its start and its end: n = 4096, 16 sweeps and two checks: 358 us of a solve -> 227 (21.2 -> 8.5 us a
 // sweep under ncu; F, 67 MB, comes from the L2)
 constexpr int MVS_THREADS = 1024;
-constexpr uint32_t MVS_MAX_N = 16384;   // the iterate in shared memory: 64 KB
+// the iterate in shared memory: 64 KB. A solve, a launch per sweep and here: n = 500 192 and 142 us, 5000 500 and 402, 9001 1.10 and 1.02 ms,
+// 12288 1.95 and 1.50, 16384 2.94 and 2.64
+constexpr uint32_t MVS_MAX_N = 16384;
 
 // wait for every block's arrival (`target` arrivals since the counter was cleared, counted modulo 2^32: blocks are at most a
 // barrier apart); false in every thread when it runs out
@@ -506,9 +508,10 @@ void launch_jacobi_gemm_fp32(const float* F, const float* rho, const float* E, c
 // ---------------------------------------------------------------------------------------------- FP32 tensor-core sweep
 // The same sweep with F B on the tensor cores in FP32 accuracy (vt_tc.cu tc_gemm_f32_kernel). F must come by TMA: rows
 // 16-byte aligned. An n that is no multiple of 4 is copied once per solve to rows that are (less than half a sweep of the FMA
-// kernel). Below 1536 nodes the FMA kernel stays: a sweep
-// is a few microseconds of work either way (n = 1000, 64 columns: 20.9 us there, 24.4 here; n = 2000: 29.4 and 25.7; n =
-// 4096: 73.6 and 30.4; n = 32768: 3197 and 755), and up to about there its rounding errors are the smaller ones.
+// kernel). Below 1536 nodes the FMA kernel stays: with 64 columns a sweep there takes as long or less (n = 1000 20.9 us, 24.4 here; 2000 29.4
+// and 25.7; 4096 73.6 and 30.4; 32768 3197 and 755), and up to about there its rounding errors are the smaller ones. Fewer columns move the line
+// down, not up, since the FMA kernel's tile is 64 wide whatever their number. Solves to 1e-5, FMA and here: 1537 x 4 493 and 375 us, 1537
+// x 60 517 and 467, 1999 x 16 534 and 393, 3001 x 4 1013 and 388, 9001 x 8 4.56 and 1.30 ms.
 constexpr uint32_t TC_F32_MIN = 1536;
 bool jacobi_tc_f32_ok(const float* F, uint32_t n, uint32_t R) {
   return R > 1 && n >= TC_F32_MIN && (n % 4u != 0u || (reinterpret_cast<uintptr_t>(F) & 15u) == 0u);

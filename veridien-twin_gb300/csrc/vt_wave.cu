@@ -685,11 +685,6 @@ void launch_dependent(void (*kernel)(P...), int blocks, cudaStream_t st, bool de
 // A bounce's closest hits read nothing that the previous bounce's light samples write, nor the other way round: their
 // kernel is launched over that one's tail (programmatic launch: its blocks start where the other's have ended, and wait
 // for the whole of it before they end themselves, so that what follows in the stream follows both)
-template <int VAR, bool HC>
-void extend_over(const Scene& S, const CamParams& cp, const WaveBufs& w, int blocks, cudaStream_t st, bool over) {
-  launch_dependent(wave_extend<VAR, HC>, blocks, st, over, S, cp, w);
-}
-
 template <int VAR>
 void wave_bounces_of(const Scene& S, const CamParams& cp, const WaveBufs& wb, int blocks, cudaStream_t st, uint64_t* launches, KernelTimer* timer) {
   const uint32_t depth = cp.mode == VT_SHADE_TWIN ? 2u : cp.max_depth;
@@ -702,8 +697,8 @@ void wave_bounces_of(const Scene& S, const CamParams& cp, const WaveBufs& wb, in
       bounce_view(w, b);
       TimedLaunch tl(timer, st, 0);
       const bool over = b > 1 && !timer;   // the kernels' own times need them apart
-      if (PLAIN && w.hcache) extend_over<VAR, PLAIN>(S, cp, w, blocks, st, over);
-      else extend_over<VAR, false>(S, cp, w, blocks, st, over);
+      if (PLAIN && w.hcache) launch_dependent(wave_extend<VAR, PLAIN>, blocks, st, over, S, cp, w);
+      else launch_dependent(wave_extend<VAR, false>, blocks, st, over, S, cp, w);
       // before the shading, which moves the rays on
       if (cull) cull_extend_kernel<<<blocks * 2, WAVE_THREADS, 0, st>>>(cp, w);
     }
@@ -734,7 +729,7 @@ void wave_bounces(const Scene& S, const CamParams& cp, WaveBufs wb, int var, int
 }
 
 void launch_wave_extend(const Scene& S, const CamParams& cp, const WaveBufs& wb, int blocks, cudaStream_t st, bool over) {
-  extend_over<WAVE_PLAIN, false>(S, cp, wb, blocks, st, over);
+  launch_dependent(wave_extend<WAVE_PLAIN, false>, blocks, st, over, S, cp, wb);
 }
 
 void launch_wave_gen(const CamParams& cp, WaveBufs wb, uint32_t i0, uint32_t n_i, uint32_t n_pix, int blocks, cudaStream_t st) {

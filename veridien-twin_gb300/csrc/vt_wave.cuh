@@ -46,7 +46,7 @@ struct WaveBufs {
   float4* acc2;     // per refined pixel: running sum of the refinement waves
   uint32_t* rlist;  // refined pixel ids
   uint32_t* rcount; // their number (refinement only)
-  uint32_t* counts; // WAVE_COUNTS words: queue lengths and entries taken (bounce_view)
+  uint32_t* counts; // 8 words: queue lengths and entries taken (bounce_view)
   // the current bounce's view
   uint32_t* q_in;
   uint32_t* q_out;
@@ -73,9 +73,8 @@ struct KernelTimer {
   int cap, n;
 };
 
-// Words of WaveBufs::counts, and a bounce's view of them and of the queues. The first bounce begins with words 1 to 3
-// clear; a bounce's closest-hit kernel clears the next one's.
-constexpr uint32_t WAVE_COUNTS = 8;
+// A bounce's view of the queues and of WaveBufs::counts. The first bounce begins with words 1 to 3 clear; a bounce's
+// closest-hit kernel clears the next one's four.
 void bounce_view(WaveBufs& w, uint32_t b);
 
 size_t wave_bytes(uint32_t paths, uint32_t n_light, uint32_t n_pix);
@@ -90,10 +89,9 @@ int wave_blocks_per_sm();
 // one wave's bounces (extend, shade, shadow per bounce) over the paths queued in wb.qa / counts[0]
 void wave_bounces(const vtd::Scene& S, const CamParams& cp, WaveBufs wb, int var, int blocks, cudaStream_t st, uint64_t* launches,
                   KernelTimer* timer = nullptr);
-// the closest-hit kernel over wb.qa / counts (plain scene) and the camera rays of sub-samples [i0, i0 + n_i) of all
-// n_pix pixel ids (path p = (i - i0) n_pix + id), queued in wb.qa / counts[0]
-// over: beside the tail of the light-sample kernel launched just before (wave_bounces_of), whose blocks have to trigger it
+// the closest-hit kernel over a bounce's queue (plain scene); over: beside the tail of the light-sample kernel launched just before (wave_bounces_of), whose blocks have to trigger it
 void launch_wave_extend(const vtd::Scene& S, const CamParams& cp, const WaveBufs& wb, int blocks, cudaStream_t st, bool over = false);
+// the camera rays of sub-samples [i0, i0 + n_i) of all n_pix pixel ids (path p = (i - i0) n_pix + id), queued in wb.qa / counts[0]
 void launch_wave_gen(const CamParams& cp, WaveBufs wb, uint32_t i0, uint32_t n_i, uint32_t n_pix, int blocks, cudaStream_t st);
 // camera rays of a batch wave: paths p = i * n_pw + lp, i < spp, pixel id px0 + lp; clears the dirty masks
 void wave_gen_batch(const CamParams& cp, WaveBufs wb, int blocks, cudaStream_t st);
