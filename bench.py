@@ -292,7 +292,7 @@ def main():
             rays_per_launch = kt["extend_rays"] / max(kt["extend_launches"], 1)
             per_launch = cnt["bytes_per_extension_ray"] * rays_per_launch
             ach = per_launch / (launch_ms / 1e3) / 1e9
-            line["roofline"] = {"bound": "hbm", "achieved": ach, "peak": hbm, "unit": "GB/s", "frac": ach / hbm,
+            line["roofline"] = {"bound": "l1", "achieved": ach, "peak": hbm, "unit": "GB/s", "frac": ach / hbm,
                                 "traffic": EXTEND_DRAM_PER_RAY * rays_per_launch, "kernel": "wave_extend",
                                 "traffic_source": TRAFFIC_SOURCE,
                                 "issue_frac": EXTEND_IPC / 4.0,
@@ -302,7 +302,7 @@ def main():
                                 "launch_ms": launch_ms, "rays_per_launch": rays_per_launch, "bytes_per_launch": per_launch,
                                 "note": "algorithmic bytes per launch = rays x (64 B per BVH node visit + 48 B per triangle test), "
                                         "counted by the oracle on extension rays of the same frame; the scene is L2-resident, so "
-                                        "the DRAM traffic (ncu, scaled by rays) is far below it",
+                                        "the DRAM traffic (ncu, scaled by rays) is far below it; the peak beside them is the HBM copy rate",
                                 "peak_source": "measured" if "hbm_gbs" in peaks else "fallback",
                                 "frame_logical_gbs": bps * W_ * H_ * SPP / (ms / args.steps / 1e3) / 1e9, **cnt,
                                 "kernel_share": {"extend_ms": kt["extend_ms"], "shade_ms": kt["shade_ms"], "shadow_ms": kt["shadow_ms"]}}
